@@ -26,6 +26,7 @@
 #include "sample_wide.cuh"      // gs::w1024: 1024 threads, one CTA per SM (latency)
 #include "sample_vocab.cuh"
 #include "index_ops.cuh"
+#include "topk_large.cuh"
 #include "generate_control.cuh"
 #include "row_softmax.cuh"
 #include "lm_head.cuh"
@@ -539,6 +540,12 @@ int launch_lm_head(Ctx* c, gs::LmHeadArgs& a, char** errOut) {
   return GORCH_CUDA_OK;
 }
 
+template <typename SH>
+cudaError_t topk_large_attributes() {
+  const cudaError_t e = cudaFuncSetAttribute(gs::topk_large_kernel<float, SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::DYN_BYTES);
+  return e != cudaSuccess ? e : cudaFuncSetAttribute(gs::topk_large_kernel<uint16_t, SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, SH::DYN_BYTES);
+}
+
 }  // namespace
 
 extern "C" {
@@ -613,8 +620,8 @@ GorchCudaCtxRef gorch_cuda_create_ctx(int device, char** errOut) {
   if ((e = cudaFuncSetAttribute(gs::n128::narrow_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n128::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::n128::narrow_rows_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n128::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::multinomial_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::MN_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
-  if ((e = cudaFuncSetAttribute(gs::topk_large_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::TKL_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
-  if ((e = cudaFuncSetAttribute(gs::topk_large_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::TKL_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = topk_large_attributes<gs::TklSmall>()) != cudaSuccess || (e = topk_large_attributes<gs::TklFew>()) != cudaSuccess ||
+      (e = topk_large_attributes<gs::TklMid>()) != cudaSuccess || (e = topk_large_attributes<gs::TklLarge>()) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::vocab_merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::VM_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::w256::wide_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::w256::W_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::w1024::wide_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::w1024::W_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
@@ -1077,6 +1084,16 @@ int gorch_cuda_sample_vocab_sharded_ex_dev(GorchCudaCtxRef ctx, const void* logi
                               cfgs, uniforms, out_ids, out_flags, errOut);
 }
 
+}  // extern "C"
+template <typename SH>
+static void launch_topk_large(Ctx* c, const gs::TopKLargeArgs& ta, int dtype) {
+  const int64_t slots = static_cast<int64_t>(SH::MINB) * c->sm_count;
+  const unsigned g = static_cast<unsigned>(ta.B < slots ? ta.B : slots);
+  if (dtype == GORCH_CUDA_F32) gs::topk_large_kernel<float, SH><<<g, SH::NT, SH::DYN_BYTES, c->stream>>>(ta);
+  else gs::topk_large_kernel<uint16_t, SH><<<g, SH::NT, SH::DYN_BYTES, c->stream>>>(ta);
+}
+extern "C" {
+
 int gorch_cuda_topk_dev(GorchCudaCtxRef ctx, const void* x, int dtype, int64_t B, int64_t V,
                         int64_t row_stride, int64_t k, float* out_values, int32_t* out_indices,
                         uint32_t* out_flags, char** errOut) {
@@ -1099,9 +1116,11 @@ int gorch_cuda_topk_dev(GorchCudaCtxRef ctx, const void* x, int dtype, int64_t B
     gs::TopKLargeArgs ta;
     ta.x = x; ta.row_stride = row_stride; ta.V = static_cast<int32_t>(V); ta.k = static_cast<int32_t>(k);
     ta.out_values = out_values; ta.out_indices = out_indices; ta.out_flags = out_flags; ta.B = B;
-    const unsigned g = static_cast<unsigned>(B < c->sm_count ? B : c->sm_count);
-    if (dtype == GORCH_CUDA_F32) gs::topk_large_kernel<float><<<g, gs::TKL_NT, gs::TKL_DYN_BYTES, c->stream>>>(ta);
-    else gs::topk_large_kernel<uint16_t><<<g, gs::TKL_NT, gs::TKL_DYN_BYTES, c->stream>>>(ta);
+    // by the list that k needs; up to one row per SM a row gets all of an SM's threads
+    if (k > gs::TKL_MID_K) launch_topk_large<gs::TklLarge>(c, ta, dtype);
+    else if (k > gs::TKL_SMALL_K) launch_topk_large<gs::TklMid>(c, ta, dtype);
+    else if (B <= c->sm_count) launch_topk_large<gs::TklFew>(c, ta, dtype);
+    else launch_topk_large<gs::TklSmall>(c, ta, dtype);
     CUDA_TRY(cudaGetLastError(), errOut);
     c->counters.kernel_launches += 1;
     return GORCH_CUDA_OK;

@@ -65,6 +65,26 @@ def test_topk_large_k_matches_oracle(_sampler_session, oracle, B, V, k):
     assert np.array_equal(vals, wv) and np.array_equal(idx.astype(np.int64), wi)
 
 
+@pytest.mark.parametrize("B,V,k", [(3, 3328, 1000), (3, 3329, 1000), (160, 3329, 1024), (2, 9000, 1025), (2, 151936, 4096), (2, 30001, 4097),
+                                   (160, 50257, 257), (2, 20000, 16384), (2, 20001, 16384)])
+def test_topk_large_k_instances(_sampler_session, oracle, B, V, k):
+    """The edges between the kernel's instances (by k and by rows) and of their candidate lists, on rows
+    that start anywhere, rise from end to end, or hold their largest logits in one short run."""
+    s = _sampler_session
+    rng = np.random.Generator(np.random.Philox(key=V * 31 + k))
+    x = (rng.standard_normal((B, V)) * 2.0).astype(np.float32)
+    x[0] = np.sort(x[0])
+    x[1, : min(V // 2, 2 * k)] += 20.0
+    x[B - 1, 3] = np.nan
+    vals, idx = s.topk(x, k)
+    wv, wi = oracle.topk(np.where(np.isnan(x), -np.inf, x), k)
+    assert np.array_equal(vals, wv) and np.array_equal(idx.astype(np.int64), wi)
+    bits = oracle.f32_to_bf16_bits(np.where(np.isnan(x), 0.5, x).astype(np.float32))
+    vals, idx = s.topk(bits, k)
+    wv, wi = oracle.topk(oracle.bf16_bits_to_f32(bits), k)
+    assert np.array_equal(vals, wv) and np.array_equal(idx.astype(np.int64), wi)
+
+
 def test_topk_k_limit(_sampler_session):
     with pytest.raises(GorchCudaError, match="k <= 16384"):
         _sampler_session.topk(np.zeros((2, 20000), dtype=np.float32), 16385)
