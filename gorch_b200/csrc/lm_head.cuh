@@ -376,15 +376,14 @@ __global__ void __launch_bounds__(LMH_F_NT) lmh_threshold_kernel(LmhSampleArgs M
   }
 }
 
-__global__ void __launch_bounds__(LMH_F_NT, 4) lmh_finish_kernel(LmhSampleArgs M) {
+__global__ void __launch_bounds__(LMH_F_NT, 4) lmh_finish_kernel(const __grid_constant__ LmhSampleArgs M) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ bu::Scratch sc;
   __shared__ uint32_t s_sel[256];
   __shared__ int s_bc[4];
-  __shared__ double s_bcd[4];
   __shared__ int s_cnt;
   uint2* list = reinterpret_cast<uint2*>(dyn);                                       // the row's candidates
-  unsigned char* work = dyn + LMH_CAND_CAP * 8;                                       // 16 KB for finish_small_set
+  unsigned char* work = dyn + LMH_CAND_CAP * 8;                                       // for finish_small_set
   uint2* kept = reinterpret_cast<uint2*>(dyn + LMH_CAND_CAP * 8 + 16384);            // KEEP_MAX entries
   const KernelArgs& A = M.k;
   const int tid = threadIdx.x;
@@ -393,10 +392,6 @@ __global__ void __launch_bounds__(LMH_F_NT, 4) lmh_finish_kernel(LmhSampleArgs M
     __syncthreads();
     const RowCfg cfg = A.cfgs[row];
     const float Tm = cfg.temperature;
-    RowDebug dbg;
-    dbg.sum_exp = 0; dbg.resum = 1.0; dbg.edge_lo = 0; dbg.edge_hi = 0; dbg.kept = 0;
-    dbg.max_scaled = 0; dbg.threshold = __int_as_float(0x7fc00000); dbg.path = 4;
-    for (int q = 0; q < 8; q++) dbg.reserved[q] = 0;
     auto write_row = [&](int id, uint32_t fl) {
       if (tid == 0) {
         A.out_ids[row] = id;
@@ -445,27 +440,15 @@ __global__ void __launch_bounds__(LMH_F_NT, 4) lmh_finish_kernel(LmhSampleArgs M
     if ((nanb & 1) || !(fabsf(m) < INFINITY)) { write_row(A.V - 1, FLAG_NONFINITE | FLAG_FALLBACK); continue; }
     // ---- top_k-th largest with ties (generate.go:157-164), then the kept set
     const int topk = cfg.top_k;
-    float thr = -INFINITY;
-    if (cnt > topk) {
-      const uint32_t kkey = bu::select_kth<LMH_F_NT>(list, cnt, topk, s_sel, s_bc, tid);
-      thr = quotient_class_floor(okey_to_float(kkey), Tm);
-    }
-    __syncthreads();
-    if (tid == 0) s_cnt = 0;
-    __syncthreads();
-    for (int j = tid; j < cnt; j += LMH_F_NT) {
-      const uint2 e = list[j];
-      if (__uint_as_float(e.x) >= thr) { const int slot = atomicAdd(&s_cnt, 1); if (slot < KEEP_MAX) kept[slot] = e; }
-    }
-    __syncthreads();
-    const int nk = s_cnt;
-    // Everything at or above the exact threshold must be on the list: that holds when the exact
-    // threshold (the floor of the k-th value's class of equal quotients) is not below the list's own.
-    if (nk > KEEP_MAX || cnt <= topk || !(thr >= M.thr[row])) { give_up(); continue; }
+    const int nk = narrow_list<LMH_F_NT>(list, cnt, topk, Tm, 0u, M.rowmax_key[row], kept, s_sel, s_bc, &s_cnt, tid);
+    if (nk > KEEP_MAX || cnt <= topk) { give_up(); continue; }
     const bool topp_on = (cfg.top_p > 0.0f && cfg.top_p < 1.0f);
     const int mode = cfg.topp_mode;
     const double plim = (mode == 0) ? static_cast<double>(cfg.top_p) * 1.5 : static_cast<double>(cfg.top_p);
-    finish_small_set<LMH_F_NT>(A, row, kept, nk, m, Tm, topp_on, mode, plim, A.uniforms[row], work, sc, s_bcd, dbg, 0u);
+    // Everything at or above the exact threshold must be on the list: that holds when the exact
+    // threshold (the floor of the k-th value's class of equal quotients) is not below the list's own.
+    if (!finish_small_set<LMH_F_NT, false>(A, row, kept, nk, topk, m, Tm, topp_on, mode, plim, A.uniforms[row], M.thr[row], work, nullptr, 0u))
+      give_up();
   }
 }
 

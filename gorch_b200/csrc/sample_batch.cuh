@@ -88,147 +88,6 @@ __device__ __forceinline__ void hand_to_single(const BatchArgs& BA, int64_t row_
   BA.list_single[1 + atomicAdd(&BA.list_single[0], 1)] = static_cast<int32_t>(row_id);
 }
 
-// ---------------------------------------------------------------------------
-// Finish a row whose kept set (nk <= 512 entries of (logit bits, index)) sits in
-// shared memory: softmax over the kept set, top-p, draw. Work arrays: 16 KB.
-// ---------------------------------------------------------------------------
-template <int NTHREADS>
-__device__ void finish_small_set(const KernelArgs& A, int64_t row_id, const uint2* kp, int nk, float m, float Tm,
-                                 bool topp_on, int mode, double plim, double u, unsigned char* work,
-                                 bu::Scratch& sc, double* bc_d, RowDebug& dbg, uint32_t flags) {
-  constexpr int NWARPS = NTHREADS / 32;
-  constexpr int PER = (KEEP_MAX + NTHREADS - 1) / NTHREADS;
-  const int tid = threadIdx.x;
-  const int V = A.V;
-  const double QNAN = __longlong_as_double(0x7ff8000000000000ll);
-  float* sx = reinterpret_cast<float*>(work);                 // [512] scaled value, index order
-  int* sidx = reinterpret_cast<int*>(work + 2048);            // [512]
-  double* se = reinterpret_cast<double*>(work + 4096);        // [512] probability
-  double* sf = reinterpret_cast<double*>(work + 8192);        // [512] scratch / final probability
-  int* rnk = reinterpret_cast<int*>(work + 12288);            // [512]
-  int* ord = reinterpret_cast<int*>(work + 14336);            // [512]
-  auto write_row = [&](int id, uint32_t fl) {
-    if (tid == 0) {
-      A.out_ids[row_id] = id;
-      if (A.out_flags) A.out_flags[row_id] = fl;
-      if (A.out_debug) A.out_debug[row_id] = dbg;
-    }
-  };
-  auto fill_probs_row = [&](double v) {
-    if (A.out_probs) {
-      double* pr = A.out_probs + row_id * static_cast<int64_t>(V);
-      for (int i = tid; i < V; i += NTHREADS) pr[i] = v;
-    }
-  };
-  __syncthreads();
-  float thr_s = INFINITY;
-  for (int j = tid; j < nk; j += NTHREADS) {
-    const uint32_t myi = kp[j].y;
-    int r = 0;
-    for (int l = 0; l < nk; l++) r += (kp[l].y < myi) ? 1 : 0;
-    const float s = scale_t(__uint_as_float(kp[j].x), Tm);
-    sx[r] = s;
-    sidx[r] = static_cast<int>(myi);
-    thr_s = fminf(thr_s, s);
-  }
-  dbg.threshold = okey_to_float(static_cast<uint32_t>(bu::min_u64<NWARPS>(static_cast<unsigned long long>(okey(thr_s)), sc, tid)));
-  __syncthreads();
-  double e_loc = 0.0;
-  for (int j = tid; j < nk; j += NTHREADS) {
-    const double e = exp(static_cast<double>(sx[j] - m));     // f32 subtract, f64 exp (generate.go:176)
-    se[j] = e;
-    e_loc += e;
-  }
-  const double S = bu::sum_d<NWARPS>(e_loc, sc, tid);
-  dbg.sum_exp = S;
-  for (int j = tid; j < nk; j += NTHREADS) { const double q = se[j] / S; se[j] = q; sf[j] = q; }   // generate.go:179-181
-  __syncthreads();
-  if (topp_on) {
-    // order by probability; equal probabilities by index, ascending in both flavours
-    // (mode A removes the lowest index first, mode B keeps it first)
-    for (int j = tid; j < nk; j += NTHREADS) {
-      const double qj = se[j];
-      int r = 0;
-      if (mode == 0) { for (int l = 0; l < nk; l++) { const double ql = se[l]; r += (ql < qj || (ql == qj && l < j)) ? 1 : 0; } }
-      else           { for (int l = 0; l < nk; l++) { const double ql = se[l]; r += (ql > qj || (ql == qj && l < j)) ? 1 : 0; } }
-      ord[r] = j;
-      rnk[j] = r;
-    }
-    __syncthreads();
-    if (mode == 0) {
-      // generate.go:184-228: the mass left after removing the r smallest is a suffix sum.
-      // sf[t] = probability of rank nk-1-t, scanned: sf[t] = mass of the t+1 largest.
-      for (int t = tid; t < nk; t += NTHREADS) sf[t] = se[ord[nk - 1 - t]];
-      __syncthreads();
-      bu::smem_scan_incl<NWARPS, PER>(sf, nk, sc, tid);
-      // left after removing r smallest = sf[nk-1-r]
-      int rs = nk;
-      for (int r = tid; r < nk; r += NTHREADS) if (sf[nk - 1 - r] <= plim) rs = min(rs, r);
-      const int rstar = bu::min_i<NWARPS>(rs, sc, tid);
-      if (rstar == nk) {                                      // everything removed: 0/0 (generate.go:221-227)
-        dbg.resum = 0.0;
-        fill_probs_row(QNAN);
-        write_row(V - 1, flags | FLAG_NONFINITE | FLAG_FALLBACK);
-        return;
-      }
-      const double resum = sf[nk - 1 - rstar];
-      if (fabs(resum - plim) <= 1e-12) flags |= FLAG_TOPP_EDGE;
-      if (rstar > 0 && fabs(sf[nk - rstar] - plim) <= 1e-12) flags |= FLAG_TOPP_EDGE;
-      dbg.resum = resum;
-      __syncthreads();
-      for (int j = tid; j < nk; j += NTHREADS) sf[j] = (rnk[j] >= rstar) ? se[j] / resum : 0.0;
-    } else {
-      // qwen/generate.go:123-153: shortest descending prefix with mass >= p
-      for (int t = tid; t < nk; t += NTHREADS) sf[t] = se[ord[t]];
-      __syncthreads();
-      bu::smem_scan_incl<NWARPS, PER>(sf, nk, sc, tid);
-      int cl = nk;
-      for (int r = tid; r < nk; r += NTHREADS) if (sf[r] >= plim) cl = min(cl, r + 1);
-      const int cutn = bu::min_i<NWARPS>(cl, sc, tid);
-      const double resum = sf[cutn - 1];
-      if (fabs(resum - plim) <= 1e-12) flags |= FLAG_TOPP_EDGE;
-      if (cutn >= 2 && fabs(sf[cutn - 2] - plim) <= 1e-12) flags |= FLAG_TOPP_EDGE;
-      if (cutn < nk && se[ord[cutn]] == se[ord[cutn - 1]]) flags |= FLAG_TIE_CUT;
-      dbg.resum = resum;
-      __syncthreads();
-      for (int j = tid; j < nk; j += NTHREADS) sf[j] = (rnk[j] < cutn) ? se[j] / resum : 0.0;
-    }
-    __syncthreads();
-  }
-  int kept_loc = 0;
-  for (int j = tid; j < nk; j += NTHREADS) kept_loc += (sf[j] > 0) ? 1 : 0;
-  dbg.kept = bu::sum_i<NWARPS>(kept_loc, sc, tid);
-  if (A.out_probs) {
-    fill_probs_row(0.0);
-    __syncthreads();
-    double* pr = A.out_probs + row_id * static_cast<int64_t>(V);
-    for (int j = tid; j < nk; j += NTHREADS) pr[sidx[j]] = sf[j];
-  }
-  // draw (generate.go:231-239): first index with u < cumulative
-  for (int j = tid; j < nk; j += NTHREADS) se[j] = sf[j];
-  __syncthreads();
-  bu::smem_scan_incl<NWARPS, PER>(se, nk, sc, tid);
-  int pl = nk;
-  for (int j = tid; j < nk; j += NTHREADS) if (u < se[j]) pl = min(pl, j);
-  const int pick = bu::min_i<NWARPS>(pl, sc, tid);
-  int id;
-  if (pick < nk) {
-    id = sidx[pick];
-    const double hi = se[pick], lo = pick > 0 ? se[pick - 1] : 0.0;
-    dbg.edge_lo = lo; dbg.edge_hi = hi;
-    if ((pick > 0 && u - lo <= 1e-6) || hi - u <= 1e-6) flags |= FLAG_BOUNDARY;
-  } else {
-    id = V - 1;
-    flags |= FLAG_FALLBACK;
-    const double tot = se[nk - 1];
-    dbg.edge_lo = dbg.edge_hi = tot;
-    if (u - tot <= 1e-6) flags |= FLAG_BOUNDARY;
-  }
-  (void)bc_d;
-  dbg.reserved[4] = static_cast<uint32_t>(clock64());       // with reserved[3]: the row's whole time on its CTA
-  write_row(id, flags);
-}
-
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 template <typename T>

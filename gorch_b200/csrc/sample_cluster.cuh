@@ -10,10 +10,10 @@
 // 77-181 (mode B). Per row:
 //   greedy         slice argmax -> rank 0 picks (max value, lowest index).
 //   top-k <= 256   pass A: slice -> smem, row max, one running max per thread.
-//                  The k-th largest of those 512 per-thread maxima bounds the
-//                  k-th largest logit from below, so pass B (shared memory)
-//                  collects a few hundred candidates at most; rank 0 merges the
-//                  CTAs' lists and finishes in shared memory.
+//                  The bucket of the k-th largest of those 512 per-thread maxima
+//                  bounds the k-th largest logit from below, so pass B (shared
+//                  memory) collects a few hundred candidates at most; rank 0
+//                  merges the CTAs' lists and finishes them (small_set.cuh).
 //   top-k off      L: slice -> smem, max and min.  P2 (only with an active
 //                  top-p cut): count histogram over 1024 linear buckets of
 //                  d = s - max; rank 0 brackets the cut from count-based mass
@@ -21,9 +21,13 @@
 //                  to running sums, the bracketed zone to an exact list that
 //                  rank 0 cuts by weighted selection.  The CTA whose slice holds
 //                  the drawn token rescans one warp's run.
-// Rows this kernel does not serve (top-k above 256, a zone or a candidate list
-// that outgrows its buffer) are appended to a work list that the single-CTA
-// kernel processes right after.
+// Rows that take another way (top-k above 256, a zone or a candidate list that
+// outgrows its buffer) are done by rank 0's CTA alone, with the single-CTA
+// kernel's routine: no work list, and no second launch that finds it empty.
+//
+// Bound: latency. A batch of a few rows moves a megabyte or two; what counts is
+// the number of dependent steps, the first of which (the slice's copies) is under
+// way before the row's configuration has been read.
 //
 // Control flow is uniform across a cluster: every CTA passes the same cluster
 // barriers, and nobody touches a peer's shared memory after the last one.
@@ -34,6 +38,7 @@
 #include <type_traits>
 
 #include "sample_kernel.cuh"
+#include "small_set.cuh"
 
 namespace gs {
 namespace cg = cooperative_groups;
@@ -42,19 +47,21 @@ constexpr int CL_MAX = 8;            // largest cluster
 constexpr int NB1 = 1024;            // buckets of width 1/32 over d in [-32, 0]
 constexpr int ZCAP = 2048;           // exact zone list capacity on rank 0 (entries of 8 B)
 constexpr int ZLOC = 1024;           // per-CTA zone list capacity
-constexpr int UCAP = 2048;           // merged top-k candidate capacity on rank 0
+constexpr int UCAP = 2048;           // merged top-k candidate capacity on rank 0 ...
+constexpr int WCAP = 4096;           // ... and with the lists in rank 0's slice (fits the smallest one)
+constexpr int LCAP = 2048;           // a rank's own candidates (region B)
 constexpr int KFAST = 256;           // largest top_k served here
-constexpr int KEEP_MAX = 512;        // largest kept set finished here
 constexpr int NSUB = 1024;           // sub-buckets of one weighted-selection round
 constexpr int REGION_A = 16384;      // bytes: zone keys / merged candidates / histogram staging
 constexpr int REGION_B = 16384;      // bytes: local lists, bucket table, selection scratch
 constexpr int MIN_SLICE_BYTES = 32768;
+static_assert(WCAP * 8 <= MIN_SLICE_BYTES && KEEP_MAX * 8 <= REGION_B && SS_WORK_BYTES <= MIN_SLICE_BYTES &&
+              POOL_BYTES <= MIN_SLICE_BYTES + REGION_A + REGION_B, "region sizes");
 
 struct ClusterArgs {
   KernelArgs k;
   int32_t slice_bytes;      // shared bytes reserved for the slice region
   const double* eb_table;   // 1024 doubles: exp(-b/32)
-  int32_t* worklist;        // [0] = count, [1..] = rows left to the single-CTA kernel
 };
 
 // Written by peers through distributed shared memory. Every slot has exactly one
@@ -68,7 +75,7 @@ struct Xchg {
   // pushed by rank 0
   float dA, dB;
   int zone_total;
-  int verdict;            // 0 owner resolves, 1 poisoned, 2 handed to the work list, 3 id written by rank 0
+  int verdict;            // 0 owner resolves, 1 poisoned, 2 rank 0 does the row alone, 3 id written by rank 0
   int owner;
   unsigned long long cut_key;   // zone entries are kept when key < cut_key, or == cut_key with cut_incl
   int cut_incl;
@@ -199,8 +206,9 @@ __device__ __forceinline__ void block_scan_excl_d2(double a, double b, double& e
   ea = ba + ia - a; eb_ = bb + ib - b; ta = sa; tb = sb;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
+// D: with the optional outputs (probabilities, debug records).
+template <typename T, bool D>
+__global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_constant__ ClusterArgs CA) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ Ctl ctl;
   __shared__ Xchg X;
@@ -231,15 +239,20 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
   unsigned char* regA = dyn + CA.slice_bytes;
   unsigned char* regB = regA + REGION_A;
 
+  // the slice's copies go out before anything else is read; a thread later looks at the vectors it copied itself
+  for (int j = tid; j < nv; j += NT)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+                 :: "r"(static_cast<uint32_t>(__cvta_generic_to_shared(slice + j))), "l"(rv.vbase + v0 + j) : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+
   RowCfg cfg;
   if (A.force_greedy) { cfg.temperature = 0.f; cfg.top_k = 0; cfg.top_p = 0.f; cfg.topp_mode = 0; }
   else cfg = A.cfgs[row_id];
   const float Tm = cfg.temperature;
+  const double u = A.force_greedy ? 0.0 : A.uniforms[row_id];
 
-  if (tid < 256) s_tab[tid] = A.exp_table[tid];
   if (tid < CL_MAX) s_zk[tid] = 0.0;
   if (tid == 0) { ctl.cand_count = 0; ctl.overflow = 0; }
-  __syncthreads();
 
   Xchg* X0 = cluster.map_shared_rank(&X, 0);
   const double QNAN = __longlong_as_double(0x7ff8000000000000ll);
@@ -247,42 +260,42 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
     if (tid == 0) {
       A.out_ids[row_id] = id;
       if (A.out_flags) A.out_flags[row_id] = flags;
-      if (A.out_debug) A.out_debug[row_id] = dbg;
+      if (D && A.out_debug) A.out_debug[row_id] = dbg;
     }
   };
   auto fill_probs_slice = [&](double v) {   // this CTA's share of the dense probability row
-    if (A.out_probs) {
+    if (D && A.out_probs) {
       double* pr = A.out_probs + row_id * static_cast<int64_t>(V);
       int i_lo = max(0, v0 * VEC - rv.shift), i_hi = min(V, v1 * VEC - rv.shift);
       for (int i = i_lo + tid; i < i_hi; i += NT) pr[i] = v;
     }
   };
   auto fill_probs_row = [&](double v) {
-    if (A.out_probs) {
+    if (D && A.out_probs) {
       double* pr = A.out_probs + row_id * static_cast<int64_t>(V);
       for (int i = tid; i < V; i += NT) pr[i] = v;
     }
   };
-  auto to_worklist = [&]() {                // rank 0 hands the row to the single-CTA kernel
-    if (tid == 0) {
-      int slot = atomicAdd(&CA.worklist[0], 1);
-      CA.worklist[1 + slot] = static_cast<int32_t>(row_id);
-    }
+  auto alone = [&]() {                      // rank 0, after the cluster's last barrier: the row from global memory
+    __syncthreads();
+    single_cta_row<T>(A, row_id, dyn);
   };
 
   RowDebug dbg;
   dbg.sum_exp = 0; dbg.resum = 1.0; dbg.edge_lo = 0; dbg.edge_hi = 0; dbg.kept = 0;
   dbg.max_scaled = 0; dbg.threshold = __int_as_float(0x7fc00000); dbg.path = 0;
   for (int q = 0; q < 8; q++) dbg.reserved[q] = 0;
-  long long tprev = clock64();
-  auto stamp = [&](int slot) { long long now = clock64(); dbg.reserved[slot] = static_cast<uint32_t>(now - tprev); tprev = now; };
+  long long tprev = D ? clock64() : 0;
+  auto stamp = [&](int slot) {
+    if (D) { const long long now = clock64(); dbg.reserved[slot] = static_cast<uint32_t>(now - tprev); tprev = now; }
+  };
 
   // ================================================================ greedy
   if (Tm == 0.0f) {
     unsigned long long best = 0ull;
-    for (int v = v0 + tid; v < v1; v += NT) {
-      uint4 raw = __ldg(rv.vbase + v);
-      rv.visit_raw(raw, v, [&](float x, int i, int) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    for (int j = tid; j < nv; j += NT) {
+      rv.visit_raw(slice[j], v0 + j, [&](float x, int i, int) {
         unsigned long long p = (static_cast<unsigned long long>(okey(x)) << 32) |
                                static_cast<uint32_t>(~static_cast<uint32_t>(i));
         best = p > best ? p : best;
@@ -300,7 +313,7 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
       float x0 = 0.f;
       rv.visit(0, [&](float x, int i) { if (i == 0) x0 = x; });
       if (x0 != x0) id = 0;     // generate.go:136: maxVal starts as NaN, nothing is greater
-      if (A.out_probs && tid == 0) A.out_probs[row_id * static_cast<int64_t>(V) + id] = 1.0;
+      if (D && A.out_probs && tid == 0) A.out_probs[row_id * static_cast<int64_t>(V) + id] = 1.0;
       dbg.kept = 1;
       finish(id, 0u, dbg);
     }
@@ -309,6 +322,7 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
   if (!(Tm > 0.0f) || !(Tm < INFINITY)) {
     fill_probs_slice(QNAN);
     if (rank == 0) finish(-1, FLAG_BAD_CFG, dbg);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     cluster.barrier_wait();
     return;
   }
@@ -316,95 +330,75 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
   const int topk = (cfg.top_k > 0 && cfg.top_k < V) ? cfg.top_k : 0;
   const bool topp_on = (cfg.top_p > 0.0f && cfg.top_p < 1.0f);
   const int mode = cfg.topp_mode;
-  const double u = A.uniforms[row_id];
   const double plim = (mode == 0) ? static_cast<double>(cfg.top_p) * 1.5 : static_cast<double>(cfg.top_p);
   const bool cut_on = topp_on && !(mode == 0 && plim >= 1.0);
   const bool t_is_one = (Tm == 1.0f);
   uint32_t flags = 0;
 
-  if (topk > KFAST || (topk > 0 && topk * C > UCAP / 2)) {
+  if (topk > KFAST) {
     // large top-k: the single-CTA kernel's counting select serves it
-    if (rank == 0) to_worklist();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     cluster.barrier_wait();
+    if (rank == 0) alone();
     return;
   }
 
-  // ---- L / pass A: slice -> shared memory; max, min, NaN, one running max per thread
+  // ---- L / pass A: the slice in shared memory; max, min, NaN, one running max per thread
+  const double tab_me = (topk == 0 && tid < 256) ? A.exp_table[tid] : 0.0;
   float xmax = -INFINITY, xmin = INFINITY;
   bool nan_seen = false;
-  // four vectors per thread in flight at a time: a slice of 50 KB is two trips to HBM, not seven
-  for (int vb = v0 + tid; vb < v1; vb += 4 * NT) {
-    uint4 r4[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) r4[q] = __ldg(rv.vbase + min(vb + q * NT, v1 - 1));
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const int v = vb + q * NT;
-      if (v < v1) slice[v - v0] = mask_and_stats(rv, v, r4[q], xmax, xmin, nan_seen);
-    }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  for (int j = tid; j < nv; j += NT) {
+    const int v = v0 + j;
+    const uint4 raw = slice[j];
+    const uint4 masked = mask_and_stats(rv, v, raw, xmax, xmin, nan_seen);
+    if (v == 0 || v >= rv.nvec - 1) slice[j] = masked;
   }
-  const float tmax = xmax;                                  // this thread's group maximum
-  const int anynan_loc = block_max_i(nan_seen ? 1 : 0, ctl, tid);
-  const unsigned long long pmax = block_max_u64(static_cast<unsigned long long>(okey(xmax)) << 32, ctl, tid);
-  const float slice_min = okey_to_float(static_cast<uint32_t>(block_min_u64(static_cast<unsigned long long>(okey(xmin)), ctl, tid)));
-  stamp(0);
+  if (topk == 0 && tid < 256) s_tab[tid] = tab_me;
 
   // ======================================================= top-k, k <= 256
   if (topk > 0) {
-    // thr0: a lower bound of the k-th largest logit = lower edge of the 16-bit key
-    // bin that holds the k-th largest of the 512 per-thread maxima.
-    uint32_t prefix = 0, mask = 0;
-    int need = topk;
-    const uint32_t mykey = okey(tmax);
-    bool have_thr = true;
-    for (int round = 0; round < 2; round++) {
-      const int sh = 24 - 8 * round;
-      __syncthreads();
-      if (tid < 256) s_sel[tid] = 0;
-      if (tid == 0) ctl.bcast_i[0] = -1;
-      __syncthreads();
-      if ((mykey & mask) == prefix) atomicAdd(&s_sel[(mykey >> sh) & 255u], 1u);
-      __syncthreads();
-      if (tid < 32) {
-        int loc[8];
-        int s = 0;
+    // thr0: a lower bound of the k-th largest logit = lower edge of the bucket (256 of them over the range
+    // of the order keys) that holds the k-th largest of the 512 per-thread maxima.
+    const uint32_t mykey = okey(xmax);
+    uint32_t klo = __reduce_min_sync(FULL, mykey), khi = __reduce_max_sync(FULL, mykey);
+    const unsigned nanw = __ballot_sync(FULL, nan_seen);
+    if (tid < 256) s_sel[tid] = 0u;
+    if (lane == 0) { ctl.red_u64[warp] = (static_cast<unsigned long long>(khi) << 32) | klo; ctl.red_i[warp] = nanw ? 1 : 0; }
+    if (tid == 0) ctl.bcast_i[0] = 0;
+    __syncthreads();                                         // every slice is complete too
+    {
+      const unsigned long long w = ctl.red_u64[lane & (NW - 1)];
+      klo = __reduce_min_sync(FULL, static_cast<uint32_t>(w));
+      khi = __reduce_max_sync(FULL, static_cast<uint32_t>(w >> 32));
+    }
+    const int anynan_loc = __reduce_max_sync(FULL, ctl.red_i[lane & (NW - 1)]);
+    const unsigned long long pmax = static_cast<unsigned long long>(khi) << 32;
+    const int bsh = max(0, 24 - __clz(khi - klo));
+    atomicAdd(&s_sel[(khi - mykey) >> bsh], 1u);
+    __syncthreads();
+    if (tid < 32) {
+      int loc[8], s = 0;
 #pragma unroll
-        for (int j = 7; j >= 0; j--) { s += static_cast<int>(s_sel[tid * 8 + j]); loc[j] = s; }
-        int run = s;
+      for (int j = 0; j < 8; j++) { s += static_cast<int>(s_sel[tid * 8 + j]); loc[j] = s; }
+      int run = s;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          int t = __shfl_down_sync(FULL, run, o);
-          if (tid + o < 32) run += t;
-        }
-        const int above = run - s;
-        if (above < need && above + s >= need) {
+      for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(FULL, run, o); if (tid >= o) run += t; }
+      const int before = run - s;
+      if (before < topk && run >= topk) {
+        int b = 0;
 #pragma unroll
-          for (int j = 7; j >= 0; j--) {
-            if (above + loc[j] >= need) {
-              ctl.bcast_i[0] = tid * 8 + j;
-              ctl.bcast_i[1] = need - (above + loc[j] - static_cast<int>(s_sel[tid * 8 + j]));
-              break;
-            }
-          }
-        }
+        for (int j = 7; j >= 0; j--) if (before + loc[j] >= topk) b = tid * 8 + j;
+        const uint32_t top = khi - (static_cast<uint32_t>(b) << bsh), width = (1u << bsh) - 1u;
+        const uint32_t edge = (top - klo > width) ? top - width : klo;
+        ctl.thr = (edge > 0x007fffffu) ? quotient_class_floor(okey_to_float(edge), Tm) : -INFINITY;   // at or below -Inf: keep everything
+        ctl.bcast_i[0] = 1;
       }
-      __syncthreads();
-      if (ctl.bcast_i[0] < 0) { have_thr = false; break; }   // fewer than k groups: keep everything
-      prefix |= static_cast<uint32_t>(ctl.bcast_i[0]) << sh;
-      mask |= 255u << sh;
-      need = ctl.bcast_i[1];
     }
-    float thr0 = -INFINITY;
-    if (prefix <= 0x007fffffu) have_thr = false;             // bound at or below -Inf: keep everything
-    if (have_thr) {
-      __syncthreads();
-      if (tid == 0) ctl.thr = quotient_class_floor(okey_to_float(prefix), Tm);
-      __syncthreads();
-      thr0 = ctl.thr;
-    }
+    __syncthreads();
+    const float thr0 = ctl.bcast_i[0] ? ctl.thr : -INFINITY;  // (fewer than k groups: keep everything)
     // pass B: candidates >= thr0 from shared memory
-    uint2* lc = reinterpret_cast<uint2*>(regB);              // up to 2048 entries
-    const int cap_r = UCAP / C;
+    uint2* lc = reinterpret_cast<uint2*>(regB);              // LCAP entries
     for (int j = tid; j < nv; j += NT) {
       float x[VEC];
       Elem<T>::unpack(slice[j], x);
@@ -418,26 +412,37 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
           int i = i0 + c;
           if (x[c] >= thr0 && i >= 0 && i < V) {
             int slot = atomicAdd(&ctl.cand_count, 1);
-            if (slot < cap_r) lc[slot] = make_uint2(__float_as_uint(x[c]), static_cast<uint32_t>(i));
+            if (slot < LCAP) lc[slot] = make_uint2(__float_as_uint(x[c]), static_cast<uint32_t>(i));
           }
         }
       }
     }
     __syncthreads();
-    const int n_loc = ctl.cand_count;
-    const bool giveup = n_loc > cap_r;
+    // Where the lists meet: rank 0's region A while UCAP entries are enough for all ranks; a larger top_k takes
+    // rank 0's slice, after one more barrier that says that rank 0 is through with it.
+    const bool wide_lists = topk * C > UCAP / 2;             // uniform over the cluster
+    const int cap_r = wide_lists ? WCAP / C : UCAP / C;
+    int n_loc = ctl.cand_count;
+    if (n_loc > cap_r && n_loc <= LCAP) {                    // more than this rank's share: only what can be kept
+      uint2* few = reinterpret_cast<uint2*>(dyn);            // (the slice has been read; peers may already write to region A)
+      n_loc = narrow_list<NT>(lc, n_loc, topk, Tm, okey(thr0), khi, few, s_sel, ctl.bcast_i, &ctl.cand_count, tid);
+      for (int j = tid; j < min(n_loc, KEEP_MAX); j += NT) lc[j] = few[j];
+      __syncthreads();
+    }
+    const bool giveup = n_loc > min(cap_r, LCAP);
     stamp(1);
     cluster.barrier_wait();
+    if (wide_lists) cluster.sync();
     if (tid == 0) {
       X0->u64[rank] = pmax | static_cast<unsigned long long>(anynan_loc);
       X0->cnt[rank] = giveup ? 0 : n_loc;
       X0->giveup[rank] = giveup ? 1 : 0;
     }
     if (!giveup) {
-      uint2* dst = cluster.map_shared_rank(reinterpret_cast<uint2*>(regA), 0) + rank * cap_r;
+      uint2* dst = cluster.map_shared_rank(reinterpret_cast<uint2*>(wide_lists ? dyn : regA), 0) + rank * cap_r;
       for (int j = tid; j < n_loc; j += NT) dst[j] = lc[j];
     }
-    cluster.sync();                                          // B1: the only barrier of this path
+    cluster.sync();                                          // B1: the last barrier of this path
     if (rank != 0) return;
     stamp(2);
     // ---------------- rank 0: merge and finish in shared memory
@@ -450,160 +455,37 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
       bad |= X.giveup[r];
       n += X.cnt[r];
     }
-    if (bad) { to_worklist(); return; }
+    if (bad) { alone(); return; }
     xmax = okey_to_float(static_cast<uint32_t>(mx >> 32));
     const float m = scale_t(xmax, Tm);
     dbg.max_scaled = m;
-    auto poison_exit = [&](bool nan_sum) {
+    if (anynan || !(fabsf(m) < INFINITY)) {
       fill_probs_row(QNAN);
-      if (nan_sum) dbg.sum_exp = QNAN;
+      dbg.sum_exp = QNAN;
       finish(V - 1, flags | FLAG_NONFINITE | FLAG_FALLBACK, dbg);
+      return;
+    }
+    const uint2* lists = reinterpret_cast<const uint2*>(wide_lists ? dyn : regA);
+    const int caplog = 31 - __clz(cap_r);                    // a power of two
+    auto each = [&](auto&& f) {
+      for (int j = tid; j < C << caplog; j += NT)
+        if ((j & (cap_r - 1)) < X.cnt[j >> caplog]) f(lists[j]);
     };
-    if (anynan || !(fabsf(m) < INFINITY)) { poison_exit(true); return; }
-    // compact the per-rank sub-ranges of region A into region B
-    uint2* uc = reinterpret_cast<uint2*>(regB);
-    {
-      const uint2* src = reinterpret_cast<const uint2*>(regA);
-      int off = 0;
-      for (int r = 0; r < C; r++) {
-        const int cr = X.cnt[r];
-        for (int j = tid; j < cr; j += NT) uc[off + j] = src[r * cap_r + j];
-        off += cr;
-      }
-    }
-    __syncthreads();
-    float keep_lo = -INFINITY;
-    if (n > topk) {
-      uint32_t kkey = block_select_kth(uc, n, topk, s_sel, ctl, tid);
-      if (tid == 0) ctl.thr = quotient_class_floor(okey_to_float(kkey), Tm);
-      __syncthreads();
-      keep_lo = ctl.thr;
-    }
-    // kept entries -> region A; order by index with a counting rank
-    uint2* kp = reinterpret_cast<uint2*>(regA);
-    __syncthreads();
-    if (tid == 0) ctl.cand_count = 0;
-    __syncthreads();
-    for (int j = tid; j < n; j += NT) {
-      uint2 e = uc[j];
-      if (__uint_as_float(e.x) >= keep_lo) {
-        int slot = atomicAdd(&ctl.cand_count, 1);
-        if (slot < KEEP_MAX) kp[slot] = e;
-      }
-    }
-    __syncthreads();
-    const int nk = ctl.cand_count;
-    if (nk > KEEP_MAX) { to_worklist(); return; }            // long run of ties at the threshold
-    // work arrays over the slice region (free now)
-    unsigned char* wr = dyn;
-    float* sx = reinterpret_cast<float*>(wr);                // [512] scaled value, index order
-    int* sidx = reinterpret_cast<int*>(wr + 2048);           // [512]
-    double* se = reinterpret_cast<double*>(wr + 4096);       // [512]
-    double* sf = reinterpret_cast<double*>(wr + 8192);       // [512]
-    int* rnk = reinterpret_cast<int*>(wr + 12288);           // [512]
-    int* ord = reinterpret_cast<int*>(wr + 14336);           // [512]
-    float thr_s = INFINITY;
-    if (tid < nk) {
-      const uint32_t myi = kp[tid].y;
-      int r = 0;
-      for (int l = 0; l < nk; l++) r += (kp[l].y < myi) ? 1 : 0;
-      float s = scale_t(__uint_as_float(kp[tid].x), Tm);
-      sx[r] = s;
-      sidx[r] = static_cast<int>(myi);
-      thr_s = s;
-    }
-    dbg.threshold = okey_to_float(static_cast<uint32_t>(block_min_u64(static_cast<unsigned long long>(okey(thr_s)), ctl, tid)));
-    __syncthreads();
-    double e_me = 0.0;
-    if (tid < nk) e_me = exp(static_cast<double>(sx[tid] - m));   // f32 subtract, f64 exp (generate.go:176)
-    double S;
-    (void)block_scan_excl_d(e_me, S, ctl, tid);
-    dbg.sum_exp = S;
-    const double q_me = e_me / S;                                 // generate.go:179-181
-    if (tid < nk) se[tid] = q_me;
-    __syncthreads();
-    double f_me = q_me;
-    if (topp_on) {
-      // order by probability; equal probabilities by index, ascending in both flavours
-      // (mode A removes the lowest index first, mode B keeps it first)
-      if (tid < nk) {
-        int r = 0;
-        if (mode == 0) { for (int l = 0; l < nk; l++) { double ql = se[l]; r += (ql < q_me || (ql == q_me && l < tid)) ? 1 : 0; } }
-        else           { for (int l = 0; l < nk; l++) { double ql = se[l]; r += (ql > q_me || (ql == q_me && l < tid)) ? 1 : 0; } }
-        ord[r] = tid;
-        rnk[tid] = r;
-      }
-      __syncthreads();
-      if (mode == 0) {
-        // generate.go:184-228: the mass left after removing the r smallest is a suffix sum.
-        // Scan from the largest down: position t holds rank nk-1-t.
-        const double v = (tid < nk) ? se[ord[nk - 1 - tid]] : 0.0;
-        double tot;
-        const double exs = block_scan_excl_d(v, tot, ctl, tid);
-        if (tid < nk) sf[nk - 1 - tid] = exs + v;                   // sf[r] = left after removing r smallest
-        __syncthreads();
-        int rs = nk;
-        if (tid < nk && sf[tid] <= plim) rs = tid;
-        const int rstar = block_min_i(rs, ctl, tid);
-        if (rstar == nk) { dbg.resum = 0.0; poison_exit(false); return; }   // everything removed: 0/0
-        const double resum = sf[rstar];
-        if (fabs(resum - plim) <= 1e-12) flags |= FLAG_TOPP_EDGE;
-        if (rstar > 0 && fabs(sf[rstar - 1] - plim) <= 1e-12) flags |= FLAG_TOPP_EDGE;
-        dbg.resum = resum;
-        f_me = (tid < nk && rnk[tid] >= rstar) ? q_me / resum : 0.0;
-      } else {
-        // qwen/generate.go:123-153: shortest descending prefix with mass >= p
-        const double v = (tid < nk) ? se[ord[tid]] : 0.0;
-        double tot;
-        const double exs = block_scan_excl_d(v, tot, ctl, tid);
-        if (tid < nk) sf[tid] = exs + v;
-        __syncthreads();
-        int cl = nk;
-        if (tid < nk && sf[tid] >= plim) cl = tid + 1;
-        const int cutn = block_min_i(cl, ctl, tid);
-        const double resum = sf[cutn - 1];
-        if (fabs(resum - plim) <= 1e-12) flags |= FLAG_TOPP_EDGE;
-        if (cutn >= 2 && fabs(sf[cutn - 2] - plim) <= 1e-12) flags |= FLAG_TOPP_EDGE;
-        if (cutn < nk && se[ord[cutn]] == se[ord[cutn - 1]]) flags |= FLAG_TIE_CUT;
-        dbg.resum = resum;
-        f_me = (tid < nk && rnk[tid] < cutn) ? q_me / resum : 0.0;
-      }
-    }
-    dbg.kept = block_sum_i((tid < nk && f_me > 0) ? 1 : 0, ctl, tid);
-    if (A.out_probs) {
-      fill_probs_row(0.0);
-      __syncthreads();
-      if (tid < nk) A.out_probs[row_id * static_cast<int64_t>(V) + sidx[tid]] = f_me;
-    }
-    // draw (generate.go:231-239): first index with u < cumulative
-    double tot;
-    const double cexcl = block_scan_excl_d(f_me, tot, ctl, tid);
-    const double c_me = cexcl + f_me;
-    int pl = nk;
-    if (tid < nk && u < c_me) pl = tid;
-    const int pick = block_min_i(pl, ctl, tid);
-    if (pick < nk && tid == pick) { ctl.bcast_d[0] = cexcl; ctl.bcast_d[1] = c_me; }
-    __syncthreads();
-    int id;
-    if (pick < nk) {
-      id = sidx[pick];
-      const double lo = ctl.bcast_d[0], hi = ctl.bcast_d[1];
-      dbg.edge_lo = lo; dbg.edge_hi = hi;
-      if ((pick > 0 && u - lo <= 1e-6) || hi - u <= 1e-6) flags |= FLAG_BOUNDARY;
-    } else {
-      id = V - 1;
-      flags |= FLAG_FALLBACK;
-      dbg.edge_lo = dbg.edge_hi = tot;
-      if (u - tot <= 1e-6) flags |= FLAG_BOUNDARY;
-    }
-    stamp(3);
-    finish(id, flags, dbg);
+    uint2* kp = reinterpret_cast<uint2*>(regB);               // the local list is done with
+    const int nk = narrow_candidates<NT>(each, n, topk, Tm, okey(thr0), static_cast<uint32_t>(mx >> 32), kp, s_sel, ctl.bcast_i,
+                                         &ctl.cand_count, tid);
+    if (nk > KEEP_MAX) { alone(); return; }                  // long run of ties at the threshold
+    finish_small_set<NT, D>(A, row_id, kp, nk, topk, m, Tm, topp_on, mode, plim, u, -INFINITY, dyn, D ? &dbg : nullptr, flags);
     return;
   }
 
   // ============================================================ full row (top-k off)
   dbg.path = 2;
   flags |= FLAG_GENERAL_PATH;
+  const int anynan_loc = block_max_i(nan_seen ? 1 : 0, ctl, tid);
+  const unsigned long long pmax = block_max_u64(static_cast<unsigned long long>(okey(xmax)) << 32, ctl, tid);
+  const float slice_min = okey_to_float(static_cast<uint32_t>(block_min_u64(static_cast<unsigned long long>(okey(xmin)), ctl, tid)));
+  stamp(0);
   cluster.barrier_wait();
   if (tid == 0) {
     const unsigned long long p = pmax | static_cast<unsigned long long>(anynan_loc);
@@ -977,7 +859,6 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
     int owner = -1;
     int code;                                                // see Xchg::verdict
     if (bad) {
-      to_worklist();
       code = 2;
     } else if (poisoned || !(Re > 0.0)) {
       // NaN/Inf in the row, or mode A removed every token (generate.go:221-227): the walk falls through
@@ -1021,14 +902,14 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
       }
       if (code == 0) {                                       // the owner adds the id, the edges and the boundary flag
         if (A.out_flags) A.out_flags[row_id] = flags;
-        if (A.out_debug) A.out_debug[row_id] = dbg;
+        if (D && A.out_debug) A.out_debug[row_id] = dbg;
       }
     }
   }
   cluster.sync();                                            // G5: last barrier
 
   const int verdict = X.verdict;
-  if (verdict == 2) return;                                  // the work list owns this row now
+  if (verdict == 2) { if (rank == 0) alone(); return; }
   if (verdict == 1) { fill_probs_slice(QNAN); return; }
   const double Re = X.Re, S = X.S;
   const unsigned long long ckey = X.cut_key;
@@ -1046,7 +927,7 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
     return exp_safe(d, s_tab);
   };
 
-  if (A.out_probs || A.out_debug) {                          // parity runs only
+  if (D && (A.out_probs || A.out_debug)) {                          // parity runs only
     double* pr = A.out_probs ? A.out_probs + row_id * static_cast<int64_t>(V) : nullptr;
     const double rq = Re / S;
     int kept_loc = 0;
@@ -1065,7 +946,7 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
       }
     }
     const int kept_cta = block_sum_i(kept_loc, ctl, tid);
-    if (A.out_debug && tid == 0) atomicAdd(&A.out_debug[row_id].kept, kept_cta);
+    if (D && A.out_debug && tid == 0) atomicAdd(&A.out_debug[row_id].kept, kept_cta);
   }
   if (verdict == 3 || rank != X.owner) return;
 
@@ -1168,7 +1049,7 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(ClusterArgs CA) {
   if (tid == 0) {
     A.out_ids[row_id] = id;
     if (A.out_flags && oflags) atomicOr(&A.out_flags[row_id], oflags);
-    if (A.out_debug) { A.out_debug[row_id].edge_lo = edge_lo; A.out_debug[row_id].edge_hi = edge_hi; }
+    if (D && A.out_debug) { A.out_debug[row_id].edge_lo = edge_lo; A.out_debug[row_id].edge_hi = edge_hi; }
   }
 }
 

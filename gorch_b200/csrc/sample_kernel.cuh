@@ -36,7 +36,8 @@ constexpr int POOL_HIST = 0;                       // 16 KB: uint32[4096] histog
 constexpr int POOL_CAND = 16384;                   // 16 KB: uint2[2048] candidates / zone list
 constexpr int POOL_X = 32768;                      // 16 KB: scratch for sorted values
 constexpr int POOL_Y = 49152;                      // 8 KB: order / rank scratch
-constexpr int POOL_BYTES = 57344;
+constexpr int POOL_STATE = 57344;                  // SingleState
+constexpr int POOL_BYTES = 57344 + 5120;
 
 struct KernelArgs {
   const void* logits;      // [B, row_stride] f32 or bf16
@@ -336,12 +337,22 @@ __device__ __forceinline__ int bucket0(float d) {
   return __float_as_int(f) & 0x1fff;
 }
 
+struct SingleState {
+  Ctl ctl;
+  Cut cut;
+  double tab[256];
+  double kseg[MAXSEG];
+};
+static_assert(POOL_STATE + sizeof(SingleState) <= POOL_BYTES, "the pool holds the row's state");
+
+// Not inlined: the kernels that fall back on it for the odd row keep their registers.
 template <typename T>
-__device__ void single_cta_row(const KernelArgs& A, const int64_t row_id, unsigned char* pool) {
-  __shared__ Ctl ctl;
-  __shared__ Cut cut;
-  __shared__ double s_tab[256];
-  __shared__ double s_kseg[MAXSEG];
+__device__ __noinline__ void single_cta_row(const KernelArgs& A, const int64_t row_id, unsigned char* pool) {
+  SingleState& state = *reinterpret_cast<SingleState*>(pool + POOL_STATE);
+  Ctl& ctl = state.ctl;
+  Cut& cut = state.cut;
+  double* s_tab = state.tab;
+  double* s_kseg = state.kseg;
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
@@ -1223,7 +1234,7 @@ __device__ void single_cta_row(const KernelArgs& A, const int64_t row_id, unsign
 
 // One CTA per row; with a work list, a fixed grid walks the listed rows.
 template <typename T>
-__global__ void __launch_bounds__(NT, 2) sample_rows_kernel(KernelArgs A) {
+__global__ void __launch_bounds__(NT, 2) sample_rows_kernel(const __grid_constant__ KernelArgs A) {
   extern __shared__ __align__(16) unsigned char pool[];
   if (A.worklist) {
     const int n = A.worklist[0];

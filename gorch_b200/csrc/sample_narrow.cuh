@@ -9,12 +9,11 @@ namespace GS_N_NS {
 constexpr int N_NT = GS_N_NT;           // threads per CTA
 constexpr int N_NW = N_NT / 32;
 constexpr int N_WARM_ELEMS = 16 * N_NT; // logits of the warm-up chunk: 16 per thread, kept in registers
-// 256 threads: five CTAs per SM (48 registers, 42 KB of dynamic shared memory: [0, 24 KB) the ring
-// the stream is staged through, whose upper 16 KB double as the work arrays of the phases that
-// run while no copy is in flight (prune, finish); then the candidate list and the hit list).
-// 128 threads: eight CTAs per SM (64 registers, 20 KB: candidate list, ring, hit list; the
-// prune's buffer is the ring, the finish's work arrays lie over the upper half of the candidate
-// list, the ring and the hit list, all of them dead by then).
+// 256 threads: five CTAs per SM (48 registers, 42 KB of dynamic shared memory: the ring that the
+// stream is staged through, the candidate list, the hit list). 128 threads: eight CTAs per SM
+// (64 registers, 20 KB: candidate list, ring, hit list). What runs while no copy is in flight works in
+// memory that is dead by then: the prune in the ring; the finish in the ring (256 threads), or over
+// the candidate list and the ring, with the kept set in the hit list's place (128 threads).
 constexpr int N_CTAS_PER_SM = (N_NT == 256) ? 5 : 8;
 constexpr int N_CAP = (N_NT == 256) ? 1536 : 1024;   // candidate capacity (entries of 8 B)
 constexpr int N_KEEP = 768;                           // a prune must get below this
@@ -23,19 +22,21 @@ constexpr int N_RING_BYTES = (N_NT == 256) ? 24576 : 8192;
 constexpr int N_RING_OFF = (N_NT == 256) ? 0 : 8192;
 constexpr int N_CAND_OFF = (N_NT == 256) ? 24576 : 0;
 constexpr int N_HITS_OFF = (N_NT == 256) ? N_CAND_OFF + N_CAP * 8 : 16384;
-constexpr int N_WORK_OFF = (N_NT == 256) ? 8192 : 4096;   // 16 KB of work arrays for the finish
+constexpr int N_KEPT_OFF = (N_NT == 256) ? 0 : N_HITS_OFF;   // what the finish works on: KEEP_MAX entries
+constexpr int N_WORK_OFF = (N_NT == 256) ? 8192 : 0;         // its work arrays
 constexpr int N_TMP_OFF = (N_NT == 256) ? 8192 : 8192;    // the prune's buffer ...
 constexpr int N_TMP_CAP = (N_NT == 256) ? 2048 : 1024;    // ... and its entries
 constexpr int N_DYN_BYTES = N_HITS_OFF + N_HITS * 4;
-static_assert(N_WORK_OFF + 16384 <= N_DYN_BYTES &&
-              (N_WORK_OFF >= N_CAND_OFF + KEEP_MAX * 8 || N_WORK_OFF + 16384 <= N_CAND_OFF),
-              "the finish's work arrays leave the kept set alone");
+static_assert((N_NT == 256) ? (N_KEPT_OFF + KEEP_MAX * 8 <= N_WORK_OFF && N_WORK_OFF + SS_WORK_BYTES <= N_RING_BYTES)
+                            : (KEEP_MAX * 8 <= N_HITS * 4 && N_WORK_OFF + SS_WORK_BYTES <= N_HITS_OFF),
+              "the finish works in memory that is dead by then");
 static_assert(N_TMP_OFF >= N_RING_OFF && N_TMP_OFF + N_TMP_CAP * 8 <= N_RING_OFF + N_RING_BYTES, "the prune's buffer lies in the ring");
 static_assert(N_TMP_CAP >= N_KEEP && N_KEEP + 8 <= N_CAP, "a pruned list fits its buffer and leaves room for a portion of hits");
 
-template <typename T>
+// D: with the optional outputs (probabilities, debug records).
+template <typename T, bool D>
 __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned char* dyn, bu::Scratch& sc,
-                           uint32_t* s_sel, int* s_bc, double* s_bcd, int* s_cnt, int* s_hcnt, float* s_thr, int* s_flag,
+                           uint32_t* s_sel, int* s_bc, int* s_cnt, int* s_hcnt, float* s_thr, int* s_flag,
                            const bool allow_tight, bool& redo) {
   const KernelArgs& A = BA.k;
   redo = false;
@@ -46,7 +47,6 @@ __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned c
   const T* row = static_cast<const T*>(A.logits) + row_id * A.row_stride;
   RowView<T> rv;
   rv.init(row, V);
-  unsigned char* work = dyn + N_WORK_OFF;                    // 16 KB of work arrays (finish)
   uint2* cand = reinterpret_cast<uint2*>(dyn + N_CAND_OFF);  // N_CAP entries
   int* hits = reinterpret_cast<int*>(dyn + N_HITS_OFF);      // N_HITS entries
   const double QNAN = __longlong_as_double(0x7ff8000000000000ll);
@@ -60,18 +60,20 @@ __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned c
   dbg.sum_exp = 0; dbg.resum = 1.0; dbg.edge_lo = 0; dbg.edge_hi = 0; dbg.kept = 0;
   dbg.max_scaled = 0; dbg.threshold = __int_as_float(0x7fc00000); dbg.path = 0;
   for (int q = 0; q < 8; q++) dbg.reserved[q] = 0;
-  long long tprev = clock64();
+  long long tprev = D ? clock64() : 0;
   dbg.reserved[3] = static_cast<uint32_t>(tprev);
-  auto stamp = [&](int slot) { const long long now = clock64(); dbg.reserved[slot] = static_cast<uint32_t>(now - tprev); tprev = now; };
+  auto stamp = [&](int slot) {
+    if (D) { const long long now = clock64(); dbg.reserved[slot] = static_cast<uint32_t>(now - tprev); tprev = now; }
+  };
   auto write_row = [&](int id, uint32_t fl) {
     if (tid == 0) {
       A.out_ids[row_id] = id;
       if (A.out_flags) A.out_flags[row_id] = fl;
-      if (A.out_debug) A.out_debug[row_id] = dbg;
+      if (D && A.out_debug) A.out_debug[row_id] = dbg;
     }
   };
   auto fill_probs_row = [&](double v) {
-    if (A.out_probs) {
+    if (D && A.out_probs) {
       double* pr = A.out_probs + row_id * static_cast<int64_t>(V);
       for (int i = tid; i < V; i += N_NT) pr[i] = v;
     }
@@ -107,7 +109,7 @@ __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned c
     }
     fill_probs_row(0.0);
     __syncthreads();
-    if (A.out_probs && tid == 0) A.out_probs[row_id * static_cast<int64_t>(V) + id] = 1.0;
+    if (D && A.out_probs && tid == 0) A.out_probs[row_id * static_cast<int64_t>(V) + id] = 1.0;
     dbg.kept = 1;
     write_row(id, 0u);
     return;
@@ -452,8 +454,9 @@ __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned c
   nan_seen |= (run != run);
   xmax = run;
   stamp(1);
-  dbg.reserved[5] = static_cast<uint32_t>(*s_cnt);
+  if (D) dbg.reserved[5] = static_cast<uint32_t>(*s_cnt);
   int nk = 0;
+  uint2* kept = cand;                                        // where the nk entries are
   if (!giveup && *s_cnt > N_CAP) giveup = true;
   if (!giveup && tight && *s_cnt < topk) {                   // the estimated threshold was too tight for this row
     if (A.vs_records || A.tk_k > 0) { redo = true; return; } // uniform: *s_cnt is read after the loop's last barrier
@@ -463,7 +466,13 @@ __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned c
   xmax = okey_to_float(static_cast<uint32_t>(bu::max_u64<N_NW>(static_cast<unsigned long long>(okey(xmax)), sc, tid)));
   if (!giveup) {
     // the row's maximum bounds the list from above, unless a thread's maximum was lost to a NaN
-    nk = prune(*s_cnt, anynan ? 0xffffffffu : okey(xmax));
+    const uint32_t hi_key = anynan ? 0xffffffffu : okey(xmax);
+    if (A.vs_records) {                                      // a record holds exactly what the slice keeps
+      nk = prune(*s_cnt, hi_key);
+    } else {
+      kept = reinterpret_cast<uint2*>(dyn + N_KEPT_OFF);
+      nk = narrow_list<N_NT>(cand, *s_cnt, topk, Tm, okey(thr), hi_key, kept, s_sel, s_bc, s_cnt, tid);
+    }
     if (nk > KEEP_MAX) giveup = true;                        // long run of ties at the threshold
   }
   const float m = scale_t(xmax, Tm);
@@ -481,13 +490,13 @@ __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned c
       return;
     }
     for (int j = tid; j < nk; j += N_NT) {
-      const uint32_t kj = okey(__uint_as_float(cand[j].x)), ij = cand[j].y;
+      const uint32_t kj = okey(__uint_as_float(kept[j].x)), ij = kept[j].y;
       int r = 0;
       for (int l = 0; l < nk; l++) {
-        const uint32_t kl = okey(__uint_as_float(cand[l].x));
-        r += (kl > kj || (kl == kj && cand[l].y < ij)) ? 1 : 0;
+        const uint32_t kl = okey(__uint_as_float(kept[l].x));
+        r += (kl > kj || (kl == kj && kept[l].y < ij)) ? 1 : 0;
       }
-      if (r < topk) { ov[r] = __uint_as_float(cand[j].x); oi[r] = static_cast<int32_t>(ij); }
+      if (r < topk) { ov[r] = __uint_as_float(kept[j].x); oi[r] = static_cast<int32_t>(ij); }
     }
     if (tid == 0 && A.out_flags) A.out_flags[row_id] = 0u;
     return;
@@ -515,17 +524,16 @@ __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned c
     return;
   }
   stamp(2);
-  finish_small_set<N_NT>(A, row_id, cand, nk, m, Tm, topp_on, mode, plim, A.uniforms[row_id],
-                         work, sc, s_bcd, dbg, 0u);
+  finish_small_set<N_NT, D>(A, row_id, kept, nk, topk, m, Tm, topp_on, mode, plim, A.uniforms[row_id], -INFINITY, dyn + N_WORK_OFF,
+                            D ? &dbg : nullptr, 0u);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(N_NT, N_CTAS_PER_SM) narrow_rows_kernel(BatchArgs BA) {
+template <typename T, bool D>
+__global__ void __launch_bounds__(N_NT, N_CTAS_PER_SM) narrow_rows_kernel(const __grid_constant__ BatchArgs BA) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ bu::Scratch sc;
   __shared__ uint32_t s_sel[256];
   __shared__ int s_bc[4];
-  __shared__ double s_bcd[4];
   __shared__ int s_cnt;
   __shared__ int s_hcnt;
   __shared__ float s_thr;
@@ -554,7 +562,7 @@ __global__ void __launch_bounds__(N_NT, N_CTAS_PER_SM) narrow_rows_kernel(BatchA
     if (row < 0) break;
     bool redo, allow_tight = true;
     for (;;) {                                               // at most twice: the second time without the estimate
-      narrow_row<T>(BA, row, dyn, sc, s_sel, s_bc, s_bcd, &s_cnt, &s_hcnt, &s_thr, &s_flag, allow_tight, redo);
+      narrow_row<T, D>(BA, row, dyn, sc, s_sel, s_bc, &s_cnt, &s_hcnt, &s_thr, &s_flag, allow_tight, redo);
       if (!redo) break;
       allow_tight = false;
       __syncthreads();

@@ -43,16 +43,15 @@ struct MergeArgs {
 // maximum}; a row this rank does not own gets a NaN target.
 constexpr int VD_NT = 256;
 
-__global__ void __launch_bounds__(VM_NT, 8) vocab_merge_kernel(MergeArgs M) {
+__global__ void __launch_bounds__(VM_NT, 8) vocab_merge_kernel(const __grid_constant__ MergeArgs M) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ bu::Scratch sc;
   __shared__ uint32_t s_sel[256];
   __shared__ int s_bc[4];
-  __shared__ double s_bcd[4];
   __shared__ int s_cnt;
   uint2* list = reinterpret_cast<uint2*>(dyn);                                   // joined candidates
   const int list_bytes = vm_list_entries(M.nranks, M.cand) * 8;
-  unsigned char* work = dyn + list_bytes;                                         // 16 KB for finish_small_set
+  unsigned char* work = dyn + list_bytes;                                         // for finish_small_set
   uint2* kept = reinterpret_cast<uint2*>(dyn + list_bytes + 16384);              // KEEP_MAX entries
   const KernelArgs& A = M.k;
   const int tid = threadIdx.x;
@@ -167,25 +166,12 @@ __global__ void __launch_bounds__(VM_NT, 8) vocab_merge_kernel(MergeArgs M) {
     }
     // ---- global k-th largest with ties (generate.go:157-164), then the kept set
     const int topk = cfg.top_k;                              // 0 < top_k <= VS_CAND (checked by the local pass)
-    float thr = -INFINITY;
-    if (cnt > topk) {
-      const uint32_t kkey = bu::select_kth<VM_NT>(list, cnt, topk, s_sel, s_bc, tid, 0u, static_cast<uint32_t>(mx));
-      thr = quotient_class_floor(okey_to_float(kkey), Tm);
-    }
-    __syncthreads();
-    if (tid == 0) s_cnt = 0;
-    __syncthreads();
-    for (int j = tid; j < cnt; j += VM_NT) {
-      const uint2 e = list[j];
-      if (__uint_as_float(e.x) >= thr) { const int slot = atomicAdd(&s_cnt, 1); if (slot < KEEP_MAX) kept[slot] = e; }
-    }
-    __syncthreads();
-    const int nk = s_cnt;
+    const int nk = narrow_list<VM_NT>(list, cnt, topk, Tm, 0u, static_cast<uint32_t>(mx), kept, s_sel, s_bc, &s_cnt, tid);
     if (nk > KEEP_MAX) { write_row(-1, FLAG_INTERNAL); continue; }
     const bool topp_on = (cfg.top_p > 0.0f && cfg.top_p < 1.0f);
     const int mode = cfg.topp_mode;
     const double plim = (mode == 0) ? static_cast<double>(cfg.top_p) * 1.5 : static_cast<double>(cfg.top_p);
-    finish_small_set<VM_NT>(A, row, kept, nk, m, Tm, topp_on, mode, plim, A.uniforms[row], work, sc, s_bcd, dbg, 0u);
+    finish_small_set<VM_NT, false>(A, row, kept, nk, topk, m, Tm, topp_on, mode, plim, A.uniforms[row], -INFINITY, work, nullptr, 0u);
   }
 }
 

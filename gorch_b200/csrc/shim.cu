@@ -227,16 +227,16 @@ size_t elem_size(int dtype) { return dtype == GORCH_CUDA_BF16 ? 2 : 4; }
 static cudaError_t launch_narrow(Ctx* c, const gs::BatchArgs& ba, int dtype, int64_t B) {
   const int64_t slots256 = static_cast<int64_t>(gs::n256::N_CTAS_PER_SM) * c->sm_count;
   const bool small_ctas = c->variant == 6 || (c->variant != 7 && B > slots256);
-  if (small_ctas) {
-    const int64_t slots = static_cast<int64_t>(gs::n128::N_CTAS_PER_SM) * c->sm_count;
-    const unsigned g = static_cast<unsigned>(B < slots ? B : slots);
-    if (dtype == GORCH_CUDA_F32) gs::n128::narrow_rows_kernel<float><<<g, gs::n128::N_NT, gs::n128::N_DYN_BYTES, c->stream>>>(ba);
-    else gs::n128::narrow_rows_kernel<uint16_t><<<g, gs::n128::N_NT, gs::n128::N_DYN_BYTES, c->stream>>>(ba);
-  } else {
-    const unsigned g = static_cast<unsigned>(B < slots256 ? B : slots256);
-    if (dtype == GORCH_CUDA_F32) gs::n256::narrow_rows_kernel<float><<<g, gs::n256::N_NT, gs::n256::N_DYN_BYTES, c->stream>>>(ba);
-    else gs::n256::narrow_rows_kernel<uint16_t><<<g, gs::n256::N_NT, gs::n256::N_DYN_BYTES, c->stream>>>(ba);
-  }
+  const int64_t slots = small_ctas ? static_cast<int64_t>(gs::n128::N_CTAS_PER_SM) * c->sm_count : slots256;
+  const unsigned g = static_cast<unsigned>(B < slots ? B : slots);
+  const bool diag = ba.k.out_probs || ba.k.out_debug;
+  auto go = [&](auto kernel, int nt, int bytes) { kernel<<<g, nt, bytes, c->stream>>>(ba); };
+  auto pick = [&](auto type) {
+    typedef decltype(type) E;
+    if (small_ctas) go(diag ? gs::n128::narrow_rows_kernel<E, true> : gs::n128::narrow_rows_kernel<E, false>, gs::n128::N_NT, gs::n128::N_DYN_BYTES);
+    else go(diag ? gs::n256::narrow_rows_kernel<E, true> : gs::n256::narrow_rows_kernel<E, false>, gs::n256::N_NT, gs::n256::N_DYN_BYTES);
+  };
+  if (dtype == GORCH_CUDA_F32) pick(float()); else pick(uint16_t());
   return cudaGetLastError();
 }
 
@@ -357,18 +357,10 @@ int launch_rows(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int
       }
       CUDA_TRY(cudaGetLastError(), errOut);
     } else {
-      int32_t* wl = fixed_lists;
-      if (!wl) {
-        int rc = ensure(c->worklist, (static_cast<size_t>(B) + 1) * sizeof(int32_t), errOut);
-        if (rc) return rc;
-        wl = static_cast<int32_t*>(c->worklist.ptr);
-      }
-      CUDA_TRY(cudaMemsetAsync(wl, 0, sizeof(int32_t), c->stream), errOut);
       gs::ClusterArgs ca;
       ca.k = a;
       ca.slice_bytes = static_cast<int32_t>(need > gs::MIN_SLICE_BYTES ? need : gs::MIN_SLICE_BYTES);
       ca.eb_table = c->eb_table;
-      ca.worklist = wl;
       const size_t dyn = static_cast<size_t>(ca.slice_bytes) + gs::REGION_A + gs::REGION_B;
       cudaLaunchConfig_t lc = {};
       lc.gridDim = dim3(static_cast<unsigned>(B * C));
@@ -382,23 +374,13 @@ int launch_rows(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int
       at[0].val.clusterDim.z = 1;
       lc.attrs = at;
       lc.numAttrs = 1;
+      const bool diag = out_probs || out_debug;
       if (dtype == GORCH_CUDA_F32) {
-        CUDA_TRY(cudaLaunchKernelEx(&lc, gs::sample_cluster_kernel<float>, ca), errOut);
+        CUDA_TRY(cudaLaunchKernelEx(&lc, diag ? gs::sample_cluster_kernel<float, true> : gs::sample_cluster_kernel<float, false>, ca), errOut);
       } else {
-        CUDA_TRY(cudaLaunchKernelEx(&lc, gs::sample_cluster_kernel<uint16_t>, ca), errOut);
-      }
-      // rows the cluster kernel handed over (rare): a fixed grid walks the list
-      gs::KernelArgs aw = a;
-      aw.worklist = ca.worklist;
-      const int64_t wg = B < 2 * c->sm_count ? B : 2 * c->sm_count;
-      dim3 grid(static_cast<unsigned>(wg)), block(gs::NT);
-      if (dtype == GORCH_CUDA_F32) {
-        gs::sample_rows_kernel<float><<<grid, block, gs::POOL_BYTES, c->stream>>>(aw);
-      } else {
-        gs::sample_rows_kernel<uint16_t><<<grid, block, gs::POOL_BYTES, c->stream>>>(aw);
+        CUDA_TRY(cudaLaunchKernelEx(&lc, diag ? gs::sample_cluster_kernel<uint16_t, true> : gs::sample_cluster_kernel<uint16_t, false>, ca), errOut);
       }
       CUDA_TRY(cudaGetLastError(), errOut);
-      klaunch = 2;
     }
   }
   c->counters.kernel_launches += static_cast<uint64_t>(klaunch);
@@ -613,12 +595,18 @@ GorchCudaCtxRef gorch_cuda_create_ctx(int device, char** errOut) {
   if ((e = cudaMemcpy(c->eb_table, ebt, sizeof ebt, cudaMemcpyHostToDevice)) != cudaSuccess) return fail("cudaMemcpy(bucket table)", e);
   if ((e = cudaFuncSetAttribute(gs::sample_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::POOL_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::sample_rows_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::POOL_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
-  if ((e = cudaFuncSetAttribute(gs::sample_cluster_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 109 * 1024)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
-  if ((e = cudaFuncSetAttribute(gs::sample_cluster_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, 109 * 1024)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
-  if ((e = cudaFuncSetAttribute(gs::n256::narrow_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n256::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
-  if ((e = cudaFuncSetAttribute(gs::n256::narrow_rows_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n256::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
-  if ((e = cudaFuncSetAttribute(gs::n128::narrow_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n128::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
-  if ((e = cudaFuncSetAttribute(gs::n128::narrow_rows_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n128::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::sample_cluster_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 109 * 1024)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::sample_cluster_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 109 * 1024)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::sample_cluster_kernel<uint16_t, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 109 * 1024)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::sample_cluster_kernel<uint16_t, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 109 * 1024)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::n256::narrow_rows_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n256::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::n256::narrow_rows_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n256::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::n256::narrow_rows_kernel<uint16_t, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n256::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::n256::narrow_rows_kernel<uint16_t, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n256::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::n128::narrow_rows_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n128::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::n128::narrow_rows_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n128::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::n128::narrow_rows_kernel<uint16_t, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n128::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::n128::narrow_rows_kernel<uint16_t, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n128::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::multinomial_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::MN_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = topk_large_attributes<gs::TklSmall>()) != cudaSuccess || (e = topk_large_attributes<gs::TklFew>()) != cudaSuccess ||
       (e = topk_large_attributes<gs::TklMid>()) != cudaSuccess || (e = topk_large_attributes<gs::TklLarge>()) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
