@@ -8,7 +8,7 @@
 //   different order than the reference's sequential loop: a row whose uniform lies within 1e-6 of
 //   an edge of the chosen interval is flagged FLAG_BOUNDARY.
 //   TopK (index_ops.go:153-190): the narrow kernel of sample_batch.cuh with KernelArgs::tk_k set for
-//   k <= 256, topk_large.cuh beyond.
+//   k <= 64, topk_large.cuh beyond.
 #pragma once
 
 #include "sample_batch.cuh"

@@ -7,21 +7,32 @@
 // HBM: here the rows of a batch tile stay in tensor memory until the epilogue has taken what sampling
 // needs from them.
 //
-// One CTA per SM, persistent over vocabulary tiles of 128 columns; a batch tile is 128 rows (rows
-// beyond B are zero-filled by TMA and ignored). Per tile, K is walked in chunks of 64:
-//   warp 0      producer: two TMA loads per chunk (x tile and w tile, 128 x 64 bf16 each, 128-byte
-//               swizzle) into a ring of shared-memory stages, completion on the stage's mbarrier
-//   warp 1      issuer: one elected thread issues tcgen05.mma (M = 128 batch rows, N = 128 vocabulary
-//               columns, K = 16; both operands K-major from shared memory) into one of two accumulator
-//               buffers in tensor memory; tcgen05.commit frees the stage / publishes the accumulator
-//   warps 2-5   epilogue: thread = batch row (a TMEM lane), its 128 logits of the tile by tcgen05.ld;
-//               optional store of the logits, row maximum and NaN flag, and (fused sampling) the logits
-//               at or above the row's threshold appended to the row's candidate list
+// A pair of CTAs (a cluster of two, tcgen05 cta_group::2) works on one tile of 256 vocabulary rows x up
+// to 256 batch rows; the vocabulary is the M side, so that a TMEM lane is a vocabulary column of the
+// output and a warp writes 32 neighbouring logits of a batch row at a time. CTA r of the pair holds
+// vocabulary rows 128 r .. of the tile, half of the batch rows, and the accumulator of its own vocabulary
+// rows. Per item K is walked in chunks of 128:
+//   warp 0      producer (both CTAs): TMA loads (w: 128 x 64, x: N / 2 x 64, 128-byte swizzle; two of each per
+//               chunk, so that 256 neighbouring bytes of a row are asked for together: 6.2 TB/s of weights
+//               against 5.5) into a ring of shared-memory stages; the bytes of both CTAs complete on the
+//               leader's mbarrier
+//   warp 1      issuer (leader): one elected thread issues tcgen05.mma (M = 256, N, K = 16) into one of two
+//               accumulators of 256 TMEM columns; tcgen05.commit frees the stage / publishes the
+//               accumulator in both CTAs
+//   warps 2-9   epilogue (both CTAs): thread = vocabulary row (a TMEM lane), the batch rows' logits by
+//               tcgen05.ld; either stores them, or (fused sampling) appends those at or above their batch
+//               row's threshold to that row's candidate list
+//
+// Bound: at 512 rows the L2-to-SM traffic, the tensor pipe and HBM ask for about the same time each. A
+// tile of 128 x 128 per CTA moves 2.5 GB from L2 for 512 x 1024 x 151,936 (4.1 ms of it per PFLOP; 10 TB/s
+// measured: 250 us); a pair's 256 x 256 moves 1.25 GB. At 64 rows it is HBM, the weights' one read.
+// Items are dealt out round by round over the pairs; what the last round would leave to a few pairs is cut
+// into 32-row items for all of them.
 // Every CTA fetches its own tiles (plain TMA loads), and every tensor map covers this GPU's own memory.
 //
-// Every wait on an mbarrier is bounded: a wait that runs out sets an abort flag that the other roles
-// see in their own waits, the kernel reports LMH_ERR_TIMEOUT in its status word, frees its tensor
-// memory and returns.
+// Every wait on an mbarrier is bounded: a wait that runs out sets an abort flag that the CTA's other roles
+// see in their own waits (the other CTA's run out by themselves), the kernel reports LMH_ERR_TIMEOUT in its
+// status word, frees its tensor memory and returns.
 #pragma once
 
 #include <cuda.h>
@@ -30,42 +41,82 @@
 
 namespace gs {
 
-constexpr int LMH_BM = 128;              // batch rows per tile (UMMA M)
-constexpr int LMH_BN = 128;              // vocabulary columns per tile (UMMA N)
-constexpr int LMH_BK = 64;               // K per stage: 64 bf16 = one 128-byte swizzle row
-constexpr int LMH_STAGES = 5;
-constexpr int LMH_NT = 192;              // warp 0 producer, warp 1 issuer, warps 2-5 epilogue
-constexpr int LMH_STAGE_BYTES = (LMH_BM + LMH_BN) * LMH_BK * 2;     // 32 KB
-constexpr int LMH_ROWS_S = 4096;         // rows whose running maximum, NaN bits and candidate count a CTA keeps in shared memory
-constexpr int LMH_DYN_BYTES = LMH_STAGES * LMH_STAGE_BYTES + 1024 + LMH_ROWS_S * 12;  // ring (+ room to align it to 1024 bytes) + the per-row words
-constexpr int LMH_TMEM_COLS = 256;       // two accumulators of 128 f32 columns
+constexpr int LMH_TILE_V = 256;          // vocabulary rows of a tile (UMMA M over the pair); 128 per CTA
+constexpr int LMH_CTA_V = 128;
+constexpr int LMH_MAX_N = 256;           // batch rows of an item (UMMA N)
+constexpr int LMH_BK = 64;               // K of one TMA box: 64 bf16 = one 128-byte swizzle row
+constexpr int LMH_SUB = 2;               // boxes of either operand per stage
+constexpr int LMH_EPI = 8;               // epilogue warps: two for each quarter of the TMEM lanes
+constexpr int LMH_NT = 64 + 32 * LMH_EPI;   // warp 0 producer, warp 1 issuer, then the epilogue
+constexpr int LMH_MAX_STAGES = 12;
+constexpr int LMH_RING_BYTES = 208 * 1024;
+constexpr int LMH_W_BYTES = LMH_CTA_V * LMH_BK * 2;                 // a box of w: 16 KB
+constexpr int LMH_DYN_BYTES = LMH_RING_BYTES + 1024;                // + room to align the swizzled tiles to 1024 bytes
+constexpr int LMH_TMEM_COLS = 512;       // two accumulators of 256 f32 columns
 constexpr uint32_t LMH_WAIT_LIMIT = 4000000u;
-constexpr int LMH_CAND_CAP = 2048;       // candidates per row that the finish kernel takes (entries of 8 bytes)
-constexpr int LMH_SEG = 32;              // candidates per row and CTA: every CTA of the projection has its own segment of a row's list
 
 constexpr uint32_t LMH_ERR_TIMEOUT = 1u;
 
 // tcgen05 instruction descriptor (kind::f16): D = F32 (bits 4-5 = 1), A = B = BF16 (bits 7-9, 10-12 = 1),
 // both K-major (bits 15, 16 = 0), N / 8 at bits 17-22, M / 16 at bits 24-28.
-constexpr uint32_t LMH_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(LMH_BN >> 3) << 17) |
-                               (static_cast<uint32_t>(LMH_BM >> 4) << 24);
+__host__ __device__ constexpr uint32_t lmh_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(LMH_TILE_V >> 4) << 24);
+}
+
+constexpr int LMH_CAND_CAP = 2048;       // candidates per row (entries of 8 bytes)
+struct LmhRow {
+  int32_t cnt;             // candidates so far (those beyond LMH_CAND_CAP are not stored)
+  int32_t nan;             // 1: a NaN in the row; 2: at index 0
+};
 
 struct LmHeadArgs {
-  CUtensorMap map_x;       // x [B, K] bf16, box 64 x 128, 128-byte swizzle
-  CUtensorMap map_w;       // w [V, K] bf16, box 64 x 128, 128-byte swizzle
+  CUtensorMap map_x;       // x [B, K] bf16, box 64 x box_n, 128-byte swizzle
+  CUtensorMap map_w;       // w [V, K] bf16, box 64 x cta_v, 128-byte swizzle
   int32_t B, V, K;
-  int32_t tile0, tile_step, ntile;   // vocabulary tiles tile0 + i * tile_step, i < ntile
+  int32_t box_n;           // batch rows that one TMA load of x brings: half of the largest item
+  int32_t item_n;          // batch rows of a full item, a multiple of 32
+  int32_t stages;          // of the ring
+  int32_t cta_v;           // vocabulary rows of a tile that each CTA takes, at most LMH_CTA_V
+  int32_t tile0, tile_step, ntile;   // vocabulary tiles (of 2 cta_v rows) tile0 + i * tile_step, i < ntile
   float* out_logits;       // [B, ld_out] f32, or null
   int64_t ld_out;
-  int32_t out_col0;        // column of out_logits that vocabulary tile i starts at: i * LMH_BN when compact, else its own
-  int32_t compact;         // 1: tile i goes to columns [i * 128, ...) of out_logits (the sample of tiles)
+  int32_t compact;         // 1: tile i goes to columns [i * 2 cta_v, ...) of out_logits (the sample of tiles)
   // fused sampling (all null when unused)
   const float* thr;        // [B] candidate threshold per row (raw logit units)
-  uint2* cand;             // [B, gridDim.x, LMH_SEG] (logit bits, index); needs B <= LMH_ROWS_S
-  int32_t* cand_cnt;       // [B, gridDim.x], written by every CTA for every row
-  uint32_t* rowmax_key;    // [B] order key of the row maximum (atomicMax)
-  int32_t* row_nan;        // [B] a NaN was seen
-  uint32_t* status;        // [1] LMH_ERR_* bits
+  uint2* cand;             // [B][LMH_CAND_CAP] (logit bits, index)
+  LmhRow* rows;            // [B]
+  uint32_t* status;        // [1] LMH_ERR_* bits, in host memory
+  int32_t clear_status;    // 1: this launch clears it first
+  int32_t chained;         // 1: launched as a dependent of the kernel that fills thr
+};
+
+// Work items in the order in which pair p takes them: p, p + npairs, ...: first the whole rounds of full
+// items (all batch rows of `full` vocabulary tiles, item_n at a time), then the remaining tiles in items
+// of small_n batch rows, at most one round of them.
+struct LmhItem { int vt, b0, n; };
+struct LmhPlan {
+  int nb, full, nfull, nsmall, total, item_n, small_n, B;
+  __host__ __device__ LmhPlan(int B_, int ntile, int item_n_, int npairs) {
+    B = B_; item_n = item_n_;
+    nb = (B + item_n - 1) / item_n;
+    full = (ntile * nb / npairs) * npairs / nb;
+    nfull = full * nb;
+    const int rest = (ntile - full) * nb;
+    int s = 1;
+    while (rest > 0 && 2 * s * rest <= npairs && item_n / (2 * s) >= 32) s *= 2;
+    small_n = (item_n / s + 31) & ~31;
+    nsmall = (B + small_n - 1) / small_n;
+    total = nfull + (ntile - full) * nsmall;
+  }
+  __device__ __forceinline__ LmhItem at(int i) const {
+    LmhItem it;
+    const bool f = i < nfull;
+    const int q = f ? i : i - nfull, per = f ? nb : nsmall, n = f ? item_n : small_n;
+    it.vt = (f ? 0 : full) + q / per;
+    it.b0 = (q % per) * n;
+    it.n = min(n, ((B - it.b0) + 31) & ~31);
+    return it;
+  }
 };
 
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -83,7 +134,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     if (done) return true;
@@ -92,9 +143,19 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-               :: "r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
+// The address of this CTA's shared variable in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" :: "r"(cluster_addr) : "memory");
+}
+// A tile into this CTA's shared memory; its bytes complete on a barrier that may be the pair's other CTA's.
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, unsigned long long pol) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+               :: "r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "l"(pol) : "memory");
 }
 // Shared-memory matrix descriptor of a K-major tile of 128-byte rows with the 128-byte swizzle: start
 // address / 16, leading byte offset 1 (unused for swizzled K-major), stride byte offset 1024 / 16 (eight
@@ -102,15 +163,17 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
 __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr_bytes) {
   return static_cast<uint64_t>((smem_addr_bytes & 0x3ffffu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      :: "r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" :: "r"(bar) : "memory");
+// Arrives on the barrier at this offset in both CTAs of the pair when the MMAs issued so far are done.
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               :: "r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -124,206 +187,219 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr) : "memory");
 }
 
-__global__ void __launch_bounds__(LMH_NT, 1) lm_head_kernel(const __grid_constant__ LmHeadArgs A) {
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(LMH_NT, 1) lm_head_kernel(const __grid_constant__ LmHeadArgs A) {
   extern __shared__ __align__(16) unsigned char lmh_dyn[];
-  __shared__ __align__(8) unsigned long long full_bar[LMH_STAGES], empty_bar[LMH_STAGES], acc_full[2], acc_empty[2];
+  __shared__ __align__(8) unsigned long long full_bar[LMH_MAX_STAGES], empty_bar[LMH_MAX_STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
+  __shared__ __align__(16) float stash_thr[LMH_EPI][32];
+  __shared__ uint2 stash[LMH_EPI][64];
+  __shared__ int stash_row[LMH_EPI][64];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = blockIdx.x & 1u;                                // in the pair; 0 leads
+  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
   const uint32_t ring = (smem_addr(lmh_dyn) + 1023u) & ~1023u;          // the swizzled tiles need 1024-byte alignment
-  // per-row running maximum and NaN bits of this CTA's tiles (a row always belongs to the same epilogue
-  // thread, so no atomics here); flushed to global memory once at the end
-  float* rowmax_s = reinterpret_cast<float*>(lmh_dyn + LMH_STAGES * LMH_STAGE_BYTES + 1024);
-  int* rownan_s = reinterpret_cast<int*>(rowmax_s + LMH_ROWS_S);
-  int* rowcnt_s = rownan_s + LMH_ROWS_S;
-  const bool rows_in_smem = A.rowmax_key != nullptr && A.B <= LMH_ROWS_S;
-  if (rows_in_smem) for (int r = tid; r < A.B; r += LMH_NT) { rowmax_s[r] = -INFINITY; rownan_s[r] = 0; rowcnt_s[r] = 0; }
   volatile int* abort_flag = &abort_s;
-  const int nkc = A.K / LMH_BK;                                        // K chunks per tile
-  const int nbt = (A.B + LMH_BM - 1) / LMH_BM;                         // batch tiles
-  // this CTA's work items: (vocabulary tile, batch tile) pairs, vocabulary-major
-  const int my_first = blockIdx.x, my_step = gridDim.x;
+  const int nk64 = A.K / LMH_BK, nkc = (nk64 + LMH_SUB - 1) / LMH_SUB;  // K boxes and chunks per item
+  const int nst = A.stages;
+  const uint32_t x_bytes = static_cast<uint32_t>(A.box_n) * LMH_BK * 2, stage_bytes = LMH_SUB * (LMH_W_BYTES + x_bytes);
+  const LmhPlan plan(A.B, A.ntile, A.item_n, npairs);
+  pdl_launch();
 
   if (tid == 0) {
-    for (int s = 0; s < LMH_STAGES; s++) { mbar_init(smem_addr(&full_bar[s]), 1); mbar_init(smem_addr(&empty_bar[s]), 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(smem_addr(&acc_full[b]), 1); mbar_init(smem_addr(&acc_empty[b]), 4); }
+    for (int s = 0; s < nst; s++) { mbar_init(smem_addr(&full_bar[s]), 1); mbar_init(smem_addr(&empty_bar[s]), 1); }
+    for (int b = 0; b < 2; b++) { mbar_init(smem_addr(&acc_full[b]), 1); mbar_init(smem_addr(&acc_empty[b]), 2 * LMH_EPI); }
     abort_s = 0;
+    if (A.clear_status && blockIdx.x == 0) *A.status = 0u;              // (a wait runs out seconds later, if ever)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {                                                      // the issuer's warp owns the tensor memory
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_addr(&tmem_base_s)), "r"(LMH_TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  if (warp == 1) {                                                      // one warp of each CTA takes the tensor memory
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_addr(&tmem_base_s)), "r"(LMH_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");   // both CTAs' barriers exist
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = tmem_base_s;
 
   if (warp == 0) {
-    // ---- producer
+    // ---- producer: this CTA's share of every stage; its bytes complete on the leader's barrier
     if (lane == 0) {
+      unsigned long long pol_w, pol_x;                                  // the weights pass once per batch tile, x stays
+      asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_w));
+      asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_x));
+      if (plan.nb > 1) asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol_w));
       uint32_t stage = 0, phase = 0;
       bool ok = true;
-      for (int t = my_first; t < A.ntile && ok; t += my_step) {
-        const int vt = A.tile0 + t * A.tile_step;
-        for (int bt = 0; bt < nbt && ok; bt++) {
-          for (int kc = 0; kc < nkc; kc++) {
-            if (!mbar_wait(smem_addr(&empty_bar[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
-            const uint32_t bar = smem_addr(&full_bar[stage]);
-            const uint32_t sa = ring + stage * LMH_STAGE_BYTES, sb = sa + LMH_BM * LMH_BK * 2;
-            mbar_expect_tx(bar, LMH_STAGE_BYTES);
-            tma_load_2d(sa, &A.map_x, bar, kc * LMH_BK, bt * LMH_BM);
-            tma_load_2d(sb, &A.map_w, bar, kc * LMH_BK, vt * LMH_BN);
-            if (++stage == LMH_STAGES) { stage = 0; phase ^= 1u; }
-          }
+      for (int i = pair; i < plan.total && ok; i += npairs) {
+        const LmhItem it = plan.at(i);
+        const int v0 = ((A.tile0 + it.vt * A.tile_step) * 2 + static_cast<int>(rank)) * A.cta_v;
+        const int xb = it.b0 + static_cast<int>(rank) * (it.n >> 1);
+        for (int kc = 0; kc < nkc; kc++) {
+          if (!mbar_wait(smem_addr(&empty_bar[stage]), phase ^ 1u, abort_flag)) { ok = false; break; }
+          const uint32_t own = smem_addr(&full_bar[stage]), bar = map_rank(own, 0);
+          const uint32_t sw = ring + stage * stage_bytes, sx = sw + LMH_SUB * LMH_W_BYTES;
+          const int subs = min(LMH_SUB, nk64 - kc * LMH_SUB);
+          if (rank == 0) mbar_expect_tx(own, 2 * subs * (static_cast<uint32_t>(A.cta_v) * LMH_BK * 2 + x_bytes));
+          for (int u = 0; u < subs; u++) tma_load_2d_pair(sw + u * LMH_W_BYTES, &A.map_w, bar, (kc * LMH_SUB + u) * LMH_BK, v0, pol_w);
+          for (int u = 0; u < subs; u++) tma_load_2d_pair(sx + u * x_bytes, &A.map_x, bar, (kc * LMH_SUB + u) * LMH_BK, xb, pol_x);
+          if (++stage == static_cast<uint32_t>(nst)) { stage = 0; phase ^= 1u; }
         }
       }
     }
   } else if (warp == 1) {
     // ---- issuer
-    if (lane == 0) {
+    if (rank == 0 && lane == 0) {
       uint32_t stage = 0, phase = 0, acc = 0, acc_phase = 0;
       bool ok = true;
-      for (int t = my_first; t < A.ntile && ok; t += my_step) {
-        for (int bt = 0; bt < nbt && ok; bt++) {
-          if (!mbar_wait(smem_addr(&acc_empty[acc]), acc_phase ^ 1u, abort_flag)) { ok = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t d_tmem = tmem_base + acc * LMH_BN;
-          for (int kc = 0; kc < nkc; kc++) {
-            if (!mbar_wait(smem_addr(&full_bar[stage]), phase, abort_flag)) { ok = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t sa = ring + stage * LMH_STAGE_BYTES, sb = sa + LMH_BM * LMH_BK * 2;
-#pragma unroll
-            for (int k = 0; k < LMH_BK / 16; k++) {
-              umma_f16(d_tmem, umma_desc(sa + k * 32), umma_desc(sb + k * 32), LMH_IDESC, (kc > 0 || k > 0) ? 1u : 0u);
-            }
-            umma_commit(smem_addr(&empty_bar[stage]));                  // the stage is free once these MMAs have read it
-            if (++stage == LMH_STAGES) { stage = 0; phase ^= 1u; }
-          }
-          if (ok) umma_commit(smem_addr(&acc_full[acc]));               // the accumulator is complete
-          if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
-        }
-      }
-    }
-  } else {
-    // ---- epilogue: warp w reads TMEM lanes 32 * (w % 4) .. + 31; thread = batch row
-    const int q = warp & 3;
-    uint32_t acc = 0, acc_phase = 0;
-    bool ok = true;
-    for (int t = my_first; t < A.ntile && ok; t += my_step) {
-      const int vt = A.tile0 + t * A.tile_step;
-      const int v0 = vt * LMH_BN;
-      const int oc0 = A.compact ? t * LMH_BN : v0;
-      for (int bt = 0; bt < nbt && ok; bt++) {
-        if (!mbar_wait(smem_addr(&acc_full[acc]), acc_phase, abort_flag)) { ok = false; break; }
+      for (int i = pair; i < plan.total && ok; i += npairs) {
+        const uint32_t idesc = lmh_idesc(plan.at(i).n);
+        if (!mbar_wait(smem_addr(&acc_empty[acc]), acc_phase ^ 1u, abort_flag)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int row = bt * LMH_BM + q * 32 + lane;
-        const bool live = row < A.B;
-        const float thr = (A.thr && live) ? A.thr[row] : INFINITY;
-        float vmax = -INFINITY;
-        int nan_bits = 0;                                             // 1: a NaN in the row; 2: at index 0
-#pragma unroll 1
-        for (int c = 0; c < LMH_BN; c += 32) {
-          uint32_t r[32];
-          tmem_ld32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * LMH_BN + c, r);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (live) {
-            const int nvalid = min(32, A.V - (v0 + c));                 // columns past the vocabulary hold zeros
-            if (A.out_logits) {
-              float* dst = A.out_logits + static_cast<int64_t>(row) * A.ld_out + oc0 + c;
-              if (nvalid == 32 && ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0)) {
+        const uint32_t d_tmem = tmem_base + acc * LMH_MAX_N;
+        for (int kc = 0; kc < nkc; kc++) {
+          if (!mbar_wait(smem_addr(&full_bar[stage]), phase, abort_flag)) { ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t sw = ring + stage * stage_bytes, sx = sw + LMH_SUB * LMH_W_BYTES;
+          const int subs = min(LMH_SUB, nk64 - kc * LMH_SUB);
+          for (int u = 0; u < subs; u++) {
 #pragma unroll
-                for (int j = 0; j < 32; j += 4) *reinterpret_cast<uint4*>(dst + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 32; j++) if (j < nvalid) dst[j] = __uint_as_float(r[j]);
-              }
-            }
-            if (A.rowmax_key) {
-              // the chunk's maximum first (NaN-propagating): only a chunk that holds a candidate, a NaN
-              // or columns past the vocabulary is looked at logit by logit
-              float cm = max3nan(__uint_as_float(r[0]), __uint_as_float(r[1]), __uint_as_float(r[2]));
-#pragma unroll
-              for (int j = 3; j + 1 < 32; j += 2) cm = max3nan(cm, __uint_as_float(r[j]), __uint_as_float(r[j + 1]));
-              cm = maxnan(cm, __uint_as_float(r[31]));
-              if (nvalid == 32 && cm < thr) {                          // (false for a NaN maximum)
-                vmax = fmaxf(vmax, cm);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 32; j++) {
-                  const float x = __uint_as_float(r[j]);
-                  if (j >= nvalid) continue;
-                  if (x != x) nan_bits |= (v0 + c + j == 0) ? 3 : 1;
-                  vmax = fmaxf(vmax, x);
-                  if (x >= thr && rows_in_smem) {
-                    // this CTA's own segment of the row's list, and a count that only this thread
-                    // touches: nothing to wait for (an atomic on a count shared by all CTAs made
-                    // every warp wait in nearly every chunk, a quarter more time for the kernel)
-                    const int slot = rowcnt_s[row]++;
-                    if (slot < LMH_SEG) A.cand[(static_cast<int64_t>(row) * gridDim.x + blockIdx.x) * LMH_SEG + slot] = make_uint2(r[j], static_cast<uint32_t>(v0 + c + j));
-                  }
-                }
-              }
-            }
+            for (int k = 0; k < LMH_BK / 16; k++)
+              umma_f16_pair(d_tmem, umma_desc(sw + u * LMH_W_BYTES + k * 32), umma_desc(sx + u * x_bytes + k * 32), idesc, (kc > 0 || u > 0 || k > 0) ? 1u : 0u);
           }
+          umma_commit_pair(smem_addr(&empty_bar[stage]));               // the stage is free once these MMAs have read it
+          if (++stage == static_cast<uint32_t>(nst)) { stage = 0; phase ^= 1u; }
         }
-        // the accumulator is free again: one arrival per epilogue warp
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_addr(&acc_empty[acc]));
-        if (A.rowmax_key && live) {
-          if (rows_in_smem) {
-            rowmax_s[row] = fmaxf(rowmax_s[row], vmax);
-            rownan_s[row] |= nan_bits;
-          } else {
-            atomicMax(&A.rowmax_key[row], okey(vmax));
-            if (nan_bits) atomicOr(&A.row_nan[row], nan_bits);
-          }
-        }
+        if (ok) umma_commit_pair(smem_addr(&acc_full[acc]));            // the accumulator is complete
         if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
       }
     }
+  } else {
+    // ---- epilogue: warp w reads TMEM lanes 32 * (w % 4) .. + 31; thread = vocabulary row
+    const int q = warp & 3, half = (warp - 2) >> 2;                     // this warp's lanes, and its share of the columns
+    uint32_t acc = 0, acc_phase = 0;
+    bool ok = true;
+    int nstash = 0;
+    auto flush = [&](int count) {                                       // the stash's first `count` entries to their rows' lists
+      __syncwarp();
+      if (lane < count) {
+        const uint2 e = stash[warp - 2][lane];
+        const int b = stash_row[warp - 2][lane];
+        const float x = __uint_as_float(e.x);
+        if (x != x) {
+          atomicOr(&A.rows[b].nan, (e.y == 0u) ? 3 : 1);
+        } else {
+          const int slot = atomicAdd(&A.rows[b].cnt, 1);
+          if (slot < LMH_CAND_CAP) A.cand[static_cast<int64_t>(b) * LMH_CAND_CAP + slot] = e;
+        }
+      }
+      __syncwarp();
+    };
+    if (A.chained) pdl_wait();                                          // the thresholds; tiles and MMAs are under way meanwhile
+    for (int i = pair; i < plan.total && ok; i += npairs) {
+      const LmhItem it = plan.at(i);
+      if (!mbar_wait(smem_addr(&acc_full[acc]), acc_phase, abort_flag)) { ok = false; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int in_tile = static_cast<int>(rank) * A.cta_v + q * 32 + lane;
+      const int v = (A.tile0 + it.vt * A.tile_step) * 2 * A.cta_v + in_tile;
+      const bool live = q * 32 + lane < A.cta_v && v < A.V;
+      const int ocol = A.compact ? it.vt * 2 * A.cta_v + in_tile : v;
+#pragma unroll 1
+      for (int c = half * 32; c < it.n; c += 64) {
+        uint32_t r[32];
+        tmem_ld32(tmem_base + (static_cast<uint32_t>(q * 32) << 16) + acc * LMH_MAX_N + c, r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        const int b0 = it.b0 + c, nb = min(32, A.B - b0);              // batch rows of these columns (uniform)
+        if (A.out_logits && live) {
+          float* dst = A.out_logits + static_cast<int64_t>(b0) * A.ld_out + ocol;
+          if (nb == 32) {
+#pragma unroll
+            for (int j = 0; j < 32; j++) __stcs(dst + j * A.ld_out, __uint_as_float(r[j]));
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; j++) if (j < nb) __stcs(dst + j * A.ld_out, __uint_as_float(r[j]));
+          }
+        }
+        if (A.thr) {
+          // a batch row's threshold is the same for all lanes, and few lanes hold a logit that reaches it: those go to
+          // the warp's stash, and from there, 32 at a time, to their rows' lists (an atomic on a row's count per
+          // logit where it is found made every warp wait in nearly every chunk)
+          stash_thr[warp - 2][lane] = (lane < nb) ? A.thr[b0 + lane] : INFINITY;
+          __syncwarp();
+          const float4* t4 = reinterpret_cast<const float4*>(stash_thr[warp - 2]);
+          uint32_t m = 0u;                                             // columns of this lane that reach their threshold
+#pragma unroll
+          for (int j = 0; j < 32; j++) {
+            const float4 t = t4[j >> 2];
+            const float tj = (j & 3) == 0 ? t.x : (j & 3) == 1 ? t.y : (j & 3) == 2 ? t.z : t.w;
+            m |= !(__uint_as_float(r[j]) < tj) ? (1u << j) : 0u;       // (true for a NaN)
+          }
+          if (!live) m = 0u;
+          for (uint32_t votes; (votes = __ballot_sync(FULL, m != 0u)) != 0u;) {   // one hit of every lane that has any
+            if (m) {
+              const int j = __ffs(m) - 1;
+              m &= m - 1;
+              uint32_t x = r[0];
+#pragma unroll
+              for (int jj = 1; jj < 32; jj++) x = (j == jj) ? r[jj] : x;
+              const int at = nstash + __popc(votes & ((1u << lane) - 1u));
+              stash[warp - 2][at] = make_uint2(x, static_cast<uint32_t>(v));
+              stash_row[warp - 2][at] = b0 + j;
+            }
+            nstash += __popc(votes);
+            if (nstash >= 32) {                                        // uniform
+              flush(32);
+              nstash -= 32;
+              const uint2 e = stash[warp - 2][32 + lane];
+              const int er = stash_row[warp - 2][32 + lane];
+              __syncwarp();
+              if (lane < nstash) { stash[warp - 2][lane] = e; stash_row[warp - 2][lane] = er; }
+            }
+          }
+          __syncwarp();
+        }
+      }
+      // the accumulator is free again: one arrival per epilogue warp of either CTA at the leader's barrier
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(map_rank(smem_addr(&acc_empty[acc]), 0));
+      if (++acc == 2) { acc = 0; acc_phase ^= 1u; }
+    }
+    if (nstash > 0) flush(nstash);
   }
   // ---- teardown
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (rows_in_smem) {
-    for (int r = tid; r < A.B; r += LMH_NT) {
-      const float v = rowmax_s[r];
-      if (v > -INFINITY) atomicMax(&A.rowmax_key[r], okey(v));
-      if (rownan_s[r]) atomicOr(&A.row_nan[r], rownan_s[r]);
-      if (A.cand_cnt) A.cand_cnt[static_cast<int64_t>(r) * gridDim.x + blockIdx.x] = rowcnt_s[r];
-    }
-  }
   if (abort_s) {
     // a wait ran out: give the copies and MMAs still in flight time to land before the shared and
     // tensor memory they target is given back (bounded: about a millisecond)
     for (int it = 0; it < 1000; it++) __nanosleep(1000);
-    if (tid == 0 && A.status) atomicOr(A.status, LMH_ERR_TIMEOUT);
-    __syncthreads();
+    if (tid == 0) atomicOr_system(A.status, LMH_ERR_TIMEOUT);
   }
+  // neither CTA leaves while the other may still arrive on its barriers or read its tiles
+  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(LMH_TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(LMH_TMEM_COLS) : "memory");
   }
 }
 
 
 // ---- fused sampling on top of the projection (greedy and top-k rows) --------------------------------
 //
-//   1. the projection over a sample of vocabulary tiles (1/32 of them, 8 to 32 tiles spread over the
-//      vocabulary) gives each row 1024 to 4096 of its logits;
+//   1. the projection over a sample of vocabulary tiles (1/32 of the vocabulary, spread over it)
+//      gives each row 1024 to 4096 of its logits;
 //   2. lmh_threshold_kernel: the r-th largest of that sample, r chosen so that eight times top_k
 //      logits of the whole row (at least 256, at most a third of the list) are expected above it: an
 //      estimate, not a bound;
 //   3. the projection over all tiles: the epilogue appends every logit at or above the row's
-//      threshold to this CTA's segment of the row's candidate list (no [B, V] logits are written);
+//      threshold to the row's candidate list (no [B, V] logits are written);
 //   4. lmh_finish_kernel: the exact top_k-th largest of the candidates with ties kept
 //      (model/generate.go:157-164), then softmax / top-p / draw on the kept set exactly as the
 //      one-GPU narrow kernel does. A row whose estimate failed (fewer than top_k candidates, or more
-//      than a segment or the list holds) or whose config the fused path does not serve is counted in nfail; the
+//      than the list holds) or whose config the fused path does not serve is counted in nfail; the
 //      host then recomputes the batch through the unfused path.
-constexpr int LMH_SAMPLE_TILES_MIN = 8, LMH_SAMPLE_TILES_MAX = 32;   // the sample: 1/32 of the tiles, within these bounds
+constexpr int LMH_SAMPLE_MIN = 1024, LMH_SAMPLE_MAX = 4096;   // logits of a row's sample
 constexpr int LMH_F_NT = 256;
 constexpr int LMH_F_DYN_BYTES = LMH_CAND_CAP * 8 + 16384 + KEEP_MAX * 8;
 
@@ -333,12 +409,9 @@ struct LmhSampleArgs {
   int32_t nsample;
   int32_t fuse_top_k;       // rows with 0 < top_k <= fuse_top_k (or temperature 0) are served
   float* thr;               // [B]
-  const uint2* cand;        // [B, nseg, LMH_SEG]
-  const int32_t* cand_cnt;  // [B, nseg]
-  int32_t nseg;             // CTAs of the projection that filled the lists
-  const uint32_t* rowmax_key;
-  const int32_t* row_nan;
-  int32_t* nfail;           // [1]
+  const uint2* cand;        // [B, LMH_CAND_CAP]
+  LmhRow* rows;             // [B]
+  int32_t* nfail;           // [1], in host memory
   int64_t B;
 };
 
@@ -350,30 +423,42 @@ __device__ __forceinline__ bool lmh_row_served(const RowCfg& c, int V, int fuse_
   return topk > 0 && topk <= fuse_top_k;
 }
 
-__global__ void __launch_bounds__(LMH_F_NT) lmh_threshold_kernel(LmhSampleArgs M) {
-  __shared__ uint2 list[LMH_SAMPLE_TILES_MAX * LMH_BN];
-  __shared__ uint32_t s_sel[256];
-  __shared__ int s_bc[4];
+__global__ void __launch_bounds__(LMH_F_NT) lmh_threshold_kernel(const __grid_constant__ LmhSampleArgs M) {
+  constexpr int PER = LMH_SAMPLE_MAX / LMH_F_NT;              // sample logits per thread
+  __shared__ bu::Scratch sc;
+  __shared__ uint32_t cnts[1024];
+  __shared__ int bc[4];
   const int tid = threadIdx.x;
-  for (int64_t row = blockIdx.x; row < M.B; row += gridDim.x) {
-    __syncthreads();
-    const RowCfg cfg = M.k.cfgs[row];
-    if (!lmh_row_served(cfg, M.k.V, M.fuse_top_k)) { if (tid == 0) M.thr[row] = INFINITY; continue; }
+  pdl_launch();
+  const int64_t row = blockIdx.x;
+  const RowCfg cfg = M.k.cfgs[row];
+  const bool served = lmh_row_served(cfg, M.k.V, M.fuse_top_k);
+  pdl_wait();                                                 // the sample's logits
+  float thr = served ? -INFINITY : INFINITY;                  // -Inf: a sample too small to say, everything is a candidate
+  if (served) {
     const int keff = (cfg.temperature == 0.0f || !(cfg.temperature > 0.0f) || !(cfg.temperature < INFINITY)) ? 1 : cfg.top_k;
     const int n = M.nsample;
-    for (int j = tid; j < n; j += LMH_F_NT) list[j] = make_uint2(__float_as_uint(M.sample[row * n + j]), static_cast<uint32_t>(j));
+    uint32_t key[PER], tmin = 0xffffffffu, tmax = 0u;
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+      const int i = j * LMH_F_NT + tid;
+      key[j] = (i < n) ? okey(M.sample[row * n + i]) : 0u;    // (0, a NaN's key, is below every other)
+      tmin = min(tmin, key[j]);
+      tmax = max(tmax, key[j]);
+    }
     // expected logits of the whole row above the threshold: eight times top_k, at least 256, at most a
     // third of the list; the r-th largest of the sample stands for the (r V / n)-th largest of the row
     const long long want = min(max(8ll * keff, 256ll), static_cast<long long>(LMH_CAND_CAP / 3));
     const int r = max(2, static_cast<int>((want * n + M.k.V / 2) / M.k.V));
-    float thr = -INFINITY;                                    // a sample too small to say: everything is a candidate
     if (r < n) {
-      const uint32_t key = bu::select_kth<LMH_F_NT>(list, n, r, s_sel, s_bc, tid);
-      thr = okey_to_float(key);
-      if (!(thr == thr)) thr = -INFINITY;                     // NaNs order lowest: a NaN threshold would collect nothing
+      const uint32_t lo = sample_threshold<LMH_F_NT, 1024>([&](auto&& g) {
+#pragma unroll
+        for (int j = 0; j < PER; j++) g(key[j]);
+      }, r, tmin, tmax, cnts, bc, sc, tid);
+      if (lo > 0x007fffffu) thr = okey_to_float(lo);          // NaNs order lowest: a NaN threshold would collect nothing
     }
-    if (tid == 0) M.thr[row] = thr;
   }
+  if (tid == 0) { M.thr[row] = thr; M.rows[row].cnt = 0; M.rows[row].nan = 0; }
 }
 
 __global__ void __launch_bounds__(LMH_F_NT, 4) lmh_finish_kernel(const __grid_constant__ LmhSampleArgs M) {
@@ -388,6 +473,7 @@ __global__ void __launch_bounds__(LMH_F_NT, 4) lmh_finish_kernel(const __grid_co
   const KernelArgs& A = M.k;
   const int tid = threadIdx.x;
   constexpr int NW = LMH_F_NT / 32;
+  pdl_wait();                                                 // the candidates
   for (int64_t row = blockIdx.x; row < M.B; row += gridDim.x) {
     __syncthreads();
     const RowCfg cfg = A.cfgs[row];
@@ -398,28 +484,19 @@ __global__ void __launch_bounds__(LMH_F_NT, 4) lmh_finish_kernel(const __grid_co
         if (A.out_flags) A.out_flags[row] = fl;
       }
     };
-    auto give_up = [&]() { if (tid == 0) atomicAdd(M.nfail, 1); write_row(-1, FLAG_INTERNAL); };
+    auto give_up = [&]() { if (tid == 0) atomicAdd_system(M.nfail, 1); write_row(-1, FLAG_INTERNAL); };
     if (!lmh_row_served(cfg, A.V, M.fuse_top_k)) { give_up(); continue; }
     if (Tm != 0.0f && (!(Tm > 0.0f) || !(Tm < INFINITY))) { write_row(-1, FLAG_BAD_CFG); continue; }
-    // the row's candidates: one segment per CTA of the projection
-    if (tid == 0) s_cnt = 0;
-    __syncthreads();
-    int over = 0;
-    for (int c = tid; c < M.nseg; c += LMH_F_NT) {
-      const int n = M.cand_cnt[row * M.nseg + c];
-      if (n > LMH_SEG) over = 1;
-      const int take = min(n, LMH_SEG);
-      const int base = atomicAdd(&s_cnt, take);
-      if (base + take <= LMH_CAND_CAP) {
-        const uint2* seg = M.cand + (row * M.nseg + c) * LMH_SEG;
-        for (int j = 0; j < take; j++) list[base + j] = seg[j];
-      }
+    const int cnt = M.rows[row].cnt, nanb = M.rows[row].nan;
+    uint32_t kmax = 0x007fffffu;                                // -Inf
+    for (int j = tid; j < min(cnt, LMH_CAND_CAP); j += LMH_F_NT) {
+      const uint2 e = M.cand[row * LMH_CAND_CAP + j];
+      list[j] = e;
+      kmax = max(kmax, okey(__uint_as_float(e.x)));
     }
-    over = __syncthreads_or(over);
-    const int cnt = s_cnt;
-    const int nanb = M.row_nan[row];
+    kmax = static_cast<uint32_t>(bu::max_u64<NW>(kmax, sc, tid));   // (its barriers publish the list)
     const int keff = (Tm == 0.0f) ? 1 : cfg.top_k;
-    if (over || cnt > LMH_CAND_CAP || (cnt < keff && !(nanb & 1))) { give_up(); continue; }   // the estimate failed for this row
+    if (cnt > LMH_CAND_CAP || (cnt < keff && !(nanb & 1))) { give_up(); continue; }   // the estimate failed for this row
     // ---- greedy (generate.go:134-144): largest logit, lowest index; a NaN at index 0 is never beaten
     if (Tm == 0.0f) {
       unsigned long long best = 0ull;
@@ -434,13 +511,12 @@ __global__ void __launch_bounds__(LMH_F_NT, 4) lmh_finish_kernel(const __grid_co
       write_row(id, 0u);
       continue;
     }
-    const float xmax = okey_to_float(M.rowmax_key[row]);
-    const float m = scale_t(xmax, Tm);
+    const float m = scale_t(okey_to_float(kmax), Tm);
     // A NaN anywhere, or an infinite maximum: the walk of generate.go:231-239 falls through
     if ((nanb & 1) || !(fabsf(m) < INFINITY)) { write_row(A.V - 1, FLAG_NONFINITE | FLAG_FALLBACK); continue; }
     // ---- top_k-th largest with ties (generate.go:157-164), then the kept set
     const int topk = cfg.top_k;
-    const int nk = narrow_list<LMH_F_NT>(list, cnt, topk, Tm, 0u, M.rowmax_key[row], kept, s_sel, s_bc, &s_cnt, tid);
+    const int nk = narrow_list<LMH_F_NT>(list, cnt, topk, Tm, 0u, kmax, kept, s_sel, s_bc, &s_cnt, tid);
     if (nk > KEEP_MAX || cnt <= topk) { give_up(); continue; }
     const bool topp_on = (cfg.top_p > 0.0f && cfg.top_p < 1.0f);
     const int mode = cfg.topp_mode;

@@ -72,7 +72,8 @@ struct Ctx {
   double* eb_table = nullptr;
   Scratch worklist;        // int32[1 + rows]: rows the cluster kernel leaves to the single-CTA kernel
   Scratch st_logits, st_cfgs, st_uniforms, st_ids, st_flags;
-  Scratch lmh_scratch;       // status word, thresholds, candidate lists, sample logits of the LM-head path
+  Scratch lmh_scratch;       // thresholds, candidate lists, sample logits of the LM-head path
+  uint32_t* host_words = nullptr;   // pinned, written by kernels: [0] LM-head status, [1] rows its fused form handed back
   Scratch lmh_logits;        // [B, V] f32 when rows need the unfused samplers
   Scratch vs_local, vs_all;  // records of the vocab-sharded call: this rank's, and every rank's after the all-gather
   Scratch vs_req;            // [B][3] doubles: what the owner's draw of a row without top-k needs
@@ -455,6 +456,23 @@ int host_run(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int64_
   return GORCH_CUDA_OK;
 }
 
+// A launch on the context's stream; dependent: it may start while the kernel before it runs, and waits for
+// that itself (griddepcontrol.wait) where it needs what it wrote.
+template <typename... P, typename... A>
+cudaError_t launch(Ctx* c, void (*kernel)(P...), unsigned grid, unsigned block, size_t dyn, bool dependent, const A&... args) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(grid);
+  lc.blockDim = dim3(block);
+  lc.dynamicSmemBytes = dyn;
+  lc.stream = c->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&lc, kernel, args...);
+}
+
 // ---- LM-head projection (lm_head.cuh) ----
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -474,12 +492,12 @@ int load_encode_tiled(char** errOut) {
   return GORCH_CUDA_OK;
 }
 
-// Tensor map of a row-major [rows, K] bf16 matrix: boxes of 64 columns x 128 rows, 128-byte swizzle,
+// Tensor map of a row-major [rows, K] bf16 matrix: boxes of 64 columns x box_rows rows, 128-byte swizzle,
 // zero fill outside the matrix.
-int make_bf16_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t ld, char** errOut) {
+int make_bf16_map(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t ld, int box_rows, char** errOut) {
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(gs::LMH_BK), static_cast<cuuint32_t>(gs::LMH_BM)};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(gs::LMH_BK), static_cast<cuuint32_t>(box_rows)};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = g_encode_tiled(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
@@ -508,16 +526,46 @@ int check_lm_head(Ctx* c, const void* x, const void* w, int64_t B, int64_t V, in
   return GORCH_CUDA_OK;
 }
 
+// Shapes of a projection: batch rows of a full item, vocabulary rows per CTA, the ring's stages, the tensor maps.
+int lm_head_args(const Ctx* c, gs::LmHeadArgs& a, const void* x, int64_t ldx, const void* w, int64_t ldw, int64_t B, int64_t V, int64_t K,
+                 bool writes_logits, char** errOut) {
+  memset(&a, 0, sizeof a);
+  a.B = static_cast<int32_t>(B); a.V = static_cast<int32_t>(V); a.K = static_cast<int32_t>(K);
+  a.item_n = B >= gs::LMH_MAX_N ? gs::LMH_MAX_N : static_cast<int32_t>((B + 31) & ~31ll);
+  a.box_n = a.item_n / 2;
+  // Up to 128 batch rows the weights' read decides: tiles as high as make the rounds over all SMs come out even
+  // (151,936 rows on 148 SMs: nine rounds of 115 rows instead of eight of 128 and one for two pairs). Beyond,
+  // the tensor pipe does, and a tile with fewer rows costs it as much as a full one.
+  a.cta_v = gs::LMH_CTA_V;
+  if (B <= 128) {
+    const int64_t sms = c->sm_count & ~1, rounds = (V + sms * gs::LMH_CTA_V - 1) / (sms * gs::LMH_CTA_V);
+    a.cta_v = static_cast<int32_t>((V + sms * rounds - 1) / (sms * rounds));
+    // whole 32-byte sectors of the output, where that is worth a few rows of padding (32 batch rows: 59.2 us with 115
+    // vocabulary rows per CTA, 60.4 with 120; 128 batch rows: 83 and 79)
+    if (writes_logits && B > 32) a.cta_v = (a.cta_v + 7) & ~7;
+  }
+  const int stage = gs::LMH_SUB * (gs::LMH_W_BYTES + a.box_n * gs::LMH_BK * 2);
+  a.stages = gs::LMH_RING_BYTES / stage;
+  if (a.stages > gs::LMH_MAX_STAGES) a.stages = gs::LMH_MAX_STAGES;
+  int rc = make_bf16_map(&a.map_x, x, B, K, ldx, a.box_n, errOut);
+  if (rc) return rc;
+  return make_bf16_map(&a.map_w, w, V, K, ldw, a.cta_v, errOut);
+}
+
 // One launch of lm_head_kernel over the vocabulary tiles tile0 + i * step, i < ntile.
-int launch_lm_head(Ctx* c, gs::LmHeadArgs& a, char** errOut) {
-  const int64_t ntile_total = (static_cast<int64_t>(a.V) + gs::LMH_BN - 1) / gs::LMH_BN;
+int launch_lm_head(Ctx* c, gs::LmHeadArgs& a, char** errOut, bool dependent = false) {
+  const int64_t ntile_total = (static_cast<int64_t>(a.V) + 2 * a.cta_v - 1) / (2 * a.cta_v);
   if (a.ntile < 1 || a.tile0 + static_cast<int64_t>(a.ntile - 1) * a.tile_step >= ntile_total) {
     set_err(errOut, "gorch_cuda: LM head tile range outside the vocabulary");
     return GORCH_CUDA_ERR_BAD_ARG;
   }
-  const unsigned grid = static_cast<unsigned>(a.ntile < c->sm_count ? a.ntile : c->sm_count);
-  gs::lm_head_kernel<<<grid, gs::LMH_NT, gs::LMH_DYN_BYTES, c->stream>>>(a);
-  CUDA_TRY(cudaGetLastError(), errOut);
+  const int most = c->sm_count / 2;
+  int npairs = gs::LmhPlan(a.B, a.ntile, a.item_n, most).total;
+  if (npairs > most) npairs = most;
+  a.status = c->host_words;
+  a.chained = dependent ? 1 : 0;
+  a.clear_status = dependent ? 0 : 1;
+  CUDA_TRY(launch(c, gs::lm_head_kernel, static_cast<unsigned>(2 * npairs), gs::LMH_NT, gs::LMH_DYN_BYTES, dependent, a), errOut);
   c->counters.kernel_launches += 1;
   return GORCH_CUDA_OK;
 }
@@ -585,6 +633,8 @@ GorchCudaCtxRef gorch_cuda_create_ctx(int device, char** errOut) {
       return nullptr;
     }
   }
+  if ((e = cudaHostAlloc(reinterpret_cast<void**>(&c->host_words), 64, cudaHostAllocMapped | cudaHostAllocPortable)) != cudaSuccess) return fail("cudaHostAlloc", e);
+  memset(c->host_words, 0, 64);
   double tab[256];
   for (int j = 0; j < 256; j++) tab[j] = static_cast<double>(exp2l(static_cast<long double>(j) / 256.0L));
   if ((e = cudaMalloc(&c->exp_table, sizeof tab)) != cudaSuccess) return fail("cudaMalloc(exp table)", e);
@@ -630,6 +680,7 @@ void gorch_cuda_release(GorchCudaCtxRef ctx) {
   for (Scratch* s : {&c->st_logits, &c->st_cfgs, &c->st_uniforms, &c->st_ids, &c->st_flags}) {
     if (s->ptr) cudaFree(s->ptr);
   }
+  if (c->host_words) cudaFreeHost(c->host_words);
   if (c->exp_table) cudaFree(c->exp_table);
   if (c->eb_table) cudaFree(c->eb_table);
   if (c->worklist.ptr) cudaFree(c->worklist.ptr);
@@ -1100,7 +1151,9 @@ int gorch_cuda_topk_dev(GorchCudaCtxRef ctx, const void* x, int dtype, int64_t B
   if (B == 0) return GORCH_CUDA_OK;
   if (!x || !out_values || !out_indices) { set_err(errOut, "gorch_cuda: null pointer argument"); return GORCH_CUDA_ERR_BAD_ARG; }
   CUDA_TRY(cudaSetDevice(c->device), errOut);
-  if (k > gs::KFAST) {                                       // beyond the one-pass kernel's lists: select, gather, sort
+  // The narrow kernel (a row per CTA of 128 threads) while its lists stay short: 512 x 151,936 f32 takes 91 us with it
+  // at k = 64 and 160 us at k = 256, where the other one takes 92.
+  if (k > gs::TKL_MIN_K) {
     gs::TopKLargeArgs ta;
     ta.x = x; ta.row_stride = row_stride; ta.V = static_cast<int32_t>(V); ta.k = static_cast<int32_t>(k);
     ta.out_values = out_values; ta.out_indices = out_indices; ta.out_flags = out_flags; ta.B = B;
@@ -1375,16 +1428,10 @@ int gorch_cuda_lm_head_logits_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
   if (!out_logits || ld_out < V) { set_err(errOut, "gorch_cuda: LM head output missing or its pitch below V"); return GORCH_CUDA_ERR_BAD_ARG; }
   CUDA_TRY(cudaSetDevice(c->device), errOut);
   if ((rc = load_encode_tiled(errOut))) return rc;
-  if ((rc = ensure(c->lmh_scratch, 256, errOut))) return rc;
   gs::LmHeadArgs a;
-  memset(&a, 0, sizeof a);
-  if ((rc = make_bf16_map(&a.map_x, x, B, K, ldx, errOut))) return rc;
-  if ((rc = make_bf16_map(&a.map_w, w, V, K, ldw, errOut))) return rc;
-  a.B = static_cast<int32_t>(B); a.V = static_cast<int32_t>(V); a.K = static_cast<int32_t>(K);
-  a.tile0 = 0; a.tile_step = 1; a.ntile = static_cast<int32_t>((V + gs::LMH_BN - 1) / gs::LMH_BN);
+  if ((rc = lm_head_args(c, a, x, ldx, w, ldw, B, V, K, true, errOut))) return rc;
+  a.tile0 = 0; a.tile_step = 1; a.ntile = static_cast<int32_t>((V + 2 * a.cta_v - 1) / (2 * a.cta_v));
   a.out_logits = out_logits; a.ld_out = ld_out; a.compact = 0;
-  a.status = static_cast<uint32_t*>(c->lmh_scratch.ptr);
-  CUDA_TRY(cudaMemsetAsync(a.status, 0, sizeof(uint32_t), c->stream), errOut);
   return launch_lm_head(c, a, errOut);
 }
 
@@ -1400,48 +1447,41 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
   CUDA_TRY(cudaSetDevice(c->device), errOut);
   if ((rc = load_encode_tiled(errOut))) return rc;
   gs::LmHeadArgs a;
-  memset(&a, 0, sizeof a);
-  if ((rc = make_bf16_map(&a.map_x, x, B, K, ldx, errOut))) return rc;
-  if ((rc = make_bf16_map(&a.map_w, w, V, K, ldw, errOut))) return rc;
-  a.B = static_cast<int32_t>(B); a.V = static_cast<int32_t>(V); a.K = static_cast<int32_t>(K);
-  const int ntile = static_cast<int>((V + gs::LMH_BN - 1) / gs::LMH_BN);
+  if ((rc = lm_head_args(c, a, x, ldx, w, ldw, B, V, K, false, errOut))) return rc;
+  const int ntile = static_cast<int>((V + 2 * a.cta_v - 1) / (2 * a.cta_v));
   // the unfused form: logits to scratch, then the ordinary sampling kernels
   auto unfused = [&]() -> int {
-    const int64_t ld = (V + 3) & ~3ll;
+    const int64_t ld = (V + 31) & ~31ll;
     int r2 = ensure(c->lmh_logits, static_cast<size_t>(B) * ld * sizeof(float), errOut);
     if (r2) return r2;
-    if ((r2 = ensure(c->lmh_scratch, 256, errOut))) return r2;
-    gs::LmHeadArgs u = a;
-    u.tile0 = 0; u.tile_step = 1; u.ntile = ntile;
+    gs::LmHeadArgs u;
+    if ((r2 = lm_head_args(c, u, x, ldx, w, ldw, B, V, K, true, errOut))) return r2;
+    u.tile0 = 0; u.tile_step = 1; u.ntile = static_cast<int32_t>((V + 2 * u.cta_v - 1) / (2 * u.cta_v));
     u.out_logits = static_cast<float*>(c->lmh_logits.ptr); u.ld_out = ld; u.compact = 0;
-    u.thr = nullptr; u.cand = nullptr; u.cand_cnt = nullptr; u.rowmax_key = nullptr; u.row_nan = nullptr;
-    u.status = static_cast<uint32_t*>(c->lmh_scratch.ptr);
-    CUDA_TRY(cudaMemsetAsync(u.status, 0, sizeof(uint32_t), c->stream), errOut);
     if ((r2 = launch_lm_head(c, u, errOut))) return r2;
     return launch_rows(c, c->lmh_logits.ptr, GORCH_CUDA_F32, B, V, ld, cfgs, uniforms, out_ids, out_flags, nullptr, nullptr, 0, errOut);
   };
-  if (fuse_top_k < 1 || fuse_top_k > gs::KFAST || ntile < 4 * gs::LMH_SAMPLE_TILES_MIN || B > gs::LMH_ROWS_S) return unfused();
-  int stiles = ntile / 32;
-  if (stiles < gs::LMH_SAMPLE_TILES_MIN) stiles = gs::LMH_SAMPLE_TILES_MIN;
-  if (stiles > gs::LMH_SAMPLE_TILES_MAX) stiles = gs::LMH_SAMPLE_TILES_MAX;
+  if (fuse_top_k < 1 || fuse_top_k > gs::KFAST || V < 4096 || B > 4096) return unfused();
+  // the sample: 1/32 of the vocabulary, but 1024 to 4096 logits, in whole tiles
+  int64_t want = V / 32;
+  if (want < gs::LMH_SAMPLE_MIN) want = gs::LMH_SAMPLE_MIN;
+  if (want > gs::LMH_SAMPLE_MAX) want = gs::LMH_SAMPLE_MAX;
+  const int stiles = static_cast<int>(want / (2 * a.cta_v) > 1 ? want / (2 * a.cta_v) : 1);
 
-  // ---- the fused form: scratch = [status, nfail | thr | rowmax | nan | count | sample logits | candidates]
-  const int nsample = stiles * gs::LMH_BN;
-  // (candidates: one segment of LMH_SEG entries per row and CTA of the projection, and its count)
-  const size_t nseg = static_cast<size_t>(ntile < c->sm_count ? ntile : c->sm_count);
-  const size_t off_thr = 256, off_max = off_thr + 4 * B, off_nan = off_max + 4 * B;
-  const size_t off_smp = (off_nan + 4 * B + 255) & ~static_cast<size_t>(255);
-  const size_t off_cnt = (off_smp + sizeof(float) * B * nsample + 255) & ~static_cast<size_t>(255);
-  const size_t off_cand = (off_cnt + 4 * static_cast<size_t>(B) * nseg + 255) & ~static_cast<size_t>(255);
-  const size_t total = off_cand + sizeof(uint2) * static_cast<size_t>(B) * nseg * gs::LMH_SEG;
+  // ---- the fused form: scratch = [row state | thresholds | sample logits | candidates]; every kernel starts while the
+  // one before it runs: the projection's first tiles are under way before the thresholds are there
+  const int nsample = stiles * 2 * a.cta_v;
+  const size_t off_rows = 0, off_thr = off_rows + sizeof(gs::LmhRow) * static_cast<size_t>(B);
+  const size_t off_smp = (off_thr + 4 * static_cast<size_t>(B) + 255) & ~static_cast<size_t>(255);
+  const size_t off_cand = (off_smp + sizeof(float) * static_cast<size_t>(B) * nsample + 255) & ~static_cast<size_t>(255);
+  const size_t total = off_cand + sizeof(uint2) * static_cast<size_t>(B) * gs::LMH_CAND_CAP;
   if ((rc = ensure(c->lmh_scratch, total, errOut))) return rc;
   unsigned char* base = static_cast<unsigned char*>(c->lmh_scratch.ptr);
-  CUDA_TRY(cudaMemsetAsync(base, 0, off_smp, c->stream), errOut);          // status, nfail, maxima, NaN bits (every CTA of the projection writes its counts)
+  c->host_words[0] = c->host_words[1] = 0u;                                  // (the call before this one was waited for)
   // 1. a sample of the vocabulary's tiles (all of them full tiles)
   gs::LmHeadArgs sa = a;
   sa.tile0 = 0; sa.tile_step = (ntile - 1) / stiles; sa.ntile = stiles;
   sa.out_logits = reinterpret_cast<float*>(base + off_smp); sa.ld_out = nsample; sa.compact = 1;
-  sa.status = reinterpret_cast<uint32_t*>(base);
   if ((rc = launch_lm_head(c, sa, errOut))) return rc;
   // 2. thresholds
   gs::LmhSampleArgs fa;
@@ -1452,35 +1492,28 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
   fa.sample = reinterpret_cast<const float*>(base + off_smp); fa.nsample = nsample; fa.fuse_top_k = fuse_top_k;
   fa.thr = reinterpret_cast<float*>(base + off_thr);
   fa.cand = reinterpret_cast<const uint2*>(base + off_cand);
-  fa.cand_cnt = reinterpret_cast<const int32_t*>(base + off_cnt);
-  fa.rowmax_key = reinterpret_cast<const uint32_t*>(base + off_max);
-  fa.row_nan = reinterpret_cast<const int32_t*>(base + off_nan);
-  fa.nfail = reinterpret_cast<int32_t*>(base + 4);
-  fa.nseg = static_cast<int32_t>(nseg);
+  fa.rows = reinterpret_cast<gs::LmhRow*>(base + off_rows);
+  fa.nfail = reinterpret_cast<int32_t*>(c->host_words + 1);
   fa.B = B;
   const unsigned g = static_cast<unsigned>(B < 4 * c->sm_count ? B : 4 * c->sm_count);
-  gs::lmh_threshold_kernel<<<g, gs::LMH_F_NT, 0, c->stream>>>(fa);
+  CUDA_TRY(launch(c, gs::lmh_threshold_kernel, static_cast<unsigned>(B), gs::LMH_F_NT, 0, true, fa), errOut);
   // 3. the whole vocabulary, candidates out of the epilogue
   gs::LmHeadArgs ma = a;
   ma.tile0 = 0; ma.tile_step = 1; ma.ntile = ntile;
   ma.out_logits = nullptr; ma.ld_out = 0; ma.compact = 0;
-  ma.thr = fa.thr; ma.cand = reinterpret_cast<uint2*>(base + off_cand); ma.cand_cnt = reinterpret_cast<int32_t*>(base + off_cnt);
-  ma.rowmax_key = reinterpret_cast<uint32_t*>(base + off_max); ma.row_nan = reinterpret_cast<int32_t*>(base + off_nan);
-  ma.status = reinterpret_cast<uint32_t*>(base);
-  if ((rc = launch_lm_head(c, ma, errOut))) return rc;
+  ma.thr = fa.thr; ma.cand = reinterpret_cast<uint2*>(base + off_cand); ma.rows = fa.rows;
+  if ((rc = launch_lm_head(c, ma, errOut, true))) return rc;
   // 4. finish every row from its candidates
-  gs::lmh_finish_kernel<<<g, gs::LMH_F_NT, gs::LMH_F_DYN_BYTES, c->stream>>>(fa);
-  CUDA_TRY(cudaGetLastError(), errOut);
+  CUDA_TRY(launch(c, gs::lmh_finish_kernel, g, gs::LMH_F_NT, gs::LMH_F_DYN_BYTES, true, fa), errOut);
   c->counters.kernel_launches += 2;
   c->counters.sample_launches += 1;
   c->counters.rows += static_cast<uint64_t>(B);
   // rows the fused form could not finish (their estimate failed, or their config is not served): the
   // count comes back to the host, which then recomputes the batch through the unfused form
-  int32_t host_word[2] = {0, 0};
-  CUDA_TRY(cudaMemcpyAsync(host_word, base, sizeof host_word, cudaMemcpyDeviceToHost, c->stream), errOut);
   CUDA_TRY(cudaStreamSynchronize(c->stream), errOut);
+  const volatile uint32_t* host_word = c->host_words;
   if (host_word[0] != 0) {
-    set_err(errOut, "gorch_cuda: the LM-head kernel gave up a bounded wait (status %d)", host_word[0]);
+    set_err(errOut, "gorch_cuda: the LM-head kernel gave up a bounded wait (status %u)", host_word[0]);
     return GORCH_CUDA_ERR_CUDA;
   }
   if (host_word[1] > 0) {
@@ -1493,11 +1526,9 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
 int gorch_cuda_lm_head_status(GorchCudaCtxRef ctx, uint32_t* status, char** errOut) {
   Ctx* c = static_cast<Ctx*>(ctx);
   if (!c || !status) { set_err(errOut, "gorch_cuda: null argument"); return GORCH_CUDA_ERR_BAD_ARG; }
-  *status = 0;
-  if (!c->lmh_scratch.ptr) return GORCH_CUDA_OK;
   CUDA_TRY(cudaSetDevice(c->device), errOut);
-  CUDA_TRY(cudaMemcpyAsync(status, c->lmh_scratch.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream), errOut);
   CUDA_TRY(cudaStreamSynchronize(c->stream), errOut);
+  *status = *static_cast<const volatile uint32_t*>(c->host_words);
   return GORCH_CUDA_OK;
 }
 

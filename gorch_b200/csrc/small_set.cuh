@@ -18,6 +18,59 @@ namespace gs {
 constexpr int KEEP_MAX = 512;        // largest kept set finished in shared memory
 constexpr int SS_WORK_BYTES = 13344; // work arrays of finish_small_set
 
+// Programmatic dependent launch: wait for the kernel before this one in the stream; let the next one start.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Lower edge of a narrow bucket of order keys that holds the r-th largest key of a sample (every thread calls
+// f(key) for its keys, the same ones on every call); tmax: the largest of the thread's own keys, tmin: the
+// smallest. cnts: NBINS counters. Buckets of equal width are counted until the one of the r-th largest
+// holds few.
+template <int NT_, int NBINS, typename F>
+__device__ __forceinline__ uint32_t sample_threshold(F&& for_each_key, int r, uint32_t tmin, uint32_t tmax, uint32_t* cnts, int* bc,
+                                                     bu::Scratch& sc, int tid) {
+  constexpr int NW_ = NT_ / 32, PER = NBINS / NT_, LOGB = 31 - __builtin_clz(NBINS);
+  const int lane = tid & 31, warp = tid >> 5;
+  // r threads hold r largest ones of their own: the smallest of the thread maxima is not above the r-th largest
+  // while r <= NT_, and keeps the buckets off the keys that nobody asks for
+  uint32_t lo = __reduce_min_sync(FULL, (r <= NT_) ? tmax : tmin), hi = __reduce_max_sync(FULL, tmax);
+  for (int b = tid; b < NBINS; b += NT_) cnts[b] = 0u;
+  if (lane == 0) { sc.i0[warp] = static_cast<int>(lo); sc.i1[warp] = static_cast<int>(hi); }
+  __syncthreads();
+  lo = __reduce_min_sync(FULL, static_cast<uint32_t>(sc.i0[lane < NW_ ? lane : 0]));
+  hi = __reduce_max_sync(FULL, static_cast<uint32_t>(sc.i1[lane < NW_ ? lane : 0]));
+  int need = r;
+  for (;;) {                                                   // uniform
+    const int sh = max(0, 32 - __clz(hi - lo) - LOGB);
+    for_each_key([&](uint32_t key) { if (key - lo <= hi - lo) atomicAdd(&cnts[(hi - key) >> sh], 1u); });
+    __syncthreads();
+    uint32_t mine = 0u;
+#pragma unroll
+    for (int q = 0; q < PER; q++) mine += cnts[tid * PER + q];
+    uint32_t incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(FULL, incl, o); if (lane >= o) incl += t; }
+    if (lane == 31) sc.i0[warp] = static_cast<int>(incl);
+    __syncthreads();
+    uint32_t before = __reduce_add_sync(FULL, (lane < warp) ? static_cast<uint32_t>(sc.i0[lane]) : 0u) + incl - mine;
+    if (before < static_cast<uint32_t>(need) && before + mine >= static_cast<uint32_t>(need)) {   // one thread
+      int q = 0;
+      while (before + cnts[tid * PER + q] < static_cast<uint32_t>(need)) before += cnts[tid * PER + q++];
+      bc[0] = tid * PER + q; bc[1] = static_cast<int>(before); bc[2] = static_cast<int>(cnts[tid * PER + q]);
+    }
+    __syncthreads();
+    const uint32_t top = hi - (static_cast<uint32_t>(bc[0]) << sh), width = (1u << sh) - 1u;
+    lo = (top - lo > width) ? top - width : lo;
+    hi = top;
+    need -= bc[1];
+    if (sh == 0 || bc[2] <= max(2, r >> 3)) break;
+    __syncthreads();
+    for (int b = tid; b < NBINS; b += NT_) cnts[b] = 0u;
+    __syncthreads();
+  }
+  return lo;
+}
+
 // Leaves in out[] (KEEP_MAX entries) every candidate whose scaled value is not below that of the
 // top_k-th largest, and little more. for_each(f) calls f(entry) for every candidate of the calling thread
 // (the same ones on every call), n of them in the block. Every key lies in [lo, hi], except keys below lo that

@@ -1,4 +1,4 @@
-// TopK (index_ops.go:153-190) for 256 < k <= TKL_MAX_K: the k largest of each row, descending, equal
+// TopK (index_ops.go:153-190) for TKL_MIN_K < k <= TKL_MAX_K: the k largest of each row, descending, equal
 // values by ascending index; NaNs last (the reference's comparator leaves them unspecified), -0 and
 // +0 equal. The values written are the row's own bits.
 //
@@ -22,6 +22,7 @@
 
 namespace gs {
 
+constexpr int TKL_MIN_K = 64;           // up to here the narrow kernel serves TopK
 constexpr int TKL_MAX_K = 16384;
 
 struct TopKLargeArgs {
@@ -102,7 +103,9 @@ __device__ __noinline__ void topk_exact_row(const TopKLargeArgs& A, int64_t row,
     });
   }
   __syncthreads();
-  const bool ok = (*s_cnt == k);                             // an invariant of the two selects
+  // an invariant of the two selects; and a k that is promised an answer only while at most KEEP_MAX logits reach the
+  // k-th value (gorch_cuda_topk_dev: k <= KFAST) gets none beyond, whichever kernel serves it
+  const bool ok = (*s_cnt == k) && !(k <= KFAST && above + ties > KEEP_MAX);
   // bitonic sort, descending (a larger key first: larger value, then lower index)
   for (int size = 2; size <= P; size <<= 1) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -227,56 +230,16 @@ __global__ void __launch_bounds__(SH::NT, SH::MINB) topk_large_kernel(TopKLargeA
 #pragma unroll
           for (int c = 0; c < VEC; c++) { const uint32_t key = okey(x[c]); kmin = min(kmin, key); kmax = max(kmax, key); }
         }
-        // r threads hold r largest ones of their own: the smallest of NT thread maxima is below the r-th
-        // largest while r <= NT, and keeps the buckets off the keys that nobody asks for
-        uint32_t lo = (r <= NT) ? kmax : kmin;
-        uint32_t hi = static_cast<uint32_t>(bu::max_u64<NW>(kmax, sc, tid));
-        lo = ~static_cast<uint32_t>(bu::max_u64<NW>(~lo, sc, tid));
-        if (r < nsv * VEC) {
-          // buckets of equal width over [lo, hi], narrowed until the r-th largest shares its bucket with
-          // few others; the bucket's lower edge is the threshold
-          constexpr int LOGB = 31 - __builtin_clz(NBINS);
-          uint32_t* cnts = reinterpret_cast<uint32_t*>(dyn);             // the candidate list's memory: empty yet
-          int need = r;
-          for (;;) {                                         // uniform
-            const int sh = max(0, 32 - __clz(hi - lo) - LOGB);
-            for (int b = tid; b < NBINS; b += NT) cnts[b] = 0u;
-            __syncthreads();
+        if (r < nsv * VEC) {                                 // uniform
+          const uint32_t lo = sample_threshold<NT, NBINS>([&](auto&& g) {
 #pragma unroll
             for (int j = 0; j < J; j++) {
               float x[VEC];
               Elem<T>::unpack(smp[j], x);
 #pragma unroll
-              for (int c = 0; c < VEC; c++) {
-                const uint32_t key = okey(x[c]);
-                if (key - lo <= hi - lo) atomicAdd(&cnts[(hi - key) >> sh], 1u);
-              }
+              for (int c = 0; c < VEC; c++) g(okey(x[c]));
             }
-            __syncthreads();
-            constexpr int PER = NBINS / NT;
-            uint32_t mine = 0u;
-#pragma unroll
-            for (int q = 0; q < PER; q++) mine += cnts[tid * PER + q];
-            uint32_t incl = mine;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const uint32_t t = __shfl_up_sync(FULL, incl, o); if (lane >= o) incl += t; }
-            if (lane == 31) sc.i0[warp] = static_cast<int>(incl);
-            __syncthreads();
-            uint32_t before = __reduce_add_sync(FULL, (lane < warp) ? static_cast<uint32_t>(sc.i0[lane]) : 0u) + incl - mine;
-            if (before < static_cast<uint32_t>(need) && before + mine >= static_cast<uint32_t>(need)) {   // one thread
-              int q = 0;
-              while (before + cnts[tid * PER + q] < static_cast<uint32_t>(need)) before += cnts[tid * PER + q++];
-              bc[0] = tid * PER + q; bc[1] = static_cast<int>(before); bc[2] = static_cast<int>(cnts[tid * PER + q]);
-            }
-            __syncthreads();
-            const uint32_t top = hi - (static_cast<uint32_t>(bc[0]) << sh);
-            const uint32_t width = (1u << sh) - 1u;
-            lo = (top - lo > width) ? top - width : lo;
-            hi = top;
-            need -= bc[1];
-            if (sh == 0 || bc[2] <= max(2, r >> 3)) break;
-            __syncthreads();
-          }
+          }, r, kmin, kmax, reinterpret_cast<uint32_t*>(dyn), bc, sc, tid);   // counters in the candidate list's memory: empty yet
           if (lo != 0u) thr = okey_to_float(lo);
         }
         __syncthreads();
@@ -378,7 +341,7 @@ __global__ void __launch_bounds__(SH::NT, SH::MINB) topk_large_kernel(TopKLargeA
 #pragma unroll
       for (int q = 0; q < PER; q++) { bins[tid * PER + q] = run; run += loc[q]; }
       __syncthreads();
-      exact = most > 512u;                                   // long runs of near-equal logits: the places within a bucket take its size squared
+      exact = most > (k <= KFAST ? 256u : 512u);             // long runs of near-equal logits: the places within a bucket take its size squared
       if (!exact) {
         for (int j = tid; j < n; j += NT) perm[atomicAdd(&bins[bin_of(cand[j])], 1u)] = static_cast<uint16_t>(j);
         __syncthreads();                                     // bins[b] is now the end of bucket b
