@@ -22,7 +22,7 @@
 
 #include <cstdint>
 
-#include "block_util.cuh"
+#include "small_set.cuh"   // pdl_wait, pdl_launch
 
 namespace gs {
 
@@ -57,26 +57,29 @@ struct GenControlArgs {
   int B;
 };
 
-__global__ void __launch_bounds__(GC_NT) generate_control_kernel(const GenControlArgs A) {
+// Bound: latency, a launch and two trips to L2: a row's words are read at once, before any decision. The kernel
+// starts beside the sampling kernel's last CTAs and waits for them here.
+__global__ void __launch_bounds__(GC_NT) generate_control_kernel(const __grid_constant__ GenControlArgs A) {
   __shared__ bu::Scratch sc;
   const int tid = threadIdx.x;
   int live = 0;
+  pdl_launch();
+  pdl_wait();
   for (int b = tid; b < A.B; b += GC_NT) {
-    if (A.done[b] != GC_LIVE) continue;
+    const int done = A.done[b], id = A.ids[b], len = A.lengths[b], cl = A.cached ? A.cache_len[b] : 0;
+    const uint32_t fl = (A.flags != nullptr) ? A.flags[b] : 0u;
     int n = A.n_new[b];
+    if (done != GC_LIVE) continue;
     if (n >= A.max_new) { A.done[b] = GC_MAX_NEW; continue; }
-    const int id = A.ids[b];
-    if (id < 0 || (A.flags != nullptr && (A.flags[b] & A.bad_flags) != 0u)) { A.done[b] = GC_ERROR; continue; }
+    if (id < 0 || (fl & A.bad_flags) != 0u) { A.done[b] = GC_ERROR; continue; }
     bool stop = false;
     for (int s = 0; s < A.n_stop; s++) stop |= (id == A.stops[s]);
     if (stop) { A.done[b] = GC_STOP; continue; }
-    const int len = A.lengths[b];
     if (len >= A.capacity) { A.done[b] = GC_ERROR; continue; }
     A.tokens[static_cast<long long>(b) * A.capacity + len] = id;
     A.lengths[b] = len + 1;
     A.n_new[b] = ++n;
     if (A.cached) {
-      const int cl = A.cache_len[b];
       if (cl >= A.max_seq) { A.done[b] = GC_MAX_SEQ; continue; }
       A.cache_len[b] = cl + 1;
     } else if (A.window_start != nullptr) {

@@ -218,6 +218,8 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
   __shared__ uint32_t s_sel[256];
 
   cg::cluster_group cluster = cg::this_cluster();
+  pdl_launch();                       // (the next kernel waits for this one's end by itself)
+  pdl_wait();                         // whatever fills the inputs
   // a row whose sequence has ended (model/generate.go:82-84) is skipped by its whole cluster, before any barrier
   if (CA.k.row_done && CA.k.row_done[CA.k.row_offset + blockIdx.x / cluster.num_blocks()] != 0) return;
   cluster.barrier_arrive();          // matched by the wait before the first remote store

@@ -15,7 +15,9 @@
 #include <cstdlib>
 #include <cstring>
 #include <limits>
+#include <mutex>
 #include <new>
+#include <vector>
 
 #include "../../include/gorch_cuda_shim.h"
 #define GS_W_NS w256
@@ -53,7 +55,63 @@ struct Buffer {
   int device;
   void* ptr;
   uint64_t bytes;
+  uint64_t block;         // bytes that the pool holds for it (a power of two), or 0: not the pool's
 };
+
+// Small device blocks that released buffers leave for the next ones, so that a generation or a call that
+// needs a few arrays for a moment does not pay for cudaMalloc and cudaFree (tens of microseconds each, and
+// cudaFree waits for the device). At most kPoolBytes per process; given back when the last context goes.
+// A block may still be in use by work queued before its buffer was released, on any stream: before a
+// block is handed out again that was released after the device was last waited for, the device is waited
+// for (as cudaFree would have done), once for all such blocks.
+struct BufferPool {
+  static constexpr uint64_t kMaxBlock = 1ull << 20, kPoolBytes = 32ull << 20;
+  struct Block { int device; void* ptr; uint64_t bytes; bool in_doubt; };
+  std::mutex lock;
+  std::vector<Block> free_blocks;
+  uint64_t held = 0;
+  int contexts = 0;
+
+  static uint64_t block_of(uint64_t bytes) {
+    uint64_t b = 256;
+    while (b < bytes) b <<= 1;
+    return b <= kMaxBlock ? b : 0;
+  }
+  // A block of exactly `bytes`, or null. The device is current.
+  void* take(int device, uint64_t bytes) {
+    std::lock_guard<std::mutex> g(lock);
+    size_t at = free_blocks.size();
+    for (size_t i = 0; i < free_blocks.size(); i++) {
+      if (free_blocks[i].device == device && free_blocks[i].bytes == bytes && (at == free_blocks.size() || !free_blocks[i].in_doubt)) at = i;
+    }
+    if (at == free_blocks.size()) return nullptr;
+    if (free_blocks[at].in_doubt) {
+      if (cudaDeviceSynchronize() != cudaSuccess) return nullptr;
+      for (Block& b : free_blocks) if (b.device == device) b.in_doubt = false;
+    }
+    void* p = free_blocks[at].ptr;
+    free_blocks[at] = free_blocks.back();
+    free_blocks.pop_back();
+    held -= bytes;
+    return p;
+  }
+  bool put(int device, void* ptr, uint64_t bytes) {
+    std::lock_guard<std::mutex> g(lock);
+    if (contexts == 0 || held + bytes > kPoolBytes) return false;
+    free_blocks.push_back(Block{device, ptr, bytes, true});
+    held += bytes;
+    return true;
+  }
+  void enter() { std::lock_guard<std::mutex> g(lock); contexts++; }
+  void leave() {
+    std::lock_guard<std::mutex> g(lock);
+    if (--contexts > 0) return;
+    for (Block& b : free_blocks) { cudaSetDevice(b.device); cudaFree(b.ptr); }
+    free_blocks.clear();
+    held = 0;
+  }
+};
+BufferPool g_pool;
 
 struct Scratch {  // grow-only device allocation
   void* ptr = nullptr;
@@ -368,13 +426,15 @@ int launch_rows(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int
       lc.blockDim = dim3(gs::NT);
       lc.dynamicSmemBytes = dyn;
       lc.stream = c->stream;
-      cudaLaunchAttribute at[1];
+      cudaLaunchAttribute at[2];
       at[0].id = cudaLaunchAttributeClusterDimension;
       at[0].val.clusterDim.x = static_cast<unsigned>(C);
       at[0].val.clusterDim.y = 1;
       at[0].val.clusterDim.z = 1;
+      at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // launch beside the kernel before it; it waits for that itself
+      at[1].val.programmaticStreamSerializationAllowed = 1;
       lc.attrs = at;
-      lc.numAttrs = 1;
+      lc.numAttrs = 2;
       const bool diag = out_probs || out_debug;
       if (dtype == GORCH_CUDA_F32) {
         CUDA_TRY(cudaLaunchKernelEx(&lc, diag ? gs::sample_cluster_kernel<float, true> : gs::sample_cluster_kernel<float, false>, ca), errOut);
@@ -600,6 +660,7 @@ GorchCudaCtxRef gorch_cuda_create_ctx(int device, char** errOut) {
   Ctx* c = new (std::nothrow) Ctx();
   if (!c) { set_err(errOut, "gorch_cuda: out of host memory"); return nullptr; }
   c->device = device;
+  g_pool.enter();
   auto fail = [&](const char* what, cudaError_t err) -> GorchCudaCtxRef {
     set_err(errOut, "gorch_cuda: %s failed: %s", what, cudaGetErrorString(err));
     gorch_cuda_release(c);
@@ -699,6 +760,7 @@ void gorch_cuda_release(GorchCudaCtxRef ctx) {
   if (c->side_stream) cudaStreamDestroy(c->side_stream);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
+  g_pool.leave();
   delete c;
 }
 
@@ -748,10 +810,11 @@ int gorch_cuda_get_counters(GorchCudaCtxRef ctx, GorchCudaCounters* out) {
 GorchCudaBufferRef gorch_cuda_buffer_alloc(GorchCudaCtxRef ctx, uint64_t bytes, char** errOut) {
   Ctx* c = static_cast<Ctx*>(ctx);
   if (!c) { set_err(errOut, "gorch_cuda: null context"); return nullptr; }
-  Buffer* b = new (std::nothrow) Buffer{c->device, nullptr, bytes};
+  Buffer* b = new (std::nothrow) Buffer{c->device, nullptr, bytes, BufferPool::block_of(bytes)};
   if (!b) { set_err(errOut, "gorch_cuda: out of host memory"); return nullptr; }
   cudaError_t e = cudaSetDevice(c->device);
-  if (e == cudaSuccess) e = cudaMalloc(&b->ptr, bytes ? bytes : 1);
+  if (e == cudaSuccess && b->block) b->ptr = g_pool.take(c->device, b->block);
+  if (e == cudaSuccess && !b->ptr) e = cudaMalloc(&b->ptr, b->block ? b->block : bytes);
   if (e != cudaSuccess) {
     set_err(errOut, "gorch_cuda: cudaMalloc(%llu) failed: %s", (unsigned long long)bytes, cudaGetErrorString(e));
     delete b;
@@ -763,8 +826,10 @@ GorchCudaBufferRef gorch_cuda_buffer_alloc(GorchCudaCtxRef ctx, uint64_t bytes, 
 void gorch_cuda_buffer_free(GorchCudaBufferRef buf) {
   Buffer* b = static_cast<Buffer*>(buf);
   if (!b) return;
-  cudaSetDevice(b->device);
-  cudaFree(b->ptr);
+  if (!b->block || !g_pool.put(b->device, b->ptr, b->block)) {
+    cudaSetDevice(b->device);
+    cudaFree(b->ptr);
+  }
   delete b;
 }
 
@@ -1239,8 +1304,7 @@ static int launch_generate_control(Ctx* c, const int32_t* ids, const uint32_t* f
   a.n_stop = gc->n_stop; a.max_new = gc->max_new; a.max_seq = gc->max_seq; a.cached = gc->cached ? 1 : 0;
   a.bad_flags = GORCH_FLAG_INTERNAL | GORCH_FLAG_BAD_CFG;
   a.B = static_cast<int>(B);
-  gs::generate_control_kernel<<<1, gs::GC_NT, 0, c->stream>>>(a);
-  CUDA_TRY(cudaGetLastError(), errOut);
+  CUDA_TRY(launch(c, gs::generate_control_kernel, 1, gs::GC_NT, 0, true, a), errOut);
   c->counters.kernel_launches += 1;
   return GORCH_CUDA_OK;
 }

@@ -20,7 +20,7 @@ import numpy as np
 
 from . import _lib
 from .config import CFG_DTYPE
-from .sampling import CudaSampler, _check
+from .sampling import BufferPart, CudaSampler, _check
 
 LOOP_UNCACHED = 0   # GenerateWithConfig without KV cache (model/generate.go:57-88)
 LOOP_CACHED = 1     # generateCached (model/generate.go:93-131)
@@ -62,33 +62,42 @@ class DeviceGenerateState:
         start = np.maximum(lengths - self.max_seq, 0).astype(np.int32)
         last = np.array([p[-1] if p else 0 for p in prompts], dtype=np.int32)
         zeros = np.zeros(B, dtype=np.int32)
-        self._bufs = {}
-        for name, arr in (("tokens", tokens), ("lengths", lengths), ("n_new", zeros), ("cache_len", lengths.copy()),
-                          ("done", zeros), ("next_input", last), ("window_start", start),
-                          ("live_count", np.array([B], dtype=np.int32)), ("ids", zeros), ("flags", zeros)):
-            buf = sampler._buf(max(arr.nbytes, 16))
-            self._bufs[name] = buf
-            if arr.nbytes:
-                sampler._upload(buf, np.ascontiguousarray(arr))
-        ptr = sampler._lib.gorch_cuda_buffer_device_ptr
+        # one allocation, one upload and one download for everything: a state's arrays are small, and each
+        # separate call costs a round trip to the device
+        self._layout, size = {}, 0
+        parts = (("tokens", tokens), ("lengths", lengths), ("n_new", zeros), ("cache_len", lengths), ("done", zeros),
+                 ("next_input", last), ("window_start", start), ("live_count", np.array([B], dtype=np.int32)), ("ids", zeros),
+                 ("flags", zeros))
+        for name, arr in parts:
+            self._layout[name] = (size, arr.shape)
+            size += max((arr.nbytes + 255) & ~255, 256)
+        packed = np.zeros(size, dtype=np.uint8)
+        for name, arr in parts:
+            at = self._layout[name][0]
+            packed[at:at + arr.nbytes] = arr.view(np.uint8).reshape(-1)
+        self._buf = sampler._buf(size)
+        sampler._upload(self._buf, packed)
+        self._bufs = {name: BufferPart(self._buf, at) for name, (at, _) in self._layout.items()}
+        base = sampler._lib.gorch_cuda_buffer_device_ptr(self._buf)
+        ptr = {name: base + at for name, (at, _) in self._layout.items()}
         self.gc = _lib.GenControl()
-        self.gc.tokens = ptr(self._bufs["tokens"])
+        self.gc.tokens = ptr["tokens"]
         self.gc.capacity = cap
-        self.gc.lengths = ptr(self._bufs["lengths"])
-        self.gc.n_new = ptr(self._bufs["n_new"])
-        self.gc.cache_len = ptr(self._bufs["cache_len"])
-        self.gc.done = ptr(self._bufs["done"])
-        self.gc.next_input = ptr(self._bufs["next_input"])
-        self.gc.window_start = ptr(self._bufs["window_start"])
-        self.gc.live_count = ptr(self._bufs["live_count"])
+        self.gc.lengths = ptr["lengths"]
+        self.gc.n_new = ptr["n_new"]
+        self.gc.cache_len = ptr["cache_len"]
+        self.gc.done = ptr["done"]
+        self.gc.next_input = ptr["next_input"]
+        self.gc.window_start = ptr["window_start"]
+        self.gc.live_count = ptr["live_count"]
         for i in range(_lib.GEN_MAX_STOPS):
             self.gc.stop_tokens[i] = stops[i] if i < len(stops) else -1
         self.gc.n_stop = len(stops)
         self.gc.max_new = self.max_new
         self.gc.max_seq = self.max_seq
         self.gc.cached = 0 if loop == LOOP_UNCACHED else 1
-        self.ids_ptr = ptr(self._bufs["ids"])
-        self.flags_ptr = ptr(self._bufs["flags"])
+        self.ids_ptr = ptr["ids"]
+        self.flags_ptr = ptr["flags"]
 
     # what a model's forward reads
     next_input_ptr = property(lambda self: self.gc.next_input)
@@ -98,9 +107,9 @@ class DeviceGenerateState:
     lengths_ptr = property(lambda self: self.gc.lengths)
 
     def release(self) -> None:
-        for b in self._bufs.values():
-            self.s._lib.gorch_cuda_buffer_free(b)
-        self._bufs = {}
+        if self._buf:
+            self.s._lib.gorch_cuda_buffer_free(self._buf)
+        self._buf, self._bufs = None, {}
 
     def control(self, ids_ptr: int, flags_ptr: int | None = None) -> None:
         """One loop iteration over ids some sampling call has left on the device."""
@@ -127,12 +136,19 @@ class DeviceGenerateState:
         return int(self._get("live_count", 1)[0])
 
     def results(self) -> dict:
-        tokens = self._get("tokens", (self.B, self.capacity))
-        lengths = self._get("lengths", self.B)
+        whole = np.empty(max(at for at, _ in self._layout.values()), dtype=np.uint8)   # all but the sampler's flags
+        self.s.sync()
+        self.s._download(self._buf, whole)
+
+        def get(name):
+            at, shape = self._layout[name]
+            n = int(np.prod(shape))
+            return whole[at:at + 4 * n].view(np.int32).reshape(shape).copy()
+
+        tokens, lengths = get("tokens"), get("lengths")
         return {"tokens": [tokens[b, : lengths[b]].tolist() for b in range(self.B)],
-                "done": self._get("done", self.B), "n_new": self._get("n_new", self.B),
-                "cache_len": self._get("cache_len", self.B), "next_input": self._get("next_input", self.B),
-                "window_start": self._get("window_start", self.B)}
+                "done": get("done"), "n_new": get("n_new"), "cache_len": get("cache_len"), "next_input": get("next_input"),
+                "window_start": get("window_start")}
 
 
 def generate_on_device(model, prompts, cfgs, uniforms, sampler: CudaSampler, max_new: int, max_seq: int,
@@ -148,15 +164,14 @@ def generate_on_device(model, prompts, cfgs, uniforms, sampler: CudaSampler, max
     if uniforms.shape[1] != st.B or cfgs.shape[0] != st.B:
         st.release()
         raise ValueError("cfgs must hold B records and uniforms max_new x B values")
-    b_cfg = sampler._buf(max(cfgs.nbytes, 16))
-    b_uni = sampler._buf(max(uniforms.nbytes, 16))
+    inputs = np.zeros(((cfgs.nbytes + 255) & ~255) + max(uniforms.nbytes, 16), dtype=np.uint8)
+    inputs[: cfgs.nbytes] = cfgs.view(np.uint8)
+    inputs[len(inputs) - max(uniforms.nbytes, 16):][: uniforms.nbytes] = uniforms.view(np.uint8).reshape(-1)
+    b_in = sampler._buf(inputs.nbytes)
     try:
-        if cfgs.nbytes:
-            sampler._upload(b_cfg, cfgs)
-        if uniforms.nbytes:
-            sampler._upload(b_uni, uniforms)
-        ptr = sampler._lib.gorch_cuda_buffer_device_ptr
-        p_cfg, p_uni = ptr(b_cfg), ptr(b_uni)
+        sampler._upload(b_in, inputs)
+        p_cfg = sampler._lib.gorch_cuda_buffer_device_ptr(b_in)
+        p_uni = p_cfg + len(inputs) - max(uniforms.nbytes, 16)
         steps = 0
         if st.B and max_new > 0:
             logits_ptr, dtype, V, stride = model.prefill_dev(st)
@@ -172,6 +187,5 @@ def generate_on_device(model, prompts, cfgs, uniforms, sampler: CudaSampler, max
         out["steps"] = steps
         return out
     finally:
-        sampler._lib.gorch_cuda_buffer_free(b_cfg)
-        sampler._lib.gorch_cuda_buffer_free(b_uni)
+        sampler._lib.gorch_cuda_buffer_free(b_in)
         st.release()

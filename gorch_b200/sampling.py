@@ -62,6 +62,17 @@ VS_RECORD_BYTES = 16 + 8 * VS_CAND  # GORCH_VS_RECORD_BYTES
 UNIQUE_ID_BYTES = 128              # GORCH_CUDA_UNIQUE_ID_BYTES
 
 
+class BufferPart:
+    """A place inside a device buffer, for uploads to it and downloads from it."""
+
+    def __init__(self, buf: int, offset: int):
+        self.buf, self.offset = buf, offset
+
+
+def _place(buf):
+    return (buf.buf, buf.offset) if isinstance(buf, BufferPart) else (buf, 0)
+
+
 class CudaSampler:
     """One device context (cf. metal.NewDevice, metal/metal.go:228-234): a
     device, a stream and grow-only staging buffers."""
@@ -168,13 +179,15 @@ class CudaSampler:
             raise GorchCudaError(2, _take_err(self._lib, err))
         return b
 
-    def _upload(self, buf: int, arr: np.ndarray) -> None:
+    def _upload(self, buf, arr: np.ndarray) -> None:
         err = C.c_void_p()
-        _check(self._lib, self._lib.gorch_cuda_buffer_upload(buf, 0, arr.ctypes.data, arr.nbytes, C.byref(err)), err)
+        handle, at = _place(buf)
+        _check(self._lib, self._lib.gorch_cuda_buffer_upload(handle, at, arr.ctypes.data, arr.nbytes, C.byref(err)), err)
 
-    def _download(self, buf: int, arr: np.ndarray) -> None:
+    def _download(self, buf, arr: np.ndarray) -> None:
         err = C.c_void_p()
-        _check(self._lib, self._lib.gorch_cuda_buffer_download(buf, 0, arr.ctypes.data, arr.nbytes, C.byref(err)), err)
+        handle, at = _place(buf)
+        _check(self._lib, self._lib.gorch_cuda_buffer_download(handle, at, arr.ctypes.data, arr.nbytes, C.byref(err)), err)
 
     def sample_batch_debug(self, logits, cfgs, uniforms, want_probs: bool = True,
                            pad_elems: int = 0):
