@@ -90,9 +90,6 @@ __device__ __forceinline__ void hand_to_single(const BatchArgs& BA, int64_t row_
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
-template <typename T>
-__device__ __forceinline__ uint4 mask_edges(const RowView<T>& rv, int v, uint4 raw);
-
 // The narrow kernel, compiled twice from one source (sample_narrow.cuh): n256 with 256 threads and
 // five CTAs per SM for batches of at most one row per CTA slot (a row is then streamed by eight
 // warps), n128 with 128 threads and eight CTAs per SM beyond that (1184 rows in flight: the phases
@@ -107,24 +104,5 @@ __device__ __forceinline__ uint4 mask_edges(const RowView<T>& rv, int v, uint4 r
 #include "sample_narrow.cuh"
 #undef GS_N_NS
 #undef GS_N_NT
-
-template <typename T>
-__device__ __forceinline__ uint4 mask_edges(const RowView<T>& rv, int v, uint4 raw) {
-  if (v > 0 && v < rv.nvec - 1) return raw;
-  constexpr int VEC = Elem<T>::VEC;
-  uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
-  const int i0 = v * VEC - rv.shift;
-#pragma unroll
-  for (int c = 0; c < VEC; c++) {
-    const int i = i0 + c;
-    if (i < 0 || i >= rv.V) {
-      if (sizeof(T) == 4) w[c] = 0xff800000u;
-      else if (c & 1) w[c >> 1] = (w[c >> 1] & 0x0000ffffu) | 0xff800000u;
-      else w[c >> 1] = (w[c >> 1] & 0xffff0000u) | 0x0000ff80u;
-    }
-  }
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
-
 
 }  // namespace gs

@@ -169,6 +169,41 @@ __device__ __forceinline__ uint4 mask_and_stats(const RowView<T>& rv, int v, uin
   }
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
+// The same without the statistics.
+template <typename T>
+__device__ __forceinline__ uint4 mask_edges(const RowView<T>& rv, int v, uint4 raw) {
+  if (v > 0 && v < rv.nvec - 1) return raw;
+  constexpr int VEC = Elem<T>::VEC;
+  uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+  const int i0 = v * VEC - rv.shift;
+#pragma unroll
+  for (int c = 0; c < VEC; c++) {
+    const int i = i0 + c;
+    if (i < 0 || i >= rv.V) {
+      if (sizeof(T) == 4) w[c] = 0xff800000u;
+      else if (c & 1) w[c >> 1] = (w[c >> 1] & 0x0000ffffu) | 0xff800000u;
+      else w[c >> 1] = (w[c >> 1] & 0xffff0000u) | 0x0000ff80u;
+    }
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// NaN-propagating maximum of a vector's logits.
+template <typename T> __device__ __forceinline__ float vec_max_nan(const uint4& a);
+template <> __device__ __forceinline__ float vec_max_nan<float>(const uint4& a) {
+  float m;
+  asm("{\n\t.reg .f32 t;\n\tmax.NaN.f32 t, %1, %2, %3;\n\tmax.NaN.f32 %0, t, %4;\n\t}"
+      : "=f"(m) : "f"(__uint_as_float(a.x)), "f"(__uint_as_float(a.y)), "f"(__uint_as_float(a.z)), "f"(__uint_as_float(a.w)));
+  return m;
+}
+template <> __device__ __forceinline__ float vec_max_nan<uint16_t>(const uint4& a) {
+  uint32_t p;
+  asm("{\n\t.reg .b32 t, u;\n\tmax.NaN.bf16x2 t, %1, %2;\n\tmax.NaN.bf16x2 u, %3, %4;\n\tmax.NaN.bf16x2 %0, t, u;\n\t}"
+      : "=r"(p) : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w));
+  float m;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(__uint_as_float(p << 16)), "f"(__uint_as_float(p & 0xffff0000u)));
+  return m;
+}
 template <typename T>
 __device__ __forceinline__ uint4 load_masked(const RowView<T>& rv, int v, float& vmax, float& vmin, bool& nan_seen) {
   return mask_and_stats(rv, v, __ldg(rv.vbase + v), vmax, vmin, nan_seen);
@@ -350,6 +385,17 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
   float xmax = -INFINITY, xmin = INFINITY;
   bool nan_seen = false;
   asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (topk > 0) {
+    // a top-k row needs the maxima only: a few packed instructions per vector
+    for (int j = tid; j < nv; j += NT) {
+      const int v = v0 + j;
+      uint4 raw = slice[j];
+      if (v == 0 || v >= rv.nvec - 1) { raw = mask_edges(rv, v, raw); slice[j] = raw; }
+      const float m = vec_max_nan<T>(raw);
+      nan_seen |= (m != m);
+      xmax = fmaxf(xmax, m);                                 // (a NaN poisons the row: what its vector's maximum would be is no matter)
+    }
+  } else
   for (int j = tid; j < nv; j += NT) {
     const int v = v0 + j;
     const uint4 raw = slice[j];
@@ -402,23 +448,22 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
     // pass B: candidates >= thr0 from shared memory
     uint2* lc = reinterpret_cast<uint2*>(regB);              // LCAP entries
     for (int j = tid; j < nv; j += NT) {
+      const uint4 raw = slice[j];
+      if (!(vec_max_nan<T>(raw) >= thr0)) continue;
       float x[VEC];
-      Elem<T>::unpack(slice[j], x);
-      bool any = false;
+      Elem<T>::unpack(raw, x);
+      const int i0 = (v0 + j) * VEC - rv.shift;
+      uint32_t hits = 0u;
 #pragma unroll
-      for (int c = 0; c < VEC; c++) any |= (x[c] >= thr0);
-      if (any) {
-        const int i0 = (v0 + j) * VEC - rv.shift;
-#pragma unroll
-        for (int c = 0; c < VEC; c++) {
-          int i = i0 + c;
-          if (x[c] >= thr0 && i >= 0 && i < V) {
-            int slot = atomicAdd(&ctl.cand_count, 1);
-            if (slot < LCAP) lc[slot] = make_uint2(__float_as_uint(x[c]), static_cast<uint32_t>(i));
-          }
-        }
+      for (int c = 0; c < VEC; c++) hits |= (x[c] >= thr0 && static_cast<uint32_t>(i0 + c) < static_cast<uint32_t>(V)) ? 1u << c : 0u;
+      int slot = atomicAdd(&ctl.cand_count, __popc(hits));
+      const T* src = reinterpret_cast<const T*>(slice + j);
+      for (; hits; hits &= hits - 1, slot++) {
+        const int c = __ffs(hits) - 1;
+        if (slot < LCAP) lc[slot] = make_uint2(__float_as_uint(Elem<T>::to_float(src[c])), static_cast<uint32_t>(i0 + c));
       }
     }
+    if (tid < 256) s_sel[tid] = 0u;                          // narrow_candidates wants it cleared (and a count: ctl.overflow still is)
     __syncthreads();
     // Where the lists meet: rank 0's region A while UCAP entries are enough for all ranks; a larger top_k takes
     // rank 0's slice, after one more barrier that says that rank 0 is through with it.
@@ -429,6 +474,7 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
       uint2* few = reinterpret_cast<uint2*>(dyn);            // (the slice has been read; peers may already write to region A)
       n_loc = narrow_list<NT>(lc, n_loc, topk, Tm, okey(thr0), khi, few, s_sel, ctl.bcast_i, &ctl.cand_count, tid);
       for (int j = tid; j < min(n_loc, KEEP_MAX); j += NT) lc[j] = few[j];
+      if (tid < 256) s_sel[tid] = 0u;
       __syncthreads();
     }
     const bool giveup = n_loc > min(cap_r, LCAP);
@@ -469,13 +515,21 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
     }
     const uint2* lists = reinterpret_cast<const uint2*>(wide_lists ? dyn : regA);
     const int caplog = 31 - __clz(cap_r);                    // a power of two
+    constexpr int PER = WCAP / NT;
+    uint2 mine[PER];                                         // this thread's entries; (x: NaN) where there is none
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+      const int j = q * NT + tid;
+      const bool there = j < (C << caplog) && (j & (cap_r - 1)) < X.cnt[j >> caplog];
+      mine[q] = there ? lists[j] : make_uint2(0x7fc00000u, 0u);
+    }
     auto each = [&](auto&& f) {
-      for (int j = tid; j < C << caplog; j += NT)
-        if ((j & (cap_r - 1)) < X.cnt[j >> caplog]) f(lists[j]);
+#pragma unroll
+      for (int q = 0; q < PER; q++) if (mine[q].x != 0x7fc00000u) f(mine[q]);
     };
     uint2* kp = reinterpret_cast<uint2*>(regB);               // the local list is done with
     const int nk = narrow_candidates<NT>(each, n, topk, Tm, okey(thr0), static_cast<uint32_t>(mx >> 32), kp, s_sel, ctl.bcast_i,
-                                         &ctl.cand_count, tid);
+                                         &ctl.overflow, tid);
     if (nk > KEEP_MAX) { alone(); return; }                  // long run of ties at the threshold
     finish_small_set<NT, D>(A, row_id, kp, nk, topk, m, Tm, topp_on, mode, plim, u, -INFINITY, dyn, D ? &dbg : nullptr, flags);
     return;

@@ -113,6 +113,9 @@ struct BufferPool {
 };
 BufferPool g_pool;
 
+// Logits in pageable host memory that go through the context's pinned block, and the piece of them that is copied at a time.
+constexpr size_t kStageBytes = 1ull << 20, kStagePiece = 128ull << 10;
+
 struct Scratch {  // grow-only device allocation
   void* ptr = nullptr;
   size_t cap = 0;
@@ -129,7 +132,8 @@ struct Ctx {
   double* exp_table = nullptr;
   double* eb_table = nullptr;
   Scratch worklist;        // int32[1 + rows]: rows the cluster kernel leaves to the single-CTA kernel
-  Scratch st_logits, st_cfgs, st_uniforms, st_ids, st_flags;
+  Scratch st_logits;       // logits of the host-memory calls
+  Scratch pinned;          // host memory: their configurations, uniforms, ids, flags, and logits on their way
   Scratch lmh_scratch;       // thresholds, candidate lists, sample logits of the LM-head path
   uint32_t* host_words = nullptr;   // pinned, written by kernels: [0] LM-head status, [1] rows its fused form handed back
   Scratch lmh_logits;        // [B, V] f32 when rows need the unfused samplers
@@ -262,6 +266,27 @@ int ensure(Scratch& s, size_t bytes, char** errOut) {
   return GORCH_CUDA_OK;
 }
 
+// Grow-only pinned host memory of the context.
+int ensure_pinned(Ctx* c, size_t bytes, char** errOut) {
+  Scratch& s = c->pinned;
+  if (bytes <= s.cap) return GORCH_CUDA_OK;
+  if (s.ptr) {
+    CUDA_TRY(cudaFreeHost(s.ptr), errOut);
+    s.ptr = nullptr;
+    s.cap = 0;
+  }
+  const size_t want = bytes + (bytes >> 2) + 4096;
+  CUDA_TRY(cudaHostAlloc(&s.ptr, want, cudaHostAllocMapped | cudaHostAllocPortable), errOut);
+  s.cap = want;
+  return GORCH_CUDA_OK;
+}
+
+bool is_pinned(const void* p) {
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return false; }
+  return at.type == cudaMemoryTypeHost;
+}
+
 int check_shape(int dtype, int64_t B, int64_t V, int64_t row_stride, char** errOut) {
   if (dtype != GORCH_CUDA_F32 && dtype != GORCH_CUDA_BF16) {
     set_err(errOut, "gorch_cuda: unknown dtype %d", dtype);
@@ -297,6 +322,25 @@ static cudaError_t launch_narrow(Ctx* c, const gs::BatchArgs& ba, int dtype, int
   };
   if (dtype == GORCH_CUDA_F32) pick(float()); else pick(uint16_t());
   return cudaGetLastError();
+}
+
+// 16-byte vectors of a row, at most.
+int64_t row_vectors(int64_t V, int dtype) {
+  const int vec = dtype == GORCH_CUDA_F32 ? 4 : 8;
+  return (V + 2 * (vec - 1)) / vec + 1;
+}
+int64_t slice_bytes(int64_t V, int dtype, int C) { return ((row_vectors(V, dtype) + C - 1) / C) * 16; }
+
+// CTAs per row of the cluster kernel: the smallest power of two whose slice fits the shared-memory budget, raised for
+// small batches so that the whole GPU has work; 0 when no size keeps the row in shared memory.
+int cluster_size(const Ctx* c, int64_t B, int64_t V, int dtype) {
+  int C = 1;
+  while (C < gs::CL_MAX && slice_bytes(V, dtype, C) > kSliceCap) C *= 2;
+  // (two CTAs of this kernel fit an SM: stop while all clusters are still resident at once;
+  // measured on 64 rows of 50257 f32: 43 us with 4 CTAs per row, 55 us with 8)
+  while (C < gs::CL_MAX && B * 2 * C <= 2 * c->sm_count && row_vectors(V, dtype) / (2 * C) >= 64) C *= 2;
+  if (c->force_cluster) C = c->force_cluster;
+  return (slice_bytes(V, dtype, C) > kSliceCap || B * C > 0x7fffffffll) ? 0 : C;
 }
 
 int launch_rows(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int64_t row_stride,
@@ -395,18 +439,8 @@ int launch_rows(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int
     }
     CUDA_TRY(cudaGetLastError(), errOut);
   } else {
-    // Cluster size: smallest power of two whose slice fits the shared-memory
-    // budget, raised for small batches so that the whole GPU has work.
-    const int vec = dtype == GORCH_CUDA_F32 ? 4 : 8;
-    const int64_t nvec_max = (V + 2 * (vec - 1)) / vec + 1;
-    int C = 1;
-    while (C < gs::CL_MAX && ((nvec_max + C - 1) / C) * 16 > kSliceCap) C *= 2;
-    // (two CTAs of this kernel fit an SM: stop while all clusters are still resident at once;
-    // measured on 64 rows of 50257 f32: 43 us with 4 CTAs per row, 55 us with 8)
-    while (C < gs::CL_MAX && B * 2 * C <= 2 * c->sm_count && ((nvec_max + 2 * C - 1) / (2 * C)) >= 64) C *= 2;
-    if (c->force_cluster) C = c->force_cluster;
-    const int64_t need = ((nvec_max + C - 1) / C) * 16;
-    if (need > kSliceCap || B * C > 0x7fffffffll) {
+    const int C = cluster_size(c, B, V, dtype);
+    if (C == 0) {
       // rows too wide to keep in shared memory: the single-CTA kernel reads global memory
       dim3 grid(static_cast<unsigned>(B)), block(gs::NT);
       if (dtype == GORCH_CUDA_F32) {
@@ -418,6 +452,7 @@ int launch_rows(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int
     } else {
       gs::ClusterArgs ca;
       ca.k = a;
+      const int64_t need = slice_bytes(V, dtype, C);
       ca.slice_bytes = static_cast<int32_t>(need > gs::MIN_SLICE_BYTES ? need : gs::MIN_SLICE_BYTES);
       ca.eb_table = c->eb_table;
       const size_t dyn = static_cast<size_t>(ca.slice_bytes) + gs::REGION_A + gs::REGION_B;
@@ -488,31 +523,55 @@ int host_run(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int64_
   CUDA_TRY(cudaSetDevice(c->device), errOut);
   const size_t es = elem_size(dtype);
   const size_t lbytes = (static_cast<size_t>(B - 1) * row_stride + V) * es;
+  // Everything that is small goes through one pinned block of the context: the kernels read configurations and
+  // uniforms from it and leave ids and flags in it, so no copy but that of the logits is needed, and the
+  // call waits once. Logits of up to kStageBytes in pageable memory take the same way, a piece being copied into the block
+  // while the one before it crosses the link; larger ones are left to the driver.
+  const size_t off_flags = (static_cast<size_t>(B) * sizeof(int32_t) + 255) & ~static_cast<size_t>(255);
+  const size_t off_cfgs = (off_flags + static_cast<size_t>(B) * sizeof(uint32_t) + 255) & ~static_cast<size_t>(255);
+  const size_t off_uni = off_cfgs + static_cast<size_t>(B) * sizeof(GorchSampleCfg);
+  const size_t off_logits = (off_uni + static_cast<size_t>(B) * sizeof(double) + 255) & ~static_cast<size_t>(255);
+  const bool staged = lbytes <= kStageBytes && !is_pinned(logits);
+  if ((rc = ensure_pinned(c, off_logits + (staged ? lbytes : 0), errOut))) return rc;
+  unsigned char* pin = static_cast<unsigned char*>(c->pinned.ptr);
   if ((rc = ensure(c->st_logits, lbytes, errOut))) return rc;
-  if ((rc = ensure(c->st_ids, B * sizeof(int32_t), errOut))) return rc;
-  if ((rc = ensure(c->st_flags, B * sizeof(uint32_t), errOut))) return rc;
-  CUDA_TRY(cudaMemcpyAsync(c->st_logits.ptr, logits, lbytes, cudaMemcpyHostToDevice, c->stream), errOut);
-  c->counters.h2d_bytes += lbytes;
   if (!force_greedy) {
-    if ((rc = ensure(c->st_cfgs, B * sizeof(GorchSampleCfg), errOut))) return rc;
-    if ((rc = ensure(c->st_uniforms, B * sizeof(double), errOut))) return rc;
-    CUDA_TRY(cudaMemcpyAsync(c->st_cfgs.ptr, cfgs, B * sizeof(GorchSampleCfg), cudaMemcpyHostToDevice, c->stream), errOut);
-    CUDA_TRY(cudaMemcpyAsync(c->st_uniforms.ptr, uniforms, B * sizeof(double), cudaMemcpyHostToDevice, c->stream), errOut);
+    memcpy(pin + off_cfgs, cfgs, B * sizeof(GorchSampleCfg));
+    memcpy(pin + off_uni, uniforms, B * sizeof(double));
     c->counters.h2d_bytes += B * (sizeof(GorchSampleCfg) + sizeof(double));
   }
-  rc = launch_rows(c, c->st_logits.ptr, dtype, B, V, row_stride,
-                   static_cast<const GorchSampleCfg*>(c->st_cfgs.ptr),
-                   static_cast<const double*>(c->st_uniforms.ptr),
-                   static_cast<int32_t*>(c->st_ids.ptr), static_cast<uint32_t*>(c->st_flags.ptr),
-                   nullptr, nullptr, force_greedy, errOut);
+  const void* dev_logits = c->st_logits.ptr;
+  // The cluster kernel reads each logit once: it can do that from the pinned block, over the link (one GPT-2 row: 45 us a
+  // call, 53 with a copy to device memory first). Kernels that read a row again, and rows that need one, get the copy.
+  bool once = staged && c->variant == 0 && !use_batch_mode(B, V * static_cast<int64_t>(es)) && cluster_size(c, B, V, dtype) > 0;
+  if (!force_greedy) for (int64_t b = 0; b < B && once; b++) once = !(cfgs[b].top_k > gs::KFAST && cfgs[b].top_k < V);
+  if (once) {
+    memcpy(pin + off_logits, logits, lbytes);
+    dev_logits = pin + off_logits;
+  } else if (staged) {
+    for (size_t at = 0; at < lbytes; at += kStagePiece) {
+      const size_t n = lbytes - at < kStagePiece ? lbytes - at : kStagePiece;
+      memcpy(pin + off_logits + at, static_cast<const unsigned char*>(logits) + at, n);
+      CUDA_TRY(cudaMemcpyAsync(static_cast<unsigned char*>(c->st_logits.ptr) + at, pin + off_logits + at, n, cudaMemcpyHostToDevice, c->stream), errOut);
+    }
+  } else {
+    CUDA_TRY(cudaMemcpyAsync(c->st_logits.ptr, logits, lbytes, cudaMemcpyHostToDevice, c->stream), errOut);
+  }
+  c->counters.h2d_bytes += lbytes;
+  int32_t* pin_ids = reinterpret_cast<int32_t*>(pin);
+  uint32_t* pin_flags = reinterpret_cast<uint32_t*>(pin + off_flags);
+  rc = launch_rows(c, dev_logits, dtype, B, V, row_stride, reinterpret_cast<const GorchSampleCfg*>(pin + off_cfgs),
+                   reinterpret_cast<const double*>(pin + off_uni), pin_ids, out_flags ? pin_flags : nullptr, nullptr, nullptr, force_greedy, errOut);
+  // (also after an error: the block is the next call's, and copies out of it may be under way)
+  const cudaError_t waited = cudaStreamSynchronize(c->stream);
   if (rc) return rc;
-  CUDA_TRY(cudaMemcpyAsync(out_ids, c->st_ids.ptr, B * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream), errOut);
+  CUDA_TRY(waited, errOut);
+  memcpy(out_ids, pin_ids, B * sizeof(int32_t));
   c->counters.d2h_bytes += B * sizeof(int32_t);
   if (out_flags) {
-    CUDA_TRY(cudaMemcpyAsync(out_flags, c->st_flags.ptr, B * sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream), errOut);
+    memcpy(out_flags, pin_flags, B * sizeof(uint32_t));
     c->counters.d2h_bytes += B * sizeof(uint32_t);
   }
-  CUDA_TRY(cudaStreamSynchronize(c->stream), errOut);
   return GORCH_CUDA_OK;
 }
 
@@ -738,9 +797,8 @@ void gorch_cuda_release(GorchCudaCtxRef ctx) {
   if (!c) return;
   cudaSetDevice(c->device);
   if (c->own_stream) { cudaStreamSynchronize(c->own_stream); }
-  for (Scratch* s : {&c->st_logits, &c->st_cfgs, &c->st_uniforms, &c->st_ids, &c->st_flags}) {
-    if (s->ptr) cudaFree(s->ptr);
-  }
+  if (c->st_logits.ptr) cudaFree(c->st_logits.ptr);
+  if (c->pinned.ptr) cudaFreeHost(c->pinned.ptr);
   if (c->host_words) cudaFreeHost(c->host_words);
   if (c->exp_table) cudaFree(c->exp_table);
   if (c->eb_table) cudaFree(c->eb_table);

@@ -76,19 +76,16 @@ __device__ __forceinline__ uint32_t sample_threshold(F&& for_each_key, int r, ui
 // (the same ones on every call), n of them in the block. Every key lies in [lo, hi], except keys below lo that
 // are known not to be wanted; 256 buckets between the two are counted until the bucket of the top_k-th
 // largest holds few. Returns how many there are; more than KEEP_MAX (then they are not all there) only
-// when that many tie with the top_k-th. hist: 256 counters, bc: 3 ints.
+// when that many tie with the top_k-th. hist: 256 counters, bc: 3 ints. The caller has cleared hist and s_cnt, with
+// a barrier since.
 template <int NTHREADS, typename F>
 __device__ __forceinline__ int narrow_candidates(F&& for_each, int n, int topk, float Tm, uint32_t lo, uint32_t hi,
                                                  uint2* out, uint32_t* hist, int* bc, int* s_cnt, int tid) {
-  float smin = -INFINITY;                                      // scaled value of the lowest key that may be kept
-  __syncthreads();
-  if (tid == 0) *s_cnt = 0;
+  uint32_t low = 0u;                                           // the lowest key that may be kept
   if (n > topk) {
     int need = topk, above_all = 0;
     for (;;) {                                                 // uniform
       const int sh = max(0, 24 - __clz(hi - lo));              // 256 buckets
-      for (int j = tid; j < 256; j += NTHREADS) hist[j] = 0u;
-      __syncthreads();
       for_each([&](const uint2& e) {
         const uint32_t key = okey(__uint_as_float(e.x));
         if (key - lo <= hi - lo) atomicAdd(&hist[(hi - key) >> sh], 1u);
@@ -117,13 +114,17 @@ __device__ __forceinline__ int narrow_candidates(F&& for_each, int n, int topk, 
       above_all += bc[1];
       need -= bc[1];
       if (sh == 0 || above_all + bc[2] <= topk + 24) break;
+      __syncthreads();
+      for (int j = tid; j < 256; j += NTHREADS) hist[j] = 0u;
+      __syncthreads();
     }
-    smin = scale_t(okey_to_float(lo), Tm);
-  } else {
-    __syncthreads();
+    // Logits that the division by T makes equal to the bucket's lower edge belong to its class: the two keys below
+    // it, as long as quotients keep 24 bits; whatever has the same quotient otherwise.
+    const float edge = okey_to_float(lo), q = fabsf(scale_t(edge, Tm));
+    low = (q > 1e-30f && q < 1e30f) ? lo - 4u : okey(quotient_class_floor(edge, Tm));
   }
   for_each([&](const uint2& e) {
-    if (scale_t(__uint_as_float(e.x), Tm) >= smin) { const int slot = atomicAdd(s_cnt, 1); if (slot < KEEP_MAX) out[slot] = e; }
+    if (okey(__uint_as_float(e.x)) >= low) { const int slot = atomicAdd(s_cnt, 1); if (slot < KEEP_MAX) out[slot] = e; }
   });
   __syncthreads();
   return *s_cnt;
@@ -132,6 +133,10 @@ __device__ __forceinline__ int narrow_candidates(F&& for_each, int n, int topk, 
 template <int NTHREADS>
 __device__ __noinline__ int narrow_list(const uint2* list, int n, int topk, float Tm, uint32_t lo, uint32_t hi,
                                                  uint2* out, uint32_t* hist, int* bc, int* s_cnt, int tid) {
+  __syncthreads();
+  for (int j = tid; j < 256; j += NTHREADS) hist[j] = 0u;
+  if (tid == 0) *s_cnt = 0;
+  __syncthreads();
   return narrow_candidates<NTHREADS>([&](auto&& f) { for (int j = tid; j < n; j += NTHREADS) f(list[j]); },
                                      n, topk, Tm, lo, hi, out, hist, bc, s_cnt, tid);
 }
