@@ -624,11 +624,9 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
       for (int j = 0; j < PER; j++) {
         const int b = tid * PER + j;
         const double a_lo = ex_lo + lo_inc[j], a_hi = ex_hi + hi_inc[j];
-        const double r_hi = a_hi / (a_hi + (tot_lo - a_lo));   // largest possible mass fraction through bucket b
-        const double r_lo = a_lo / (a_lo + (tot_hi - a_hi));   // smallest possible
-        bool c1, c2;
-        if (mode == 0) { c1 = r_hi > plim * (1.0 - 1e-9); c2 = r_lo > plim * (1.0 + 1e-9); }
-        else           { c1 = r_hi >= plim * (1.0 - 1e-9); c2 = r_lo >= plim * (1.0 + 1e-9); }
+        // largest and smallest possible mass fraction through bucket b, against the limit
+        const double l_hi = plim * (1.0 - 1e-9) * (a_hi + (tot_lo - a_lo)), l_lo = plim * (1.0 + 1e-9) * (a_lo + (tot_hi - a_hi));
+        const bool c1 = (mode == 0) ? a_hi > l_hi : a_hi >= l_hi, c2 = (mode == 0) ? a_lo > l_lo : a_lo >= l_lo;
         if (c1) b1 = min(b1, b);
         if (c2) b2 = min(b2, b);
       }
@@ -652,6 +650,96 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
     stamp(3);
     cluster.sync();                                          // G3
     dA = X.dA; dB = X.dB; nzone = X.zone_total;
+    if (nzone > NT) {                                        // uniform over the cluster
+      // The counts alone leave an uncertain mass of some 3 % around the cut, and in a large or flat vocabulary
+      // that is more logits than the list holds. Now the zone's own range of d is cut into 1024 buckets, and the
+      // masses on either side of it are summed (f32 exponentials, good to 1e-6; the bounds allow 1e-5): the zone
+      // that remains is a few buckets, tens of logits. One more look at the slice (shared memory) and two more
+      // barriers, where the row used to be left to the single-CTA routine (151,936 logits, sigma 2, p = 0.9, eight
+      // CTAs: 376 us).
+      const uint32_t klo = (dA == INFINITY) ? 0u : dkey_of(dA) + 1u, khi = (dB == -INFINITY) ? 0x7f7fffffu : dkey_of(dB);
+      const int ksh = max(0, 22 - __clz(khi - klo));         // (khi - klo) >> ksh < 1024
+      uint32_t* fine = (rank == 0) ? reinterpret_cast<uint32_t*>(regA) : reinterpret_cast<uint32_t*>(regB);
+      __syncthreads();
+      for (int j = tid; j < NB1; j += NT) fine[j] = 0;
+      __syncthreads();
+      float ks = 0.f, zs = 0.f, ds = 0.f;
+      for (int j = tid; j < nv; j += NT) {
+        float x[VEC];
+        Elem<T>::unpack(slice[j], x);
+#pragma unroll
+        for (int c = 0; c < VEC; c++) {
+          const float d = (t_is_one ? x[c] : __fdiv_rn(x[c], Tm)) - m;
+          float e;
+          asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(d * 1.44269502162933349609375f));
+          if (d >= dA) ks += e;
+          else if (d >= dB && d > -INFINITY) { zs += e; atomicAdd(&fine[(dkey_of(d) - klo) >> ksh], 1u); }
+          else ds += e;
+        }
+      }
+      const double kw = warp_sum_d(ks), rw = warp_sum_d(static_cast<double>(zs) + ds);
+      if (lane == 0) { ctl.red_d[warp] = kw; ctl.red_d2[warp] = rw; }
+      __syncthreads();
+      if (warp == 0) {
+        const double kr = warp_sum_d(lane < NW ? ctl.red_d[lane] : 0.0), sr = warp_sum_d(lane < NW ? ctl.red_d2[lane] : 0.0);
+        if (lane == 0) { X0->K[rank] = kr; X0->Z[rank] = sr; }
+      }
+      if (rank != 0) {
+        uint32_t* dst = cluster.map_shared_rank(reinterpret_cast<uint32_t*>(regA), 0) + rank * NB1;
+        for (int j = tid; j < NB1; j += NT) dst[j] = fine[j];
+      }
+      cluster.sync();
+      if (rank == 0) {
+        const uint32_t* all = reinterpret_cast<const uint32_t*>(regA);
+        double K = 0.0, S = 0.0;
+        for (int r = 0; r < C; r++) { K += X.K[r]; S += X.K[r] + X.Z[r]; }
+        const double lim_lo = plim * S * (1.0 - 1e-5), lim_hi = plim * S * (1.0 + 1e-5);
+        constexpr int PER = NB1 / NT;
+        double lo_inc[PER], hi_inc[PER], slo = 0.0, shi = 0.0;
+        int cb[PER];
+        auto key_at = [&](int b) { return klo + (static_cast<uint32_t>(b) << ksh); };
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+          const int b = tid * PER + j;
+          uint32_t cnt = 0;
+          for (int r = 0; r < C; r++) cnt += all[r * NB1 + b];
+          cb[j] = static_cast<int>(cnt);
+          if (cnt) {
+            shi += cnt * exp_safe(-__uint_as_float(key_at(b)), s_tab);
+            slo += cnt * exp_safe(-__uint_as_float(min(key_at(b + 1) - 1u, khi)), s_tab);
+          }
+          lo_inc[j] = slo; hi_inc[j] = shi;
+        }
+        double ex_lo, ex_hi, tot_lo, tot_hi;
+        block_scan_excl_d2(slo, shi, ex_lo, ex_hi, tot_lo, tot_hi, ctl, tid);
+        int b1 = NB1 - 1, b2 = NB1 - 1;
+#pragma unroll
+        for (int j = PER - 1; j >= 0; j--) {
+          // largest and smallest possible mass through the bucket, against the limit
+          const double a_hi = K * (1.0 + 1e-5) + ex_hi + hi_inc[j], a_lo = K * (1.0 - 1e-5) + ex_lo + lo_inc[j];
+          const bool c1 = (mode == 0) ? a_hi > lim_lo : a_hi >= lim_lo, c2 = (mode == 0) ? a_lo > lim_hi : a_lo >= lim_hi;
+          if (c1) b1 = tid * PER + j;
+          if (c2) b2 = tid * PER + j;
+        }
+        block_min_i2(b1, b2, ctl, tid);
+        b2 = max(b1, b2);
+        int nz_part = 0;
+#pragma unroll
+        for (int j = 0; j < PER; j++) if (tid * PER + j >= b1 && tid * PER + j <= b2) nz_part += cb[j];
+        const int nz = block_sum_i(nz_part, ctl, tid);
+        if (tid == 0) {
+          const float tA = (key_at(b1) == 0u) ? INFINITY : -__uint_as_float(key_at(b1) - 1u);
+          const float tB = (b2 == NB1 - 1 || key_at(b2 + 1) > khi) ? dB : -__uint_as_float(key_at(b2 + 1) - 1u);
+          for (int r = 0; r < C; r++) {
+            Xchg* xr = cluster.map_shared_rank(&X, r);
+            xr->dA = tA; xr->dB = tB; xr->zone_total = nz;
+          }
+        }
+      }
+      cluster.sync();
+      dA = X.dA; dB = X.dB; nzone = X.zone_total;
+      stamp(7);
+    }
   }
   // the zone count includes masked lanes when the zone reaches the last bucket; they are never listed
   const bool zone_ok = nzone <= ZCAP + 2 * VEC;
@@ -728,10 +816,14 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
   // certainly-kept mass of this warp's run. With dA = +Inf nothing is certainly kept (exactly 0);
   // otherwise the row maximum is, and the subtraction's rounding is far below that mass.
   const double kw = (dA == INFINITY) ? 0.0 : tot_w - dsum - zsum;
-  if (lane == 0) s_kseg[warp] = kw;
-  const double Kr = block_sum_d(lane == 0 ? kw : 0.0, ctl, tid);
-  const double Dr = block_sum_d(lane == 0 ? dsum : 0.0, ctl, tid);
-  const double Zr = block_sum_d(lane == 0 ? zsum : 0.0, ctl, tid);
+  if (lane == 0) { s_kseg[warp] = kw; ctl.red_d[warp] = dsum; ctl.red_d2[warp] = zsum; }
+  __syncthreads();
+  double Kr = 0.0, Dr = 0.0, Zr = 0.0;                       // the slice's masses, in the first warp
+  if (warp == 0) {
+    Kr = warp_sum_d(lane < NW ? s_kseg[lane] : 0.0);
+    Dr = warp_sum_d(lane < NW ? ctl.red_d[lane] : 0.0);
+    Zr = warp_sum_d(lane < NW ? ctl.red_d2[lane] : 0.0);
+  }
   const int nz_cta = ctl.cand_count;
   // Rank r owns the sub-range [r*ZCAP/C, (r+1)*ZCAP/C) of rank 0's region A.
   const int zcap_r = ZCAP / C;
@@ -776,16 +868,19 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
       if (Ktot > 0.0 && crossed(Ktot)) bad = 1;              // the bracket was wrong
       double* sm = reinterpret_cast<double*>(regB);           // [NSUB] mass per sub-bucket
       int* sc = reinterpret_cast<int*>(regB + 8192);          // [NSUB] count per sub-bucket
+      const bool few_keys = nz <= NT;                          // uniform
       unsigned long long lo = ~0ull, hi = 0ull;
-      for (int t = tid; t < ZCAP; t += NT) {
-        if (zlive(t)) { const unsigned long long k = zk[t]; lo = k < lo ? k : lo; hi = k > hi ? k : hi; }
+      if (!few_keys) {
+        for (int t = tid; t < ZCAP; t += NT) {
+          if (zlive(t)) { const unsigned long long k = zk[t]; lo = k < lo ? k : lo; hi = k > hi ? k : hi; }
+        }
+        lo = block_min_u64(lo, ctl, tid);
+        hi = block_max_u64(hi, ctl, tid);
       }
-      lo = block_min_u64(lo, ctl, tid);
-      hi = block_max_u64(hi, ctl, tid);
       double gbase = Ktot;                                     // Ktot + mass of keys below lo; never crossed
       int inrange = nz;
       bool all_in = false;
-      for (int iter = 0; iter < 8 && inrange > 32 && !bad && !all_in; iter++) {
+      for (int iter = 0; iter < 8 && !few_keys && inrange > 32 && !bad && !all_in; iter++) {
         const unsigned long long span = hi - lo;
         int sh = 0;
         while (sh < 63 && (span >> sh) >= static_cast<unsigned long long>(NSUB)) sh++;
@@ -830,10 +925,47 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
         if (nhi < nlo || nhi > hi) nhi = hi;
         lo = nlo; hi = nhi;
       }
-      if (inrange > 32 && !all_in) bad = 1;
+      if (!few_keys && inrange > 32 && !all_in) bad = 1;
       double g_at = gbase;                                     // G(c*) and G just before c*
       double g_before = gbase;
-      if (!bad && !all_in) {
+      if (few_keys && !bad) {
+        // Every key adds up the masses that come no later than its own, all at once: a few thousand cycles
+        // for some hundred keys, where narrowing the range takes several rounds of barriers and f64
+        // atomics (151,936 logits, sigma 2, p = 0.9, mode B: 31,000 cycles, 16 us).
+        unsigned long long* zkeys = reinterpret_cast<unsigned long long*>(regB);
+        double* zmass = reinterpret_cast<double*>(regB + 8 * NT);
+        __syncthreads();
+        if (tid == 0) ctl.cand_count = 0;
+        __syncthreads();
+        for (int t = tid; t < ZCAP; t += NT) {
+          if (zlive(t)) { const int slot = atomicAdd(&ctl.cand_count, 1); const unsigned long long k = zk[t]; zkeys[slot] = k; zmass[slot] = exp_safe(zone_key_d(k), s_tab); }
+        }
+        __syncthreads();
+        const unsigned long long k = (tid < nz) ? zkeys[tid] : ~0ull;
+        double g = 0.0, g2 = 0.0;
+        if (tid < nz) {
+          int l = 0;
+#pragma unroll 2
+          for (; l + 1 < nz; l += 2) {
+            g += (zkeys[l] <= k) ? zmass[l] : 0.0;
+            g2 += (zkeys[l + 1] <= k) ? zmass[l + 1] : 0.0;
+          }
+          if (l < nz) g += (zkeys[l] <= k) ? zmass[l] : 0.0;
+          g = Ktot + (g + g2);
+        }
+        const bool cr = tid < nz && crossed(g);
+        const unsigned long long cstar = block_min_u64(cr ? k : ~0ull, ctl, tid);
+        if (cr && k == cstar) { ctl.bcast_d[1] = g; ctl.bcast_d[2] = g - zmass[tid]; }   // keys are distinct
+        __syncthreads();
+        if (cstar != ~0ull) {
+          g_at = ctl.bcast_d[1];
+          g_before = ctl.bcast_d[2];
+          cut_key = cstar;
+          cut_incl = (mode == 0) ? 0 : 1;
+        } else {
+          all_in = true;                                       // nothing in the zone crosses
+        }
+      } else if (!bad && !all_in) {
         unsigned long long* few = reinterpret_cast<unsigned long long*>(regB);   // [32]
         __syncthreads();
         if (tid == 0) ctl.cand_count = 0;

@@ -215,6 +215,24 @@ def test_c5_rows(sampler, oracle):
     run_both(sampler, oracle, w.logits, w.cfgs, w.uniforms, fast=True, allow_tie_cut=True)
 
 
+# (mode A on short rows: the oracle removes one token at a time)
+@pytest.mark.parametrize("V,dtype,mode", [(9001, "f32", MODE_A), (9001, "bf16", MODE_A), (50257, "f32", MODE_B),
+                                          (151936, "f32", MODE_B), (151936, "bf16", MODE_B)])
+def test_top_p_cut_among_many_equal_logits(sampler, oracle, V, dtype, mode):
+    """Rows whose cut lies among thousands of logits that counts alone cannot separate: the zone around it is
+    counted again in finer buckets. Flat and steep rows, cuts near either end, a masked tail, temperatures."""
+    rng = np.random.default_rng(V + mode)
+    sigmas = [0.02, 0.25, 0.25, 2.0, 2.0, 2.0, 12.0, 0.25]
+    x = np.stack([rng.standard_normal(V).astype(np.float32) * np.float32(s) for s in sigmas])
+    x[7, V // 2:] = -np.inf
+    if dtype == "bf16":
+        x = (x.view(np.uint32) >> 16).astype(np.uint16)
+    cfgs = cfgs_of(8, 1.0, 0, 0.0, mode)
+    cfgs["temperature"] = [1.0, 1.0, 0.7, 1.0, 0.7, 1.3, 1.0, 1.0]
+    cfgs["top_p"] = np.array([0.9, 0.01, 0.9, 0.9, 0.5, 0.99, 0.99999, 0.97], dtype=np.float32) / (1.5 if mode == MODE_A else 1.0)
+    run_both(sampler, oracle, x, cfgs, rng.random(8), allow_tie_cut=True)
+
+
 def test_host_entry_matches_device_entry(sampler):
     w = workloads.mixed_rows(64)
     ids, flags = sampler.sample_batch(w.logits, w.cfgs, w.uniforms)
