@@ -68,7 +68,7 @@ __device__ __forceinline__ double vs_exp(float d, const double* __restrict__ eb,
 struct BatchArgs {
   KernelArgs k;
   const double* eb_table;   // 1024 doubles: exp(-b/32)
-  int32_t* hdr;             // [2] narrow kernel's row cursor, [3] wide kernel's row cursor
+  int32_t* hdr;             // HDR_NARROW, HDR_WIDE: the kernels' row cursors
   int32_t* list_single;     // [0] = count, [1..] rows for the single-CTA kernel
   int64_t B;
 };

@@ -53,6 +53,7 @@ struct KernelArgs {
   const double* exp_table; // 256 doubles: 2^(j/256)
   int64_t row_offset;      // first row handled by this launch (for chunked launches)
   const int32_t* worklist; // single-CTA kernel only: [0] = count, [1..] = rows to process (null: every row)
+  int32_t* batch_hdr;      // set for the last kernel of a sorted batch: the header that it leaves cleared (see leave_batch)
   void* vs_records;        // vocab-sharded local pass (narrow kernel only): [B] VsRecord to fill instead of drawing
   int32_t vs_col_offset;   // global index of this slice's first column
   int32_t vs_cand;         // candidates per record (records are 16 + 8 * vs_cand bytes apart), at most VS_CAND
@@ -1233,15 +1234,34 @@ __device__ __noinline__ void single_cta_row(const KernelArgs& A, const int64_t r
 }
 
 // One CTA per row; with a work list, a fixed grid walks the listed rows.
+// Programmatic dependent launch: wait for the kernel before this one in the stream; let the next one start.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Header of a sorted batch: row cursors and the count of handed-over rows (BatchArgs). Every call finds it cleared: the
+// last CTA of the call's last kernel leaves it so, which a memset before the call's first kernel did at the price
+// of one more step on the GPU's queue (about 2 us).
+constexpr int HDR_NARROW = 2, HDR_WIDE = 3, HDR_LEFT = 4, HDR_COUNT = 15;
+__device__ __forceinline__ void leave_batch(int32_t* hdr) {
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicInc(reinterpret_cast<unsigned*>(hdr + HDR_LEFT), gridDim.x - 1) == gridDim.x - 1) {   // (and wraps to 0)
+      hdr[HDR_NARROW] = 0; hdr[HDR_WIDE] = 0; hdr[HDR_COUNT] = 0;
+    }
+  }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(NT, 2) sample_rows_kernel(const __grid_constant__ KernelArgs A) {
   extern __shared__ __align__(16) unsigned char pool[];
+  pdl_wait();                                                // the kernels that hand rows over
   if (A.worklist) {
     const int n = A.worklist[0];
     for (int w = blockIdx.x; w < n; w += gridDim.x) {
       single_cta_row<T>(A, A.worklist[1 + w], pool);
       __syncthreads();
     }
+    if (A.batch_hdr) leave_batch(A.batch_hdr);
   } else {
     const int64_t row = A.row_offset + blockIdx.x;
     if (A.row_done && A.row_done[row] != 0) return;        // the sequence has ended (model/generate.go:82-84)

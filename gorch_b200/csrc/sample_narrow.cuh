@@ -539,6 +539,7 @@ __global__ void __launch_bounds__(N_NT, N_CTAS_PER_SM) narrow_rows_kernel(const 
   __shared__ float s_thr;
   __shared__ int s_flag;
   __shared__ int s_row;
+  pdl_launch();                                              // the hand-over kernel, which waits for this one's end
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -549,7 +550,7 @@ __global__ void __launch_bounds__(N_NT, N_CTAS_PER_SM) narrow_rows_kernel(const 
       // the step; the second gains nothing.)
       int w;
       for (;;) {
-        w = atomicAdd(&BA.hdr[2], 1);
+        w = atomicAdd(&BA.hdr[HDR_NARROW], 1);
         if (w >= BA.B) { w = -1; break; }
         const int kind = row_kind(BA.k, w);
         if (kind == 0) break;
@@ -568,6 +569,9 @@ __global__ void __launch_bounds__(N_NT, N_CTAS_PER_SM) narrow_rows_kernel(const 
       __syncthreads();
     }
   }
+  // Whoever waits for this kernel waits for the one it was launched beside, too: one CTA sees to that.
+  if (blockIdx.x == 0) pdl_wait();
+  if (BA.k.batch_hdr) leave_batch(BA.k.batch_hdr);
 }
 
 }  // namespace GS_N_NS

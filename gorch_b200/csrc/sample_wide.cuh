@@ -1493,7 +1493,7 @@ __global__ void __launch_bounds__(W_NT, W_CTAS) wide_rows_kernel(BatchArgs BA) {
     if (threadIdx.x == 0) {
       int w;                                                 // next row of this kernel's kind
       for (;;) {
-        w = atomicAdd(&BA.hdr[3], 1);
+        w = atomicAdd(&BA.hdr[HDR_WIDE], 1);
         if (w >= BA.B) { w = -1; break; }
         if (row_kind(BA.k, w) == 1) break;
       }
@@ -1502,6 +1502,9 @@ __global__ void __launch_bounds__(W_NT, W_CTAS) wide_rows_kernel(BatchArgs BA) {
     __syncthreads();
     const int row = sh.row;
     if (row < 0) break;
+    // The narrow kernel may start: every CTA of this one has a row, or has gone. (Started together, the two kernels'
+    // CTAs mix at random, and some SMs end up with more rows of this kind than others.)
+    pdl_launch();
     wide_row<T>(BA, row, dyn, sh, pol_keep, pol_drop);
   }
 }

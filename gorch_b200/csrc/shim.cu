@@ -127,11 +127,9 @@ struct Ctx {
   int64_t l2_bytes = 126ll << 20;
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
-  cudaStream_t side_stream = nullptr;     // the wide kernel of a mixed batch runs here, beside the narrow one
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   double* exp_table = nullptr;
   double* eb_table = nullptr;
-  Scratch worklist;        // int32[1 + rows]: rows the cluster kernel leaves to the single-CTA kernel
+  Scratch worklist;        // int32[16 + rows + 1]: header of a sorted batch, rows that its kernels leave to the single-CTA kernel
   Scratch st_logits;       // logits of the host-memory calls
   Scratch pinned;          // host memory: their configurations, uniforms, ids, flags, and logits on their way
   Scratch lmh_scratch;       // thresholds, candidate lists, sample logits of the LM-head path
@@ -306,22 +304,50 @@ int check_shape(int dtype, int64_t B, int64_t V, int64_t row_stride, char** errO
 
 size_t elem_size(int dtype) { return dtype == GORCH_CUDA_BF16 ? 2 : 4; }
 
+// A launch on the context's stream; dependent: it may start while the kernel before it runs, and waits for
+// that itself (griddepcontrol.wait) where it needs what it wrote.
+template <typename... P, typename... A>
+cudaError_t launch(Ctx* c, void (*kernel)(P...), unsigned grid, unsigned block, size_t dyn, bool dependent, const A&... args) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(grid);
+  lc.blockDim = dim3(block);
+  lc.dynamicSmemBytes = dyn;
+  lc.stream = c->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = dependent ? 1 : 0;
+  return cudaLaunchKernelEx(&lc, kernel, args...);
+}
+
+// The context's row work lists of a sorted batch: 16 header words, all zero between calls, and B + 1 for the rows.
+int batch_lists(Ctx* c, int64_t B, int32_t** base, char** errOut) {
+  const size_t had = c->worklist.cap;
+  int rc = ensure(c->worklist, (16 + static_cast<size_t>(B) + 1) * sizeof(int32_t), errOut);
+  if (rc) return rc;
+  *base = static_cast<int32_t*>(c->worklist.ptr);
+  if (c->worklist.cap != had) CUDA_TRY(cudaMemsetAsync(*base, 0, 16 * sizeof(int32_t), c->stream), errOut);
+  return GORCH_CUDA_OK;
+}
+
 // The narrow kernel's two instances: 256-thread CTAs (five per SM) while every row gets a CTA slot
 // of its own, 128-thread CTAs (eight per SM) beyond that. Variants 6 / 7 force one of them (tests).
-static cudaError_t launch_narrow(Ctx* c, const gs::BatchArgs& ba, int dtype, int64_t B) {
+static cudaError_t launch_narrow(Ctx* c, const gs::BatchArgs& ba, int dtype, int64_t B, bool dependent) {
   const int64_t slots256 = static_cast<int64_t>(gs::n256::N_CTAS_PER_SM) * c->sm_count;
   const bool small_ctas = c->variant == 6 || (c->variant != 7 && B > slots256);
   const int64_t slots = small_ctas ? static_cast<int64_t>(gs::n128::N_CTAS_PER_SM) * c->sm_count : slots256;
   const unsigned g = static_cast<unsigned>(B < slots ? B : slots);
   const bool diag = ba.k.out_probs || ba.k.out_debug;
-  auto go = [&](auto kernel, int nt, int bytes) { kernel<<<g, nt, bytes, c->stream>>>(ba); };
+  cudaError_t e = cudaSuccess;
+  auto go = [&](auto kernel, int nt, int bytes) { e = launch(c, kernel, g, nt, bytes, dependent, ba); };
   auto pick = [&](auto type) {
     typedef decltype(type) E;
     if (small_ctas) go(diag ? gs::n128::narrow_rows_kernel<E, true> : gs::n128::narrow_rows_kernel<E, false>, gs::n128::N_NT, gs::n128::N_DYN_BYTES);
     else go(diag ? gs::n256::narrow_rows_kernel<E, true> : gs::n256::narrow_rows_kernel<E, false>, gs::n256::N_NT, gs::n256::N_DYN_BYTES);
   };
   if (dtype == GORCH_CUDA_F32) pick(float()); else pick(uint16_t());
-  return cudaGetLastError();
+  return e;
 }
 
 // 16-byte vectors of a row, at most.
@@ -370,6 +396,7 @@ int launch_rows(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int
   a.exp_table = c->exp_table;
   a.row_offset = 0;
   a.worklist = nullptr;
+  a.batch_hdr = nullptr;
   a.vs_records = nullptr;
   a.vs_col_offset = 0;
   a.vs_cand = gs::VS_CAND;
@@ -382,22 +409,18 @@ int launch_rows(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int
   int klaunch = 1;
   const bool batch_mode = c->variant == 2 || c->variant >= 4 || (c->variant == 0 && use_batch_mode(B, V * static_cast<int64_t>(elem_size(dtype))));
   if (batch_mode) {
-    // narrow (greedy / top-k) beside wide (top-k off), then single-CTA (whatever was handed over)
-    const size_t ints = 16 + static_cast<size_t>(B) + 1;
+    // wide (top-k off) with narrow (greedy / top-k) beside it, then single-CTA (whatever was handed over): one stream, each
+    // launched while the one before it runs (programmatic dependent launch). The wide kernel goes first and lets the
+    // narrow one start when its CTAs have their rows; the narrow kernel ends after the wide one; the third waits for that.
     int32_t* base = fixed_lists;
-    if (!base) {
-      int rc = ensure(c->worklist, ints * sizeof(int32_t), errOut);
-      if (rc) return rc;
-      base = static_cast<int32_t*>(c->worklist.ptr);
-    }
+    if (base) CUDA_TRY(cudaMemsetAsync(base, 0, 16 * sizeof(int32_t), c->stream), errOut);   // (shared by the contexts of a device)
+    else if (int rc = batch_lists(c, B, &base, errOut)) return rc;
     gs::BatchArgs ba;
     ba.k = a;
     ba.eb_table = c->eb_table;
     ba.hdr = base;
-    // the hand-over list's count is the header's last word, its rows follow: one memset clears all
-    ba.list_single = base + 15;
+    ba.list_single = base + gs::HDR_COUNT;
     ba.B = B;
-    CUDA_TRY(cudaMemsetAsync(base, 0, 16 * sizeof(int32_t), c->stream), errOut);
     // at most one row per SM: a 1024-thread CTA finishes its row sooner than a 256-thread one, and no SM
     // would have held a second row anyway. Beyond that the 256-thread instance wins (measured), also
     // because a 1024-thread CTA takes the whole register file and keeps the narrow kernel off its SM
@@ -407,28 +430,18 @@ int launch_rows(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int
     const unsigned gsgl = static_cast<unsigned>(B < 2 * c->sm_count ? B : 2 * c->sm_count);
     gs::KernelArgs aw = a;
     aw.worklist = ba.list_single;
-    // The narrow and the wide kernel work on disjoint rows: the wide one runs on a side stream
-    // (fork before, join before the hand-over kernel), so that a mixed batch
-    // does not pay for them one after the other.
+    aw.batch_hdr = base;
+    if (force_greedy) ba.k.batch_hdr = base;
+    const bool f32 = dtype == GORCH_CUDA_F32;
+    cudaError_t e = cudaSuccess;
     if (!force_greedy) {
-      CUDA_TRY(cudaEventRecord(c->ev_fork, c->stream), errOut);
-      CUDA_TRY(cudaStreamWaitEvent(c->side_stream, c->ev_fork, 0), errOut);
-      if (dtype == GORCH_CUDA_F32) {
-        if (wide_big_ctas) gs::w1024::wide_rows_kernel<float><<<gw, gs::w1024::W_NT, gs::w1024::W_DYN_BYTES, c->side_stream>>>(ba);
-        else gs::w256::wide_rows_kernel<float><<<gw, gs::w256::W_NT, gs::w256::W_DYN_BYTES, c->side_stream>>>(ba);
-      } else {
-        if (wide_big_ctas) gs::w1024::wide_rows_kernel<uint16_t><<<gw, gs::w1024::W_NT, gs::w1024::W_DYN_BYTES, c->side_stream>>>(ba);
-        else gs::w256::wide_rows_kernel<uint16_t><<<gw, gs::w256::W_NT, gs::w256::W_DYN_BYTES, c->side_stream>>>(ba);
-      }
+      if (wide_big_ctas) e = launch(c, f32 ? gs::w1024::wide_rows_kernel<float> : gs::w1024::wide_rows_kernel<uint16_t>, gw, gs::w1024::W_NT, gs::w1024::W_DYN_BYTES, false, ba);
+      else e = launch(c, f32 ? gs::w256::wide_rows_kernel<float> : gs::w256::wide_rows_kernel<uint16_t>, gw, gs::w256::W_NT, gs::w256::W_DYN_BYTES, false, ba);
     }
-    CUDA_TRY(launch_narrow(c, ba, dtype, B), errOut);
-    if (!force_greedy) {
-      CUDA_TRY(cudaEventRecord(c->ev_join, c->side_stream), errOut);
-      CUDA_TRY(cudaStreamWaitEvent(c->stream, c->ev_join, 0), errOut);
-      if (dtype == GORCH_CUDA_F32) gs::sample_rows_kernel<float><<<gsgl, gs::NT, gs::POOL_BYTES, c->stream>>>(aw);
-      else gs::sample_rows_kernel<uint16_t><<<gsgl, gs::NT, gs::POOL_BYTES, c->stream>>>(aw);
-    }
-    CUDA_TRY(cudaGetLastError(), errOut);
+    if (e == cudaSuccess) e = launch_narrow(c, ba, dtype, B, !force_greedy);
+    if (e == cudaSuccess && !force_greedy) e = launch(c, f32 ? gs::sample_rows_kernel<float> : gs::sample_rows_kernel<uint16_t>, gsgl, gs::NT, gs::POOL_BYTES, true, aw);
+    if (e != cudaSuccess) { cudaGetLastError(); cudaMemsetAsync(base, 0, 16 * sizeof(int32_t), c->stream); }   // nobody has left the header cleared
+    CUDA_TRY(e, errOut);
     klaunch = force_greedy ? 1 : 3;
   } else if (c->variant == 1) {
     dim3 grid(static_cast<unsigned>(B)), block(gs::NT);
@@ -573,23 +586,6 @@ int host_run(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int64_
     c->counters.d2h_bytes += B * sizeof(uint32_t);
   }
   return GORCH_CUDA_OK;
-}
-
-// A launch on the context's stream; dependent: it may start while the kernel before it runs, and waits for
-// that itself (griddepcontrol.wait) where it needs what it wrote.
-template <typename... P, typename... A>
-cudaError_t launch(Ctx* c, void (*kernel)(P...), unsigned grid, unsigned block, size_t dyn, bool dependent, const A&... args) {
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(grid);
-  lc.blockDim = dim3(block);
-  lc.dynamicSmemBytes = dyn;
-  lc.stream = c->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  lc.attrs = at;
-  lc.numAttrs = dependent ? 1 : 0;
-  return cudaLaunchKernelEx(&lc, kernel, args...);
 }
 
 // ---- LM-head projection (lm_head.cuh) ----
@@ -738,9 +734,6 @@ GorchCudaCtxRef gorch_cuda_create_ctx(int device, char** errOut) {
   if (prop.l2CacheSize > 0) c->l2_bytes = prop.l2CacheSize;
   if ((e = cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking)) != cudaSuccess) return fail("cudaStreamCreate", e);
   c->stream = c->own_stream;
-  if ((e = cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking)) != cudaSuccess) return fail("cudaStreamCreate", e);
-  if ((e = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming)) != cudaSuccess) return fail("cudaEventCreate", e);
-  if ((e = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming)) != cudaSuccess) return fail("cudaEventCreate", e);
   if ((e = cudaEventCreate(&c->ev0)) != cudaSuccess) return fail("cudaEventCreate", e);
   if ((e = cudaEventCreate(&c->ev1)) != cudaSuccess) return fail("cudaEventCreate", e);
   {
@@ -815,9 +808,6 @@ void gorch_cuda_release(GorchCudaCtxRef ctx) {
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
-  if (c->side_stream) cudaStreamDestroy(c->side_stream);
-  if (c->ev_fork) cudaEventDestroy(c->ev_fork);
-  if (c->ev_join) cudaEventDestroy(c->ev_join);
   g_pool.leave();
   delete c;
 }
@@ -974,23 +964,20 @@ static int vocab_local_launch(Ctx* c, const void* logits, int dtype, int64_t B, 
   }
   CUDA_TRY(cudaSetDevice(c->device), errOut);
   // every row goes through the narrow kernel (row_kind says so when vs_records is set)
-  const size_t ints = 16 + static_cast<size_t>(B) + 1;
-  rc = ensure(c->worklist, ints * sizeof(int32_t), errOut);
-  if (rc) return rc;
-  int32_t* base = static_cast<int32_t*>(c->worklist.ptr);
+  int32_t* base = nullptr;
+  if ((rc = batch_lists(c, B, &base, errOut))) return rc;
   gs::BatchArgs ba;
   ba.k.logits = logits; ba.k.row_stride = row_stride; ba.k.V = static_cast<int32_t>(Vslice);
   ba.k.force_greedy = 0; ba.k.cfgs = reinterpret_cast<const gs::RowCfg*>(cfgs); ba.k.uniforms = nullptr;
   ba.k.out_ids = nullptr; ba.k.out_flags = nullptr; ba.k.out_probs = nullptr; ba.k.out_debug = nullptr;
-  ba.k.exp_table = c->exp_table; ba.k.row_offset = 0; ba.k.worklist = nullptr;
+  ba.k.exp_table = c->exp_table; ba.k.row_offset = 0; ba.k.worklist = nullptr; ba.k.batch_hdr = base;
   ba.k.vs_records = records; ba.k.vs_col_offset = static_cast<int32_t>(col_offset); ba.k.vs_cand = cand;
   ba.k.vs_sumexp = sumexp_rows ? 1 : 0;
   ba.k.tk_values = nullptr; ba.k.tk_indices = nullptr; ba.k.tk_k = 0; ba.k.row_done = nullptr;
   ba.eb_table = c->eb_table;
-  ba.hdr = base; ba.list_single = base + 15;
+  ba.hdr = base; ba.list_single = base + gs::HDR_COUNT;
   ba.B = B;
-  CUDA_TRY(cudaMemsetAsync(base, 0, 16 * sizeof(int32_t), c->stream), errOut);
-  CUDA_TRY(launch_narrow(c, ba, dtype, B), errOut);
+  CUDA_TRY(launch_narrow(c, ba, dtype, B, false), errOut);
   c->counters.kernel_launches += 1;
   if (sumexp_rows) {                                         // the records of rows without top-k: disjoint rows, same stream
     const unsigned g = static_cast<unsigned>(B < 4 * c->sm_count ? B : 4 * c->sm_count);
@@ -1018,7 +1005,7 @@ static int vocab_merge_launch(Ctx* c, const void* all_records, int nranks, int c
   m.k.logits = nullptr; m.k.row_stride = V; m.k.V = static_cast<int32_t>(V); m.k.force_greedy = 0;
   m.k.cfgs = reinterpret_cast<const gs::RowCfg*>(cfgs); m.k.uniforms = uniforms;
   m.k.out_ids = out_ids; m.k.out_flags = out_flags; m.k.out_probs = nullptr; m.k.out_debug = nullptr;
-  m.k.exp_table = c->exp_table; m.k.row_offset = 0; m.k.worklist = nullptr; m.k.vs_records = nullptr; m.k.vs_col_offset = 0;
+  m.k.exp_table = c->exp_table; m.k.row_offset = 0; m.k.worklist = nullptr; m.k.batch_hdr = nullptr; m.k.vs_records = nullptr; m.k.vs_col_offset = 0;
   m.k.vs_cand = cand;
   m.k.vs_sumexp = 0;
   m.k.tk_values = nullptr; m.k.tk_indices = nullptr; m.k.tk_k = 0; m.k.row_done = nullptr;
@@ -1289,22 +1276,19 @@ int gorch_cuda_topk_dev(GorchCudaCtxRef ctx, const void* x, int dtype, int64_t B
     c->counters.kernel_launches += 1;
     return GORCH_CUDA_OK;
   }
-  const size_t ints = 16 + static_cast<size_t>(B) + 1;
-  rc = ensure(c->worklist, ints * sizeof(int32_t), errOut);
-  if (rc) return rc;
-  int32_t* base = static_cast<int32_t*>(c->worklist.ptr);
+  int32_t* base = nullptr;
+  if ((rc = batch_lists(c, B, &base, errOut))) return rc;
   gs::BatchArgs ba;
   ba.k.logits = x; ba.k.row_stride = row_stride; ba.k.V = static_cast<int32_t>(V);
   ba.k.force_greedy = 0; ba.k.cfgs = nullptr; ba.k.uniforms = nullptr;
   ba.k.out_ids = nullptr; ba.k.out_flags = out_flags; ba.k.out_probs = nullptr; ba.k.out_debug = nullptr;
-  ba.k.exp_table = c->exp_table; ba.k.row_offset = 0; ba.k.worklist = nullptr;
+  ba.k.exp_table = c->exp_table; ba.k.row_offset = 0; ba.k.worklist = nullptr; ba.k.batch_hdr = base;
   ba.k.vs_records = nullptr; ba.k.vs_col_offset = 0; ba.k.vs_sumexp = 0;
   ba.k.tk_values = out_values; ba.k.tk_indices = out_indices; ba.k.tk_k = static_cast<int32_t>(k); ba.k.row_done = nullptr;
   ba.eb_table = c->eb_table;
-  ba.hdr = base; ba.list_single = base + 15;
+  ba.hdr = base; ba.list_single = base + gs::HDR_COUNT;
   ba.B = B;
-  CUDA_TRY(cudaMemsetAsync(base, 0, 16 * sizeof(int32_t), c->stream), errOut);
-  CUDA_TRY(launch_narrow(c, ba, dtype, B), errOut);
+  CUDA_TRY(launch_narrow(c, ba, dtype, B, false), errOut);
   CUDA_TRY(cudaGetLastError(), errOut);
   c->counters.kernel_launches += 1;
   return GORCH_CUDA_OK;

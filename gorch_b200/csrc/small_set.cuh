@@ -18,10 +18,6 @@ namespace gs {
 constexpr int KEEP_MAX = 512;        // largest kept set finished in shared memory
 constexpr int SS_WORK_BYTES = 13344; // work arrays of finish_small_set
 
-// Programmatic dependent launch: wait for the kernel before this one in the stream; let the next one start.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // Lower edge of a narrow bucket of order keys that holds the r-th largest key of a sample (every thread calls
 // f(key) for its keys, the same ones on every call); tmax: the largest of the thread's own keys, tmin: the
 // smallest. cnts: NBINS counters. Buckets of equal width are counted until the one of the r-th largest
