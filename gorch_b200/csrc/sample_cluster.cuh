@@ -204,6 +204,17 @@ template <> __device__ __forceinline__ float vec_max_nan<uint16_t>(const uint4& 
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(m) : "f"(__uint_as_float(p << 16)), "f"(__uint_as_float(p & 0xffff0000u)));
   return m;
 }
+// Maximum of a vector's logits; a NaN counts as less than anything else.
+template <typename T> __device__ __forceinline__ float vec_max(const uint4& a);
+template <> __device__ __forceinline__ float vec_max<float>(const uint4& a) {
+  return fmaxf(fmaxf(__uint_as_float(a.x), __uint_as_float(a.y)), fmaxf(__uint_as_float(a.z), __uint_as_float(a.w)));
+}
+template <> __device__ __forceinline__ float vec_max<uint16_t>(const uint4& a) {
+  uint32_t p;
+  asm("{\n\t.reg .b32 t, u;\n\tmax.bf16x2 t, %1, %2;\n\tmax.bf16x2 u, %3, %4;\n\tmax.bf16x2 %0, t, u;\n\t}"
+      : "=r"(p) : "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w));
+  return fmaxf(__uint_as_float(p << 16), __uint_as_float(p & 0xffff0000u));
+}
 template <typename T>
 __device__ __forceinline__ uint4 load_masked(const RowView<T>& rv, int v, float& vmax, float& vmin, bool& nan_seen) {
   return mask_and_stats(rv, v, __ldg(rv.vbase + v), vmax, vmin, nan_seen);
@@ -329,15 +340,15 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
 
   // ================================================================ greedy
   if (Tm == 0.0f) {
-    unsigned long long best = 0ull;
+    // per vector a maximum and one compare (a NaN is not seen); the place within the vector at the end
+    float top = -INFINITY;
+    int tv = 0;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     for (int j = tid; j < nv; j += NT) {
-      rv.visit_raw(slice[j], v0 + j, [&](float x, int i, int) {
-        unsigned long long p = (static_cast<unsigned long long>(okey(x)) << 32) |
-                               static_cast<uint32_t>(~static_cast<uint32_t>(i));
-        best = p > best ? p : best;
-      });
+      const float x = vec_max<T>(mask_edges(rv, v0 + j, slice[j]));
+      if (x > top) { top = x; tv = v0 + j; }
     }
+    unsigned long long best = (top > -INFINITY) ? (static_cast<unsigned long long>(okey(top)) << 32) | static_cast<uint32_t>(~static_cast<uint32_t>(tv)) : 0ull;
     best = block_max_u64(best, ctl, tid);
     fill_probs_slice(0.0);
     cluster.barrier_wait();
@@ -346,7 +357,10 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
     if (rank == 0) {
       unsigned long long b = 0;
       for (int r = 0; r < C; r++) b = X.u64[r] > b ? X.u64[r] : b;
-      int id = static_cast<int>(~static_cast<uint32_t>(b & 0xffffffffull));
+      int id = 0x7fffffff;
+      if (b != 0ull)
+        rv.visit(static_cast<int>(~static_cast<uint32_t>(b & 0xffffffffull)), [&](float x, int i) { if (okey(x) == static_cast<uint32_t>(b >> 32)) id = min(id, i); });
+      if (id == 0x7fffffff) id = 0;                          // nothing above -Inf: no logit beats the first one
       float x0 = 0.f;
       rv.visit(0, [&](float x, int i) { if (i == 0) x0 = x; });
       if (x0 != x0) id = 0;     // generate.go:136: maxVal starts as NaN, nothing is greater

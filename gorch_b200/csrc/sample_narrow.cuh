@@ -33,6 +33,35 @@ static_assert((N_NT == 256) ? (N_KEPT_OFF + KEEP_MAX * 8 <= N_WORK_OFF && N_WORK
 static_assert(N_TMP_OFF >= N_RING_OFF && N_TMP_OFF + N_TMP_CAP * 8 <= N_RING_OFF + N_RING_BYTES, "the prune's buffer lies in the ring");
 static_assert(N_TMP_CAP >= N_KEEP && N_KEEP + 8 <= N_CAP, "a pruned list fits its buffer and leaves room for a portion of hits");
 
+// This thread's largest logit above -Inf, as (order key, ~vector): the lowest vector of equals; 0: none. NaNs are not
+// seen (maxima leave them out). Latency bounds a row that one CTA reads by itself, so what counts is the bytes in
+// flight: GREEDY_U vectors per thread are asked for before the first is looked at, and a look is a maximum per
+// vector and one compare (384 rows of 151,936 f32: 114 us with one vector at a time and a 64-bit key per logit). Not
+// inlined: the streaming code keeps its registers.
+template <typename T>
+__device__ __noinline__ unsigned long long greedy_scan(const RowView<T> rv, int tid) {
+  constexpr int GREEDY_U = 6;
+  float best = -INFINITY;
+  int bv = 0;
+  auto look = [&](const uint4& raw, int v) {
+    const float m = vec_max<T>(raw);
+    if (m > best) { best = m; bv = v; }
+  };
+  if (tid == 0) look(mask_edges(rv, 0, __ldg(rv.vbase)), 0);
+  int v = 1 + tid;
+  for (; v + (GREEDY_U - 1) * N_NT < rv.nvec - 1; v += GREEDY_U * N_NT) {
+    uint4 raw[GREEDY_U];
+#pragma unroll
+    for (int q = 0; q < GREEDY_U; q++) raw[q] = __ldg(rv.vbase + v + q * N_NT);
+#pragma unroll
+    for (int q = 0; q < GREEDY_U; q++) look(raw[q], v + q * N_NT);
+  }
+  for (; v < rv.nvec - 1; v += N_NT) look(__ldg(rv.vbase + v), v);
+  if (tid == N_NT - 1 && rv.nvec > 1) look(mask_edges(rv, rv.nvec - 1, __ldg(rv.vbase + rv.nvec - 1)), rv.nvec - 1);
+  if (!(best > -INFINITY)) return 0ull;
+  return (static_cast<unsigned long long>(okey(best)) << 32) | static_cast<uint32_t>(~static_cast<uint32_t>(bv));
+}
+
 // D: with the optional outputs (probabilities, debug records).
 template <typename T, bool D>
 __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned char* dyn, bu::Scratch& sc,
@@ -81,17 +110,12 @@ __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned c
 
   // ---- greedy (generate.go:75-76, 134-144): strict '>' from index 0, lowest index wins ties
   if (Tm == 0.0f) {
-    unsigned long long best = 0ull;
-    for (int v = tid; v < rv.nvec; v += N_NT) {
-      const uint4 raw = __ldg(rv.vbase + v);
-      rv.visit_raw(raw, v, [&](float x, int i, int) {
-        const unsigned long long p = (static_cast<unsigned long long>(okey(x)) << 32) |
-                                     static_cast<uint32_t>(~static_cast<uint32_t>(i));
-        best = p > best ? p : best;
-      });
-    }
-    best = bu::max_u64<N_NW>(best, sc, tid);
-    int id = static_cast<int>(~static_cast<uint32_t>(best & 0xffffffffull));
+    // the largest logit's vector (the lowest of them), then its place in there
+    const unsigned long long best = bu::max_u64<N_NW>(greedy_scan<T>(rv, tid), sc, tid);
+    const int gv = static_cast<int>(~static_cast<uint32_t>(best & 0xffffffffull));
+    int id = 0x7fffffff;
+    if (best != 0ull) rv.visit(gv, [&](float x, int i) { if (okey(x) == static_cast<uint32_t>(best >> 32)) id = min(id, i); });
+    if (id == 0x7fffffff) id = 0;                            // nothing above -Inf: no logit beats the first one
     float x0 = 0.f;
     rv.visit(0, [&](float x, int i) { if (i == 0) x0 = x; });
     // a NaN at index 0 is never beaten (index 0 of the whole row: a later slice has no such column)

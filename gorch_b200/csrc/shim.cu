@@ -1263,7 +1263,9 @@ int gorch_cuda_topk_dev(GorchCudaCtxRef ctx, const void* x, int dtype, int64_t B
   CUDA_TRY(cudaSetDevice(c->device), errOut);
   // The narrow kernel (a row per CTA of 128 threads) while its lists stay short: 512 x 151,936 f32 takes 91 us with it
   // at k = 64 and 160 us at k = 256, where the other one takes 92.
-  if (k > gs::TKL_MIN_K) {
+  // Up to one row per SM the other one wins for every k: all of an SM's threads read the row (us, narrow | this, f32,
+  // k = 40: 32 x 4,000: 23 | 14; 32 x 50,257: 33 | 20; 8 x 151,936: 45 | 25; 128 x 151,936: 49 | 31).
+  if (k > gs::TKL_MIN_K || B <= c->sm_count) {
     gs::TopKLargeArgs ta;
     ta.x = x; ta.row_stride = row_stride; ta.V = static_cast<int32_t>(V); ta.k = static_cast<int32_t>(k);
     ta.out_values = out_values; ta.out_indices = out_indices; ta.out_flags = out_flags; ta.B = B;
