@@ -1039,17 +1039,26 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
           if (block_max_i(tie, ctl, tid)) flags |= FLAG_TIE_CUT;
         }
       }
-      // kept zone mass per owning rank
+      // kept zone mass per owning rank: rank r's part of the list by NW / C warps (f64 atomics of shared memory on a few
+      // addresses took longer than the selection: 16,000 logits, sigma 2, p = 0.9: 19,000 cycles of the step, 10,000 so)
+      const int wlog = 31 - __clz(max(1, NW / C)), per_r = 1 << wlog;
       __syncthreads();
       if (!bad) {
-        for (int t = tid; t < ZCAP; t += NT) {
-          if (zlive(t)) {
-            const unsigned long long k = zk[t];
-            if (k < cut_key || (cut_incl && k == cut_key)) {
-              const int idx = zone_key_index(k, mode);
-              atomicAdd(&s_zk[min(C - 1, rv.vec_of(idx) / SV)], exp_safe(zone_key_d(k), s_tab));
-            }
+        const int r = warp >> wlog;
+        double e = 0.0;
+        if (r < C) {
+          for (int t = (warp & (per_r - 1)) * 32 + lane; t < X.cnt[r]; t += per_r * 32) {
+            const unsigned long long k = zk[r * zcap_r + t];
+            if (k < cut_key || (cut_incl && k == cut_key)) e += exp_safe(zone_key_d(k), s_tab);
           }
+        }
+        e = warp_sum_d(e);
+        if (lane == 0) ctl.red_d[warp] = e;
+        __syncthreads();
+        if (tid < C) {
+          double z = 0.0;
+          for (int q = 0; q < per_r; q++) z += ctl.red_d[(tid << wlog) + q];
+          s_zk[tid] = z;
         }
       }
       __syncthreads();
@@ -1155,29 +1164,20 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
   // ---- owner: kept mass per warp run = certain mass + kept zone entries, then one run is rescanned
   __syncthreads();
   if (cut_on) {
-    if (rank == 0) {
-      // rank 0's region B was reused by the selection: it filters the staged list instead
-      const unsigned long long* zk = reinterpret_cast<const unsigned long long*>(regA);
-      for (int t = tid; t < ZCAP; t += NT) {
-        if ((t & (zcap_r - 1)) < X.cnt[t >> zlog]) {
-          const unsigned long long k = zk[t];
-          const int jj = rv.vec_of(zone_key_index(k, mode)) - v0;
-          if ((k < ckey || (cincl && k == ckey)) && jj >= 0 && jj < nv) {
-            atomicAdd(&s_kseg[min(NW - 1, jj / max(wv, 1))], exp_safe(zone_key_d(k), s_tab));
-          }
-        }
-      }
-    } else {
-      for (int j = tid; j < nz_loc; j += NT) {
-        const uint2 e = lz[j];
-        const float d = __uint_as_float(e.x);
-        const int i = static_cast<int>(e.y);
-        const unsigned long long k = zone_key(d, i, mode);
-        if (k < ckey || (cincl && k == ckey)) {
-          atomicAdd(&s_kseg[min(NW - 1, (rv.vec_of(i) - v0) / max(wv, 1))], exp_safe(d, s_tab));
-        }
-      }
+    // (rank 0's region B was reused by the selection: it takes its part of the staged list instead)
+    const unsigned long long* zk = reinterpret_cast<const unsigned long long*>(regA);
+    const int n = (rank == 0) ? X.cnt[0] : nz_loc;
+    const int j0 = v0 + warp * wv, j1 = (warp == NW - 1) ? v1 : j0 + wv;   // this warp's run: it adds its own entries, no atomics
+    double e = 0.0;
+    for (int j = lane; j < n; j += 32) {
+      unsigned long long k;
+      if (rank == 0) k = zk[j];
+      else { const uint2 z = lz[j]; k = zone_key(__uint_as_float(z.x), static_cast<int>(z.y), mode); }
+      const int v = rv.vec_of(zone_key_index(k, mode));
+      if (v >= j0 && v < j1 && (k < ckey || (cincl && k == ckey))) e += exp_safe(zone_key_d(k), s_tab);
     }
+    e = warp_sum_d(e);
+    if (lane == 0) s_kseg[warp] += e;
   }
   __syncthreads();
   const double ltgt = X.local_target;
