@@ -4,12 +4,15 @@
 //   (f32 probabilities, f64 running sum), else V-1. multinomial_rows_kernel: 256 threads, rows
 //   pulled by a grid-stride loop; every warp sums its span of the row step by step (one f64 sum
 //   per warp-step of 256 probabilities), a block scan over the steps finds the step the uniform
-//   falls into, and one warp rescans that step in index order. The running sum is formed in a
+//   falls into, and one warp rescans that step in index order. A row is shared out over a cluster of one to
+//   eight CTAs, each with its own part of the row; they exchange the sums of their parts. The running sum is formed in a
 //   different order than the reference's sequential loop: a row whose uniform lies within 1e-6 of
 //   an edge of the chosen interval is flagged FLAG_BOUNDARY.
 //   TopK (index_ops.go:153-190): the narrow kernel of sample_batch.cuh with KernelArgs::tk_k set for
 //   k <= 64, topk_large.cuh beyond.
 #pragma once
+
+#include <cooperative_groups.h>
 
 #include "sample_batch.cuh"
 
@@ -18,6 +21,7 @@ namespace gs {
 constexpr int MN_NT = 256;
 constexpr int MN_NW = MN_NT / 32;
 constexpr int MN_MAX_STEPS = 256;                          // steps per warp: rows up to 8 * 256 * 256 = 524288 probabilities
+constexpr int MN_MAX_C = 8;                                // CTAs per row, at most
 constexpr int MN_NQ = 3;                                   // steps of the row in flight per thread
 constexpr int MN_RING_OFF = MN_NW * MN_MAX_STEPS * 8;      // after the 16 KB of step sums
 constexpr int MN_DYN_BYTES = MN_RING_OFF + MN_NQ * 2 * MN_NT * 16;   // + 24 KB of ring
@@ -37,17 +41,22 @@ __global__ void __launch_bounds__(MN_NT, 4) multinomial_rows_kernel(MultinomialA
   __shared__ bu::Scratch sc;
   __shared__ double s_bcd[4];
   __shared__ int s_bc[2];
+  __shared__ double s_part[MN_MAX_C];                      // sums of the row's parts
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = static_cast<int>(cluster.num_blocks()), rank = static_cast<int>(cluster.block_rank());
   double* stepsum = reinterpret_cast<double*>(dyn);        // [warp][step], row order
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int SV = 64;                                   // vectors per warp-step (two per lane)
   unsigned long long pol;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
-  for (int64_t row = blockIdx.x; row < M.B; row += gridDim.x) {
+  for (int64_t row = blockIdx.x / C; row < M.B; row += gridDim.x / C) {
     __syncthreads();
     RowView<float> rv;
     rv.init(M.probs + row * M.row_stride, M.V);
     const double u = M.uniforms[row];
-    const int span = (((rv.nvec + MN_NW - 1) / MN_NW + SV - 1) / SV) * SV;
+    const int span = (((rv.nvec + MN_NW * C - 1) / (MN_NW * C) + SV - 1) / SV) * SV;
+    const int w0 = rank * MN_NW;                           // this CTA's first warp among the row's
     const int steps = span / SV;
     int id = -1;
     uint32_t fl = 0u;
@@ -55,7 +64,7 @@ __global__ void __launch_bounds__(MN_NT, 4) multinomial_rows_kernel(MultinomialA
       if (tid == 0) { M.out_ids[row] = -1; if (M.out_flags) M.out_flags[row] = FLAG_INTERNAL; }
       continue;
     }
-    const WSpan sp = make_span<float>(rv, warp * span, span, lane);
+    const WSpan sp = make_span<float>(rv, min((w0 + warp) * span, rv.nvec), span, lane);
     for (int j = tid; j < MN_NW * steps; j += MN_NT) stepsum[j] = 0.0;
     __syncthreads();
     // masked value of element c of this lane's vectors in step st (0 outside the row)
@@ -112,17 +121,31 @@ __global__ void __launch_bounds__(MN_NT, 4) multinomial_rows_kernel(MultinomialA
     for (int q = 0; q < PER; q++) { const int j = tid * PER + q; acc += (j < nsteps) ? stepsum[j] : 0.0; loc[q] = acc; }
     double total;
     const double ex = bu::scan_excl_d<MN_NW>(acc, total, sc, tid);
+    double before_me = 0.0, whole = total;                 // the row's mass ahead of this part, and all of it
+    if (C > 1) {
+      if (tid < C) *cluster.map_shared_rank(&s_part[rank], tid) = total;
+      cluster.sync();
+      int owner = -1;
+      whole = 0.0;
+      for (int r = 0; r < C; r++) {
+        if (r == rank) before_me = whole;
+        whole += s_part[r];
+        if (owner < 0 && (u < whole || whole != whole)) owner = r;   // (a NaN: what lies ahead of it in this part still counts)
+      }
+      cluster.sync();                                      // everyone has read: the next row may write
+      if (rank != (owner < 0 ? C - 1 : owner)) continue;
+    }
     int mine = 0x7fffffff;
 #pragma unroll
-    for (int q = PER - 1; q >= 0; q--) { const int j = tid * PER + q; if (j < nsteps && u < ex + loc[q]) mine = j; }
+    for (int q = PER - 1; q >= 0; q--) { const int j = tid * PER + q; if (j < nsteps && u < before_me + (ex + loc[q])) mine = j; }
     const int jsel = bu::min_i<MN_NW>(mine, sc, tid);
-    if (jsel != 0x7fffffff && tid == jsel / PER) s_bcd[0] = ex + ((jsel % PER) ? loc[jsel % PER - 1] : 0.0);
+    if (jsel != 0x7fffffff && tid == jsel / PER) s_bcd[0] = before_me + (ex + ((jsel % PER) ? loc[jsel % PER - 1] : 0.0));
     if (tid == 0) s_bc[0] = -1;
     __syncthreads();
     if (jsel != 0x7fffffff && warp == 0) {
       // rescan the chosen warp-step in index order: first vectors of lanes 0..31, then the second
       const int w = jsel / steps, st = jsel % steps;
-      const WSpan sw = make_span<float>(rv, w * span, span, lane);
+      const WSpan sw = make_span<float>(rv, min((w0 + w) * span, rv.nvec), span, lane);
       uint4 a, b;
       w_load<float, 0>(sw, st, pol, a, b);
       double v[8];
@@ -172,10 +195,14 @@ __global__ void __launch_bounds__(MN_NT, 4) multinomial_rows_kernel(MultinomialA
     if (jsel != 0x7fffffff && s_bc[0] >= 0) {
       id = s_bc[0];
       if ((s_bcd[1] > 0.0 && u - s_bcd[1] <= 1e-6) || s_bcd[2] - u <= 1e-6) fl |= FLAG_BOUNDARY;
+    } else if (C > 1 && u < whole) {
+      // the parts' sums put u inside this part, the scan over its steps just past its end, to within rounding
+      id = min(M.V, (w0 + MN_NW) * span * 4 - rv.shift) - 1;
+      fl |= FLAG_BOUNDARY;
     } else {
       id = M.V - 1;                                        // index_ops.go: falls through to the last index
       fl |= FLAG_FALLBACK;
-      if (u - total <= 1e-6) fl |= FLAG_BOUNDARY;
+      if (u - whole <= 1e-6) fl |= FLAG_BOUNDARY;
     }
     if (tid == 0) { M.out_ids[row] = id; if (M.out_flags) M.out_flags[row] = fl; }
   }

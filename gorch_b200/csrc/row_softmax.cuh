@@ -23,6 +23,7 @@
 #include <cstdint>
 
 #include "block_util.cuh"
+#include "sample_cluster.cuh"   // mask_edges, vec_max
 #include "sample_common.cuh"
 #include "sample_kernel.cuh"   // Elem, RowView
 
@@ -58,6 +59,13 @@ __device__ __forceinline__ uint32_t bf16_bits_rne(float v) {
   const uint32_t b = __float_as_uint(v);
   if (((b >> 23) & 0xffu) == 0xffu && (b & 0x7fffffu) != 0u) return (b >> 16) | 0x40u;
   return (b + 0x7fffu + ((b >> 16) & 1u)) >> 16;
+}
+
+// The same for two at once, lo in the lower half (every NaN here comes out of arithmetic: 0x7fffffff, so 0x7fff)
+__device__ __forceinline__ uint32_t bf16x2_rne(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
 }
 
 // Two f32 in one 64-bit register for the packed FMA pipe (half the issue slots per element).
@@ -220,10 +228,10 @@ __device__ __forceinline__ void rs_store(TO* orow, bool vec_ok, int V, int i0, c
       }
     } else {
       uint4 o;
-      o.x = bf16_bits_rne(y[0]) | (bf16_bits_rne(y[1]) << 16);
-      o.y = bf16_bits_rne(y[2]) | (bf16_bits_rne(y[3]) << 16);
-      o.z = bf16_bits_rne(y[N - 4]) | (bf16_bits_rne(y[N - 3]) << 16);
-      o.w = bf16_bits_rne(y[N - 2]) | (bf16_bits_rne(y[N - 1]) << 16);
+      o.x = bf16x2_rne(y[0], y[1]);
+      o.y = bf16x2_rne(y[2], y[3]);
+      o.z = bf16x2_rne(y[N - 4], y[N - 3]);
+      o.w = bf16x2_rne(y[N - 2], y[N - 1]);
       __stcs(reinterpret_cast<uint4*>(orow + i0), o);
     }
   } else {
@@ -371,6 +379,105 @@ __global__ void __launch_bounds__(RS_NT, 1) row_softmax_kernel(const RowSoftmaxA
   }
   // the other CTA may still be reading this one's last (M, S): no CTA leaves before both are done
   if (C > 1 && A.mode != RS_CE_BWD) cluster.sync();
+}
+
+// ---- Softmax and log-softmax with the row resident in shared memory: a cluster of C CTAs takes a row, every CTA
+// copies its slice in once, and the slices' (M, S) meet through distributed shared memory before the outputs are
+// written from the copies. Two CTAs of different rows share an SM: one reads while the other writes. The two-pass kernel
+// above reads the row from L2 a second time and gives a row to at most two CTAs: it stays for rows that fit no cluster
+// and where the clusters' packing costs more (the host's rule). us, two-pass | this, f32: 8 x 151,936: 23 | 12;
+// 512 x 16,000: 31 | 18; 512 x 50,257: 64 | 53 (of 32 at copy speed); 512 x 151,936: 141 | 137 (of 96).
+constexpr int RR_NT = 512;
+constexpr int RR_MAX_C = 8;
+constexpr int RR_SLICE = 110 * 1024;                           // of shared memory per CTA, two CTAs per SM
+// vectors per CTA, cut at a 128-byte line
+__host__ __device__ inline int64_t rr_per(int64_t nvec, int C) { return ((nvec + C - 1) / C + 7) & ~static_cast<int64_t>(7); }
+
+template <typename T>
+__global__ void __launch_bounds__(RR_NT, 2) row_softmax_resident_kernel(const __grid_constant__ RowSoftmaxArgs A) {
+  namespace cg = cooperative_groups;
+  extern __shared__ __align__(16) unsigned char rs_dyn[];
+  __shared__ bu::Scratch sc;
+  __shared__ RsHalf xch[RR_MAX_C];
+  constexpr int VEC = Elem<T>::VEC, NW = RR_NT / 32;
+  uint4* slice = reinterpret_cast<uint4*>(rs_dyn);
+  const int tid = threadIdx.x;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = static_cast<int>(cluster.num_blocks());
+  const int rank = static_cast<int>(cluster.block_rank());
+  const int64_t row = blockIdx.x / C;
+  RowView<T> rv;
+  rv.init(static_cast<const T*>(A.x) + row * A.row_stride, A.V);
+  const int per = static_cast<int>(rr_per(rv.nvec, C));
+  const int v0 = min(rank * per, rv.nvec), nv = min(v0 + per, rv.nvec) - v0;
+  // a thread looks at the vectors it copied itself: no barrier before the first pass
+  const uint32_t at = static_cast<uint32_t>(__cvta_generic_to_shared(slice));
+  for (int j = tid; j < nv; j += RR_NT)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(at + static_cast<uint32_t>(j) * 16u), "l"(rv.vbase + v0 + j) : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  if (C > 1) cluster.barrier_arrive();
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  float m = -INFINITY;                                         // this thread's maximum (NaNs ignored)
+  for (int j = tid; j < nv; j += RR_NT) {
+    const int v = v0 + j;
+    uint4 raw = slice[j];
+    if (v == 0 || v >= rv.nvec - 1) { raw = mask_edges(rv, v, raw); slice[j] = raw; }
+    m = fmaxf(m, vec_max<T>(raw));
+  }
+  rs_f2 s2 = rs_pk(0.0f, 0.0f);
+  const float mm = (m > -INFINITY) ? m : 0.0f;                 // (only -Inf and NaN: exp(-Inf - 0) = 0, and a NaN shows in the sum)
+  const rs_f2 NM = rs_pk(-mm, -mm), L = rs_pk(1.44269502162933349609375f, 1.44269502162933349609375f);
+  for (int j = tid; j < nv; j += RR_NT) {
+    float x[VEC];
+    Elem<T>::unpack(slice[j], x);
+#pragma unroll
+    for (int c = 0; c < VEC; c += 2) {
+      float t0, t1;
+      rs_upk(rs_mul2(rs_add2(rs_pk(x[c], x[c + 1]), NM), L), t0, t1);
+      s2 = rs_add2(s2, rs_pk(rs_ex2(t0), rs_ex2(t1)));         // the terms' precision: see rs_max_sum
+    }
+  }
+  float M = okey_to_float(static_cast<uint32_t>(bu::max_u64<NW>(static_cast<unsigned long long>(okey(m)), sc, tid)));
+  float sa, sb;
+  rs_upk(s2, sa, sb);
+  const float s = sa + sb;
+  const double part = (m > -INFINITY || s != s) ? static_cast<double>(s) * static_cast<double>(expf(mm - M)) : 0.0;
+  double S = bu::sum_d<NW>(part, sc, tid);
+  if (C > 1) {
+    cluster.barrier_wait();
+    if (tid < C) { RsHalf* p = cluster.map_shared_rank(&xch[rank], tid); p->m = M; p->s = S; }
+    cluster.sync();                                            // the last remote access: no CTA waits for another after it
+    float Mt = -INFINITY;
+    for (int r = 0; r < C; r++) Mt = fmaxf(Mt, xch[r].m);
+    double St = 0.0;                                           // the same expression on every CTA, in rank order: the same bits
+    for (int r = 0; r < C; r++) {
+      const double sr = xch[r].s;
+      if (xch[r].m > -INFINITY || sr != sr) St += sr * static_cast<double>(expf(xch[r].m - Mt));
+    }
+    M = Mt;
+    S = St;
+  }
+  if (!(M > -INFINITY)) S = __longlong_as_double(0x7ff8000000000000ll);   // a row of -Inf only: upstream's -Inf - -Inf
+  const float Sf = static_cast<float>(S);
+  T* orow = static_cast<T*>(A.out) + row * A.out_stride;
+  const bool vec_ok = ((reinterpret_cast<uintptr_t>(orow) - static_cast<uintptr_t>(rv.shift) * sizeof(T)) & 15u) == 0;
+  auto map = [&](auto&& f) {
+#pragma unroll 2
+    for (int j = tid; j < nv; j += RR_NT) {
+      float x[VEC], y[VEC];
+      Elem<T>::unpack(slice[j], x);
+#pragma unroll
+      for (int c = 0; c < VEC; c += 2) f(x[c], x[c + 1], y[c], y[c + 1]);
+      rs_store<T, VEC>(orow, vec_ok, rv.V, (v0 + j) * VEC - rv.shift, y);
+    }
+  };
+  if (A.mode == RS_SOFTMAX) {
+    const float inv = 1.0f / Sf;
+    map([&](float xa, float xb, float& ya, float& yb) { rs_upk(rs_mul2(rs_exp2(xa - M, xb - M), rs_pk(inv, inv)), ya, yb); });
+  } else {
+    const float logS = static_cast<float>(log(static_cast<double>(Sf)));
+    map([&](float xa, float xb, float& ya, float& yb) { ya = xa - M - logS; yb = xb - M - logS; });
+  }
 }
 
 // Mean of the row losses in row order (loss.go:83: total / batch), one warp-sized CTA.

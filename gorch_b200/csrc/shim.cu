@@ -51,6 +51,12 @@ inline bool use_batch_mode(int64_t B, int64_t row_bytes) {
   return B >= 32 && B * row_bytes >= kBatchModeBytes;
 }
 
+// LM head with sampling: up to this many bytes of logits they are written to scratch, where the cluster kernel finds them in
+// L2. The fused form saves that traffic and pays for it with two more kernels and a second run over part of the weights
+// (us, fused | this: 64 x 50,257, K = 1024: 65 | 48; 96: 67 | 52; 16 x 151,936, K = 512: 75 | 60; 32: 76 | 65; K = 2048,
+// 16: 150 | 133). Beyond it the batch kernels would serve the rows: 128 x 50,257: 70 | 77. Measured from K = 512 on.
+constexpr int64_t kLmhUnfusedBytes = 20ll << 20, kLmhUnfusedK = 512;
+
 struct Buffer {
   int device;
   void* ptr;
@@ -305,7 +311,25 @@ int check_shape(int dtype, int64_t B, int64_t V, int64_t row_stride, char** errO
 size_t elem_size(int dtype) { return dtype == GORCH_CUDA_BF16 ? 2 : 4; }
 
 // A launch on the context's stream; dependent: it may start while the kernel before it runs, and waits for
-// that itself (griddepcontrol.wait) where it needs what it wrote.
+// that itself (griddepcontrol.wait) where it needs what it wrote. cluster: CTAs per cluster.
+template <typename... P, typename... A>
+cudaError_t launch_clusters(Ctx* c, void (*kernel)(P...), unsigned grid, unsigned block, size_t dyn, bool dependent, int cluster, const A&... args) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(grid);
+  lc.blockDim = dim3(block);
+  lc.dynamicSmemBytes = dyn;
+  lc.stream = c->stream;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = dependent ? 2 : 1;
+  return cudaLaunchKernelEx(&lc, kernel, args...);
+}
 template <typename... P, typename... A>
 cudaError_t launch(Ctx* c, void (*kernel)(P...), unsigned grid, unsigned block, size_t dyn, bool dependent, const A&... args) {
   cudaLaunchConfig_t lc = {};
@@ -469,26 +493,10 @@ int launch_rows(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int
       ca.slice_bytes = static_cast<int32_t>(need > gs::MIN_SLICE_BYTES ? need : gs::MIN_SLICE_BYTES);
       ca.eb_table = c->eb_table;
       const size_t dyn = static_cast<size_t>(ca.slice_bytes) + gs::REGION_A + gs::REGION_B;
-      cudaLaunchConfig_t lc = {};
-      lc.gridDim = dim3(static_cast<unsigned>(B * C));
-      lc.blockDim = dim3(gs::NT);
-      lc.dynamicSmemBytes = dyn;
-      lc.stream = c->stream;
-      cudaLaunchAttribute at[2];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = static_cast<unsigned>(C);
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = 1;
-      at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // launch beside the kernel before it; it waits for that itself
-      at[1].val.programmaticStreamSerializationAllowed = 1;
-      lc.attrs = at;
-      lc.numAttrs = 2;
       const bool diag = out_probs || out_debug;
-      if (dtype == GORCH_CUDA_F32) {
-        CUDA_TRY(cudaLaunchKernelEx(&lc, diag ? gs::sample_cluster_kernel<float, true> : gs::sample_cluster_kernel<float, false>, ca), errOut);
-      } else {
-        CUDA_TRY(cudaLaunchKernelEx(&lc, diag ? gs::sample_cluster_kernel<uint16_t, true> : gs::sample_cluster_kernel<uint16_t, false>, ca), errOut);
-      }
+      auto* kernel = (dtype == GORCH_CUDA_F32) ? (diag ? gs::sample_cluster_kernel<float, true> : gs::sample_cluster_kernel<float, false>)
+                                               : (diag ? gs::sample_cluster_kernel<uint16_t, true> : gs::sample_cluster_kernel<uint16_t, false>);
+      CUDA_TRY(launch_clusters(c, kernel, static_cast<unsigned>(B * C), gs::NT, dyn, true, C, ca), errOut);
       CUDA_TRY(cudaGetLastError(), errOut);
     }
   }
@@ -781,6 +789,8 @@ GorchCudaCtxRef gorch_cuda_create_ctx(int device, char** errOut) {
   if ((e = cudaFuncSetAttribute(gs::lmh_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::LMH_F_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::row_softmax_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::RS_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::row_softmax_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::RS_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::row_softmax_resident_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::RR_SLICE)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::row_softmax_resident_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::RR_SLICE)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::w256::wide_rows_kernel<uint16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::w256::W_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   return c;
 }
@@ -1261,11 +1271,12 @@ int gorch_cuda_topk_dev(GorchCudaCtxRef ctx, const void* x, int dtype, int64_t B
   if (B == 0) return GORCH_CUDA_OK;
   if (!x || !out_values || !out_indices) { set_err(errOut, "gorch_cuda: null pointer argument"); return GORCH_CUDA_ERR_BAD_ARG; }
   CUDA_TRY(cudaSetDevice(c->device), errOut);
-  // The narrow kernel (a row per CTA of 128 threads) while its lists stay short: 512 x 151,936 f32 takes 91 us with it
-  // at k = 64 and 160 us at k = 256, where the other one takes 92.
+  // The narrow kernel (a row per CTA, phases that grow with k) for small k over rows that are not long: us, narrow | the
+  // other, 512 rows: 50,257 f32, k = 16: 47 | 53; 40: 53 | 53; 64: 57 | 53; bf16, k = 64: 43 | 47; 151,936 f32, k = 4: 92 | 86.
   // Up to one row per SM the other one wins for every k: all of an SM's threads read the row (us, narrow | this, f32,
   // k = 40: 32 x 4,000: 23 | 14; 32 x 50,257: 33 | 20; 8 x 151,936: 45 | 25; 128 x 151,936: 49 | 31).
-  if (k > gs::TKL_MIN_K || B <= c->sm_count) {
+  const int64_t min_k = V * static_cast<int64_t>(elem_size(dtype)) >= (400 << 10) ? 0 : (dtype == GORCH_CUDA_F32 ? gs::TKL_MIN_K / 2 : gs::TKL_MIN_K);
+  if (k > min_k || B <= c->sm_count) {
     gs::TopKLargeArgs ta;
     ta.x = x; ta.row_stride = row_stride; ta.V = static_cast<int32_t>(V); ta.k = static_cast<int32_t>(k);
     ta.out_values = out_values; ta.out_indices = out_indices; ta.out_flags = out_flags; ta.B = B;
@@ -1314,9 +1325,17 @@ int gorch_cuda_multinomial_dev(GorchCudaCtxRef ctx, const float* probs, int64_t 
   gs::MultinomialArgs m;
   m.probs = probs; m.row_stride = row_stride; m.V = static_cast<int32_t>(V);
   m.uniforms = uniforms; m.out_ids = out_ids; m.out_flags = out_flags; m.B = B;
-  const unsigned g = static_cast<unsigned>(B < 4 * c->sm_count ? B : 4 * c->sm_count);
-  gs::multinomial_rows_kernel<<<g, gs::MN_NT, gs::MN_DYN_BYTES, c->stream>>>(m);
-  CUDA_TRY(cudaGetLastError(), errOut);
+  // CTAs per row: more while the batch still fits the GPU at two CTAs per SM and a thread keeps four vectors (us, one CTA |
+  // so: 8 x 151,936: 34 | 12; 64 x 151,936: 35 | 23; 8 x 50,257: 15 | 9). Long rows of large batches go by halves, for the
+  // sake of the last round (512 x 151,936: 87 | 79).
+  const int64_t slots = 4 * c->sm_count;
+  int C = 1;
+  while (C < gs::MN_MAX_C && B * 2 * C <= 2 * c->sm_count && V / (2 * C) >= 4 * 4 * gs::MN_NT) C *= 2;
+  if (B > 2 * c->sm_count && V >= 100000) C = 2;
+  const int64_t clusters = (C > 1 || B < slots) ? B : slots;
+  // (not beside the end of the kernel before it: its CTAs would crowd on the SMs that are free first. 64 x 151,936 behind a
+  // softmax: 105 us instead of 60)
+  CUDA_TRY(launch_clusters(c, gs::multinomial_rows_kernel, static_cast<unsigned>(clusters * C), gs::MN_NT, gs::MN_DYN_BYTES, false, C, m), errOut);
   c->counters.kernel_launches += 1;
   return GORCH_CUDA_OK;
 }
@@ -1385,6 +1404,21 @@ int gorch_cuda_generate_step_dev(GorchCudaCtxRef ctx, const void* logits, int dt
   return launch_generate_control(c, out_ids, out_flags, gc, B, errOut);
 }
 
+// CTAs per row of the resident softmax: the smallest power of two whose slice leaves room for two CTAs per SM, more while
+// the whole batch is resident at once; 0 when eight are too few.
+static int softmax_cluster(const Ctx* c, int64_t B, int64_t V, int dtype) {
+  const int64_t nvec = row_vectors(V, dtype);
+  int C = 1;
+  while (C < gs::RR_MAX_C && gs::rr_per(nvec, C) * 16 > gs::RR_SLICE) C++;
+  while (2 * C <= gs::RR_MAX_C && B * 2 * C <= 2 * c->sm_count && nvec / (2 * C) >= 2 * gs::RR_NT) C *= 2;
+  if (gs::rr_per(nvec, C) * 16 > gs::RR_SLICE || B * C > 0x7fffffffll) return 0;
+  // Rows that need three CTAs and more leave slots of a GPC empty; the two-pass kernel then wins (us, two-pass | this)
+  // between one wave of clusters and one row per SM (64 x 151,936 f32: 27 | 29; 128 x 100,000: 32 | 33; beyond: 256 x 151,936:
+  // 84 | 78, 512 x 100,000: 102 | 92), and for bf16, whose rows are half as long, throughout (256 x 151,936: 50 | 55).
+  if (C >= 3 && B * C > 2 * c->sm_count && (B <= c->sm_count || dtype == GORCH_CUDA_BF16)) return 0;
+  return C;
+}
+
 static int launch_row_softmax(Ctx* c, int dtype, const gs::RowSoftmaxArgs& a, char** errOut) {
   CUDA_TRY(cudaSetDevice(c->device), errOut);
   // A pair of CTAs per row where it was measured to pay: the two-pass ops when one row per SM in
@@ -1395,23 +1429,20 @@ static int launch_row_softmax(Ctx* c, int dtype, const gs::RowSoftmaxArgs& a, ch
   bool pair = false;
   if (a.mode == gs::RS_SOFTMAX || a.mode == gs::RS_LOG_SOFTMAX) pair = row_bytes * c->sm_count > (static_cast<int64_t>(c->l2_bytes) / 2);
   else if (a.mode == gs::RS_CE_BWD) pair = row_bytes >= 262144;
+  if (a.mode == gs::RS_SOFTMAX || a.mode == gs::RS_LOG_SOFTMAX) {
+    const int RC = softmax_cluster(c, a.B, a.V, dtype);
+    if (RC > 0) {
+      auto* kernel = (dtype == GORCH_CUDA_F32) ? gs::row_softmax_resident_kernel<float> : gs::row_softmax_resident_kernel<uint16_t>;
+      CUDA_TRY(launch_clusters(c, kernel, static_cast<unsigned>(a.B * RC), gs::RR_NT, static_cast<size_t>(gs::rr_per(row_vectors(a.V, dtype), RC)) * 16,
+                               false, RC, a), errOut);
+      c->counters.kernel_launches += 1;
+      return GORCH_CUDA_OK;
+    }
+  }
   const int C = (pair && c->sm_count >= 2) ? 2 : 1;
   const int64_t clusters = a.B < c->sm_count / C ? a.B : c->sm_count / C;
-  cudaLaunchConfig_t lc = {};
-  lc.gridDim = dim3(static_cast<unsigned>(clusters * C));
-  lc.blockDim = dim3(gs::RS_NT);
-  lc.dynamicSmemBytes = gs::RS_DYN_BYTES;
-  lc.stream = c->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = static_cast<unsigned>(C);
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  lc.attrs = at;
-  lc.numAttrs = 1;
-  if (dtype == GORCH_CUDA_F32) { CUDA_TRY(cudaLaunchKernelEx(&lc, gs::row_softmax_kernel<float>, a), errOut); }
-  else { CUDA_TRY(cudaLaunchKernelEx(&lc, gs::row_softmax_kernel<uint16_t>, a), errOut); }
-  CUDA_TRY(cudaGetLastError(), errOut);
+  auto* kernel = (dtype == GORCH_CUDA_F32) ? gs::row_softmax_kernel<float> : gs::row_softmax_kernel<uint16_t>;
+  CUDA_TRY(launch_clusters(c, kernel, static_cast<unsigned>(clusters * C), gs::RS_NT, gs::RS_DYN_BYTES, false, C, a), errOut);
   c->counters.kernel_launches += 1;
   return GORCH_CUDA_OK;
 }
@@ -1569,7 +1600,7 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
     if ((r2 = launch_lm_head(c, u, errOut))) return r2;
     return launch_rows(c, c->lmh_logits.ptr, GORCH_CUDA_F32, B, V, ld, cfgs, uniforms, out_ids, out_flags, nullptr, nullptr, 0, errOut);
   };
-  if (fuse_top_k < 1 || fuse_top_k > gs::KFAST || V < 4096 || B > 4096) return unfused();
+  if (fuse_top_k < 1 || fuse_top_k > gs::KFAST || V < 4096 || B > 4096 || (K >= kLmhUnfusedK && B * V * 4 <= kLmhUnfusedBytes && !use_batch_mode(B, V * 4))) return unfused();
   // the sample: 1/32 of the vocabulary, but 1024 to 4096 logits, in whole tiles
   int64_t want = V / 32;
   if (want < gs::LMH_SAMPLE_MIN) want = gs::LMH_SAMPLE_MIN;
