@@ -8,6 +8,7 @@
 //   pass 1   one read of the row: every thread keeps a running maximum m and the sum s of
 //            exp(x - m) over its own elements (rescaled when m grows), then the block combines
 //            them: M = max m, S = sum s * exp(m - M) in f64.
+// (Rows that fit the shared memory of a few CTAs take the second kernel below, which reads them once.)
 //   pass 2   softmax: exp(x - M) / S; log-softmax: (x - M) - log S; cross-entropy backward:
 //            exp(x - lse) * scale, minus scale at the target. Written with streaming stores.
 // Cross-entropy forward needs pass 1 only: lse = M + log S, loss = lse - x[target].
@@ -271,13 +272,25 @@ __device__ __forceinline__ void rs_map(const RowView<T>& rv, int v0, int v1, TO*
   for (; v < v1; v += RS_NT) put(v, __ldg(rv.vbase + v));
 }
 
+// loss.go:118-120: l = rowMax + f32(log(f64(sumExp))); loss = l - row[target]
+template <typename T>
+__device__ __forceinline__ void rs_ce_loss(const RowSoftmaxArgs& A, int64_t row, float M, float Sf) {
+  const T* x = static_cast<const T*>(A.x) + row * A.row_stride;
+  const float lse = M + static_cast<float>(log(static_cast<double>(Sf)));
+  const int t = A.targets[row];
+  float xt = __int_as_float(0x7fc00000);                       // a target outside the row: upstream panics; NaN here
+  if (t >= 0 && t < A.V) xt = Elem<T>::to_float(x[t]);
+  A.row_lse[row] = lse;
+  A.row_loss[row] = lse - xt;
+}
+
 // What one CTA of a pair tells the other about its half of a row.
 struct RsHalf {
   float m;
   double s;
 };
 
-// Launched as clusters of C = 1 or 2 CTAs; cluster c takes rows c, c + #clusters, ... With two
+// Launched as clusters of C = 1 or 2 CTAs (the cross-entropy backward, which exchanges nothing: up to 8); cluster c takes rows c, c + #clusters, ... With two
 // CTAs each handles half of the row's vectors and the two exchange (M, S) of their halves through
 // distributed shared memory, one cluster barrier per row. Two CTAs per row halve the rows in
 // flight (74 x 608 KB: what the second pass re-reads fits in the part of L2 an SM reads at full
@@ -296,11 +309,13 @@ __global__ void __launch_bounds__(RS_NT, 1) row_softmax_kernel(const RowSoftmaxA
   const int C = static_cast<int>(cluster.num_blocks());
   const int rank = static_cast<int>(cluster.block_rank());
   const int64_t ncl = gridDim.x / C;
+  if (A.mode == RS_CE_FWD) pdl_launch();                     // the mean's kernel, which waits for the losses
+  if (A.mode == RS_CE_BWD) pdl_wait();
   int k = 0;
   bool primed = false;
   // this CTA's vectors of a row: halves cut at a 128-byte line
   auto range = [&](const RowView<T>& r, int& a0, int& a1) {
-    const int per = (C == 1) ? r.nvec : (((r.nvec + 1) / 2 + 7) & ~7);
+    const int per = (C == 1) ? r.nvec : (((r.nvec + C - 1) / C + 7) & ~7);
     a0 = min(rank * per, r.nvec);
     a1 = min(a0 + per, r.nvec);
   };
@@ -348,18 +363,7 @@ __global__ void __launch_bounds__(RS_NT, 1) row_softmax_kernel(const RowSoftmaxA
     if (!(M > -INFINITY)) S = __longlong_as_double(0x7ff8000000000000ll);   // a row of -Inf only: upstream's -Inf - -Inf
     const float Sf = static_cast<float>(S);                  // the reference's f32 sum
     if (A.mode == RS_CE_FWD) {
-      if (tid == 0 && rank == 0) {
-        // loss.go:118-120: l = rowMax + f32(log(f64(sumExp))); loss = l - row[target]
-        const float lse = M + static_cast<float>(log(static_cast<double>(Sf)));
-        const int t = A.targets[row];
-        float xt = __int_as_float(0x7fc00000);               // a target outside the row: upstream panics; NaN here
-        if (t >= 0 && t < A.V) {
-          if (sizeof(T) == 4) xt = reinterpret_cast<const float*>(x)[row * A.row_stride + t];
-          else xt = __uint_as_float(static_cast<uint32_t>(reinterpret_cast<const uint16_t*>(x)[row * A.row_stride + t]) << 16);
-        }
-        A.row_lse[row] = lse;
-        A.row_loss[row] = lse - xt;
-      }
+      if (tid == 0 && rank == 0) rs_ce_loss<T>(A, row, M, Sf);
     } else if (A.mode == RS_SOFTMAX) {
       // ops.go:544-550: f32(exp(f64(x - max))) / sum; the quotient as a product with 1 / sum (within 1 ulp of it)
       const float inv = 1.0f / Sf;
@@ -415,6 +419,7 @@ __global__ void __launch_bounds__(RR_NT, 2) row_softmax_resident_kernel(const __
   for (int j = tid; j < nv; j += RR_NT)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(at + static_cast<uint32_t>(j) * 16u), "l"(rv.vbase + v0 + j) : "memory");
   asm volatile("cp.async.commit_group;" ::: "memory");
+  if (A.mode == RS_CE_FWD) pdl_launch();
   if (C > 1) cluster.barrier_arrive();
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   float m = -INFINITY;                                         // this thread's maximum (NaNs ignored)
@@ -459,6 +464,10 @@ __global__ void __launch_bounds__(RR_NT, 2) row_softmax_resident_kernel(const __
   }
   if (!(M > -INFINITY)) S = __longlong_as_double(0x7ff8000000000000ll);   // a row of -Inf only: upstream's -Inf - -Inf
   const float Sf = static_cast<float>(S);
+  if (A.mode == RS_CE_FWD) {
+    if (tid == 0 && rank == 0) rs_ce_loss<T>(A, row, M, Sf);
+    return;
+  }
   T* orow = static_cast<T*>(A.out) + row * A.out_stride;
   const bool vec_ok = ((reinterpret_cast<uintptr_t>(orow) - static_cast<uintptr_t>(rv.shift) * sizeof(T)) & 15u) == 0;
   auto map = [&](auto&& f) {
@@ -484,6 +493,7 @@ __global__ void __launch_bounds__(RR_NT, 2) row_softmax_resident_kernel(const __
 __global__ void __launch_bounds__(256) mean_loss_kernel(const float* row_loss, int64_t B, float* out) {
   __shared__ bu::Scratch sc;
   double acc = 0.0;
+  pdl_wait();
   for (int64_t i = threadIdx.x; i < B; i += 256) acc += static_cast<double>(row_loss[i]);
   acc = bu::sum_d<8>(acc, sc, threadIdx.x);
   if (threadIdx.x == 0) *out = static_cast<float>(acc / static_cast<double>(B));

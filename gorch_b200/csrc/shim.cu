@@ -1429,9 +1429,12 @@ static int launch_row_softmax(Ctx* c, int dtype, const gs::RowSoftmaxArgs& a, ch
   bool pair = false;
   if (a.mode == gs::RS_SOFTMAX || a.mode == gs::RS_LOG_SOFTMAX) pair = row_bytes * c->sm_count > (static_cast<int64_t>(c->l2_bytes) / 2);
   else if (a.mode == gs::RS_CE_BWD) pair = row_bytes >= 262144;
-  if (a.mode == gs::RS_SOFTMAX || a.mode == gs::RS_LOG_SOFTMAX) {
+  if (a.mode != gs::RS_CE_BWD) {
+    // Cross-entropy forward writes nothing, and the persistent kernel then has the next row's copies in flight: the
+    // clusters win where a row fits one CTA (us: 1500 x 16,000 f32: 52 | 34; 1500 x 50,257 bf16: 75 | 55) or the whole batch
+    // is resident (16 x 151,936 f32: 24 | 17), and lose beyond (256 x 151,936: 48 | 58).
     const int RC = softmax_cluster(c, a.B, a.V, dtype);
-    if (RC > 0) {
+    if (RC == 1 || (RC > 1 && (a.mode != gs::RS_CE_FWD || a.B * RC <= 2 * c->sm_count))) {
       auto* kernel = (dtype == GORCH_CUDA_F32) ? gs::row_softmax_resident_kernel<float> : gs::row_softmax_resident_kernel<uint16_t>;
       CUDA_TRY(launch_clusters(c, kernel, static_cast<unsigned>(a.B * RC), gs::RR_NT, static_cast<size_t>(gs::rr_per(row_vectors(a.V, dtype), RC)) * 16,
                                false, RC, a), errOut);
@@ -1439,10 +1442,13 @@ static int launch_row_softmax(Ctx* c, int dtype, const gs::RowSoftmaxArgs& a, ch
       return GORCH_CUDA_OK;
     }
   }
-  const int C = (pair && c->sm_count >= 2) ? 2 : 1;
+  int C = (pair && c->sm_count >= 2) ? 2 : 1;
+  const bool bwd = a.mode == gs::RS_CE_BWD;
+  if (bwd)                                                   // few rows: more CTAs each, while they fit at once (16 x 151,936 f32: 17 us by pairs, 14 by eights)
+    while (C < gs::RR_MAX_C && a.B * 2 * C <= c->sm_count && row_bytes / (2 * C) >= 16 * gs::RS_NT) C *= 2;
   const int64_t clusters = a.B < c->sm_count / C ? a.B : c->sm_count / C;
   auto* kernel = (dtype == GORCH_CUDA_F32) ? gs::row_softmax_kernel<float> : gs::row_softmax_kernel<uint16_t>;
-  CUDA_TRY(launch_clusters(c, kernel, static_cast<unsigned>(clusters * C), gs::RS_NT, gs::RS_DYN_BYTES, false, C, a), errOut);
+  CUDA_TRY(launch_clusters(c, kernel, static_cast<unsigned>(clusters * C), gs::RS_NT, gs::RS_DYN_BYTES, bwd, C, a), errOut);
   c->counters.kernel_launches += 1;
   return GORCH_CUDA_OK;
 }
@@ -1489,8 +1495,7 @@ int gorch_cuda_cross_entropy_fwd_dev(GorchCudaCtxRef ctx, const void* logits, in
   rc = launch_row_softmax(c, dtype, a, errOut);
   if (rc) return rc;
   if (mean_loss) {
-    gs::mean_loss_kernel<<<1, 256, 0, c->stream>>>(row_loss, B, mean_loss);
-    CUDA_TRY(cudaGetLastError(), errOut);
+    CUDA_TRY(launch(c, gs::mean_loss_kernel, 1, 256, 0, true, static_cast<const float*>(row_loss), B, mean_loss), errOut);
     c->counters.kernel_launches += 1;
   }
   return GORCH_CUDA_OK;

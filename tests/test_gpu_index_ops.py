@@ -131,6 +131,36 @@ def test_multinomial_nan_row_falls_through(sampler, oracle):
     assert ids.tolist() == oracle.multinomial(p, u).tolist()
 
 
+@pytest.mark.parametrize("B,V", [(1, 32767), (3, 32768), (8, 151936), (36, 65536), (37, 65537), (148, 50257), (297, 100001), (2, 524000)])
+def test_multinomial_rows_shared_by_several_ctas(sampler, oracle, B, V):
+    """Edges of the rule that shares rows out; uniforms at the row's ends; a NaN ahead of the drawn token and behind it."""
+    rng = np.random.Generator(np.random.Philox(key=B * 31 + V))
+    p = rng.random((B, V), dtype=np.float32) ** 8
+    p /= p.sum(axis=1, keepdims=True, dtype=np.float64).astype(np.float32)
+    u = rng.random(B)
+    u[B - 1] = 1.0 - 1e-12
+    if B > 2:
+        u[0], u[1] = 0.0, 0.25
+        p[1, 3 * V // 4] = np.nan
+        p[2, V // 8] = np.nan
+    ids, flags = sampler.multinomial(p, u)
+    ok = (flags & FLAG_BOUNDARY) == 0
+    assert np.array_equal(ids[ok].astype(np.int64), oracle.multinomial(p, u)[ok])
+
+
+@pytest.mark.parametrize("B,V,k", [(1, 64, 64), (3, 3327, 1), (148, 3329, 40), (149, 3329, 40), (5, 151936, 1), (160, 102400, 8), (150, 50257, 33)])
+def test_topk_small_k_dispatch(_sampler_session, oracle, B, V, k):
+    """Few rows or long ones take the one-pass kernel for small k too."""
+    rng = np.random.Generator(np.random.Philox(key=V * 17 + k))
+    x = (rng.integers(-3000, 3000, (B, V)) * 0.01).astype(np.float32)    # many ties
+    x[0, V // 2] = np.nan
+    vals, idx = _sampler_session.topk(x, k)
+    wv, wi = oracle.topk(np.where(np.isnan(x), -np.inf, x), k)
+    if B == 1:                                                           # every logit wanted: the NaN comes last
+        vals, wv, idx, wi = vals[:, :-1], wv[:, :-1], idx[:, :-1], wi[:, :-1]
+    assert np.array_equal(vals, wv) and np.array_equal(idx.astype(np.int64), wi)
+
+
 def test_topk_rows_whose_start_is_not_typical(sampler, oracle):
     """The streaming kernel guesses a threshold from the first 4096 logits of a row. Rows whose
     largest values all sit there make the guess too high (fewer than k logits pass it) and are

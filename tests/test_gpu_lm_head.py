@@ -99,6 +99,30 @@ def test_fused_sampling_matches_the_oracle_on_the_same_logits(_sampler_session, 
     assert s.counters()["lm_head_refused_rows"] == refused0, "the fused form should have served every row"
 
 
+@pytest.mark.parametrize("B", [31, 32, 33, 65, 127, 128, 129, 255, 256, 257, 511, 512])
+@pytest.mark.parametrize("V,K", [(1000, 64), (4161, 192)])
+def test_projection_at_the_edges_of_its_tiles(_sampler_session, B, V, K):
+    import torch
+    xb, wb = _inputs(B, V, K, 7300 + B)
+    got = _project(_sampler_session, torch, xb, wb)
+    want = _bf16_to_f64(xb) @ _bf16_to_f64(wb).T
+    assert (np.abs(got - want) <= 1e-3 * np.abs(want).max(axis=1, keepdims=True)).all()
+
+
+@pytest.mark.parametrize("B,V,K", [(100, 50257, 512), (110, 50257, 512), (100, 50257, 448), (4, 4096, 512), (400, 4200, 512)])
+def test_few_logits_are_sampled_from_scratch(_sampler_session, oracle, B, V, K):
+    """Either side of the rule that writes the logits instead of fusing."""
+    import torch
+    s = _sampler_session
+    xb, wb = _inputs(B, V, K, 7400 + B)
+    uniforms = np.random.default_rng(B).random(B)
+    cfgs = _cfgs(B, [(0.8, 40, 0.0, MODE_A), (0.7, 64, 0.95, MODE_B)])
+    ora = oracle.sample_batch(_project(s, torch, xb, wb), cfgs, uniforms, flags=oracle.FAST_KTH, threads=oracle.hw_threads())
+    ids, flags = _sample_call(s, torch, xb, wb, cfgs, uniforms, 100)
+    rep = compare({"ids": ids, "flags": flags}, ora, uniforms, check_probs=False, allow_tie_cut=True)
+    assert rep["id_mismatch"] == rep["boundary_mismatch"]
+
+
 def test_rows_the_fused_form_does_not_serve_fall_back(_sampler_session, oracle):
     import torch
     s = _sampler_session

@@ -233,6 +233,13 @@ def test_top_p_cut_among_many_equal_logits(sampler, oracle, V, dtype, mode):
     run_both(sampler, oracle, x, cfgs, rng.random(8), allow_tie_cut=True)
 
 
+@pytest.mark.parametrize("B,V,k", [(1, 50257, 129), (4, 50257, 200), (8, 151936, 256), (2, 30000, 128)])
+def test_wide_top_k_in_small_batches(sampler, oracle, B, V, k):
+    rng = np.random.default_rng(V + k)
+    x = (rng.standard_normal((B, V)) * 2).astype(np.float32)
+    run_both(sampler, oracle, x, cfgs_of(B, 0.9, k, 0.97, MODE_B), rng.random(B), allow_tie_cut=True)
+
+
 def test_host_entry_matches_device_entry(sampler):
     w = workloads.mixed_rows(64)
     ids, flags = sampler.sample_batch(w.logits, w.cfgs, w.uniforms)

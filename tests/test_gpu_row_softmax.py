@@ -88,6 +88,29 @@ def test_bf16_logits(_sampler_session, oracle, batch, classes):
     assert np.allclose(dx, oracle.cross_entropy_bwd(xf, tgt, o_lse, 0.25), rtol=2e-6, atol=1e-7)
 
 
+@pytest.mark.parametrize("batch,classes", [(2, 28148), (300, 28153), (297, 28170), (2, 56300), (40, 84500), (60, 112632), (2, 225290), (2, 225400), (16, 16385)])
+def test_rows_at_the_edges_of_their_slices(_sampler_session, batch, classes):
+    """Rows that just fit the shared memory of one CTA, two, eight, or no longer fit; one wave of clusters and more."""
+    s = _sampler_session
+    x, tgt = _case(batch, classes, 5)
+    x[0, classes // 2] = -np.inf
+    x[1, classes - 1] = np.nan
+    keep = np.arange(batch) != 1
+    want_sm, want_ls = _f64_softmax(x[keep])
+    sm, ls = row_ops.softmax(s, x), row_ops.softmax(s, x, log=True)
+    assert np.isnan(sm[1]).all() and np.isnan(ls[1]).all()
+    assert np.allclose(sm[keep], want_sm, rtol=2e-6, atol=1e-37)
+    fin = np.isfinite(want_ls)
+    assert np.abs(ls[keep][fin] - want_ls[fin]).max() <= 2e-6 * np.abs(want_ls[fin]).max()
+    _, row_loss, row_lse = row_ops.cross_entropy(s, x, tgt)
+    lse = np.log(np.exp(x[keep].astype(np.float64)).sum(axis=1))
+    assert np.abs(row_lse[keep] - lse).max() <= 4e-6 * np.abs(lse).max() and np.isnan(row_lse[1])
+    dx = row_ops.cross_entropy_backward(s, x, tgt, row_lse, 0.5)
+    want_dx = 0.5 * want_sm
+    want_dx[np.arange(batch - 1), tgt[keep]] -= 0.5
+    assert np.abs(dx[keep] - want_dx).max() <= 1e-5
+
+
 def test_special_values_match_the_go_loops(_sampler_session, oracle):
     s = _sampler_session
     rng = np.random.default_rng(3)
