@@ -8,8 +8,8 @@
 //   eight CTAs, each with its own part of the row; they exchange the sums of their parts. The running sum is formed in a
 //   different order than the reference's sequential loop: a row whose uniform lies within 1e-6 of
 //   an edge of the chosen interval is flagged FLAG_BOUNDARY.
-//   TopK (index_ops.go:153-190): the narrow kernel of sample_batch.cuh with KernelArgs::tk_k set for
-//   k <= 64, topk_large.cuh beyond.
+//   TopK (index_ops.go:153-190): topk_large.cuh; the narrow kernel of sample_batch.cuh with KernelArgs::tk_k set for small
+//   k over many rows that are not long.
 #pragma once
 
 #include <cooperative_groups.h>

@@ -39,11 +39,11 @@ namespace {
 // (two CTAs per SM) minus the two 16 KB work regions.
 constexpr int64_t kSliceCap = 109 * 1024 - gs::REGION_A - gs::REGION_B;
 
-// Batches of at least this many rows are sorted by kind and served by the narrow / wide
-// kernels; smaller ones use one cluster per row so that every SM still has work.
 // Batches go to the sorted-batch kernels (one CTA per row) from this many rows on; smaller ones to
-// the cluster kernel (several CTAs per row), whose latency is lower while the GPU is not full.
-// Measured crossovers on B200: 40 rows of 608 KB, ~120 rows of 200 KB.
+// the cluster kernel (several CTAs per row), whose latency is lower while the GPU is not full. The rows' kinds are
+// on the device, so one line serves them all. us, batch | cluster: 128 x 50,257 f32: top-k 44 | 31, greedy 28 | 18, mixed
+// 52 | 37, nucleus without a cut 44 | 43, with one 69 | 96; 64 x 151,936 f32: 54 | 33, 48 | 20, 69 | 42, 71 | 50, 101 | 102: it lies
+// where rows with a cut would lose. 512 x 4,000 f32: 37 | 27, 19 | 16, 54 | 40, 38 | 33, 54 | 66.
 constexpr int64_t kBatchModeRows = 384;
 constexpr int64_t kBatchModeBytes = 24ll << 20;
 inline bool use_batch_mode(int64_t B, int64_t row_bytes) {

@@ -1,4 +1,4 @@
-// TopK (index_ops.go:153-190) for TKL_MIN_K < k <= TKL_MAX_K: the k largest of each row, descending, equal
+// TopK (index_ops.go:153-190), k <= TKL_MAX_K (the narrow kernel takes small k over many rows): the k largest of each row, descending, equal
 // values by ascending index; NaNs last (the reference's comparator leaves them unspecified), -0 and
 // +0 equal. The values written are the row's own bits.
 //
@@ -22,7 +22,7 @@
 
 namespace gs {
 
-constexpr int TKL_MIN_K = 64;           // up to here the narrow kernel serves TopK
+constexpr int TKL_MIN_K = 64;           // up to here (f32: half of it) the narrow kernel serves TopK of many rows that are not long
 constexpr int TKL_MAX_K = 16384;
 
 struct TopKLargeArgs {
