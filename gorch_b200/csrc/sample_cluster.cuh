@@ -226,10 +226,9 @@ __device__ __forceinline__ void block_min_i2(int& a_min, int& b_min, Ctl& c, int
   __syncthreads();
   if ((tid & 31) == 0) { c.red_i[tid >> 5] = a_min; c.red_u64[tid >> 5] = static_cast<unsigned long long>(static_cast<uint32_t>(b_min)); }
   __syncthreads();
-  int a = c.red_i[0], b = static_cast<int>(c.red_u64[0]);
-#pragma unroll
-  for (int w = 1; w < NW; w++) { a = min(a, c.red_i[w]); b = min(b, static_cast<int>(c.red_u64[w])); }
-  a_min = a; b_min = b;
+  const int l = tid & (NW - 1);
+  a_min = __reduce_min_sync(FULL, c.red_i[l]);
+  b_min = __reduce_min_sync(FULL, static_cast<int>(c.red_u64[l]));
 }
 __device__ __forceinline__ unsigned long long block_min_u64(unsigned long long v, Ctl& c, int tid) {
   return ~block_max_u64(~v, c, tid);
@@ -242,14 +241,11 @@ __device__ __forceinline__ void block_scan_excl_d2(double a, double b, double& e
   __syncthreads();
   if (lane == 31) { c.red_d[w] = ia; c.red_d2[w] = ib; }
   __syncthreads();
-  double ba = 0, bb = 0, sa = 0, sb = 0;
-#pragma unroll
-  for (int j = 0; j < NW; j++) {
-    double va = c.red_d[j], vb = c.red_d2[j];
-    if (j < w) { ba += va; bb += vb; }
-    sa += va; sb += vb;
-  }
-  ea = ba + ia - a; eb_ = bb + ib - b; ta = sa; tb = sb;
+  const double va = (lane < NW) ? c.red_d[lane] : 0.0, vb = (lane < NW) ? c.red_d2[lane] : 0.0;
+  const double sa = warp_scan_incl_d(va, lane), sb = warp_scan_incl_d(vb, lane);
+  ta = __shfl_sync(FULL, sa, NW - 1); tb = __shfl_sync(FULL, sb, NW - 1);
+  ea = __shfl_sync(FULL, sa - va, w) + ia - a;
+  eb_ = __shfl_sync(FULL, sb - vb, w) + ib - b;
 }
 
 // D: with the optional outputs (probabilities, debug records).
@@ -395,7 +391,10 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
   }
 
   // ---- L / pass A: the slice in shared memory; max, min, NaN, one running max per thread
+  // (the tables' words are on their way before they are wanted: a trip to L2 in front of the bracket and one in front of the
+  // exponentials otherwise)
   const double tab_me = (topk == 0 && tid < 256) ? A.exp_table[tid] : 0.0;
+  const double2 eb_me = (topk == 0) ? __ldg(reinterpret_cast<const double2*>(CA.eb_table) + tid) : make_double2(0.0, 0.0);
   float xmax = -INFINITY, xmin = INFINITY;
   bool nan_seen = false;
   asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -552,17 +551,21 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
   // ============================================================ full row (top-k off)
   dbg.path = 2;
   flags |= FLAG_GENERAL_PATH;
-  const int anynan_loc = block_max_i(nan_seen ? 1 : 0, ctl, tid);
-  const unsigned long long pmax = block_max_u64(static_cast<unsigned long long>(okey(xmax)) << 32, ctl, tid);
-  const float slice_min = okey_to_float(static_cast<uint32_t>(block_min_u64(static_cast<unsigned long long>(okey(xmin)), ctl, tid)));
-  stamp(0);
-  cluster.barrier_wait();
-  if (tid == 0) {
-    const unsigned long long p = pmax | static_cast<unsigned long long>(anynan_loc);
-    for (int r = 0; r < C; r++) {
-      Xchg* xr = cluster.map_shared_rank(&X, r);
-      xr->u64[rank] = p;
-      xr->mn[rank] = slice_min;
+  {
+    uint32_t khi = __reduce_max_sync(FULL, okey(xmax)), klo = __reduce_min_sync(FULL, okey(xmin));
+    const unsigned nanw = __ballot_sync(FULL, nan_seen);
+    if (lane == 0) { ctl.red_u64[warp] = (static_cast<unsigned long long>(khi) << 32) | klo; ctl.red_i[warp] = nanw ? 1 : 0; }
+    __syncthreads();                                         // every slice is complete too
+    const unsigned long long w = ctl.red_u64[lane & (NW - 1)];
+    khi = __reduce_max_sync(FULL, static_cast<uint32_t>(w >> 32));
+    klo = __reduce_min_sync(FULL, static_cast<uint32_t>(w));
+    const int anynan_loc = __reduce_max_sync(FULL, ctl.red_i[lane & (NW - 1)]);
+    stamp(0);
+    cluster.barrier_wait();
+    if (tid < C) {                                           // one thread per receiver, here and below
+      Xchg* xr = cluster.map_shared_rank(&X, tid);
+      xr->u64[rank] = (static_cast<unsigned long long>(khi) << 32) | static_cast<unsigned long long>(anynan_loc);
+      xr->mn[rank] = okey_to_float(klo);
     }
   }
   cluster.sync();                                            // G1
@@ -612,7 +615,8 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
     cluster.sync();                                          // G2
     if (rank == 0) {
       const uint32_t* all = reinterpret_cast<const uint32_t*>(regA);
-      constexpr int PER = NB1 / NT;                          // 2 buckets per thread
+      constexpr int PER = NB1 / NT;                          // 2 buckets per thread: those of eb_me
+      static_assert(PER == 2, "eb_me");
       double lo_inc[PER], hi_inc[PER];
       int cb[PER];
       double slo = 0.0, shi = 0.0;
@@ -625,7 +629,7 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
         const double c = static_cast<double>(cnt);
         // bucket b holds d in [-(b+.5)/32, -(b-.5)/32]; the last one everything below.
         // Masked lanes (-Inf) are counted there too; their mass bound starts at 0.
-        const double eb = __ldg(CA.eb_table + b);
+        const double eb = (j == 0) ? eb_me.x : eb_me.y;
         const double elo = (b == NB1 - 1) ? 0.0 : eb * 0.98449643700540845 * (1.0 - 1e-7);   // exp(-1/64)
         const double ehi = fmin(1.0, eb * 1.0157477085866857 * (1.0 + 1e-7));                 // exp(+1/64)
         slo += c * elo; shi += c * ehi;
@@ -653,12 +657,9 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
         if (b >= b1 && b <= b2) nz_part += cb[j];
       }
       const int nz = block_sum_i(nz_part, ctl, tid);
-      if (tid == 0) {
-        const float tA = bucket_floor(b1 - 1), tB = bucket_floor(b2);
-        for (int r = 0; r < C; r++) {
-          Xchg* xr = cluster.map_shared_rank(&X, r);
-          xr->dA = tA; xr->dB = tB; xr->zone_total = nz;
-        }
+      if (tid < C) {
+        Xchg* xr = cluster.map_shared_rank(&X, tid);
+        xr->dA = bucket_floor(b1 - 1); xr->dB = bucket_floor(b2); xr->zone_total = nz;
       }
     }
     stamp(3);
@@ -741,13 +742,11 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
 #pragma unroll
         for (int j = 0; j < PER; j++) if (tid * PER + j >= b1 && tid * PER + j <= b2) nz_part += cb[j];
         const int nz = block_sum_i(nz_part, ctl, tid);
-        if (tid == 0) {
+        if (tid < C) {
           const float tA = (key_at(b1) == 0u) ? INFINITY : -__uint_as_float(key_at(b1) - 1u);
           const float tB = (b2 == NB1 - 1 || key_at(b2 + 1) > khi) ? dB : -__uint_as_float(key_at(b2 + 1) - 1u);
-          for (int r = 0; r < C; r++) {
-            Xchg* xr = cluster.map_shared_rank(&X, r);
-            xr->dA = tA; xr->dB = tB; xr->zone_total = nz;
-          }
+          Xchg* xr = cluster.map_shared_rank(&X, tid);
+          xr->dA = tA; xr->dB = tB; xr->zone_total = nz;
         }
       }
       cluster.sync();
@@ -762,7 +761,7 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
   double* ebs = reinterpret_cast<double*>(regB + 8192);     // bucket table exp(-b/32), 8 KB
   uint2* lz = reinterpret_cast<uint2*>(regB);               // local zone list (d bits, idx), 1024 entries
   __syncthreads();
-  if (fast_ok) for (int j = tid; j < NB1; j += NT) ebs[j] = __ldg(CA.eb_table + j);
+  if (fast_ok) reinterpret_cast<double2*>(ebs)[tid] = eb_me;
   if (tid == 0) ctl.cand_count = 0;
   __syncthreads();
   const int wv = (nv + NW - 1) / NW;                        // vectors per warp run
@@ -949,13 +948,11 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
         unsigned long long* zkeys = reinterpret_cast<unsigned long long*>(regB);
         double* zmass = reinterpret_cast<double*>(regB + 8 * NT);
         __syncthreads();
-        if (tid == 0) ctl.cand_count = 0;
+        int src = -1;                                          // thread t takes the t-th live entry
+        for (int r = 0, off = 0; r < C; r++) { const int c = X.cnt[r]; if (tid >= off && tid < off + c) src = r * zcap_r + tid - off; off += c; }
+        unsigned long long k = ~0ull;
+        if (src >= 0) { k = zk[src]; zkeys[tid] = k; zmass[tid] = exp_safe(zone_key_d(k), s_tab); }
         __syncthreads();
-        for (int t = tid; t < ZCAP; t += NT) {
-          if (zlive(t)) { const int slot = atomicAdd(&ctl.cand_count, 1); const unsigned long long k = zk[t]; zkeys[slot] = k; zmass[slot] = exp_safe(zone_key_d(k), s_tab); }
-        }
-        __syncthreads();
-        const unsigned long long k = (tid < nz) ? zkeys[tid] : ~0ull;
         double g = 0.0, g2 = 0.0;
         if (tid < nz) {
           int l = 0;
@@ -1094,23 +1091,21 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
         finish(V - 1, flags, dbg);
         code = 3;
       }
-      if (tid == 0) {
-        for (int r = 0; r < C; r++) {
-          Xchg* xr = cluster.map_shared_rank(&X, r);
-          xr->local_target = tgt - base;
-          xr->base_mass = base;
-        }
+      if (tid < C) {
+        Xchg* xr = cluster.map_shared_rank(&X, tid);
+        xr->local_target = tgt - base;
+        xr->base_mass = base;
       }
     }
     stamp(6);
+    if (tid < C) {
+      Xchg* xr = cluster.map_shared_rank(&X, tid);
+      xr->owner = owner;
+      xr->cut_key = cut_key; xr->cut_incl = cut_incl;
+      xr->Re = Re; xr->S = S;
+      xr->verdict = code;
+    }
     if (tid == 0) {
-      for (int r = 0; r < C; r++) {
-        Xchg* xr = cluster.map_shared_rank(&X, r);
-        xr->owner = owner;
-        xr->cut_key = cut_key; xr->cut_incl = cut_incl;
-        xr->Re = Re; xr->S = S;
-        xr->verdict = code;
-      }
       if (code == 0) {                                       // the owner adds the id, the edges and the boundary flag
         if (A.out_flags) A.out_flags[row_id] = flags;
         if (D && A.out_debug) A.out_debug[row_id] = dbg;
