@@ -39,16 +39,21 @@ namespace {
 // (two CTAs per SM) minus the two 16 KB work regions.
 constexpr int64_t kSliceCap = 109 * 1024 - gs::REGION_A - gs::REGION_B;
 
-// Batches go to the sorted-batch kernels (one CTA per row) from this many rows on; smaller ones to
+// Batches go to the sorted-batch kernels (one CTA per row) from this many rows or bytes on; smaller ones to
 // the cluster kernel (several CTAs per row), whose latency is lower while the GPU is not full. The rows' kinds are
-// on the device, so one line serves them all. us, batch | cluster: 128 x 50,257 f32: top-k 44 | 31, greedy 28 | 18, mixed
-// 52 | 37, nucleus without a cut 44 | 43, with one 69 | 96; 64 x 151,936 f32: 54 | 33, 48 | 20, 69 | 42, 71 | 50, 101 | 102: it lies
-// where rows with a cut would lose. 512 x 4,000 f32: 37 | 27, 19 | 16, 54 | 40, 38 | 33, 54 | 66.
+// on the device, so one line serves them all, and it lies where rows with a top-p cut do not lose. us, batch | cluster:
+//   128 x 50,257 f32: top-k 44 | 31, greedy 28 | 18, mixed 52 | 37, nucleus without a cut 44 | 37, with one 67 | 85
+//   64 x 151,936 f32: 54 | 33, 48 | 20, 69 | 42, 71 | 45, 101 | 93; at 96 rows the last pair is 110 | 137
+// Short rows stay with the clusters for longer: two waves of them (one CTA per row, two per SM) up to 4,096 logits
+//   512 x 4,000 f32: 38 | 27, 19 | 16, 52 | 40, 38 | 29, 54 | 57 (16,000: 44 | 31, 28 | 19, 79 | 38, 43 | 40, 65 | 76)
+// and, where the batch kernels need a second round of wide rows, three waves up to 16,384:
+//   768 x 16,000 f32: 46 | 42, 28 | 25, 122 | 49, 75 | 57, 116 | 108; 1024: 50 | 52, 32 | 29, 134 | 59, 79 | 69, 118 | 137
+// An argmax is one launch of the narrow kernel and keeps the lower line.
 constexpr int64_t kBatchModeRows = 384;
 constexpr int64_t kBatchModeBytes = 24ll << 20;
-inline bool use_batch_mode(int64_t B, int64_t row_bytes) {
-  if (B >= kBatchModeRows) return true;
-  return B >= 32 && B * row_bytes >= kBatchModeBytes;
+inline bool use_batch_mode(int sm_count, int64_t B, int64_t V, int64_t elem_bytes, bool argmax) {
+  const bool many_short = B >= kBatchModeRows && !argmax && B <= 6 * sm_count && V <= (B > 4 * sm_count ? 16384 : 4096);
+  return !many_short && (B >= kBatchModeRows || (B >= 32 && B * V * elem_bytes >= kBatchModeBytes));
 }
 
 // LM head with sampling: up to this many bytes of logits they are written to scratch, where the cluster kernel finds them in
@@ -431,7 +436,7 @@ int launch_rows(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int
   a.tk_k = 0;
   if (c->timing) CUDA_TRY(cudaEventRecord(c->ev0, c->stream), errOut);
   int klaunch = 1;
-  const bool batch_mode = c->variant == 2 || c->variant >= 4 || (c->variant == 0 && use_batch_mode(B, V * static_cast<int64_t>(elem_size(dtype))));
+  const bool batch_mode = c->variant == 2 || c->variant >= 4 || (c->variant == 0 && use_batch_mode(c->sm_count, B, V, static_cast<int64_t>(elem_size(dtype)), force_greedy != 0));
   if (batch_mode) {
     // wide (top-k off) with narrow (greedy / top-k) beside it, then single-CTA (whatever was handed over): one stream, each
     // launched while the one before it runs (programmatic dependent launch). The wide kernel goes first and lets the
@@ -564,7 +569,7 @@ int host_run(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int64_
   const void* dev_logits = c->st_logits.ptr;
   // The cluster kernel reads each logit once: it can do that from the pinned block, over the link (one GPT-2 row: 45 us a
   // call, 53 with a copy to device memory first). Kernels that read a row again, and rows that need one, get the copy.
-  bool once = staged && c->variant == 0 && !use_batch_mode(B, V * static_cast<int64_t>(es)) && cluster_size(c, B, V, dtype) > 0;
+  bool once = staged && c->variant == 0 && !use_batch_mode(c->sm_count, B, V, static_cast<int64_t>(es), force_greedy != 0) && cluster_size(c, B, V, dtype) > 0;
   if (!force_greedy) for (int64_t b = 0; b < B && once; b++) once = !(cfgs[b].top_k > gs::KFAST && cfgs[b].top_k < V);
   if (once) {
     memcpy(pin + off_logits, logits, lbytes);
@@ -1605,7 +1610,7 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
     if ((r2 = launch_lm_head(c, u, errOut))) return r2;
     return launch_rows(c, c->lmh_logits.ptr, GORCH_CUDA_F32, B, V, ld, cfgs, uniforms, out_ids, out_flags, nullptr, nullptr, 0, errOut);
   };
-  if (fuse_top_k < 1 || fuse_top_k > gs::KFAST || V < 4096 || B > 4096 || (K >= kLmhUnfusedK && B * V * 4 <= kLmhUnfusedBytes && !use_batch_mode(B, V * 4))) return unfused();
+  if (fuse_top_k < 1 || fuse_top_k > gs::KFAST || V < 4096 || B > 4096 || (K >= kLmhUnfusedK && B * V * 4 <= kLmhUnfusedBytes && !use_batch_mode(c->sm_count, B, V, 4, false))) return unfused();
   // the sample: 1/32 of the vocabulary, but 1024 to 4096 logits, in whole tiles
   int64_t want = V / 32;
   if (want < gs::LMH_SAMPLE_MIN) want = gs::LMH_SAMPLE_MIN;

@@ -240,6 +240,17 @@ def test_wide_top_k_in_small_batches(sampler, oracle, B, V, k):
     run_both(sampler, oracle, x, cfgs_of(B, 0.9, k, 0.97, MODE_B), rng.random(B), allow_tie_cut=True)
 
 
+@pytest.mark.parametrize("B,V", [(592, 4096), (593, 4097), (888, 1500), (700, 16384)])
+def test_many_short_rows(sampler, oracle, B, V):
+    """Either side of the rule that leaves short rows of large batches to the clusters."""
+    rng = np.random.default_rng(V)
+    x = (rng.standard_normal((B, V)) * 2).astype(np.float32)
+    cfgs = np.zeros(B, dtype=CFG_DTYPE)
+    for b in range(B):
+        cfgs[b] = [(0.8, 40, 0.0, MODE_A), (1.0, 0, 0.9, MODE_B), (0.0, 0, 0.0, MODE_A), (0.7, 200, 0.95, MODE_B), (0.9, 300, 0.0, MODE_A)][b % 5]
+    run_both(sampler, oracle, x, cfgs, rng.random(B), want_probs=False, allow_tie_cut=True)
+
+
 def test_host_entry_matches_device_entry(sampler):
     w = workloads.mixed_rows(64)
     ids, flags = sampler.sample_batch(w.logits, w.cfgs, w.uniforms)
