@@ -482,15 +482,16 @@ __global__ void __launch_bounds__(NT, 2) sample_cluster_kernel(const __grid_cons
     // rank 0's slice, after one more barrier that says that rank 0 is through with it.
     const bool wide_lists = topk * C > UCAP / 2;             // uniform over the cluster
     const int cap_r = wide_lists ? WCAP / C : UCAP / C;
-    int n_loc = ctl.cand_count;
+    int n_loc = ctl.cand_count, n_most = cap_r;              // what this rank has, and may send
     if (n_loc > cap_r && n_loc <= LCAP) {                    // more than this rank's share: only what can be kept
       uint2* few = reinterpret_cast<uint2*>(dyn);            // (the slice has been read; peers may already write to region A)
       n_loc = narrow_list<NT>(lc, n_loc, topk, Tm, okey(thr0), khi, few, s_sel, ctl.bcast_i, &ctl.cand_count, tid);
+      n_most = min(cap_r, KEEP_MAX);                         // (a larger count is of ties that are not all there; two CTAs' share is 1024)
       for (int j = tid; j < min(n_loc, KEEP_MAX); j += NT) lc[j] = few[j];
       if (tid < 256) s_sel[tid] = 0u;
       __syncthreads();
     }
-    const bool giveup = n_loc > min(cap_r, LCAP);
+    const bool giveup = n_loc > min(n_most, LCAP);
     stamp(1);
     cluster.barrier_wait();
     if (wide_lists) cluster.sync();

@@ -240,6 +240,30 @@ def test_wide_top_k_in_small_batches(sampler, oracle, B, V, k):
     run_both(sampler, oracle, x, cfgs_of(B, 0.9, k, 0.97, MODE_B), rng.random(B), allow_tie_cut=True)
 
 
+@pytest.mark.parametrize("ties", [511, 512, 513, 740, 1023, 1024, 1025])
+def test_more_ties_in_one_slice_than_a_kept_list_holds(sampler, oracle, ties):
+    """Rows of 75 and more that a pair of CTAs shares: the first slice's k-th largest logit is tied more often than a
+    kept list has entries (512), the second slice raises the row's k-th largest above those ties. Each row has its
+    own places; every third row keeps the ties."""
+    rng = np.random.default_rng(ties)
+    B, V = 75, 50257
+    half = V // 2 - 200
+    x = np.tile(-20.0 - 0.05 * (np.arange(V) % 97), (B, 1)).astype(np.float32)
+    for b in range(B):
+        c = rng.permutation(half)[:40 + ties + 600]
+        x[b, c[:40]] = 5.0 + 0.0625 * np.arange(40)
+        x[b, c[40:40 + ties]] = 1.0
+        x[b, c[40 + ties:]] = 0.97
+        if b % 3:
+            x[b, V // 2 + 200 + rng.permutation(half)[:60]] = 4.0
+    bits = oracle.f32_to_bf16_bits(x)
+    cfgs = cfgs_of(B, 0.8, 50, 0.0, MODE_A)
+    cfgs["top_p"][::2] = 0.9
+    cfgs["topp_mode"][::2] = MODE_B
+    gpu, _, _ = run_both(sampler, oracle, bits, cfgs, rng.random(B), allow_tie_cut=True)
+    assert set(gpu["debug"]["kept"][1::2].tolist()) <= {100, 40 + ties}
+
+
 @pytest.mark.parametrize("B,V", [(592, 4096), (593, 4097), (888, 1500), (700, 16384)])
 def test_many_short_rows(sampler, oracle, B, V):
     """Either side of the rule that leaves short rows of large batches to the clusters."""
