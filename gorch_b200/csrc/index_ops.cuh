@@ -50,6 +50,10 @@ __global__ void __launch_bounds__(MN_NT, 4) multinomial_rows_kernel(MultinomialA
   constexpr int SV = 64;                                   // vectors per warp-step (two per lane)
   unsigned long long pol;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+  // A peer's shared memory may be written once all CTAs of the cluster run: arrived at here, waited for before the
+  // first remote store, so that it costs nothing while the row streams.
+  bool peers_run = (C == 1);
+  if (!peers_run) cluster.barrier_arrive();
   for (int64_t row = blockIdx.x / C; row < M.B; row += gridDim.x / C) {
     __syncthreads();
     RowView<float> rv;
@@ -123,6 +127,7 @@ __global__ void __launch_bounds__(MN_NT, 4) multinomial_rows_kernel(MultinomialA
     const double ex = bu::scan_excl_d<MN_NW>(acc, total, sc, tid);
     double before_me = 0.0, whole = total;                 // the row's mass ahead of this part, and all of it
     if (C > 1) {
+      if (!peers_run) { cluster.barrier_wait(); peers_run = true; }
       if (tid < C) *cluster.map_shared_rank(&s_part[rank], tid) = total;
       cluster.sync();
       int owner = -1;
@@ -206,6 +211,7 @@ __global__ void __launch_bounds__(MN_NT, 4) multinomial_rows_kernel(MultinomialA
     }
     if (tid == 0) { M.out_ids[row] = id; if (M.out_flags) M.out_flags[row] = fl; }
   }
+  if (!peers_run) cluster.barrier_wait();                  // (no row of this cluster came to its store)
 }
 
 }  // namespace gs

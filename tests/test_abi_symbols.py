@@ -77,3 +77,24 @@ def test_comm_entry_points_fail_cleanly():
     rc = lib.gorch_cuda_sample_vocab_sharded_dev(None, None, 0, 1, 1, 1, 0, 1, 0, None, None, None, None, C.byref(err))
     assert rc == 1
     lib.gorch_cuda_free_string(err)
+
+
+def test_no_kernel_touches_a_peers_shared_memory_before_it_is_known_to_run():
+    """A CTA may write to (or read from) another one's shared memory only after a cluster barrier has shown that
+    the other one has started: in every kernel a barrier's wait comes before the first access through a mapped address."""
+    csrc = os.path.join(ROOT, "gorch_b200", "csrc")
+    seen = []
+    for name in sorted(os.listdir(csrc)):
+        with open(os.path.join(csrc, name)) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        for body in re.split(r"\b__global__\b", text)[1:]:
+            if "map_shared_rank" not in body:
+                continue
+            mapped = re.findall(r"(\w+) = cluster\.map_shared_rank", body)
+            uses = [m.start() for m in re.finditer(r"\*cluster\.map_shared_rank", body)]
+            for var in mapped:
+                uses += [m.start() for m in re.finditer(rf"\b{var}\s*(->|\[)", body)]
+            waits = [m.start() for m in re.finditer(r"cluster\.(barrier_wait|sync)\(\)", body)]
+            assert waits and uses and min(waits) < min(uses), name
+            seen.append(name)
+    assert {"index_ops.cuh", "row_softmax.cuh", "sample_cluster.cuh"} <= set(seen)
