@@ -296,6 +296,13 @@ bool is_pinned(const void* p) {
   return at.type == cudaMemoryTypeHost;
 }
 
+// Whether what is queued on the stream runs or goes into a graph; Invalidated where the stream cannot be asked.
+cudaStreamCaptureStatus capture_status(cudaStream_t stream) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) { cudaGetLastError(); st = cudaStreamCaptureStatusInvalidated; }
+  return st;
+}
+
 int check_shape(int dtype, int64_t B, int64_t V, int64_t row_stride, char** errOut) {
   if (dtype != GORCH_CUDA_F32 && dtype != GORCH_CUDA_BF16) {
     set_err(errOut, "gorch_cuda: unknown dtype %d", dtype);
@@ -1610,7 +1617,21 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
     if ((r2 = launch_lm_head(c, u, errOut))) return r2;
     return launch_rows(c, c->lmh_logits.ptr, GORCH_CUDA_F32, B, V, ld, cfgs, uniforms, out_ids, out_flags, nullptr, nullptr, 0, errOut);
   };
-  if (fuse_top_k < 1 || fuse_top_k > gs::KFAST || V < 4096 || B > 4096 || (K >= kLmhUnfusedK && B * V * 4 <= kLmhUnfusedBytes && !use_batch_mode(c->sm_count, B, V, 4, false))) return unfused();
+  if (fuse_top_k < 1 || fuse_top_k > gs::KFAST || V < 4096 || B > 4096) return unfused();
+  // From here on the call returns when the ids are there, whichever form serves it, and reports a projection that gave up.
+  auto ids_there = [&]() -> int {
+    CUDA_TRY(cudaStreamSynchronize(c->stream), errOut);
+    const uint32_t status = *static_cast<const volatile uint32_t*>(c->host_words);
+    if (status != 0) {
+      set_err(errOut, "gorch_cuda: the LM-head kernel gave up a bounded wait (status %u)", status);
+      return GORCH_CUDA_ERR_CUDA;
+    }
+    return GORCH_CUDA_OK;
+  };
+  if (K >= kLmhUnfusedK && B * V * 4 <= kLmhUnfusedBytes && !use_batch_mode(c->sm_count, B, V, 4, false)) {
+    rc = unfused();
+    return (rc || capture_status(c->stream) == cudaStreamCaptureStatusActive) ? rc : ids_there();   // (recorded into a graph: nothing runs that could be waited for)
+  }
   // the sample: 1/32 of the vocabulary, but 1024 to 4096 logits, in whole tiles
   int64_t want = V / 32;
   if (want < gs::LMH_SAMPLE_MIN) want = gs::LMH_SAMPLE_MIN;
@@ -1626,7 +1647,7 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
   const size_t total = off_cand + sizeof(uint2) * static_cast<size_t>(B) * gs::LMH_CAND_CAP;
   if ((rc = ensure(c->lmh_scratch, total, errOut))) return rc;
   unsigned char* base = static_cast<unsigned char*>(c->lmh_scratch.ptr);
-  c->host_words[0] = c->host_words[1] = 0u;                                  // (the call before this one was waited for)
+  c->host_words[1] = 0u;                                                     // (written by finish kernels only, whose calls waited for them; the projections clear [0])
   // 1. a sample of the vocabulary's tiles (all of them full tiles)
   gs::LmHeadArgs sa = a;
   sa.tile0 = 0; sa.tile_step = (ntile - 1) / stiles; sa.ntile = stiles;
@@ -1659,15 +1680,12 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
   c->counters.rows += static_cast<uint64_t>(B);
   // rows the fused form could not finish (their estimate failed, or their config is not served): the
   // count comes back to the host, which then recomputes the batch through the unfused form
-  CUDA_TRY(cudaStreamSynchronize(c->stream), errOut);
-  const volatile uint32_t* host_word = c->host_words;
-  if (host_word[0] != 0) {
-    set_err(errOut, "gorch_cuda: the LM-head kernel gave up a bounded wait (status %u)", host_word[0]);
-    return GORCH_CUDA_ERR_CUDA;
-  }
-  if (host_word[1] > 0) {
-    c->counters.lm_head_refused_rows += static_cast<uint64_t>(host_word[1]);
-    return unfused();
+  if ((rc = ids_there())) return rc;
+  const uint32_t refused = *static_cast<const volatile uint32_t*>(c->host_words + 1);
+  if (refused > 0) {
+    c->counters.lm_head_refused_rows += static_cast<uint64_t>(refused);
+    rc = unfused();
+    return rc ? rc : ids_there();
   }
   return GORCH_CUDA_OK;
 }

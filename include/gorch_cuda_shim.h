@@ -369,13 +369,15 @@ int gorch_cuda_lm_head_status(GorchCudaCtxRef ctx, uint32_t* status, char** errO
  * x @ w^T under cfgs[b] with uniforms[b], as gorch_cuda_sample_dev would return on the materialised
  * logits. fuse_top_k in 1..256: the batch's largest top_k; rows with temperature 0 or 0 < top_k <=
  * fuse_top_k (DefaultGenerateConfig: T = 0.8, k = 40) are finished from candidate lists that the
- * projection's epilogue fills, and the [B, V] logits are never written; the call then blocks until
- * the ids are there, and if a row could not be finished that way (top_k off or above fuse_top_k, or
- * a row whose largest logits a sample of the vocabulary misjudged) the whole batch is redone through
- * the unfused form. fuse_top_k == 0 (or a vocabulary below 4096 columns, or more than 4096 rows): the
- * unfused form at once:
- * logits into scratch memory of the context, then the kernels of gorch_cuda_sample_dev
- * (asynchronous). */
+ * projection's epilogue fills, and the [B, V] logits are never written; a batch of few logits (at most
+ * 20 MB, and K >= 512) is served by the unfused form all the same, which is then the faster one. The
+ * call blocks until the ids are there, and returns GORCH_CUDA_ERR_CUDA when a bounded device-side wait
+ * ran out. If a row could not be finished from its list (top_k off or above fuse_top_k, or a row whose
+ * largest logits a sample of the vocabulary misjudged) the whole batch is redone through the unfused
+ * form before the call returns. fuse_top_k == 0 (or a vocabulary below 4096 columns, or more than 4096
+ * rows): the unfused form at once: logits into scratch memory of the context, then the kernels of
+ * gorch_cuda_sample_dev (asynchronous; so is a batch of few logits that is being recorded into a
+ * stream capture; the fused form cannot be recorded). */
 int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ldx, const void* w, int64_t ldw,
                                   int64_t B, int64_t V, int64_t K, int fuse_top_k, const GorchSampleCfg* cfgs,
                                   const double* uniforms, int32_t* out_ids, uint32_t* out_flags, char** errOut);

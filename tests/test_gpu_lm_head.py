@@ -123,6 +123,65 @@ def test_few_logits_are_sampled_from_scratch(_sampler_session, oracle, B, V, K):
     assert rep["id_mismatch"] == rep["boundary_mismatch"]
 
 
+@pytest.mark.parametrize("B,V,K,kinds", [(100, 50257, 512, [(0.8, 40, 0.0, MODE_A)]), (64, 50257, 128, [(0.8, 40, 0.0, MODE_A)]),
+                                         (64, 50257, 128, [(0.8, 40, 0.0, MODE_A), (1.0, 0, 0.9, MODE_B)])])
+def test_the_ids_are_there_when_the_call_returns(_sampler_session, oracle, B, V, K, kinds):
+    """Few logits (sampled from scratch), the fused form, and a batch that it hands back: behind milliseconds of work
+    that is already queued, the ids are read without a sync, on a stream that does not wait for the context's."""
+    import torch
+    s = _sampler_session
+    s.set_kernel_variant(0, 0)
+    xb, wb = _inputs(B, V, K, 7500 + B)
+    uniforms = np.random.default_rng(B).random(B)
+    cfgs = _cfgs(B, kinds)
+    ora = oracle.sample_batch(_project(s, torch, xb, wb), cfgs, uniforms, flags=oracle.FAST_KTH, threads=oracle.hw_threads())
+    dx, dw = _dev(torch, xb), _dev(torch, wb)
+    dc = torch.from_numpy(cfgs.view(np.uint8).reshape(B, 16).copy()).cuda()
+    du = torch.from_numpy(uniforms.copy()).cuda()
+    ids = torch.full((B,), -7, dtype=torch.int32, device="cuda")
+    flags = torch.zeros(B, dtype=torch.int32, device="cuda")
+    out = torch.empty((B, V), dtype=torch.float32, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(100):
+        s.lm_head_logits_ptrs(dx.data_ptr(), K, dw.data_ptr(), K, B, V, K, out.data_ptr(), V)
+    s.lm_head_sample_ptrs(dx.data_ptr(), K, dw.data_ptr(), K, B, V, K, 100, dc.data_ptr(), du.data_ptr(), ids.data_ptr(), flags.data_ptr())
+    got = {"ids": ids.cpu().numpy(), "flags": flags.cpu().numpy().view(np.uint32)}
+    rep = compare(got, ora, uniforms, check_probs=False, allow_tie_cut=True)
+    assert rep["id_mismatch"] == rep["boundary_mismatch"]
+
+
+def test_few_logits_recorded_into_a_graph(_sampler_session, oracle):
+    """A batch that is sampled from scratch can be recorded: the call then waits for nothing."""
+    import torch
+    s = _sampler_session
+    B, V, K = 8, 8192, 512
+    xb, wb = _inputs(B, V, K, 7600)
+    uniforms = np.random.default_rng(B).random(B)
+    cfgs = _cfgs(B, [(0.8, 40, 0.0, MODE_A)])
+    ora = oracle.sample_batch(_project(s, torch, xb, wb), cfgs, uniforms, flags=oracle.FAST_KTH, threads=oracle.hw_threads())
+    dx, dw = _dev(torch, xb), _dev(torch, wb)
+    dc = torch.from_numpy(cfgs.view(np.uint8).reshape(B, 16).copy()).cuda()
+    du = torch.from_numpy(uniforms.copy()).cuda()
+    ids = torch.full((B,), -7, dtype=torch.int32, device="cuda")
+    flags = torch.zeros(B, dtype=torch.int32, device="cuda")
+    call = lambda: s.lm_head_sample_ptrs(dx.data_ptr(), K, dw.data_ptr(), K, B, V, K, 40, dc.data_ptr(), du.data_ptr(), ids.data_ptr(), flags.data_ptr())
+    call()                                     # (grows the context's scratch memory)
+    ids.fill_(-7)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    try:
+        with torch.cuda.graph(graph):
+            s.set_stream(torch.cuda.current_stream().cuda_stream)
+            call()
+    finally:
+        s.set_stream(None)
+    assert (ids.cpu().numpy() == -7).all()
+    graph.replay()
+    torch.cuda.synchronize()
+    rep = compare({"ids": ids.cpu().numpy(), "flags": flags.cpu().numpy().view(np.uint32)}, ora, uniforms, check_probs=False, allow_tie_cut=True)
+    assert rep["id_mismatch"] == rep["boundary_mismatch"]
+
+
 def test_rows_the_fused_form_does_not_serve_fall_back(_sampler_session, oracle):
     import torch
     s = _sampler_session
