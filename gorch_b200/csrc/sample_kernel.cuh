@@ -1233,14 +1233,14 @@ __device__ __noinline__ void single_cta_row(const KernelArgs& A, const int64_t r
   finish(id, flags, dbg);
 }
 
-// One CTA per row; with a work list, a fixed grid walks the listed rows.
 // Programmatic dependent launch: wait for the kernel before this one in the stream; let the next one start.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Header of a sorted batch: row cursors and the count of handed-over rows (BatchArgs). Every call finds it cleared: the
 // last CTA of the call's last kernel leaves it so, which a memset before the call's first kernel did at the price
-// of one more step on the GPU's queue (about 2 us).
+// of one more step on the GPU's queue (about 2 us). So no two calls of a context may overlap: they share a stream, or
+// are ordered where the context changes it (gorch_cuda_set_stream).
 constexpr int HDR_NARROW = 2, HDR_WIDE = 3, HDR_LEFT = 4, HDR_COUNT = 15;
 __device__ __forceinline__ void leave_batch(int32_t* hdr) {
   if (threadIdx.x == 0) {
@@ -1251,6 +1251,7 @@ __device__ __forceinline__ void leave_batch(int32_t* hdr) {
   }
 }
 
+// One CTA per row; with a work list, a fixed grid walks the listed rows.
 template <typename T>
 __global__ void __launch_bounds__(NT, 2) sample_rows_kernel(const __grid_constant__ KernelArgs A) {
   extern __shared__ __align__(16) unsigned char pool[];

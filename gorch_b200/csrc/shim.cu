@@ -153,6 +153,9 @@ struct Ctx {
   int comm_rank = 0, comm_nranks = 0;
   cudaEvent_t ev_vs[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t ev_left = nullptr;     // the end of the work on the stream that gorch_cuda_set_stream left ...
+  bool left_pending = false;         // ... which no later stream waits for yet
+  uint64_t waited_launches = 0;      // counters.kernel_launches when the context was last waited for
   int timing = 0;
   int variant = 0;        // 0: by batch size, 1: single-CTA kernel, 2: narrow/wide kernels, 3: cluster kernel,
                           // 4 / 5: as 2 with the wide kernel's 256- / 1024-thread instance forced,
@@ -301,6 +304,13 @@ cudaStreamCaptureStatus capture_status(cudaStream_t stream) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) { cudaGetLastError(); st = cudaStreamCaptureStatusInvalidated; }
   return st;
+}
+
+// Waits for the context's stream.
+cudaError_t wait_stream(Ctx* c) {
+  const cudaError_t e = cudaStreamSynchronize(c->stream);
+  if (e == cudaSuccess) c->waited_launches = c->counters.kernel_launches;
+  return e;
 }
 
 int check_shape(int dtype, int64_t B, int64_t V, int64_t row_stride, char** errOut) {
@@ -596,7 +606,7 @@ int host_run(Ctx* c, const void* logits, int dtype, int64_t B, int64_t V, int64_
   rc = launch_rows(c, dev_logits, dtype, B, V, row_stride, reinterpret_cast<const GorchSampleCfg*>(pin + off_cfgs),
                    reinterpret_cast<const double*>(pin + off_uni), pin_ids, out_flags ? pin_flags : nullptr, nullptr, nullptr, force_greedy, errOut);
   // (also after an error: the block is the next call's, and copies out of it may be under way)
-  const cudaError_t waited = cudaStreamSynchronize(c->stream);
+  const cudaError_t waited = wait_stream(c);
   if (rc) return rc;
   CUDA_TRY(waited, errOut);
   memcpy(out_ids, pin_ids, B * sizeof(int32_t));
@@ -756,6 +766,7 @@ GorchCudaCtxRef gorch_cuda_create_ctx(int device, char** errOut) {
   c->stream = c->own_stream;
   if ((e = cudaEventCreate(&c->ev0)) != cudaSuccess) return fail("cudaEventCreate", e);
   if ((e = cudaEventCreate(&c->ev1)) != cudaSuccess) return fail("cudaEventCreate", e);
+  if ((e = cudaEventCreateWithFlags(&c->ev_left, cudaEventDisableTiming)) != cudaSuccess) return fail("cudaEventCreate", e);
   {
     // device address of the fixed work-list array of gorch_cuda_sample_dev_static on this device
     int32_t* unused = nullptr;
@@ -829,6 +840,7 @@ void gorch_cuda_release(GorchCudaCtxRef ctx) {
   for (cudaEvent_t e : c->ev_vs) if (e) cudaEventDestroy(e);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);
+  if (c->ev_left) cudaEventDestroy(c->ev_left);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   g_pool.leave();
   delete c;
@@ -839,14 +851,29 @@ void gorch_cuda_free_string(char* s) { free(s); }
 int gorch_cuda_sync(GorchCudaCtxRef ctx, char** errOut) {
   Ctx* c = static_cast<Ctx*>(ctx);
   if (!c) { set_err(errOut, "gorch_cuda: null context"); return GORCH_CUDA_ERR_BAD_ARG; }
-  CUDA_TRY(cudaStreamSynchronize(c->stream), errOut);
+  CUDA_TRY(wait_stream(c), errOut);
   return GORCH_CUDA_OK;
 }
 
 int gorch_cuda_set_stream(GorchCudaCtxRef ctx, void* stream, int external, char** errOut) {
   Ctx* c = static_cast<Ctx*>(ctx);
   if (!c) { set_err(errOut, "gorch_cuda: null context"); return GORCH_CUDA_ERR_BAD_ARG; }
-  c->stream = external ? static_cast<cudaStream_t>(stream) : c->own_stream;
+  const cudaStream_t next = external ? static_cast<cudaStream_t>(stream) : c->own_stream;
+  if (next == c->stream) return GORCH_CUDA_OK;
+  CUDA_TRY(cudaSetDevice(c->device), errOut);
+  // Scratch memory and the header of the work lists, which a sorted batch finds cleared and leaves cleared, serve one call
+  // at a time: what is queued and was not waited for comes before whatever the next stream gets. A stream that is
+  // being recorded takes no part (its work runs when the graph does); the event then waits for the stream after it.
+  if (c->counters.kernel_launches != c->waited_launches && capture_status(c->stream) == cudaStreamCaptureStatusNone) {
+    if (c->left_pending) CUDA_TRY(cudaStreamWaitEvent(c->stream, c->ev_left, 0), errOut);
+    CUDA_TRY(cudaEventRecord(c->ev_left, c->stream), errOut);
+    c->left_pending = true;
+  }
+  c->stream = next;
+  if (c->left_pending && capture_status(next) == cudaStreamCaptureStatusNone) {
+    CUDA_TRY(cudaStreamWaitEvent(next, c->ev_left, 0), errOut);
+    c->left_pending = false;
+  }
   return GORCH_CUDA_OK;
 }
 
@@ -1142,7 +1169,7 @@ int gorch_cuda_comm_release(GorchCudaCtxRef ctx, char** errOut) {
   if (!c) { set_err(errOut, "gorch_cuda: null context"); return GORCH_CUDA_ERR_BAD_ARG; }
   if (!c->comm) return GORCH_CUDA_OK;
   CUDA_TRY(cudaSetDevice(c->device), errOut);
-  CUDA_TRY(cudaStreamSynchronize(c->stream), errOut);
+  CUDA_TRY(wait_stream(c), errOut);
   ncclComm_t comm = c->comm;
   c->comm = nullptr;
   c->comm_nranks = 0;
@@ -1620,7 +1647,7 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
   if (fuse_top_k < 1 || fuse_top_k > gs::KFAST || V < 4096 || B > 4096) return unfused();
   // From here on the call returns when the ids are there, whichever form serves it, and reports a projection that gave up.
   auto ids_there = [&]() -> int {
-    CUDA_TRY(cudaStreamSynchronize(c->stream), errOut);
+    CUDA_TRY(wait_stream(c), errOut);
     const uint32_t status = *static_cast<const volatile uint32_t*>(c->host_words);
     if (status != 0) {
       set_err(errOut, "gorch_cuda: the LM-head kernel gave up a bounded wait (status %u)", status);
@@ -1694,7 +1721,7 @@ int gorch_cuda_lm_head_status(GorchCudaCtxRef ctx, uint32_t* status, char** errO
   Ctx* c = static_cast<Ctx*>(ctx);
   if (!c || !status) { set_err(errOut, "gorch_cuda: null argument"); return GORCH_CUDA_ERR_BAD_ARG; }
   CUDA_TRY(cudaSetDevice(c->device), errOut);
-  CUDA_TRY(cudaStreamSynchronize(c->stream), errOut);
+  CUDA_TRY(wait_stream(c), errOut);
   *status = *static_cast<const volatile uint32_t*>(c->host_words);
   return GORCH_CUDA_OK;
 }

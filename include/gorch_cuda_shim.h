@@ -101,7 +101,10 @@ void gorch_cuda_free_string(char* s);
 int gorch_cuda_sync(GorchCudaCtxRef ctx, char** errOut);
 /* external != 0: run the context's work on the caller-owned CUDA stream
  * `stream` (a cudaStream_t as void*; NULL is the legacy default stream).
- * external == 0: go back to the context's own stream. */
+ * external == 0: go back to the context's own stream. Work that the context has queued on the stream it
+ * leaves, and that no gorch_cuda_sync or blocking call of the context has waited for, comes before
+ * what it queues on the new one; that stream must then still exist (without such work it is not looked
+ * at). A stream that is being recorded into a graph is left out of this order. */
 int gorch_cuda_set_stream(GorchCudaCtxRef ctx, void* stream, int external, char** errOut);
 /* Record device time of each call into counters.last_kernel_ms (adds a sync). */
 int gorch_cuda_set_timing(GorchCudaCtxRef ctx, int on);
