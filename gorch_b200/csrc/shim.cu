@@ -1365,12 +1365,17 @@ int gorch_cuda_multinomial_dev(GorchCudaCtxRef ctx, const float* probs, int64_t 
   m.probs = probs; m.row_stride = row_stride; m.V = static_cast<int32_t>(V);
   m.uniforms = uniforms; m.out_ids = out_ids; m.out_flags = out_flags; m.B = B;
   // CTAs per row: more while the batch still fits the GPU at two CTAs per SM and a thread keeps four vectors (us, one CTA |
-  // so: 8 x 151,936: 34 | 12; 64 x 151,936: 35 | 23; 8 x 50,257: 15 | 9). Long rows of large batches go by halves, for the
-  // sake of the last round (512 x 151,936: 87 | 79).
+  // so: 8 x 151,936: 34 | 12; 64 x 151,936: 35 | 23; 8 x 50,257: 15 | 9).
   const int64_t slots = 4 * c->sm_count;
   int C = 1;
   while (C < gs::MN_MAX_C && B * 2 * C <= 2 * c->sm_count && V / (2 * C) >= 4 * 4 * gs::MN_NT) C *= 2;
-  if (B > 2 * c->sm_count && V >= 100000) C = 2;
+  // Long rows of larger batches go by halves where that saves half a round over the SMs: where at most half the SMs would get one
+  // row more than the others. us, one CTA | two, 151,936: 297 rows 62 | 54, 370: 62 | 56, 512: 78 | 73, 666: 95 | 90, and
+  // without that half round 371: 62 | 63, 444: 62 | 64, 592: 78 | 82, 1024: 125 | 135. Shorter rows leave less to gain than the
+  // pair's exchange costs, and half a round is less of more rounds: 100,000: 297 rows 43 | 39, 512: 55 | 53, 666: 66 | 66, but 800:
+  // 76 | 78; 70,000: 512: 41 | 42. Beyond five rounds, 151,936: 800 rows 111 | 109, 960: 125 | 127, 1200: 170 | 162, 2400: 322 | 310.
+  const int64_t odd = B % c->sm_count;
+  if (V >= (B <= 5 * c->sm_count ? 100000 : 150000) && B > 2 * c->sm_count && odd > 0 && 2 * odd <= c->sm_count) C = 2;
   const int64_t clusters = (C > 1 || B < slots) ? B : slots;
   // (not beside the end of the kernel before it: its CTAs would crowd on the SMs that are free first. 64 x 151,936 behind a
   // softmax: 105 us instead of 60)

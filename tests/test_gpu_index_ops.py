@@ -131,7 +131,7 @@ def test_multinomial_nan_row_falls_through(sampler, oracle):
     assert ids.tolist() == oracle.multinomial(p, u).tolist()
 
 
-@pytest.mark.parametrize("B,V", [(1, 32767), (3, 32768), (8, 151936), (36, 65536), (37, 65537), (148, 50257), (297, 100001), (2, 524000)])
+@pytest.mark.parametrize("B,V", [(1, 32767), (3, 32768), (8, 151936), (36, 65536), (37, 65537), (148, 50257), (297, 100001), (370, 100000), (371, 100000), (2, 524000)])
 def test_multinomial_rows_shared_by_several_ctas(sampler, oracle, B, V):
     """Edges of the rule that shares rows out; uniforms at the row's ends; a NaN ahead of the drawn token and behind it."""
     rng = np.random.Generator(np.random.Philox(key=B * 31 + V))
