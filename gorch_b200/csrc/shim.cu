@@ -58,8 +58,9 @@ inline bool use_batch_mode(int sm_count, int64_t B, int64_t V, int64_t elem_byte
 
 // LM head with sampling: up to this many bytes of logits they are written to scratch, where the cluster kernel finds them in
 // L2. The fused form saves that traffic and pays for it with two more kernels and a second run over part of the weights
-// (us, fused | this: 64 x 50,257, K = 1024: 65 | 48; 96: 67 | 52; 16 x 151,936, K = 512: 75 | 60; 32: 76 | 65; K = 2048,
-// 16: 150 | 133). Beyond it the batch kernels would serve the rows: 128 x 50,257: 70 | 77. Measured from K = 512 on.
+// (us a call with its wait, fused | this: 64 x 50,257, K = 1024: 62 | 51; 96: 66 | 57; 104: 66 | 59; 16 x 151,936, K = 512:
+// 67 | 58; 32: 67 | 64; K = 2048, 16: 135 | 123; 16 x 4,096, K = 512: 42 | 31). Beyond it the two meet: 110 x 50,257, K = 1024:
+// 64 | 60; 128: 64 | 65; 40 x 151,936, K = 512: 68 | 69.
 constexpr int64_t kLmhUnfusedBytes = 20ll << 20, kLmhUnfusedK = 512;
 
 struct Buffer {
@@ -697,8 +698,10 @@ int lm_head_args(const Ctx* c, gs::LmHeadArgs& a, const void* x, int64_t ldx, co
   return make_bf16_map(&a.map_w, w, V, K, ldw, a.cta_v, errOut);
 }
 
-// One launch of lm_head_kernel over the vocabulary tiles tile0 + i * step, i < ntile.
-int launch_lm_head(Ctx* c, gs::LmHeadArgs& a, char** errOut, bool dependent = false) {
+// One launch of lm_head_kernel over the vocabulary tiles tile0 + i * step, i < ntile. chained: behind the kernel that fills the
+// thresholds. dependent: it may start beside the end of the kernel before it (the first one of a chain does not: the
+// chain's second projection reads x and w without waiting for what came before the chain).
+int launch_lm_head(Ctx* c, gs::LmHeadArgs& a, char** errOut, bool dependent, bool chained = false) {
   const int64_t ntile_total = (static_cast<int64_t>(a.V) + 2 * a.cta_v - 1) / (2 * a.cta_v);
   if (a.ntile < 1 || a.tile0 + static_cast<int64_t>(a.ntile - 1) * a.tile_step >= ntile_total) {
     set_err(errOut, "gorch_cuda: LM head tile range outside the vocabulary");
@@ -708,8 +711,8 @@ int launch_lm_head(Ctx* c, gs::LmHeadArgs& a, char** errOut, bool dependent = fa
   int npairs = gs::LmhPlan(a.B, a.ntile, a.item_n, most).total;
   if (npairs > most) npairs = most;
   a.status = c->host_words;
-  a.chained = dependent ? 1 : 0;
-  a.clear_status = dependent ? 0 : 1;
+  a.chained = chained ? 1 : 0;
+  a.clear_status = chained ? 0 : 1;
   CUDA_TRY(launch(c, gs::lm_head_kernel, static_cast<unsigned>(2 * npairs), gs::LMH_NT, gs::LMH_DYN_BYTES, dependent, a), errOut);
   c->counters.kernel_launches += 1;
   return GORCH_CUDA_OK;
@@ -1620,7 +1623,7 @@ int gorch_cuda_lm_head_logits_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
   if ((rc = lm_head_args(c, a, x, ldx, w, ldw, B, V, K, true, errOut))) return rc;
   a.tile0 = 0; a.tile_step = 1; a.ntile = static_cast<int32_t>((V + 2 * a.cta_v - 1) / (2 * a.cta_v));
   a.out_logits = out_logits; a.ld_out = ld_out; a.compact = 0;
-  return launch_lm_head(c, a, errOut);
+  return launch_lm_head(c, a, errOut, true);
 }
 
 int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ldx, const void* w, int64_t ldw, int64_t B,
@@ -1646,7 +1649,7 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
     if ((r2 = lm_head_args(c, u, x, ldx, w, ldw, B, V, K, true, errOut))) return r2;
     u.tile0 = 0; u.tile_step = 1; u.ntile = static_cast<int32_t>((V + 2 * u.cta_v - 1) / (2 * u.cta_v));
     u.out_logits = static_cast<float*>(c->lmh_logits.ptr); u.ld_out = ld; u.compact = 0;
-    if ((r2 = launch_lm_head(c, u, errOut))) return r2;
+    if ((r2 = launch_lm_head(c, u, errOut, true))) return r2;
     return launch_rows(c, c->lmh_logits.ptr, GORCH_CUDA_F32, B, V, ld, cfgs, uniforms, out_ids, out_flags, nullptr, nullptr, 0, errOut);
   };
   if (fuse_top_k < 1 || fuse_top_k > gs::KFAST || V < 4096 || B > 4096) return unfused();
@@ -1684,7 +1687,7 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
   gs::LmHeadArgs sa = a;
   sa.tile0 = 0; sa.tile_step = (ntile - 1) / stiles; sa.ntile = stiles;
   sa.out_logits = reinterpret_cast<float*>(base + off_smp); sa.ld_out = nsample; sa.compact = 1;
-  if ((rc = launch_lm_head(c, sa, errOut))) return rc;
+  if ((rc = launch_lm_head(c, sa, errOut, false))) return rc;
   // 2. thresholds
   gs::LmhSampleArgs fa;
   memset(&fa, 0, sizeof fa);
@@ -1704,7 +1707,7 @@ int gorch_cuda_lm_head_sample_dev(GorchCudaCtxRef ctx, const void* x, int64_t ld
   ma.tile0 = 0; ma.tile_step = 1; ma.ntile = ntile;
   ma.out_logits = nullptr; ma.ld_out = 0; ma.compact = 0;
   ma.thr = fa.thr; ma.cand = reinterpret_cast<uint2*>(base + off_cand); ma.rows = fa.rows;
-  if ((rc = launch_lm_head(c, ma, errOut, true))) return rc;
+  if ((rc = launch_lm_head(c, ma, errOut, true, true))) return rc;
   // 4. finish every row from its candidates
   CUDA_TRY(launch(c, gs::lmh_finish_kernel, g, gs::LMH_F_NT, gs::LMH_F_DYN_BYTES, true, fa), errOut);
   c->counters.kernel_launches += 2;
