@@ -10,7 +10,7 @@ entry point, CUDA events on the launching stream); `e2e` is the same metric
 through the host-pointer C-ABI call with pinned host buffers, copies inside
 the timed region. After the timed region rank 0 compares the timed call's ids
 with the CPU oracle and reports the counts under `parity`. At N=1 the same JSON
-line also carries `configs` (every other BASELINE config, 20 timed steps each,
+line also carries `configs` (every other workload, 20 timed steps each,
 with its own parity counts) and `ops` (TopK, Multinomial, softmax, log-softmax,
 cross-entropy forward / backward on 512 x 151,936 f32). `--impl reference`
 times the CPU restatement of the reference's routines on the host cores. Under
@@ -288,7 +288,7 @@ def time_steps(torch, stream, fn, steps, warmup, flush):
 
 
 def configs_leg(torch, smp, stream, flush, peak, skip):
-    """Every BASELINE config except the headline: 20 timed steps each after 3 warm-up steps, L2 flushed
+    """Every workload except the headline: 20 timed steps each after 3 warm-up steps, L2 flushed
     between steps where the batch fits in it; step time, rows/s, algorithmic GB/s, fraction of the HBM
     peak, and the parity counts of the last timed call."""
     from gorch_b200 import workloads

@@ -41,13 +41,22 @@ constexpr int64_t kSliceCap = 109 * 1024 - gs::REGION_A - gs::REGION_B;
 
 // Batches go to the sorted-batch kernels (one CTA per row) from this many rows or bytes on; smaller ones to
 // the cluster kernel (several CTAs per row), whose latency is lower while the GPU is not full. The rows' kinds are
-// on the device, so one line serves them all, and it lies where rows with a top-p cut do not lose. us, batch | cluster:
-//   128 x 50,257 f32: top-k 44 | 31, greedy 28 | 18, mixed 52 | 37, nucleus without a cut 44 | 37, with one 67 | 85
-//   64 x 151,936 f32: 54 | 33, 48 | 20, 69 | 42, 71 | 45, 101 | 93; at 96 rows the last pair is 110 | 137
-// Short rows stay with the clusters for longer: two waves of them (one CTA per row, two per SM) up to 4,096 logits
-//   512 x 4,000 f32: 38 | 27, 19 | 16, 52 | 40, 38 | 29, 54 | 57 (16,000: 44 | 31, 28 | 19, 79 | 38, 43 | 40, 65 | 76)
-// and, where the batch kernels need a second round of wide rows, three waves up to 16,384:
-//   768 x 16,000 f32: 46 | 42, 28 | 25, 122 | 49, 75 | 57, 116 | 108; 1024: 50 | 52, 32 | 29, 134 | 59, 79 | 69, 118 | 137
+// on the device, so one line serves them all. us, batch | cluster, calls back to back on inputs that are not in L2, for rows with
+// top-k, greedy ones, the two mixed with nucleus rows, plain softmax rows, and rows with a top-p cut (f32):
+//   112 x 50,257: 30 | 23, 20 | 12, 40 | 27, 33 | 30, 50 | 67;  256 x 50,257: 33 | 41, 23 | 22, 49 | 48, 49 | 58, 75 | 128
+//   32 x 151,936: 39 | 18, 31 | 9, 57 | 23, 57 | 22, 82 | 49;  64: 41 | 27, 32 | 15, 59 | 35, 63 | 39, 83 | 84;  128: 43 | 43, 35 | 25, 65 | 54,
+//   75 | 72, 101 | 159
+// Rows with a cut change sides long before the others, and the line stays near theirs. Bytes follow that only roughly: from 40 to 60
+// rows of 151,936 f32 the clusters would serve every kind sooner (48: 40 | 21, 32 | 12, 60 | 29, 58 | 36, 82 | 77), and behind the line the
+// other kinds pay (128 x 50,257: 30 | 24, 19 | 12, 41 | 30, 33 | 32, for 51 | 69).
+// Short rows stay with the clusters for longer. Up to four rows per SM of 4,096 logits, two waves of clusters:
+//   592 x 4,096: 25 | 21, 14 | 10, 36 | 28, 27 | 24, 43 | 44 (8,000 logits, 512 rows: 27 | 21, 16 | 11, 39 | 28, 29 | 27, 48 | 53)
+// Beyond four rows per SM, the wide kernel's slots, the batch kernels start a second round of wide rows (592 x 12,000: 29 | 23, 19 | 12,
+// 44 | 32, 34 | 31, 53 | 65; 593: 31 | 29, 20 | 14, 44 | 32, 47 | 38, 81 | 80): up to six rows per SM of 16,384 logits
+//   888 x 4,000: 24 | 31, 14 | 15, 46 | 39, 42 | 35, 70 | 64;  768 x 16,000: 33 | 34, 20 | 18, 107 | 43, 62 | 51, 100 | 111
+//   889 x 16,384: 34 | 41, 22 | 20, 109 | 48, 71 | 58, 128 | 128
+// Mixed batches gain most there; rows with a cut give some of it back from 15,000 f32 or 8,000 bf16 logits on (700 x 16,000: 96 | 99, bf16:
+// 90 | 98), beyond five rows per SM from 10,000 and 5,000 on, where top-k rows by themselves do too.
 // An argmax is one launch of the narrow kernel and keeps the lower line.
 constexpr int64_t kBatchModeRows = 384;
 constexpr int64_t kBatchModeBytes = 24ll << 20;
@@ -1451,8 +1460,8 @@ int gorch_cuda_generate_step_dev(GorchCudaCtxRef ctx, const void* logits, int dt
   return launch_generate_control(c, out_ids, out_flags, gc, B, errOut);
 }
 
-// CTAs per row of the resident softmax: the smallest power of two whose slice leaves room for two CTAs per SM, more while
-// the whole batch is resident at once; 0 when eight are too few.
+// CTAs per row of the resident softmax: as few as leave room for two slices per SM (any number up to eight), twice as many
+// while the whole batch is resident at once; 0 when eight are too few.
 static int softmax_cluster(const Ctx* c, int64_t B, int64_t V, int dtype) {
   const int64_t nvec = row_vectors(V, dtype);
   int C = 1;
