@@ -46,7 +46,7 @@ def test_topk_matches_oracle(sampler, oracle, B, V, k):
 @pytest.mark.parametrize("B,V,k", [(3, 300, 257), (2, 300, 300), (5, 5000, 1000), (6, 50257, 4096), (150, 151936, 300),
                                    (3, 151936, 16384), (4, 20000, 5000)])
 def test_topk_large_k_matches_oracle(_sampler_session, oracle, B, V, k):
-    """k beyond the one-pass kernel's lists: radix select of the k-th largest, gather, sort. Ties across
+    """Large k: candidates in one pass, places by bucket, and the exact form for rows tied too often. Ties across
     the k-th value (lowest indices win), a row of one value only, -Inf and NaN entries (ordered last)."""
     s = _sampler_session
     rng = np.random.Generator(np.random.Philox(key=B * 1000003 + V * 17 + k))
