@@ -80,6 +80,21 @@ __device__ __forceinline__ void min_i2(int& a, int& b, Scratch& s, int tid) {
   b = __reduce_min_sync(FULL, s.i1[l]);
 }
 
+// Three maxima with one pair of barriers.
+template <int NWARPS>
+__device__ __forceinline__ void max_u3(uint32_t& a, uint32_t& b, uint32_t& c, Scratch& s, int tid) {
+  a = __reduce_max_sync(FULL, a);
+  b = __reduce_max_sync(FULL, b);
+  c = __reduce_max_sync(FULL, c);
+  __syncthreads();
+  if ((tid & 31) == 0) { s.i0[tid >> 5] = static_cast<int>(a); s.i1[tid >> 5] = static_cast<int>(b); s.u[tid >> 5] = c; }
+  __syncthreads();
+  const int l = (tid & 31) < NWARPS ? (tid & 31) : 0;
+  a = __reduce_max_sync(FULL, static_cast<uint32_t>(s.i0[l]));
+  b = __reduce_max_sync(FULL, static_cast<uint32_t>(s.i1[l]));
+  c = __reduce_max_sync(FULL, static_cast<uint32_t>(s.u[l]));
+}
+
 __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {

@@ -44,7 +44,7 @@ constexpr int W_NW = W_NT / 32;
 constexpr int W_NB = 4096;              // histogram buckets
 constexpr int W_ZCAP = 2048;            // exact zone list capacity
 constexpr int W_D1 = 2;                 // steps of register prefetch in pass 1
-constexpr int W_G = 4;                  // steps per piece (power of two)
+constexpr int W_G = 8;                  // steps per piece (power of two)
 constexpr int W_MAX_STEPS = (W_NT >= 512) ? 64 : 128;         // steps per warp and pass; longer rows go to the single-CTA kernel
 constexpr int W_MAX_PPW = W_MAX_STEPS / W_G;
 constexpr int W_MAX_PIECES = W_NW * W_MAX_PPW;                 // 512
@@ -53,11 +53,25 @@ constexpr int W_EB_REP_ENTRIES = 128;   // entries of that layout: d > -(128-1)/
 constexpr int W_OFF_HIST = 0;
 constexpr int W_OFF_ZONE = W_OFF_HIST + W_NB * 4;
 constexpr int W_OFF_EB = W_OFF_ZONE + W_ZCAP * 8;              // 1024 entries, or 128 entries x 16 copies
-constexpr int W_OFF_PART = W_OFF_EB + W_EB_REP * W_EB_REP_ENTRIES * 8;
-constexpr int W_DYN_BYTES = W_OFF_PART + W_MAX_PIECES * 8;     // 52 KB
+// one pass: the lanes' buffers (of the last four slots only what fills one takes any), the warps' lists and where the pieces
+// begin in them, the ring of copies, the selection's buckets
+constexpr int W1_SLOTS = 16;
+constexpr int W1_WCAP = (W_NT >= 512) ? 256 : 512;
+constexpr int W1_RING_BYTES = 2 * W_NT * 32;
+constexpr int W1_BINS = W_NT;
+constexpr int W1_OFF_LIST = 0;
+constexpr int W1_OFF_BUF = W1_OFF_LIST + W_NW * W1_WCAP * 4;
+constexpr int W1_OFF_RING = W1_OFF_BUF + W1_SLOTS * W_NT * 4;
+constexpr int W1_OFF_MASS = W1_OFF_BUF;                        // after the pass: the listed logits' masses
+constexpr int W1_OFF_BINS = W1_OFF_RING + W1_RING_BYTES;
+constexpr int W1_OFF_FROM = W1_OFF_BINS + W1_BINS * 4;
+constexpr int W1_END = W1_OFF_FROM + W_NW * (W_MAX_PPW + 1) * 4;
+constexpr int W2_END = W_OFF_EB + W_EB_REP * W_EB_REP_ENTRIES * 8;
+constexpr int W_OFF_PART = W1_END > W2_END ? W1_END : W2_END;
+constexpr int W_DYN_BYTES = W_OFF_PART + W_MAX_PIECES * 8;     // 51 KB (1024 threads: 167 KB)
 static_assert(W_EB_REP * W_EB_REP_ENTRIES >= NB1, "either layout fits");
-static_assert(W_NT >= 256 && W_NT <= 1024 && W_MAX_PIECES <= W_NT && W_G * 64 <= W_NT && W_NSUB * 12 <= W_NB * 4,
-              "one piece / one vector of a piece / one sub-bucket per thread");
+static_assert(W_NT >= 256 && W_NT <= 1024 && W_MAX_PIECES <= W_NT && W_G * 64 <= 2 * W_NT && W_NSUB * 12 <= W_NB * 4,
+              "one piece / two vectors of a piece / one sub-bucket per thread");
 
 // Histogram buckets of width 1/scale (scale a power of two): bucket = round(-d * scale),
 // clamped to W_NB - 1. Multiplying by a power of two is exact, so the bucket edges are exact.
@@ -325,7 +339,130 @@ struct WideShared {
   int bc[4];
   int cnt;
   int row;
+  // one pass: the row, its window, and what the pass and the cut find
+  const uint4* vbase;
+  int V, shift, nvec;
+  int span, ppw;           // vectors of a warp's part of the row, pieces in it
+  float as, Tm, xA, xB;    // anchor in units of x / T; above the window: x >= xA; the window: xB <= x < xA
+  int low;                 // the window reaches down to where no mass is
+  double eps;              // relative error bound of the sums
+  double kw[W_NW];         // the mass above the window in each warp's part of the row (all its mass where the window is low),
+  double zw[W_NW];         // what the window adds to it,
+  double pm[W_MAX_PPW];    // kept mass of one warp's pieces
 };
+
+// How a row ends, from either form. `path`: 2 two passes, 3 one.
+struct WideResult {
+  float m;                 // largest x / T
+  double S, Re;            // all mass, kept mass
+  int path;
+};
+__device__ __forceinline__ void wide_write(const KernelArgs& A, int64_t row_id, const WideResult& r, int id, uint32_t flags,
+                                           double lo, double hi, int kept) {
+  A.out_ids[row_id] = id;
+  if (A.out_flags) A.out_flags[row_id] = flags;
+  if (A.out_debug) {
+    RowDebug d;
+    d.sum_exp = r.S; d.resum = r.Re / r.S; d.edge_lo = lo; d.edge_hi = hi; d.kept = kept;
+    d.max_scaled = r.m; d.threshold = __int_as_float(0x7fc00000); d.path = r.path;
+    for (int q = 0; q < 8; q++) d.reserved[q] = 0;
+    A.out_debug[row_id] = d;
+  }
+}
+// A row whose sum is no number (S NaN), or whose mode A cut removed every token (generate.go:221-227 divides by zero): every
+// comparison of the walk fails, result n-1 (:239).
+__device__ __noinline__ void wide_write_nothing_kept(const KernelArgs& A, int64_t row_id, float m, double S, int path, uint32_t flags) {
+  const double QNAN = __longlong_as_double(0x7ff8000000000000ll);
+  if (A.out_probs) {
+    double* pr = A.out_probs + row_id * static_cast<int64_t>(A.V);
+    for (int i = threadIdx.x; i < A.V; i += W_NT) pr[i] = QNAN;
+  }
+  WideResult r;
+  const bool number = S == S && S > 0.0;
+  r.m = m; r.S = number ? S : QNAN; r.Re = number ? 0.0 : r.S; r.path = path;
+  if (threadIdx.x == 0) wide_write(A, row_id, r, A.V - 1, flags | FLAG_NONFINITE | FLAG_FALLBACK, 0.0, 0.0, 0);
+}
+// The end of a row: u Re falls into piece `psel` or just behind it (rounding), `before` is the kept mass ahead of it
+// (psel 0x7fffffff: behind every piece). kept_mass(x, i): the kept mass of logit i, 0 when it is cut away.
+template <typename T, typename F>
+__device__ __forceinline__ void wide_draw(const KernelArgs& A, const int64_t row_id, const RowView<T>& rv, const int span, const int ppw,
+                                          const int psel, const double before, const double u, const WideResult& r, uint32_t flags,
+                                          WideShared& sh, F&& kept_mass) {
+  constexpr int VEC = Elem<T>::VEC, SV = 32 * (8 / VEC), PV = W_G * SV;
+  constexpr int NV = (PV + W_NT - 1) / W_NT;                 // vectors of a piece per thread
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int V = rv.V, npiece = W_NW * ppw;
+  int kept_n = 0;
+  if (A.out_probs || A.out_debug) {                          // parity runs only
+    double* pr = A.out_probs ? A.out_probs + row_id * static_cast<int64_t>(V) : nullptr;
+    const double rq = r.Re / r.S;
+    int kept_loc = 0;
+    for (int v = tid; v < rv.nvec; v += W_NT) {
+      float x[VEC];
+      Elem<T>::unpack(__ldg(rv.vbase + v), x);
+      const int i0 = v * VEC - rv.shift;
+#pragma unroll
+      for (int c = 0; c < VEC; c++) {
+        const int i = i0 + c;
+        if (i >= 0 && i < V) {
+          const double f = (kept_mass(x[c], i) / r.S) / rq;
+          kept_loc += (f > 0) ? 1 : 0;
+          if (pr) pr[i] = f;
+        }
+      }
+    }
+    kept_n = bu::sum_i<W_NW>(kept_loc, sh.sc, tid);
+  }
+  // draw (generate.go:231-239): u < prefix/Re is tested as u*Re < prefix
+  const double tgt = u * r.Re;
+  double run_end = before;
+  // walk pieces from the selected one (rounding can push the crossing into the next piece)
+  for (int pi = psel; pi < npiece; pi++) {                   // uniform; normally one trip
+    const int w = pi / ppw;
+    const int vb = w * span + (pi - w * ppw) * PV;
+    const int vend = min(min(vb + PV, w * span + span), rv.nvec);
+    const int j = vb + tid * NV;
+    double em[NV * VEC];
+    double tsum = 0.0;
+    const int i0 = j * VEC - rv.shift;
+#pragma unroll
+    for (int h = 0; h < NV; h++) {
+      const bool in = tid * NV + h < PV && j + h < vend;
+      float x[VEC];
+      Elem<T>::unpack(__ldg(rv.vbase + (in ? j + h : 0)), x);
+#pragma unroll
+      for (int c = 0; c < VEC; c++) { em[h * VEC + c] = in ? kept_mass(x[c], i0 + h * VEC + c) : 0.0; tsum += em[h * VEC + c]; }
+    }
+    if (tid == 0) sh.bc[3] = 0x7fffffff;
+    double totc;
+    const double ex = bu::scan_excl_d<W_NW>(tsum, totc, sh.sc, tid);
+    int pick = 0x7fffffff;
+    double run = run_end + ex, lo = 0.0, hi = 0.0;
+#pragma unroll
+    for (int c = 0; c < NV * VEC; c++) {
+      const double b = run;
+      run += em[c];
+      if (em[c] > 0.0 && tgt < run && pick == 0x7fffffff) { pick = i0 + c; lo = b; hi = run; }
+    }
+    const int first = __reduce_min_sync(FULL, pick);
+    if (lane == 0 && first != 0x7fffffff) atomicMin(&sh.bc[3], first);
+    __syncthreads();
+    const int id = sh.bc[3];
+    if (id != 0x7fffffff) {
+      if (pick == id) {
+        lo /= r.Re; hi /= r.Re;
+        if ((lo > 0.0 && u - lo <= 1e-6) || hi - u <= 1e-6) flags |= FLAG_BOUNDARY;
+        wide_write(A, row_id, r, id, flags, lo, hi, kept_n);
+      }
+      return;
+    }
+    run_end += totc;
+    __syncthreads();
+  }
+  const double end = run_end / r.Re;
+  if (u - end <= 1e-6) flags |= FLAG_BOUNDARY;
+  if (tid == 0) wide_write(A, row_id, r, V - 1, flags | FLAG_FALLBACK, end, end, kept_n);   // generate.go:239
+}
 
 // The exact cut for a zone that outgrew the shared list (long runs of equal logits around the
 // cut): the weighted selection of wide_row, with the row itself as the source of the zone's keys,
@@ -466,494 +603,11 @@ __device__ __noinline__ bool wide_big_zone(const WSpan& sp_in, const RowView<T>&
   return true;
 }
 
-// ---------------------------------------------------------------------------------------------
-// One-pass front end. Where a sample of the row (every eighth step of every warp) places the
-// top-p cut inside a narrow window of logit values, one pass over the row is enough: it sums the
-// mass of everything (S) and of what lies above the window (certainly kept, per piece) with the fast
-// exponential, relative to an anchor near the row maximum, and notes which lane-steps hold a logit
-// inside the window; those few vectors are read again (from L2) into the exact zone list, and the
-// tail decides the cut inside the window as it does after two passes. The sample only chooses the
-// window: whether the cut really lies inside it is checked on the sums of the whole row, and a row
-// whose window failed (or that the sample cannot place: a few heavy tokens, NaN, a wide window) takes
-// the two-pass front end. Rows without a cut need no window at all.
-//
-// Error budget of the fast sums against exp(d) in f64, d = x/T - max rounded to f32 as upstream:
-// ex2.approx 2.4e-7, three f32 additions per step before the f64 accumulators 1.8e-7, and per unit
-// of |x/T - anchor| the roundings of that difference, of d itself, of the product with log2(e) and
-// of the constant, 2e-7 together: W1_EPS_FIXED + W1_EPS_PER_D * (largest |d| that carries mass).
-// ---------------------------------------------------------------------------------------------
-constexpr int W1_STRIDE = 8;             // the sample: every eighth step
-#ifndef GS_W1_PF
-#define GS_W1_PF 10
-#endif
-constexpr int W1_PF = GS_W1_PF;          // steps ahead that the pass asks L2 for its lines (0: never)
-constexpr int W_ZCAP1 = 2 * W_ZCAP;      // zone list of the one-pass front end (zone + table areas)
-constexpr double W1_EPS_FIXED = 4.5e-7;
-constexpr double W1_EPS_PER_D = 2.0e-7;
-constexpr float W1_MAGIC = 2097152.0f;   // 2^21: floats in [2^21, 2^22) have an ulp of 1/4
-constexpr float W1_FCLAMP = 2097152.0f + 4095.75f;
-static_assert(W_OFF_EB == W_OFF_ZONE + W_ZCAP * 8 && W_EB_REP * W_EB_REP_ENTRIES * 8 >= W_ZCAP * 8, "the long zone list spans both areas");
+#include "sample_wide_onepass.cuh"
 
-__device__ __forceinline__ void l2_prefetch(const void* p) { asm volatile("prefetch.global.L2 [%0];" :: "l"(p)); }
-__device__ __forceinline__ float ex2_approx(float t) { float e; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t)); return e; }
-__device__ __forceinline__ float set_ge(float a, float b) { float r; asm("set.ge.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }   // 1.0f or 0.0f
-__device__ __forceinline__ float min3abs(float a, float b, float c) { float d; asm("min.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(fabsf(b)), "f"(fabsf(c))); return d; }
-
-// Histogram bucket of a raw logit: y = (anchor' - x) * hs, f = RN(hc - x * hs) rounds the exact
-// y + 2^21 to a multiple of 1/4 (one rounding, by fma); bits 2..13 of f are the bucket: y in
-// [b - 1/8, b + 7/8]. f is clamped from above (everything below the range, -Inf and NaN land in the
-// last bucket); a logit above the anchor leaves the binade and lands anywhere inside the array:
-// the caller checks the maximum it saw against the anchor.
-__device__ __forceinline__ uint32_t bucket_off1(float x, float nhs, float hc) {
-  return __float_as_uint(fminf(fmaf(x, nhs, hc), W1_FCLAMP)) & 0x3ffcu;
-}
-// Smallest float whose bucket is <= bmax (the buckets fall as x rises). +Inf: none; -Inf: every float.
-__device__ __forceinline__ float bucket_floor1(int bmax, float nhs, float hc, bool& ok) {
-  if (bmax >= W_NB - 1) return -INFINITY;
-  if (bmax < 0) return INFINITY;
-  float x = ((hc - W1_MAGIC) - (static_cast<float>(bmax) + 0.875f)) / (-nhs);
-  const uint32_t lim = static_cast<uint32_t>(bmax) * 4u + 3u;
-  int it = 0;
-  while (bucket_off1(x, nhs, hc) > lim && it < 24) { x = nextafterf(x, INFINITY); it++; }
-  while (it < 24) {
-    const float below = nextafterf(x, -INFINITY);
-    if (bucket_off1(below, nhs, hc) > lim) break;
-    x = below; it++;
-  }
-  if (it >= 24) ok = false;
-  return x;
-}
-// x / T in IEEE f32 round-to-nearest by q0 = x y, r = fma(-q0, T, x), q = fma(r, y, q0) with y = RN(1/T):
-// the correctly rounded quotient whenever T's significand is not all ones and nothing over- or underflows
-// (the caller takes this form for 2^-20 <= T <= 2^20 only and clamps x at -1e30: whatever lies below has
-// mass 0 either way).
-__device__ __forceinline__ f32x2_t div2_fast(f32x2_t X, float T, float y) {
-  const f32x2_t Y = pk2(y, y);
-  const f32x2_t Q0 = mul2(X, Y);
-  const f32x2_t R = fma2(Q0, pk2(-T, -T), X);
-  return fma2(R, Y, Q0);
-}
-
-struct OnePassOut {
-  float m;                 // row maximum of x / T
-  double S, Ktot;          // all mass; mass above the window (both relative to exp(m))
-  int nz;                  // zone entries in the list
-  float xA, xB;            // above the window: x >= xA; the window: xB <= x < xA
-  double eps;              // relative error bound of S and Ktot
-};
-struct P1Consts {
-  float as, Tm, yT;        // anchor in units of x / T; temperature and its rounded reciprocal
-  float xA, xB;            // above the window: x >= xA; the window: xB <= x < xA
-  float xmid, xhalf;       // |x - xmid| <= xhalf is a superset of the window
-  uint32_t zl_s, zcnt_s;   // shared-memory addresses of the window list (W_ZCAP1 entries of (logit bits, index)) and its counter
-};
-struct P1Acc {
-  double tot;              // running piece without a cut: all its mass; with a cut: all mass so far
-  double kep;              // with a cut: mass above the window of the running piece
-  double stot;             // without a cut: all mass of the pieces done
-  float vmax;              // NaN-propagating running maximum
-};
-
-// The window's logits of one lane-step go to the list. Only lanes that saw a logit near the window
-// come here; CHECK: the step may hold logits outside the row (index tested against V).
-template <int VEC, bool CHECK>
-__device__ __forceinline__ void p1_append(const float* x, int i_first, int V, const P1Consts& k) {
-#pragma unroll
-  for (int c = 0; c < 8; c++) {
-    if (x[c] < k.xA && x[c] >= k.xB) {                         // (masked logits are -Inf: never at or above a finite xB)
-      const int i = i_first + (c / VEC) * 32 * VEC + (c % VEC);
-      if (!CHECK || (i >= 0 && i < V)) {
-        uint32_t slot;
-        asm volatile("atom.shared.add.u32 %0, [%1], 1;" : "=r"(slot) : "r"(k.zcnt_s) : "memory");
-        if (slot < static_cast<uint32_t>(W_ZCAP1)) {
-          asm volatile("st.shared.v2.u32 [%0], {%1, %2};" :: "r"(k.zl_s + slot * 8u), "r"(__float_as_uint(x[c])), "r"(static_cast<uint32_t>(i)) : "memory");
-        }
-      }
-    }
-  }
-}
-
-// Eight logits of a lane: exp(x/T - anchor) = 2^((x/T - anchor) log2 e); masked logits are -Inf and
-// add 2^-Inf = 0. Three f32 additions per sum, then f64. Returns whether a logit lies near the window.
-template <bool TONE, bool CUT>
-__device__ __forceinline__ bool p1_body(const float* x, const P1Consts& k, P1Acc& a) {
-  const float LOG2E = 1.4426950408889634f;
-  const f32x2_t NA = pk2(-k.as, -k.as), LL = pk2(LOG2E, LOG2E);
-  a.vmax = max3nan(a.vmax, x[0], x[1]); a.vmax = max3nan(a.vmax, x[2], x[3]);
-  a.vmax = max3nan(a.vmax, x[4], x[5]); a.vmax = max3nan(a.vmax, x[6], x[7]);
-  float nearest = INFINITY;
-  f32x2_t E[4], KK[2];
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
-    const f32x2_t X = pk2(x[2 * c], x[2 * c + 1]);
-    f32x2_t S_;
-    if (TONE) S_ = X;
-    else S_ = div2_fast(pk2(fmaxf(x[2 * c], -1e30f), fmaxf(x[2 * c + 1], -1e30f)), k.Tm, k.yT);
-    float t0, t1;
-    upk2(mul2(add2(S_, NA), LL), t0, t1);
-    E[c] = pk2(ex2_approx(t0), ex2_approx(t1));
-    if (CUT) {
-      const f32x2_t M = pk2(set_ge(x[2 * c], k.xA), set_ge(x[2 * c + 1], k.xA));
-      if ((c & 1) == 0) KK[c >> 1] = mul2(E[c], M); else KK[c >> 1] = fma2(E[c], M, KK[c >> 1]);
-      float z0, z1;
-      upk2(add2(X, pk2(-k.xmid, -k.xmid)), z0, z1);
-      nearest = min3abs(nearest, z0, z1);
-    }
-  }
-  { float p, q; upk2(add2(add2(E[0], E[1]), add2(E[2], E[3])), p, q); a.tot += static_cast<double>(p + q); }
-  if (CUT) {
-    float p, q;
-    upk2(add2(KK[0], KK[1]), p, q);
-    a.kep += static_cast<double>(p + q);
-  }
-  return CUT && nearest <= k.xhalf;
-}
-template <bool CUT>
-__device__ __forceinline__ void p1_piece_end(int st, int nst, int lane, double* part_w, P1Acc& a) {
-  if ((st & (W_G - 1)) == W_G - 1 || st == nst - 1) {
-    const double kw = warp_sum_d(CUT ? a.kep : a.tot);
-    if (lane == 0) part_w[st / W_G] = kw;
-    if (CUT) { a.kep = 0.0; } else { a.stot += a.tot; a.tot = 0.0; }
-  }
-}
-// A step that holds the row's first or last vector, or vectors past the end: loaded on the spot and masked.
-template <typename T, bool TONE, bool CUT>
-__device__ __noinline__ void p1_edge_step(const WSpan& sp, const RowView<T>& rv, int lane, int st,
-                                          const P1Consts& k, double* part_w, P1Acc& a) {
-  constexpr int VEC = Elem<T>::VEC, EPI = 8 / VEC, SV = 32 * EPI;
-  const int gv = sp.first + st * SV + lane;
-  float x[8];
-#pragma unroll
-  for (int h = 0; h < EPI; h++) {
-    const int g = gv + 32 * h;
-    float xv[VEC];
-    Elem<T>::unpack(__ldg(rv.vbase + min(g, rv.nvec - 1)), xv);
-    const int i0 = g * VEC - rv.shift;
-#pragma unroll
-    for (int c = 0; c < VEC; c++) {
-      const int i = i0 + c;
-      x[h * VEC + c] = (g < rv.nvec && i >= 0 && i < rv.V) ? xv[c] : -INFINITY;
-    }
-  }
-  if (p1_body<TONE, CUT>(x, k, a)) p1_append<VEC, true>(x, gv * VEC - rv.shift, rv.V, k);
-  p1_piece_end<CUT>(st, sp.nst, lane, part_w, a);
-}
-// The pass: part_w[piece] (this warp's pieces) receives the mass of each piece (of all its logits
-// without a cut, of those above the window with one); the lane-private sum of all mass comes back
-// in Ssum, the lane's running maximum in vmax.
-template <typename T, bool TONE, bool CUT>
-__device__ __noinline__ void wide_onepass_stream(const WSpan& sp, const RowView<T>& rv, int lane, const P1Consts& k_in,
-                                                 double* part_w, double& Ssum, float& vmax) {
-  constexpr int VEC = Elem<T>::VEC, EPI = 8 / VEC, SV = 32 * EPI;
-  const P1Consts k = k_in;
-  P1Acc a;
-  a.tot = 0.0; a.kep = 0.0; a.stot = 0.0; a.vmax = -INFINITY;
-  const int nst = sp.nst, clean_lo = sp.clean_lo, clean_hi = sp.clean_hi;
-  int st = 0;
-  for (; st < clean_lo; st++) p1_edge_step<T, TONE, CUT>(sp, rv, lane, st, k, part_w, a);
-  // Clean steps: every vector exists and none is the row's first or last. Two register buffers used
-  // in turn (no copies between them): a step's vectors are asked for two steps ahead, and L2 is asked
-  // for the lines W1_PF steps ahead. The steady loop runs while both refills stay inside the clean
-  // range; what is left is loaded on the spot. (Four steps in flight, two of them in a cp.async ring
-  // in shared memory, were measured and changed nothing: the pass is bound by instruction issue.)
-  auto unpack8 = [&](const uint4& q0, const uint4& q1, float* x) {
-    if (EPI == 2) { Elem<T>::unpack(q0, x); Elem<T>::unpack(q1, x + 4 * (EPI - 1)); }
-    else Elem<T>::unpack(q0, x);
-  };
-  if (clean_hi - clean_lo >= 4) {
-    const uint4* p = sp.lane_src + clean_lo * SV;
-    int i_first = (sp.first + clean_lo * SV + lane) * VEC - rv.shift;
-    const int st_end = clean_lo + ((clean_hi - clean_lo - 2) & ~1);   // steps [clean_lo, st_end) in pairs, refills < clean_hi
-    uint4 a0 = __ldg(p), a1 = a0, b0, b1;
-    if (EPI == 2) a1 = __ldg(p + 32);
-    b0 = __ldg(p + SV); b1 = b0;
-    if (EPI == 2) b1 = __ldg(p + SV + 32);
-    const int pf_end = clean_hi - W1_PF;                      // last step that may still ask for step + W1_PF
-    float x[8];
-#pragma unroll 1
-    for (; st < st_end; st += 2) {
-      unpack8(a0, a1, x);
-      a0 = __ldg(p + 2 * SV); if (EPI == 2) a1 = __ldg(p + 2 * SV + 32);
-      if (W1_PF > 0 && st + 1 < pf_end) {
-        l2_prefetch(p + W1_PF * SV); l2_prefetch(p + (W1_PF + 1) * SV);
-        if (EPI == 2) { l2_prefetch(p + W1_PF * SV + 32); l2_prefetch(p + (W1_PF + 1) * SV + 32); }
-      }
-      if (p1_body<TONE, CUT>(x, k, a)) p1_append<VEC, false>(x, i_first, 0, k);
-      p1_piece_end<CUT>(st, nst, lane, part_w, a);
-      unpack8(b0, b1, x);
-      b0 = __ldg(p + 3 * SV); if (EPI == 2) b1 = __ldg(p + 3 * SV + 32);
-      if (p1_body<TONE, CUT>(x, k, a)) p1_append<VEC, false>(x, i_first + SV * VEC, 0, k);
-      p1_piece_end<CUT>(st + 1, nst, lane, part_w, a);
-      p += 2 * SV;
-      i_first += 2 * SV * VEC;
-    }
-    unpack8(a0, a1, x);
-    if (p1_body<TONE, CUT>(x, k, a)) p1_append<VEC, false>(x, i_first, 0, k);
-    p1_piece_end<CUT>(st, nst, lane, part_w, a);
-    unpack8(b0, b1, x);
-    if (p1_body<TONE, CUT>(x, k, a)) p1_append<VEC, false>(x, i_first + SV * VEC, 0, k);
-    p1_piece_end<CUT>(st + 1, nst, lane, part_w, a);
-    st += 2;
-  }
-  for (; st < nst; st++) p1_edge_step<T, TONE, CUT>(sp, rv, lane, st, k, part_w, a);
-  Ssum = CUT ? a.tot : a.stot;
-  vmax = a.vmax;
-}
-
-// false: the row takes the two-pass front end (nothing of the row has been decided or written).
+// Two passes over the row: for what one pass does not serve.
 template <typename T>
-__device__ __noinline__ bool wide_front_onepass(const BatchArgs& BA, const int64_t row_id, const RowView<T>& rv, const WSpan& sp,
-                                                unsigned char* dyn, WideShared& sh, const RowCfg cfg, const bool cut_on,
-                                                const int span, const int ppw, const int npiece, OnePassOut& out, uint32_t* clk) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  long long tprev = clock64();
-  auto stamp = [&](int slot) { const long long now = clock64(); clk[slot] = static_cast<uint32_t>(now - tprev); tprev = now; };
-  auto fail = [&](int why) -> bool { out.nz = why; return false; };   // why the row takes two passes (diagnostics)
-  constexpr int VEC = Elem<T>::VEC, EPI = 8 / VEC, SV = 32 * EPI;
-  bu::Scratch& sc = sh.sc;
-  const double* s_tab = sh.tab;
-  uint32_t* hist = reinterpret_cast<uint32_t*>(dyn + W_OFF_HIST);
-  uint2* zl = reinterpret_cast<uint2*>(dyn + W_OFF_ZONE);                 // W_ZCAP1 entries
-  double* part = reinterpret_cast<double*>(dyn + W_OFF_PART);
-  const float Tm = cfg.temperature;
-  const int mode = cfg.topp_mode;
-  const double plim = (mode == 0) ? static_cast<double>(cfg.top_p) * 1.5 : static_cast<double>(cfg.top_p);
-  const bool t_is_one = (Tm == 1.0f);
-  const uint32_t tb = __float_as_uint(Tm);
-  if (!t_is_one && !(Tm >= 9.5367431640625e-7f && Tm <= 1048576.0f && (tb & 0x7fffffu) != 0x7fffffu)) return fail(1);
-  if (rv.nvec < W_NW * SV * 8) return fail(2);                              // short rows: nothing to gain
-
-  // ask L2 for the sample's lines now: the sweep below then finds them there
-  if (cut_on) {
-    for (int st = 0; st < sp.nst; st += W1_STRIDE) {
-#pragma unroll
-      for (int h = 0; h < EPI; h++) {
-        const int g = sp.first + st * SV + lane + 32 * h;
-        if (g < rv.nvec) asm volatile("prefetch.global.L2::evict_last [%0];" :: "l"(rv.vbase + g));
-      }
-    }
-  }
-  // ---- a first look: every warp's first step gives a value near the row maximum and the range
-  float smax = -INFINITY, smin = INFINITY;
-  bool snan = false;
-#pragma unroll
-  for (int h = 0; h < EPI; h++) {
-    const int g = sp.first + 32 * h + lane;
-    if (sp.nst > 0 && g < rv.nvec) rv.visit(g, [&](float xv, int) { smax = fmaxf(smax, xv); smin = fminf(smin, xv); snan |= (xv != xv); });
-  }
-  if (bu::max_i<W_NW>(snan ? 1 : 0, sc, tid)) return fail(3);
-  smax = okey_to_float(static_cast<uint32_t>(bu::max_u64<W_NW>(static_cast<unsigned long long>(okey(smax)), sc, tid)));
-  smin = okey_to_float(static_cast<uint32_t>(bu::min_u64<W_NW>(static_cast<unsigned long long>(okey(smin)), sc, tid)));
-  const float r0 = smax - smin;
-  if (!(r0 >= 0.0f && r0 < 1e30f && fabsf(smax) < 1e30f)) return fail(3);
-  // the anchor of the fast exponentials: where the row maximum is expected (for bell-shaped rows the
-  // maximum of the whole row lies about an eighth of the first look's range above its maximum)
-  const float as = scale_t(smax + 0.125f * r0, Tm);
-  if (!(fabsf(as) < 1e30f)) return fail(3);
-
-  stamp(0);
-  P1Consts k;
-  k.as = as; k.Tm = Tm; k.yT = t_is_one ? 1.0f : __frcp_rn(Tm);
-  k.xA = -INFINITY; k.xmid = 0.0f; k.xhalf = -1.0f;
-  k.xB = -INFINITY; k.zl_s = smem_addr(zl); k.zcnt_s = smem_addr(&sh.cnt);
-  float xA = -INFINITY, xB = -INFINITY;
-  double eps = W1_EPS_FIXED + W1_EPS_PER_D * 9.7;
-  if (cut_on) {
-    // ---- the sample: count histogram over 4096 buckets of (anchor - x), anchor half of the first
-    // look's range above its maximum, bucket width so that the range and as much again below fit
-    const float margin = fmaxf(0.5f * r0, 1e-3f * fmaxf(1.0f, fabsf(smax)));
-    const float hs = 4094.0f / fmaxf(2.25f * r0 + margin, 1e-30f);
-    const float Tc = Tm;
-    // bucket width in units of x / T between 2^-16 and 2^-7
-    const float hs_c = fminf(fmaxf(hs, 128.0f / Tc), 65536.0f / Tc);
-    if (!(hs_c > 1e-30f && hs_c < 1e30f)) return fail(4);
-    const float nhs = -hs_c;
-    const float hc = fmaf(smax + margin, hs_c, W1_MAGIC);
-    if (!(fabsf(hc) < 1e30f)) return fail(4);
-    for (int j = tid; j < W_NB; j += W_NT) hist[j] = 0;
-    __syncthreads();
-    float svmax = -INFINITY;
-    const uint32_t hb = smem_addr(hist);
-    // four sampled steps at a time: their loads are in flight together
-    for (int st0 = 0; st0 < sp.nst; st0 += 4 * W1_STRIDE) {
-      uint4 q[4 * EPI];
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-#pragma unroll
-        for (int h = 0; h < EPI; h++) {
-          const int g = sp.first + (st0 + u * W1_STRIDE) * SV + lane + 32 * h;
-          q[u * EPI + h] = __ldg(rv.vbase + min(g, rv.nvec - 1));
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 4; u++) {
-        if (st0 + u * W1_STRIDE < sp.nst) {
-#pragma unroll
-          for (int h = 0; h < EPI; h++) {
-            const int g = sp.first + (st0 + u * W1_STRIDE) * SV + lane + 32 * h;
-            if (g < rv.nvec) {
-              rv.visit_raw(q[u * EPI + h], g, [&](float xv, int, int) {
-                svmax = maxnan(svmax, xv);
-                asm volatile("red.shared.add.u32 [%0], 1;" :: "r"(bucket_off1(xv, nhs, hc) + hb) : "memory");
-              });
-            }
-          }
-        }
-      }
-    }
-    const int bad_s = bu::max_i<W_NW>((svmax != svmax) ? 1 : 0, sc, tid);  // also orders the histogram
-    stamp(1);
-    svmax = okey_to_float(static_cast<uint32_t>(bu::max_u64<W_NW>(static_cast<unsigned long long>(okey(svmax)), sc, tid)));
-    if (bad_s || !(fmaf(svmax, nhs, hc) >= W1_MAGIC)) return fail(6);       // NaN, or a sampled logit above the anchor
-    // ---- the window from the sample's histogram: bucket b holds y = (anchor' - x) hs in
-    // [b - 1/8, b + 7/8], a width of w = 1 / (hs T) in units of x / T; masses relative to
-    // exp(anchor' / T) lie between exp(-(b + 7/8) w) and exp(-(b - 1/8) w). The bracket is the one of
-    // the two-pass front end, widened by the sampling error of a mass fraction estimated from n logits.
-    // Placing the window is a matter of speed, not of correctness (the pass checks it on the whole
-    // row): f32 and the fast exponential do.
-    constexpr int PER = W_NB / W_NT;
-    const double wd = 1.0 / (static_cast<double>(hs_c) * static_cast<double>(Tm));
-    const float wl2 = static_cast<float>(wd * 1.4426950408889634);        // bucket width in units of log2
-    const float ratio = ex2_approx(-wl2);
-    const float edge0 = ex2_approx(-(static_cast<float>(tid * PER) - 0.125f) * wl2);
-    float slo = 0.0f, shi = 0.0f;
-    int cnt_loc = 0, lowest = -1, top = W_NB;
-    uint32_t cnt[PER];                                                    // this thread's buckets, read once
-    {
-      const uint4* mine = reinterpret_cast<const uint4*>(hist) + tid * (PER / 4);
-#pragma unroll
-      for (int q = 0; q < PER / 4; q++) { const uint4 v = mine[q]; cnt[4 * q] = v.x; cnt[4 * q + 1] = v.y; cnt[4 * q + 2] = v.z; cnt[4 * q + 3] = v.w; }
-    }
-    {
-      float edge = edge0;
-#pragma unroll
-      for (int j = 0; j < PER; j++) {
-        const int b = tid * PER + j;
-        const int ci = static_cast<int>(cnt[j]);
-        const float c = static_cast<float>(ci);
-        const float ehi = edge;
-        edge *= ratio;
-        const float elo = (b == W_NB - 1) ? 0.0f : edge;
-        slo = fmaf(c, elo, slo); shi = fmaf(c, ehi, shi);
-        cnt_loc += ci;
-        if (ci) { lowest = b; top = min(top, b); }
-      }
-    }
-    double ex_lo, ex_hi, tot_lo, tot_hi;
-    bu::scan_excl_d2<W_NW>(static_cast<double>(slo), static_cast<double>(shi), ex_lo, ex_hi, tot_lo, tot_hi, sc, tid);
-    const int nsamp = bu::sum_i<W_NW>(cnt_loc, sc, tid);
-    int nlow = -lowest;                                                   // the lowest populated bucket as a minimum of negatives
-    bu::min_i2<W_NW>(top, nlow, sc, tid);
-    lowest = -nlow;
-    if (nsamp < 4096 || !(tot_lo > 0.0)) return fail(7);
-    // a few heavy tokens: the sample cannot place the cut (one token above a thousandth of the mass)
-    const double heavy = static_cast<double>(ex2_approx(-(static_cast<float>(top) - 0.125f) * wl2));
-    if (heavy > 1e-3 * tot_lo) return fail(8);
-    // five standard errors of a mass fraction estimated from nsamp logits
-    const double delta = 5.0 * sqrt(plim * fabs(1.0 - plim) / static_cast<double>(nsamp)) + 4.0 / static_cast<double>(nsamp);
-    const float p_lo = static_cast<float>(plim - delta), p_hi = static_cast<float>(plim + delta);
-    if (!(p_lo > 0.0f)) return fail(9);
-    int b1 = W_NB - 1, b2 = W_NB - 1, wcount = 0;
-    {
-      float edge = edge0, a_lo = static_cast<float>(ex_lo), a_hi = static_cast<float>(ex_hi);
-      const float t_lo = static_cast<float>(tot_lo), t_hi = static_cast<float>(tot_hi);
-#pragma unroll
-      for (int j = 0; j < PER; j++) {
-        const int b = tid * PER + j;
-        const float c = static_cast<float>(cnt[j]);
-        const float ehi = edge;
-        edge *= ratio;
-        const float elo = (b == W_NB - 1) ? 0.0f : edge;
-        a_lo = fmaf(c, elo, a_lo); a_hi = fmaf(c, ehi, a_hi);
-        const float den_hi = a_hi + (t_lo - a_lo), den_lo = a_lo + (t_hi - a_hi);
-        const bool c1 = a_hi >= p_lo * den_hi, c2 = a_lo >= p_hi * den_lo;
-        if (c1 && a_hi > 0.0f) b1 = min(b1, b);
-        if (c2 && a_lo > 0.0f) b2 = min(b2, b);
-      }
-    }
-    bu::min_i2<W_NW>(b1, b2, sc, tid);
-    if (b2 < b1) b2 = b1;
-    if (b1 > 0) b1--;                                                     // one bucket of slack for the f32 sums
-    if (b2 < W_NB - 1) b2++;
-#pragma unroll
-    for (int j = 0; j < PER; j++) { const int b = tid * PER + j; if (b >= b1 && b <= b2) wcount += static_cast<int>(cnt[j]); }
-    wcount = bu::sum_i<W_NW>(wcount, sc, tid);
-    // the window must stay small: its logits go through the exact list
-    if (static_cast<long long>(wcount) * W1_STRIDE > (W_ZCAP1 * 13) / 16) return fail(10);
-    bool ok = true;
-    xA = bucket_floor1(b1 - 1, nhs, hc, ok);
-    xB = bucket_floor1(b2, nhs, hc, ok);
-    if (!ok) return fail(11);
-    k.xA = xA; k.xB = xB;
-    const float xAc = fminf(xA, 3.0e38f), xBc = fmaxf(xB, -3.0e38f);
-    k.xmid = 0.5f * xAc + 0.5f * xBc;
-    k.xhalf = (0.5f * xAc - 0.5f * xBc) * 1.000001f + 1e-30f;
-    if (lowest >= 0 && lowest < W_NB - 1) {
-      const double dmax = (static_cast<double>(lowest) + 1.0) * wd + 1e-3;   // from the histogram's anchor down
-      eps = W1_EPS_FIXED + W1_EPS_PER_D * fmin(9.7, dmax);
-    }
-    __syncthreads();                                                      // the histogram area becomes the record list
-  }
-
-  stamp(2);
-  // ---- the pass
-  if (tid < npiece) part[tid] = 0.0;                                      // pieces past the row's end stay empty
-  if (tid == 0) sh.cnt = 0;
-  __syncthreads();
-  double Ssum = 0.0;
-  float vmax = -INFINITY;
-  double* part_w = part + warp * ppw;
-  if (cut_on) {
-    if (t_is_one) wide_onepass_stream<T, true, true>(sp, rv, lane, k, part_w, Ssum, vmax);
-    else wide_onepass_stream<T, false, true>(sp, rv, lane, k, part_w, Ssum, vmax);
-  } else {
-    if (t_is_one) wide_onepass_stream<T, true, false>(sp, rv, lane, k, part_w, Ssum, vmax);
-    else wide_onepass_stream<T, false, false>(sp, rv, lane, k, part_w, Ssum, vmax);
-  }
-  __syncthreads();
-  stamp(6);
-  const int anynan = bu::max_i<W_NW>((vmax != vmax) ? 1 : 0, sc, tid);
-  const float xmax = okey_to_float(static_cast<uint32_t>(bu::max_u64<W_NW>(static_cast<unsigned long long>(okey(vmax)), sc, tid)));
-  const float m = scale_t(xmax, Tm);
-  if (anynan || !(fabsf(m) < INFINITY)) return fail(12);                     // the two-pass front end reports such rows
-  // the fast sums round x/T - anchor where upstream rounds x/T - max: the two must be close for the
-  // heavy logits to keep the error budget (2e-7 per unit of distance)
-  if (!(fabsf(m - as) <= 2.0f)) return fail(13);
-  int nz = 0;
-  double S = bu::sum_d<W_NW>(Ssum, sc, tid);
-  nz = sh.cnt;
-  if (!(S > 0.0) || !(S < 1e300)) return fail(14);
-  // everything so far is relative to exp(anchor); the tail works relative to exp(max)
-  const double cf = exp(static_cast<double>(as) - static_cast<double>(m));
-  S *= cf;
-  if (tid < npiece) part[tid] *= cf;
-  __syncthreads();
-  double Ktot = 0.0;
-  if (cut_on) {
-    Ktot = bu::sum_d<W_NW>((tid < npiece) ? part[tid] : 0.0, sc, tid);
-    // ---- the window's logits: x -> d = x / T - max, in place, and their mass
-    if (nz > W_ZCAP1 || nz == 0) return fail(5);
-    double zmass = 0.0;
-    for (int j = tid; j < nz; j += W_NT) {
-      const uint2 e = zl[j];
-      const float d = scale_t(__uint_as_float(e.x), Tm) - m;
-      zl[j] = make_uint2(__float_as_uint(d), e.y);
-      zmass += exp_safe(d, s_tab);
-    }
-    zmass = bu::sum_d<W_NW>(zmass, sc, tid);
-    // the cut must lie inside the window by more than the error of the sums
-    const double etol = 1e-12 + 2.0 * plim * fabs(1.0 - plim) * eps + 1e-9;
-    if (!(Ktot / S < plim - etol) || !((Ktot + zmass) / S > plim + etol)) {
-      if (!(xB == -INFINITY && Ktot / S < plim - etol)) return fail(15);     // a window open at the bottom holds whatever is left
-    }
-  }
-  stamp(7);
-  out.m = m; out.S = S; out.Ktot = Ktot; out.nz = nz; out.xA = xA; out.xB = xB; out.eps = eps;
-  return true;
-}
-
-template <typename T>
-__device__ void wide_row(const BatchArgs& BA, const int64_t row_id, unsigned char* dyn, WideShared& sh,
+__device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t row_id, unsigned char* dyn, WideShared& sh,
                          unsigned long long pol_keep, unsigned long long pol_drop) {
   const KernelArgs& A = BA.k;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -971,7 +625,6 @@ __device__ void wide_row(const BatchArgs& BA, const int64_t row_id, unsigned cha
   unsigned long long* zk = reinterpret_cast<unsigned long long*>(dyn + W_OFF_ZONE);
   double* ebs = reinterpret_cast<double*>(dyn + W_OFF_EB);
   double* part = reinterpret_cast<double*>(dyn + W_OFF_PART);   // [warp][piece] kept mass, row order
-  const double QNAN = __longlong_as_double(0x7ff8000000000000ll);
 
   const RowCfg cfg = A.cfgs[row_id];
   const float Tm = cfg.temperature;
@@ -984,26 +637,6 @@ __device__ void wide_row(const BatchArgs& BA, const int64_t row_id, unsigned cha
   const bool cut_on = topp_on && !(mode == 0 && plim >= 1.0);
   const bool t_is_one = (Tm == 1.0f);
   uint32_t flags = FLAG_GENERAL_PATH;
-  RowDebug dbg;
-  dbg.sum_exp = 0; dbg.resum = 1.0; dbg.edge_lo = 0; dbg.edge_hi = 0; dbg.kept = 0;
-  dbg.max_scaled = 0; dbg.threshold = __int_as_float(0x7fc00000); dbg.path = 2;
-  for (int q = 0; q < 8; q++) dbg.reserved[q] = 0;
-  long long tprev = clock64();
-  auto stamp = [&](int slot) { const long long now = clock64(); dbg.reserved[slot] = static_cast<uint32_t>(now - tprev); tprev = now; };
-  auto write_row = [&](int id, uint32_t fl) {
-    if (tid == 0) {
-      A.out_ids[row_id] = id;
-      if (A.out_flags) A.out_flags[row_id] = fl;
-      if (A.out_debug) A.out_debug[row_id] = dbg;
-    }
-  };
-  auto fill_probs_row = [&](double v) {
-    if (A.out_probs) {
-      double* pr = A.out_probs + row_id * static_cast<int64_t>(V);
-      for (int i = tid; i < V; i += W_NT) pr[i] = v;
-    }
-  };
-
   // the warp's span: 1/W_NW of the row, rounded up to whole steps
   const int span = (((rv.nvec + W_NW - 1) / W_NW + SV - 1) / SV) * SV;
   const int steps_max = span / SV;
@@ -1015,34 +648,11 @@ __device__ void wide_row(const BatchArgs& BA, const int64_t row_id, unsigned cha
   const int npiece = W_NW * ppw;
   const WSpan sp = make_span<T>(rv, warp * span, span, lane);
 
-  // What the tail needs of the row, from either front end.
   float m = 0.0f, dlow = -INFINITY;
   float dA = -INFINITY, dB = -INFINITY;    // certainly kept: d >= dA; zone: dB <= d < dA; dropped: d < dB
   bool fast_ok = false;
   double S = 0.0, Ktot = 0.0;
   int nz = 0;
-  // one-pass front end: thresholds on the raw logits (xs), its own error bound and list capacity
-  bool xs = false;
-  int onepass_why = 0;
-  float xA = -INFINITY, xB = -INFINITY;
-  double eps_rel = W_EXP_REL_ERR;
-  int zcap = W_ZCAP;
-  {
-    OnePassOut fo;
-    fo.nz = 0;
-    if (wide_front_onepass<T>(BA, row_id, rv, sp, dyn, sh, cfg, cut_on, span, ppw, npiece, fo, dbg.reserved)) {
-      xs = true;
-      m = fo.m; S = fo.S; Ktot = fo.Ktot; nz = fo.nz; xA = fo.xA; xB = fo.xB; eps_rel = fo.eps; zcap = W_ZCAP1;
-      fast_ok = true;
-      dlow = -INFINITY;
-      dB = (xB == -INFINITY) ? -INFINITY : 0.0f;             // "logits below the zone may exist"
-      dbg.max_scaled = m;
-      dbg.path = 3;
-    } else {
-      onepass_why = fo.nz;
-    }
-  }
-  if (!xs) {
   // ---- a sample of the row (every warp's first step) gives an upper estimate of the maximum
   // and the bucket width, so that pass 1 can already count the histogram the cut needs
   bool anchored = false;
@@ -1093,14 +703,10 @@ __device__ void wide_row(const BatchArgs& BA, const int64_t row_id, unsigned cha
   xmax = okey_to_float(static_cast<uint32_t>(bu::max_u64<W_NW>(static_cast<unsigned long long>(okey(xmax)), sc, tid)));
   xmin = okey_to_float(static_cast<uint32_t>(bu::min_u64<W_NW>(static_cast<unsigned long long>(okey(xmin)), sc, tid)));
   m = scale_t(xmax, Tm);
-  dbg.max_scaled = m;
-  stamp(0);
   // A NaN anywhere, or an infinite maximum, makes the softmax sum NaN upstream
   // (generate.go:173-181): every comparison of the walk fails, result n-1 (:239).
   if (anynan || !(fabsf(m) < INFINITY)) {
-    fill_probs_row(QNAN);
-    dbg.sum_exp = QNAN;
-    write_row(V - 1, flags | FLAG_NONFINITE | FLAG_FALLBACK);
+    wide_write_nothing_kept(A, row_id, m, -1.0, 2, flags);
     return;
   }
   dlow = scale_t(xmin, Tm) - m;                  // smallest d of the row (-Inf with a -Inf logit)
@@ -1185,7 +791,6 @@ __device__ void wide_row(const BatchArgs& BA, const int64_t row_id, unsigned cha
       if (dA > 0.0f) dA = INFINITY;                          // no d reaches it: nothing is certainly kept
     }
   }
-  stamp(1);
 
   // ---- pass 3: exponentials (last use of the row: evict-first)
   // exponential table: sixteen conflict-free copies of the first 128 entries when the row's range
@@ -1217,22 +822,15 @@ __device__ void wide_row(const BatchArgs& BA, const int64_t row_id, unsigned cha
   S = Ssum; Ktot = Ksum;
   bu::sum_d3<W_NW>(S, Ktot, unused, sc, tid);
   nz = sh.cnt;
-  stamp(2);
-  dbg.reserved[6] = static_cast<uint32_t>(onepass_why);     // why the row took two passes
-  }  // two-pass front end
   // A zone that outgrew the list (long runs of equal logits around the cut): the same selection
   // runs over the row itself, one more pass per round.
-  const bool big = cut_on && nz > zcap;
-  dbg.sum_exp = S;
+  const bool big = cut_on && nz > W_ZCAP;
 
   // ---- exact cut inside the zone by weighted selection
   unsigned long long cut_key = 0ull;       // zone entries are kept when key < cut_key, or == with cut_incl
   int cut_incl = 0;
   bool bad = false;
-  if (big && xs) {
-    if (tid == 0) hand_to_single(BA, row_id);
-    return;
-  } else if (big) {
+  if (big) {
     if (!wide_big_zone<T>(sp, rv, pol_keep, sh, hist, part, s_tab, m, Tm, dA, dB, dlow, mode, plim, S, Ktot, fast_ok,
                           span, ppw, cut_key, cut_incl, flags)) {
       if (tid == 0) hand_to_single(BA, row_id);
@@ -1340,15 +938,8 @@ __device__ void wide_row(const BatchArgs& BA, const int64_t row_id, unsigned cha
     }
     if (!bad && !all_in) {
       // the sums carry exp_fast_s's error; in G/S >= p it enters as 2 p (1-p) times that bound
-      const double etol = 1e-12 + (fast_ok ? 2.0 * plim * fabs(1.0 - plim) * eps_rel : 0.0);
+      const double etol = 1e-12 + (fast_ok ? 2.0 * plim * fabs(1.0 - plim) * W_EXP_REL_ERR : 0.0);
       if (fabs(g_at / S - plim) <= etol || fabs(g_before / S - plim) <= etol) flags |= FLAG_TOPP_EDGE;
-      if (xs) {
-        // Several logits can share one d, and the order among equal d is by index: a cut whose d is also
-        // the d of a logit outside the window (at its upper or lower edge) is decided on the whole row.
-        const float dc = zone_key_d(cut_key);
-        if (xA < INFINITY && dc == scale_t(xA, Tm) - m) bad = true;
-        if (xB > -INFINITY && dc == scale_t(nextafterf(xB, -INFINITY), Tm) - m) bad = true;
-      }
       if (mode == 1) {
         // a later key with the same d as c*: the cut separates equal probabilities
         int tie = 0;
@@ -1374,114 +965,34 @@ __device__ void wide_row(const BatchArgs& BA, const int64_t row_id, unsigned cha
   }
   // ---- kept mass and the piece that holds the drawn token: prefix over the pieces in row order
   const double pm = (tid < npiece) ? part[tid] : 0.0;
-  double Re;
-  const double pex = bu::scan_excl_d<W_NW>(pm, Re, sc, tid);
-  dbg.resum = Re / S;
-  stamp(3);
-  if (!(S == S) || !(S > 0.0) || !(Re > 0.0)) {
-    // mode A removed every token (generate.go:221-227 divides by zero): the walk falls through
-    fill_probs_row(QNAN);
-    if (S == S && S > 0.0) dbg.resum = 0.0; else dbg.sum_exp = QNAN;
-    write_row(V - 1, flags | FLAG_NONFINITE | FLAG_FALLBACK);
+  WideResult r;
+  const double pex = bu::scan_excl_d<W_NW>(pm, r.Re, sc, tid);
+  r.m = m; r.S = S; r.path = 2;
+  if (!(S == S) || !(S > 0.0) || !(r.Re > 0.0)) {
+    wide_write_nothing_kept(A, row_id, m, S, 2, flags);
     return;
   }
+  const int psel = bu::min_i<W_NW>((tid < npiece && u * r.Re < pex + pm) ? tid : 0x7fffffff, sc, tid);
+  if (tid == psel) sh.bcd[0] = pex;
+  __syncthreads();
+  const double before = (psel != 0x7fffffff) ? sh.bcd[0] : r.Re;
   // final rule for one logit: its kept mass (0 when cut away)
   auto kept_mass = [&](float xv, int i) -> double {
     if (i < 0 || i >= V) return 0.0;
     const float s = t_is_one ? xv : __fdiv_rn(xv, Tm);
     const float d = s - m;
-    if (xs ? (cut_on && !(xv >= xA)) : (d < dA)) {
-      if (xs ? !(xv >= xB) : !(d >= dB)) return 0.0;
+    if (d < dA) {
+      if (!(d >= dB)) return 0.0;
       const unsigned long long k = zone_key(d, i, mode);
       if (!(k < cut_key || (cut_incl && k == cut_key))) return 0.0;
     }
     return exp_safe(d, s_tab);
   };
-  if (A.out_probs || A.out_debug) {                          // parity runs only
-    double* pr = A.out_probs ? A.out_probs + row_id * static_cast<int64_t>(V) : nullptr;
-    const double rq = Re / S;
-    int kept_loc = 0;
-    for (int v = tid; v < rv.nvec; v += W_NT) {
-      float x[VEC];
-      Elem<T>::unpack(__ldg(rv.vbase + v), x);
-      const int i0 = v * VEC - rv.shift;
-#pragma unroll
-      for (int c = 0; c < VEC; c++) {
-        const int i = i0 + c;
-        if (i >= 0 && i < V) {
-          const double f = (kept_mass(x[c], i) / S) / rq;
-          kept_loc += (f > 0) ? 1 : 0;
-          if (pr) pr[i] = f;
-        }
-      }
-    }
-    dbg.kept = bu::sum_i<W_NW>(kept_loc, sc, tid);
-  }
-  stamp(4);
-  // ---- draw (generate.go:231-239): u < prefix/Re is tested as u*Re < prefix
-  const double tgt = u * Re;
-  int psel = (tid < npiece && tgt < pex + pm) ? tid : 0x7fffffff;
-  psel = bu::min_i<W_NW>(psel, sc, tid);
-  if (tid == psel) sh.bcd[0] = pex;
-  __syncthreads();
-  int id = -1;
-  double edge_lo = 0.0, edge_hi = 0.0;
-  double run_end = (psel != 0x7fffffff) ? sh.bcd[0] : Re;
-  if (psel != 0x7fffffff) {
-    // walk pieces from the selected one (rounding can push the crossing into the next piece)
-    for (int pi = psel; pi < npiece && id < 0; pi++) {       // uniform; normally one trip
-      const int w = pi / ppw;
-      const int vb = w * span + (pi - w * ppw) * PV;
-      const int vend = min(min(vb + PV, w * span + span), rv.nvec);
-      const int j = vb + tid;
-      double em[VEC];
-      double tsum = 0.0;
-#pragma unroll
-      for (int c = 0; c < VEC; c++) em[c] = 0.0;
-      int i0 = 0;
-      if (j < vend) {
-        float x[VEC];
-        Elem<T>::unpack(__ldg(rv.vbase + j), x);
-        i0 = j * VEC - rv.shift;
-#pragma unroll
-        for (int c = 0; c < VEC; c++) { em[c] = kept_mass(x[c], i0 + c); tsum += em[c]; }
-      }
-      double totc;
-      const double ex = bu::scan_excl_d<W_NW>(tsum, totc, sc, tid);
-      int pick_loc = 0x7fffffff;
-      double run = run_end + ex, lo = 0.0, hi = 0.0;
-#pragma unroll
-      for (int c = 0; c < VEC; c++) {
-        const double before = run;
-        run += em[c];
-        if (em[c] > 0.0 && tgt < run && pick_loc == 0x7fffffff) { pick_loc = i0 + c; lo = before; hi = run; }
-      }
-      const int pick = bu::min_i<W_NW>(pick_loc, sc, tid);
-      if (pick != 0x7fffffff) {
-        if (pick_loc == pick) { sh.bcd[1] = lo; sh.bcd[2] = hi; }
-        __syncthreads();
-        id = pick;
-        edge_lo = sh.bcd[1] / Re;
-        edge_hi = sh.bcd[2] / Re;
-      }
-      run_end += totc;
-    }
-  }
-  if (id >= 0) {
-    dbg.edge_lo = edge_lo; dbg.edge_hi = edge_hi;
-    if ((edge_lo > 0.0 && u - edge_lo <= 1e-6) || edge_hi - u <= 1e-6) flags |= FLAG_BOUNDARY;
-  } else {
-    id = V - 1;                                              // generate.go:239
-    flags |= FLAG_FALLBACK;
-    dbg.edge_lo = dbg.edge_hi = run_end / Re;
-    if (u - run_end / Re <= 1e-6) flags |= FLAG_BOUNDARY;
-  }
-  stamp(5);
-  write_row(id, flags);
+  wide_draw<T>(A, row_id, rv, span, ppw, psel, before, u, r, flags, sh, kept_mass);
 }
 
 template <typename T>
-__global__ void __launch_bounds__(W_NT, W_CTAS) wide_rows_kernel(BatchArgs BA) {
+__global__ void __launch_bounds__(W_NT, W_CTAS) wide_rows_kernel(const __grid_constant__ BatchArgs BA) {
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ WideShared sh;
   if (threadIdx.x < 256) sh.tab[threadIdx.x] = BA.k.exp_table[threadIdx.x];
@@ -1505,7 +1016,9 @@ __global__ void __launch_bounds__(W_NT, W_CTAS) wide_rows_kernel(BatchArgs BA) {
     // The narrow kernel may start: every CTA of this one has a row, or has gone. (Started together, the two kernels'
     // CTAs mix at random, and some SMs end up with more rows of this kind than others.)
     pdl_launch();
-    wide_row<T>(BA, row, dyn, sh, pol_keep, pol_drop);
+    if (wide_onepass_row<T>(BA, row, dyn, sh) == 0) continue;
+    __syncthreads();
+    wide_twopass_row<T>(BA, row, dyn, sh, pol_keep, pol_drop);
   }
 }
 

@@ -1,0 +1,795 @@
+// The wide kernel's usual way with a row: one pass over it. (Included by sample_wide.cuh inside its namespace, once per
+// instance.)
+//
+// One pass sums the mass of everything (S) with the fast exponential relative to an anchor near the row maximum. With a top-p
+// cut, a sample of the row places the cut in a window of logit values; the window's own logits go to lists, and the cut is
+// decided exactly among them. What lies above the window is certainly kept: its mass is summed beside S (P1_MID), or, where few
+// logits lie below the window, they are listed too and the rest of S is what is kept (P1_LOW: a quarter fewer instructions
+// in a loop that is bound by their issue where an SM has four rows). The sample only chooses the window: whether the cut really
+// lies inside is checked on the sums of the whole row, and a row whose window failed (or that the sample cannot place:
+// a few heavy tokens, NaN, a wide window) takes two passes (sample_wide.cuh). Rows without a cut (P1_ALL) need neither sample
+// nor window.
+//
+// The lists. A window of 1 to 2 % of the logits puts one into a tenth of the lane-steps, so nearly every warp-step has a lane
+// that must list something, and slots from a shared counter cost every warp some ninety issue slots a step. So a lane has a
+// buffer of its own: a predicated store and a predicated addition per logit, no branch, no counter, consecutive lanes in
+// consecutive banks. At the end of a piece the warp moves what its lanes hold to its list, a vote per round. What is listed is
+// the logit alone: its piece is known, and the few indices that the cut's ties need are found by looking at one piece again.
+//
+// The loads. Four CTAs' shared memory leaves some 28 KB of L1 per SM, too little for 64 KB of register loads on their way
+// (512 rows of 151,936 f32, loads alone: 65 us; 51 with L1 free), and the loop's loads share their scoreboards with its
+// exponentials. So sample and row come by asynchronous copies to shared memory, which take no L1 (53); asking L2
+// for lines further ahead made the pass slower (98 against 90 thousand cycles). Everything uniform lies in shared memory and nothing of a thread's on its stack: the stacks of a former version
+// wrote 59 MB to HBM per 311 MB read.
+//
+// Error budget of the fast sums against exp(d) in f64, d = x/T - max rounded to f32 as upstream. With a cut the argument of
+// 2^t is one FMA, x log2 e - C: ex2.approx 2.4e-7, three f32 additions per step before the f64 accumulators 1.8e-7, and per
+// unit of |x/T - anchor| the roundings of t, of log2 e and of upstream's d, 1.4e-7 together: W1_EPS_FIXED + W1_EPS_PER_D * (largest |d|
+// that carries mass). (C is the anchor times log2 e, rounded: the anchor that this stands for is what the sums are taken
+// back from.) The anchor must lie within 2 of the maximum. Without a cut the rounding of t is made up for (p1_exp2), which leaves
+// 6e-8 per unit: the anchor may lie W1_RISE below a logit for the same error.
+constexpr int P1_ALL = 0, P1_LOW = 1, P1_MID = 2;
+constexpr int W1_SAMPLE = (W_NT >= 512) ? 16384 : 8192;        // logits of the sample
+constexpr int W1_SBINS = 1024;           // its histogram's buckets
+constexpr double W1_EPS_FIXED = 4.5e-7;
+constexpr double W1_EPS_PER_D = 2.0e-7;
+constexpr float W1_RISE = 6.0f;
+static_assert(W1_SBINS % W_NT == 0 && W1_BINS == W_NT && W1_SAMPLE * 4 + W1_SBINS * 4 <= W1_OFF_BINS, "a thread's share of the buckets; the sample and its buckets lie where lists and ring will be");
+static_assert(W_MAX_PPW <= 32 && W_NW <= 32 && W_MAX_PIECES <= W1_BINS && W1_OFF_MASS + W_NW * W1_WCAP * 8 <= W1_OFF_BINS, "memory of the selection");
+
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
+__device__ __forceinline__ float ex2_approx(float t) { float e; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t)); return e; }
+__device__ __forceinline__ float set_ge(float a, float b) { float r; asm("set.ge.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }   // 1.0f or 0.0f
+
+// x / T in IEEE f32 round-to-nearest by q0 = x y, r = fma(-q0, T, x), q = fma(r, y, q0) with y = RN(1/T):
+// the correctly rounded quotient whenever T's significand is not all ones and nothing over- or underflows
+// (the caller takes this form for 2^-20 <= T <= 2^20 only and clamps x at -1e30: whatever lies below has
+// mass 0 either way).
+__device__ __forceinline__ f32x2_t div2_fast(f32x2_t X, float T, float y) {
+  const f32x2_t Y = pk2(y, y);
+  const f32x2_t Q0 = mul2(X, Y);
+  const f32x2_t R = fma2(Q0, pk2(-T, -T), X);
+  return fma2(R, Y, Q0);
+}
+constexpr float P1_L2E = 1.4426950408889634f;
+// exp of two, the rounding of the product with log2 e recovered exactly and applied to the result (arguments at or above -1e30).
+__device__ __forceinline__ f32x2_t p1_exp2(f32x2_t D) {
+  constexpr float L2E_LO = 1.925963033500011e-8f, LN2 = 0.6931471805599453f;
+  float t0, t1;
+  const f32x2_t NT2 = mul2(D, pk2(-P1_L2E, -P1_L2E));
+  f32x2_t R = fma2(D, pk2(P1_L2E, P1_L2E), NT2);
+  R = fma2(D, pk2(L2E_LO, L2E_LO), R);
+  upk2(NT2, t0, t1);
+  const f32x2_t P = pk2(ex2_approx(-t0), ex2_approx(-t1));
+  return fma2(P, mul2(R, pk2(LN2, LN2)), P);
+}
+
+struct P1Consts {
+  float as, C, Tm, yT;     // anchor in units of x / T, and times log2 e; temperature and its rounded reciprocal
+  float xA;                // above the window: x >= xA
+  float xmid, xhalf;       // |x - xmid| <= xhalf is a superset of the window
+  uint32_t buf, buf_end;   // shared-memory addresses of this lane's buffer: its first slot, and the one that leaves room for four logits
+};
+struct P1Acc {
+  double tot;              // all mass of the running piece (P1_MID: all mass so far)
+  double kep;              // P1_MID: mass above the window of the running piece
+  double stot;             // all mass of the pieces done
+  float vmax;              // NaN-propagating running maximum
+  uint32_t at;             // the lane's next slot
+};
+
+// Eight logits of a lane; masked logits are -Inf and add 0. Three f32 additions per sum, then f64. Logits near the window go
+// to the lane's buffer.
+template <int VEC, bool TONE, int MODE>
+__device__ __forceinline__ void p1_body(const float* x, const P1Consts& k, P1Acc& a) {
+  a.vmax = max3nan(a.vmax, x[0], x[1]); a.vmax = max3nan(a.vmax, x[2], x[3]);
+  a.vmax = max3nan(a.vmax, x[4], x[5]); a.vmax = max3nan(a.vmax, x[6], x[7]);
+  f32x2_t E[4], KK[2];
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    const f32x2_t X = pk2(x[2 * c], x[2 * c + 1]);
+    f32x2_t S_ = X;
+    if (!TONE || MODE == P1_ALL) S_ = pk2(fmaxf(x[2 * c], -1e30f), fmaxf(x[2 * c + 1], -1e30f));
+    if (!TONE) S_ = div2_fast(S_, k.Tm, k.yT);
+    if (MODE == P1_ALL) {
+      E[c] = p1_exp2(add2(S_, pk2(-k.as, -k.as)));
+    } else {
+      float t0, t1;
+      upk2(fma2(S_, pk2(P1_L2E, P1_L2E), pk2(-k.C, -k.C)), t0, t1);
+      E[c] = pk2(ex2_approx(t0), ex2_approx(t1));
+      if (MODE == P1_MID) {
+        const f32x2_t M = pk2(set_ge(x[2 * c], k.xA), set_ge(x[2 * c + 1], k.xA));
+        if ((c & 1) == 0) KK[c >> 1] = mul2(E[c], M); else KK[c >> 1] = fma2(E[c], M, KK[c >> 1]);
+      }
+      float z0, z1;
+      upk2(add2(X, pk2(-k.xmid, -k.xmid)), z0, z1);
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.le.f32 p, %2, %3;\n\t@p st.shared.f32 [%0], %1;\n\t@p add.u32 %0, %0, %4;\n\t}"
+                     : "+r"(a.at) : "f"(x[2 * c + h]), "f"(fabsf(h ? z1 : z0)), "f"(k.xhalf), "n"(W_NT * 4));
+      if (c & 1) a.at = min(a.at, k.buf_end);                   // a full buffer stays full: the row takes two passes
+    }
+  }
+  { float p, q; upk2(add2(add2(E[0], E[1]), add2(E[2], E[3])), p, q); a.tot += static_cast<double>(p + q); }
+  if (MODE == P1_MID) {
+    float p, q;
+    upk2(add2(KK[0], KK[1]), p, q);
+    a.kep += static_cast<double>(p + q);
+  }
+}
+// Logits of a lane-step (first vector gv) that lie outside the row become -Inf.
+template <int VEC>
+__device__ __forceinline__ void p1_mask(float* x, int gv, int nvec, int shift, int V) {
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    const int g = gv + 32 * (c / VEC), i = g * VEC - shift + (c % VEC);
+    if (!(g < nvec && i >= 0 && i < V)) x[c] = -INFINITY;
+  }
+}
+// A piece of a row without a cut held a logit far above the warp's anchor: the anchor moves up to the warp's maximum, and the
+// piece (the n steps from that of gv) is summed again. A row of a few heavy tokens comes here a few times. Returns the lane's sum.
+template <typename T, bool TONE>
+__device__ __noinline__ double p1_raise_anchor(const WideShared& sh, int gv, int n, float vmax, float& as, float& xlim) {
+  constexpr int VEC = Elem<T>::VEC, EPI = 8 / VEC, SV = 32 * EPI;
+  const float wmax = okey_to_float(__reduce_max_sync(FULL, okey(vmax)));
+  const float up = scale_t(wmax, sh.Tm);
+  if (!(fabsf(up) < 1e30f)) { xlim = INFINITY; return 0.0; }   // the row's maximum is no number: it ends in the two-pass form
+  as = up;
+  xlim = (up + W1_RISE) * sh.Tm;
+  P1Consts k;
+  k.as = up; k.Tm = sh.Tm; k.yT = TONE ? 1.0f : __frcp_rn(sh.Tm);
+  P1Acc a;
+  a.tot = 0.0; a.vmax = -INFINITY;
+  for (int s = 0; s < n; s++, gv += SV) {
+    float x[8];
+#pragma unroll
+    for (int h = 0; h < EPI; h++) Elem<T>::unpack(__ldg(sh.vbase + min(gv + 32 * h, sh.nvec - 1)), x + h * VEC);
+    p1_mask<VEC>(x, gv, sh.nvec, sh.shift, sh.V);
+    p1_body<VEC, TONE, P1_ALL>(x, k, a);
+  }
+  return a.tot;
+}
+
+// The pass. Leaves in shared memory: part[warp * ppw + piece], the mass of each piece (P1_MID: of its logits above the window), relative to the anchor; the warps' lists, and in from[warp][piece] where a piece begins in its warp's;
+// per warp kw (sum of its pieces), sc.d0 (all mass), sc.i0 (order key of the maximum), sc.i1 (1: a NaN, 2: a list that did
+// not hold all).
+template <typename T, bool TONE, int MODE>
+__device__ __noinline__ void wide_onepass_stream(unsigned char* dyn, WideShared& sh) {
+  constexpr int VEC = Elem<T>::VEC, EPI = 8 / VEC, SV = 32 * EPI;
+  constexpr uint32_t STAGE = EPI * W_NT * 16;                  // ring: EPI vectors per thread and stage
+  constexpr int NQ = W1_RING_BYTES / STAGE;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nvec = sh.nvec, shift = sh.shift, ppw = sh.ppw;
+  const int first = warp * sh.span, end = min(nvec, first + sh.span);
+  const int nst = (end > first) ? (end - first + SV - 1) / SV : 0;
+  // steps [clean_lo, clean_hi) hold no logit outside the row: all their vectors exist, none is the row's first or last
+  const int clean_lo = (first == 0) ? 1 : 0, clean_hi = min(nst, (nvec - 1 - first) / SV);
+  P1Consts k;
+  k.as = sh.as; k.C = sh.as * P1_L2E; k.Tm = sh.Tm; k.yT = TONE ? 1.0f : __frcp_rn(sh.Tm);
+  k.xA = sh.xA;
+  k.xmid = 0.5f * sh.xA + 0.5f * sh.xB;
+  k.xhalf = (0.5f * sh.xA - 0.5f * sh.xB) * 1.000001f + 1e-30f + 2.4e-7f * fabsf(k.xmid);
+  k.buf = smem_addr(dyn + W1_OFF_BUF) + static_cast<uint32_t>(tid) * 4u;
+  k.buf_end = k.buf + (W1_SLOTS - 4) * W_NT * 4u;
+  double* part_w = reinterpret_cast<double*>(dyn + W_OFF_PART) + warp * ppw;
+  float* list = reinterpret_cast<float*>(dyn + W1_OFF_LIST) + warp * W1_WCAP;
+  int* from = reinterpret_cast<int*>(dyn + W1_OFF_FROM) + warp * (W_MAX_PPW + 1);
+  int listed = 0;                                              // by the warp, so far
+  bool full = false;
+  if (lane == 0) from[0] = 0;
+  P1Acc a;
+  a.tot = 0.0; a.kep = 0.0; a.stot = 0.0; a.vmax = -INFINITY; a.at = k.buf;
+  // without a cut: sums are relative to the warp's anchor, and f brings them to the row's
+  float xlim = (k.as + W1_RISE) * k.Tm;
+  double f = 1.0;
+  // The ring: a thread copies the vectors it will take itself, and waits for its own copies only. A vector past the row's
+  // end is replaced by the row's last one (masked below).
+  const uint4* src = sh.vbase + first + lane;
+  const int omax = nvec - 1 - first - lane;                    // of the offsets from src (negative: none of the warp's steps runs then)
+  const uint32_t ring = smem_addr(dyn + W1_OFF_RING) + static_cast<uint32_t>(tid) * 16u;
+  const uint4* ring_at = reinterpret_cast<const uint4*>(dyn + W1_OFF_RING) + tid;
+  auto piece_end = [&](int st) {
+    if (MODE == P1_ALL) {
+      if (__any_sync(FULL, a.vmax > xlim)) {
+        float as = k.as, xl = xlim;
+        const int n = (st & (W_G - 1)) + 1;
+        a.tot = p1_raise_anchor<T, TONE>(sh, first + (st + 1 - n) * SV + lane, n, a.vmax, as, xl);
+        f = exp(static_cast<double>(as) - static_cast<double>(sh.as));
+        k.as = as; xlim = xl;
+      }
+    } else {
+      full |= a.at >= k.buf_end;
+      const int n = static_cast<int>((a.at - k.buf) / (W_NT * 4u));
+      for (int r = 0;; r++) {
+        const unsigned have = __ballot_sync(FULL, r < n);
+        if (have == 0u) break;
+        const int slot = listed + __popc(have & ((1u << lane) - 1u));
+        if (r < n && slot < W1_WCAP) {
+          float v;
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(k.buf + static_cast<uint32_t>(r) * (W_NT * 4u)));
+          list[slot] = v;
+        }
+        listed += __popc(have);
+      }
+      a.at = k.buf;
+      if (lane == 0) from[st / W_G + 1] = min(listed, W1_WCAP);
+    }
+    double t = a.kep;
+    if (MODE == P1_MID) a.kep = 0.0;
+    else { t = (MODE == P1_ALL) ? a.tot * f : a.tot; a.stot += t; a.tot = 0.0; }
+    const double kw = warp_sum_d(t);
+    if (lane == 0) part_w[st / W_G] = kw;
+  };
+  auto step = [&](int st, int slot, auto&& refill, bool clean) {
+    cp_wait<NQ - 1>();
+    float x[8];
+    Elem<T>::unpack(ring_at[slot * EPI * W_NT], x);
+    if (EPI == 2) Elem<T>::unpack(ring_at[slot * EPI * W_NT + W_NT], x + 4 * (EPI - 1));
+    refill();                                                  // into the slot just read
+    cp_commit();
+    if (!clean) p1_mask<VEC>(x, first + st * SV + lane, nvec, shift, sh.V);
+    p1_body<VEC, TONE, MODE>(x, k, a);
+  };
+  auto put = [&](int slot, const uint4* p0, const uint4* p1) {
+    cp_async16(ring + slot * STAGE, p0);
+    if (EPI == 2) cp_async16(ring + slot * STAGE + W_NT * 16u, p1);
+  };
+  auto put_any = [&](int slot, int q) { if (q < nst) put(slot, src + min(q * SV, omax), src + min(q * SV + 32, omax)); };
+#pragma unroll
+  for (int q = 0; q < NQ; q++) { put_any(q, q); cp_commit(); }
+  // Pieces that hold no step at the row's edges and whose refills are clean too run without a mask, a clamp or a test; W_G steps are
+  // a multiple of the ring's NQ.
+  static_assert(W_G % NQ == 0, "a piece begins at the ring's first slot");
+  int st = 0;
+#pragma unroll 1
+  while (st < nst) {
+    if (st >= clean_lo && st + W_G + NQ <= clean_hi) {
+      const uint4* p = src + (st + NQ) * SV;
+#pragma unroll 1
+      for (int j = 0; j < W_G; j += NQ, p += NQ * SV) {
+#pragma unroll
+        for (int q = 0; q < NQ; q++) step(st, q, [&]() { put(q, p + q * SV, p + q * SV + 32); }, true);
+      }
+      st += W_G;
+    } else {
+#pragma unroll 1
+      for (int j = 0; j < W_G && st < nst; j++, st++)
+        step(st, j % NQ, [&]() { put_any(j % NQ, st + NQ); }, st >= clean_lo && st < clean_hi);
+    }
+    piece_end(st - 1);
+  }
+  cp_wait<0>();
+  if (lane == 0) {
+    for (int q = (nst + W_G - 1) / W_G; q < ppw; q++) {        // pieces past the row's end
+      from[q + 1] = min(listed, W1_WCAP);
+      part_w[q] = 0.0;
+    }
+  }
+  __syncwarp();
+  const double kw = warp_sum_d((lane < ppw) ? part_w[lane] : 0.0);
+  const double S = warp_sum_d(MODE == P1_MID ? a.tot : a.stot);
+  const uint32_t wmax = __reduce_max_sync(FULL, okey(a.vmax));
+  const int odd = (__any_sync(FULL, a.vmax != a.vmax) ? 1 : 0) | ((MODE != P1_ALL && (listed > W1_WCAP || __any_sync(FULL, full))) ? 2 : 0);
+  if (lane == 0) { sh.kw[warp] = kw; sh.sc.d0[warp] = S; sh.sc.i0[warp] = static_cast<int>(wmax); sh.sc.i1[warp] = odd; }
+  __syncthreads();
+}
+
+// Places the window of a row with a cut: sh.as, xA, xB, low and eps. 0, or why the row takes two passes.
+template <typename T>
+__device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh, const double plim) {
+  constexpr int VEC = Elem<T>::VEC;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const float Tm = sh.Tm;
+  const int V = sh.V;
+  // ---- the sample: 64-byte pieces spread evenly over the row, none of them at its edges; a thread looks at what it copied itself
+  constexpr int J = W1_SAMPLE / (W_NT * VEC), PIECES = W_NT * J / 4;
+  const int have = (sh.nvec - 2) / 4;                                     // whole pieces between the row's first and last vector
+  if (have < 2 * PIECES) return 2;                                        // short rows: nothing to gain
+  {
+    const uint4* src = sh.vbase + 1 + (tid & 3);
+    const uint32_t dst = smem_addr(dyn) + static_cast<uint32_t>(tid) * 16u;
+#pragma unroll
+    for (int j = 0; j < J; j++) {
+      const int piece = static_cast<int>(static_cast<uint32_t>((static_cast<uint64_t>((j * W_NT + tid) >> 2) * static_cast<uint32_t>(have)) / PIECES));
+      cp_async16(dst + j * W_NT * 16, src + piece * 4);
+    }
+    cp_commit();
+  }
+  uint32_t* bins = reinterpret_cast<uint32_t*>(dyn + W1_SAMPLE * 4);
+  for (int j = tid; j < W1_SBINS; j += W_NT) bins[j] = 0u;
+  auto each = [&](auto&& fn) {
+#pragma unroll 2
+    for (int j = 0; j < J; j++) {
+      float x[VEC];
+      Elem<T>::unpack(reinterpret_cast<const uint4*>(dyn)[j * W_NT + tid], x);
+#pragma unroll
+      for (int c = 0; c < VEC; c++) fn(x[c]);
+    }
+  };
+  cp_wait<0>();
+  float smax = -INFINITY, smin = INFINITY;
+  each([&](float x) { smax = maxnan(smax, x); smin = fminf(smin, x); });
+  {
+    uint32_t hi = okey(smax), lo = ~okey(smin), nan = (smax != smax) ? 1u : 0u;
+    bu::max_u3<W_NW>(hi, lo, nan, sh.sc, tid);                            // (its barriers also publish the cleared bins)
+    if (nan) return 3;
+    smax = okey_to_float(hi);
+    smin = okey_to_float(~lo);
+  }
+  const float as = scale_t(smax, Tm);
+  if (!(fabsf(smax) < 1e30f) || !(fabsf(as) < 1e30f)) return 3;
+  // ---- a count histogram of its upper 24 units of x / T (what lies lower has no mass to speak of, and shares the last bucket)
+  const float range = fmaxf(fminf(smax - smin, 24.0f * Tm), 1e-6f * fmaxf(fabsf(smax), Tm));
+  const float scale = static_cast<float>(W1_SBINS - 1) / range;
+  each([&](float x) { atomicAdd(&bins[static_cast<int>(fminf((smax - x) * scale, static_cast<float>(W1_SBINS - 1)))], 1u); });
+  if (tid == 0) { sh.bc[0] = 0; sh.bc[1] = W1_SBINS - 1; sh.bc[2] = 0; sh.bc[3] = W1_SAMPLE; }
+  __syncthreads();
+  // ---- the window: where the sample's mass passes plim, give or take five standard errors of a mass fraction
+  // estimated from weighted logits (Var = ((1-p)^2 sum of squared weights above the cut + p^2 of those below) / (sum of
+  // weights)^2). Placing it is a matter of speed, not of correctness (the pass checks it on the whole row): f32 does.
+  constexpr int PER = W1_SBINS / W_NT;
+  const float wl2 = range / (Tm * static_cast<float>(W1_SBINS - 1)) * 1.4426950408889634f;   // bucket width in units of log2
+  int cnt[PER] = {}, n = 0;
+  float mass = 0.0f, sq = 0.0f;
+  const float ratio = ex2_approx(-wl2), e0 = ex2_approx(-(static_cast<float>(tid * PER) + 0.5f) * wl2);
+  auto weight = [&](int j, float e) { return (tid * PER + j == W1_SBINS - 1) ? 0.0f : static_cast<float>(cnt[j]) * e; };
+  {
+    float e = e0;
+#pragma unroll
+    for (int j = 0; j < PER; j++) {
+      cnt[j] = static_cast<int>(bins[tid * PER + j]);
+      const float c = weight(j, e);
+      n += cnt[j]; mass += c; sq = fmaf(c, e, sq);
+      e *= ratio;
+    }
+  }
+  float im = mass, iq = sq;
+  int in = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const float a = __shfl_up_sync(FULL, im, o), b = __shfl_up_sync(FULL, iq, o);
+    const int c = __shfl_up_sync(FULL, in, o);
+    if (lane >= o) { im += a; iq += b; in += c; }
+  }
+  float* wm = reinterpret_cast<float*>(sh.sc.d0);
+  float* wq = reinterpret_cast<float*>(sh.sc.d1);
+  if (lane == 31) { wm[warp] = im; wq[warp] = iq; sh.sc.i0[warp] = in; }
+  if (tid == 0) wq[W_NW] = -1.0f;
+  __syncthreads();
+  float tot_m = 0.0f, tot_q = 0.0f;
+  im -= mass; iq -= sq; in -= n;                                          // exclusive
+#pragma unroll
+  for (int w = 0; w < W_NW; w++) {
+    const float a = wm[w], b = wq[w];
+    if (w < warp) { im += a; iq += b; in += sh.sc.i0[w]; }
+    tot_m += a; tot_q += b;
+  }
+  if (!(tot_m * 2.4e-3f >= 1.0f)) return 8;                               // heavy tokens (one above 1/400 of the mass): not for a sample to place
+  const float pl = static_cast<float>(plim), lim = pl * tot_m;
+  if (im < lim && im + mass >= lim) wq[W_NW] = iq + sq;                   // one thread (none: nothing lies below the cut)
+  __syncthreads();
+  const float q_above = (wq[W_NW] >= 0.0f) ? wq[W_NW] : tot_q, q1 = 1.0f - pl;
+  const float fpc = 1.0f - static_cast<float>(W1_SAMPLE) / static_cast<float>(V);
+  const float delta = 5.0f * sqrtf(fmaxf(q1 * q1 * q_above + pl * pl * (tot_q - q_above), 0.0f) * fpc) + 2.0f;   // in units of mass: two top tokens more
+  const float m_lo = lim - delta, m_hi = lim + delta;
+  {
+    float e = e0, acc = im;
+    int c = in;
+#pragma unroll
+    for (int j = 0; j < PER; j++) {                                       // prefixes grow: one bucket passes either limit first
+      const float next = acc + weight(j, e);
+      if (acc < m_lo && next >= m_lo) { sh.bc[0] = tid * PER + j; sh.bc[2] = c; }
+      if (acc < m_hi && next >= m_hi) { sh.bc[1] = tid * PER + j; sh.bc[3] = c + cnt[j]; }
+      c += cnt[j];
+      acc = next;
+      e *= ratio;
+    }
+  }
+  __syncthreads();
+  const int b1 = max(sh.bc[0] - 1, 0), b2 = min(sh.bc[1] + 1, W1_SBINS - 1);   // a bucket of slack for the f32 sums
+  // How many logits of the row will be listed: the window's mass over that of its last logit, or the sample's count of a hundred
+  // or so (which by itself would be off by a tenth) and three standard deviations, whichever is less; and of the buckets of slack as
+  // many as the window's have on average. The lists hold five standard deviations more, and a lane's buffer of 12 for a piece is
+  // too small in less than one of 10^8 pieces. A window that reaches down to where no mass is saves instructions.
+  auto fits = [&](float logits) {
+    const float per_warp = logits * (static_cast<float>(V) / static_cast<float>(W1_SAMPLE * W_NW));
+    const float per_visit = per_warp / static_cast<float>(32 * max(sh.nvec / (W_NT * (8 / VEC) * W_G), 1));
+    return per_warp + 5.0f * sqrtf(per_warp) <= static_cast<float>(W1_WCAP) && per_visit <= 1.5f;
+  };
+  const float seen = static_cast<float>(max(sh.bc[3] - sh.bc[2], 0));
+  const float inside = fminf(2.0f * delta / ex2_approx(-(static_cast<float>(sh.bc[1]) + 0.5f) * wl2), seen + 3.0f * sqrtf(seen)), per_bucket = inside / static_cast<float>(max(sh.bc[1] - sh.bc[0] + 1, 1));
+  const bool low = fits(static_cast<float>(W1_SAMPLE - sh.bc[2]) + per_bucket);
+  if (!low && !fits(inside + 2.0f * per_bucket)) return 10;
+  const float xA = smax - static_cast<float>(b1) / scale;
+  const float xB = (low || b2 == W1_SBINS - 1) ? smax - 40.0f * Tm : smax - static_cast<float>(b2 + 1) / scale;
+  if (!(xA > xB)) return 11;
+  if (tid == 0) {
+    sh.as = as; sh.xA = xA; sh.xB = xB; sh.low = low ? 1 : 0;
+    sh.eps = W1_EPS_FIXED + W1_EPS_PER_D * fmin(9.7, static_cast<double>(range / Tm) + 2.0);
+  }
+  return 0;
+}
+
+// One row. 0, or why it takes two passes (nothing of it has been written then).
+template <typename T>
+__device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t row_id, unsigned char* dyn, WideShared& sh) {
+  const KernelArgs& A = BA.k;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  constexpr int VEC = Elem<T>::VEC, SV = 32 * (8 / VEC), PV = W_G * SV;
+  bu::Scratch& sc = sh.sc;
+  const double* s_tab = sh.tab;
+  const RowCfg cfg = A.cfgs[row_id];
+  const float Tm = cfg.temperature;
+  const int mode = cfg.topp_mode;
+  const double plim = (mode == 0) ? static_cast<double>(cfg.top_p) * 1.5 : static_cast<double>(cfg.top_p);
+  // mode A prunes only while the mass exceeds 1.5p; the mass starts at 1 up to ~1e-11 of rounding
+  // and 1.5*float(p) is never that close to 1
+  const bool cut_on = cfg.top_p > 0.0f && cfg.top_p < 1.0f && !(mode == 0 && plim >= 1.0);
+  const bool t_is_one = (Tm == 1.0f);
+  if (!t_is_one && !(Tm >= 9.5367431640625e-7f && Tm <= 1048576.0f && (__float_as_uint(Tm) & 0x7fffffu) != 0x7fffffu)) return 1;
+  {
+    RowView<T> rv;
+    rv.init(static_cast<const T*>(A.logits) + row_id * A.row_stride, A.V);
+    const int span = (((rv.nvec + W_NW - 1) / W_NW + SV - 1) / SV) * SV;   // a warp's part of the row, in whole steps
+    if (span / SV > W_MAX_STEPS) return 17;
+    if (tid == 0) {
+      sh.vbase = rv.vbase; sh.V = rv.V; sh.shift = rv.shift; sh.nvec = rv.nvec;
+      sh.span = span; sh.ppw = (span / SV + W_G - 1) / W_G;
+      sh.Tm = Tm; sh.xA = 0.0f; sh.xB = 0.0f;
+      sh.eps = W1_EPS_FIXED + W1_EPS_PER_D * 9.7;
+    }
+    if (!cut_on) {
+      // ---- the anchor: the largest logit of the warps' first steps
+      float smax = -INFINITY;
+#pragma unroll
+      for (int h = 0; h < 8 / VEC; h++) {
+        const int g = warp * span + 32 * h + lane;
+        if (g < rv.nvec) rv.visit(g, [&](float xv, int) { smax = maxnan(smax, xv); });
+      }
+      uint32_t top = okey(smax), nan = (smax != smax) ? 1u : 0u, none = 0u;
+      bu::max_u3<W_NW>(top, nan, none, sc, tid);
+      const float as = scale_t(okey_to_float(top), Tm);
+      if (nan || !(fabsf(as) < 1e30f)) return 3;
+      if (tid == 0) sh.as = as;
+    }
+  }
+  __syncthreads();
+  if (cut_on) {
+    const int why = wide_place_window<T>(dyn, sh, plim);
+    if (why) return why;
+  }
+  __syncthreads();
+  const bool low = cut_on && sh.low;
+  if (low) {
+    if (t_is_one) wide_onepass_stream<T, true, P1_LOW>(dyn, sh); else wide_onepass_stream<T, false, P1_LOW>(dyn, sh);
+  } else if (cut_on) {
+    if (t_is_one) wide_onepass_stream<T, true, P1_MID>(dyn, sh); else wide_onepass_stream<T, false, P1_MID>(dyn, sh);
+  } else {
+    if (t_is_one) wide_onepass_stream<T, true, P1_ALL>(dyn, sh); else wide_onepass_stream<T, false, P1_ALL>(dyn, sh);
+  }
+  // ---- the row's sums and maximum
+  const bool mine = lane < W_NW;
+  const float m = scale_t(okey_to_float(__reduce_max_sync(FULL, mine ? static_cast<uint32_t>(sc.i0[lane]) : 0u)), Tm);
+  const int any = __reduce_or_sync(FULL, mine ? sc.i1[lane] : 0);
+  double S = warp_sum_d(mine ? sc.d0[lane] : 0.0);
+  double Ktot = warp_sum_d(mine ? sh.kw[lane] : 0.0);
+  if ((any & 1) || !(fabsf(m) < INFINITY)) return 12;                      // the two-pass form reports such rows
+  if (any & 2) return 5;
+  // with a cut the anchor is the sample's maximum: it must be close to the row's for the heavy logits to keep the error budget
+  if (cut_on && !(fabsf(m - sh.as) <= 2.0f)) return 13;
+  if (!(S > 0.0) || !(S < 1e300)) return 14;
+  // everything so far is relative to exp(anchor); from here on to exp(max)
+  const double anchor = cut_on ? static_cast<double>(sh.as * P1_L2E) / static_cast<double>(P1_L2E) : static_cast<double>(sh.as);
+  const double cf = exp(anchor - static_cast<double>(m));
+  S *= cf;
+  Ktot *= cf;
+  if (!(S > 0.0)) return 14;
+  const int ppw = sh.ppw, span = sh.span;
+  const float xA = sh.xA, xB = sh.xB;
+  const int* from = reinterpret_cast<const int*>(dyn + W1_OFF_FROM);
+  const double* part = reinterpret_cast<const double*>(dyn + W_OFF_PART);
+  uint32_t* bins = reinterpret_cast<uint32_t*>(dyn + W1_OFF_BINS);
+  uint32_t flags = FLAG_GENERAL_PATH;
+  RowView<T> rv;
+  rv.vbase = sh.vbase; rv.V = sh.V; rv.shift = sh.shift; rv.nvec = sh.nvec;
+
+  // ---- the cut. The order of the kept set is by d, equal ones by index: a class of equal d is kept, dropped, or divided
+  // by an index.
+  unsigned long long cut_key = 0ull;       // window entries are kept when key < cut_key, or == with cut_incl
+  int cut_incl = 0;
+  float dstar = INFINITY;
+  double estar = 0.0, zw = 0.0;            // mass of one member of the cut's class; lane w: what the window adds to warp w's part
+  bool by_piece = false, ties_in = false;  // kept members of the class: counted per piece in bins[], or all of them
+  if (cut_on) {
+    const double lim = plim * S;
+    auto crossed = [&](double g) -> bool { return mode == 0 ? (g > lim) : (g >= lim); };
+    float* list = reinterpret_cast<float*>(dyn + W1_OFF_LIST) + warp * W1_WCAP;   // every warp works on its own list
+    double* mass = reinterpret_cast<double*>(dyn + W1_OFF_MASS) + warp * W1_WCAP;
+    from += warp * (W_MAX_PPW + 1);
+    const int cnt = from[ppw];
+    const float dA = scale_t(xA, Tm) - m, dB = scale_t(xB, Tm) - m;
+    float dhi = dA, dlo = dB, scale = static_cast<float>(W1_BINS) / (dA - dB);
+    auto bucket = [&](float d) { return static_cast<int>(fminf((dhi - d) * scale, static_cast<float>(W1_BINS - 1))); };
+    bins[tid] = 0u;
+    if (tid == 0) { sh.bc[0] = W1_BINS; sh.bc[1] = W1_BINS - 1; sh.cnt = 0; }
+    __syncthreads();
+    // logits -> d, in place (1: not in the window, the lists hold a little more), their masses, and their counts by bucket of d
+    double inside = 0.0;
+    for (int j = lane; j < cnt; j += 32) {
+      const float x = list[j];
+      const float d = (x >= xB && x < xA) ? scale_t(x, Tm) - m : 1.0f;
+      list[j] = d;
+      if (d <= 0.0f) {
+        const double e = exp_safe(d, s_tab);
+        mass[j] = e;
+        inside += e;
+        atomicAdd(&bins[bucket(d)], 1u);
+      }
+    }
+    if (low) {                                               // what is not listed is kept
+      inside = bu::sum_d<W_NW>(inside, sc, tid);             // (its barriers also publish the counts)
+      Ktot = S - inside;
+    } else {
+      __syncthreads();
+    }
+    // the cut must lie below the window's upper end by more than the error of the sums
+    if (!(Ktot < lim - (1e-12 + 2.0 * plim * fabs(1.0 - plim) * sh.eps + 1e-9) * S)) return 15;
+    double gbase = Ktot;                                     // mass of everything above dhi
+    double zsum = 0.0;                                       // this lane's window mass above the crossing's buckets
+    int nc = 0;
+    bool one_class = false;
+    for (int round = 0;; round++) {                          // uniform
+      // The bucket of the crossing, from bounds of the mass through each bucket (a bucket's members lie between its edges): the
+      // first that can cross, and the first that must. The slack covers the f32 sums and edges.
+      {
+        const float need = static_cast<float>(lim - gbase), width = 1.0f / scale;
+        const float c = static_cast<float>(bins[tid]);
+        const float top = dhi - static_cast<float>(tid) * width;
+        float hi = c * ex2_approx(top * 1.44269504f) * (1.0f + 2e-5f), lo = c * ex2_approx((top - width) * 1.44269504f) * (1.0f - 2e-5f);
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const float a = __shfl_up_sync(FULL, hi, o), b = __shfl_up_sync(FULL, lo, o);
+          if (lane >= o) { hi += a; lo += b; }
+        }
+        float* wh = reinterpret_cast<float*>(sc.d0);
+        float* wl = reinterpret_cast<float*>(sc.d1);
+        if (lane == 31) { wh[warp] = hi; wl[warp] = lo; }
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < W_NW; w++) if (w < warp) { hi += wh[w]; lo += wl[w]; }
+        const unsigned may = __ballot_sync(FULL, hi >= need && c > 0.0f), must = __ballot_sync(FULL, lo >= need && c > 0.0f);
+        if (lane == 0 && may) atomicMin(&sh.bc[0], warp * 32 + __ffs(may) - 1);
+        if (lane == 0 && must) atomicMin(&sh.bc[1], warp * 32 + __ffs(must) - 1);
+        __syncthreads();
+      }
+      const int b1 = sh.bc[0], b2 = max(sh.bc[1], b1);
+      if (b1 == W1_BINS) return 16;                          // the window ends before the cut
+      // what lies above the crossing's buckets is kept; what lies in them is looked at one by one
+      double sure = 0.0;
+      float cmax = -INFINITY, cmin = 1.0f;
+      float* cd = reinterpret_cast<float*>(bins);            // the candidates: d, the warp they come from (the buckets have been read)
+      int* cl = reinterpret_cast<int*>(bins) + 32;
+      for (int j = lane; j < cnt; j += 32) {
+        const float d = list[j];
+        if (d <= dhi && d >= dlo) {
+          const int b = bucket(d);
+          if (b < b1) sure += mass[j];
+          else if (b <= b2) {
+            cmin = (cmin > 0.0f) ? d : fminf(cmin, d); cmax = fmaxf(cmax, d);
+            const int slot = atomicAdd(&sh.cnt, 1);
+            if (slot < 32) { cd[slot] = d; cl[slot] = warp; }
+          }
+        }
+      }
+      zsum += sure;
+      gbase += bu::sum_d<W_NW>(sure, sc, tid);
+      nc = sh.cnt;
+      if (nc <= 32) break;
+      uint32_t kmax = dkey_of(cmin), inv = ~dkey_of(cmax), none = 0u;      // (dkey falls as d rises)
+      if (cmin > 0.0f) { kmax = 0u; inv = 0u; }                            // none here
+      bu::max_u3<W_NW>(kmax, inv, none, sc, tid);
+      dhi = -__uint_as_float(~inv); dlo = -__uint_as_float(kmax);
+      if (dhi == dlo) { one_class = true; break; }           // a long run of equal d
+      if (round == 5) return 16;
+      scale = fminf(static_cast<float>(W1_BINS) / (dhi - dlo), 1e30f);
+      bins[tid] = 0u;
+      if (tid == 0) { sh.bc[0] = W1_BINS; sh.bc[1] = W1_BINS - 1; sh.cnt = 0; }
+      __syncthreads();
+      for (int j = lane; j < cnt; j += 32) {
+        const float d = list[j];
+        if (d <= dhi && d >= dlo) atomicAdd(&bins[bucket(d)], 1u);
+      }
+      __syncthreads();
+    }
+    // ---- the class of the crossing: its d, the mass above it, its size. Every warp finds it by itself, a candidate per lane.
+    double gb = gbase;
+    int neq = nc;
+    const float d_l = (!one_class && lane < nc) ? reinterpret_cast<const float*>(bins)[lane] : -INFINITY;
+    const int from_l = (!one_class && lane < nc) ? reinterpret_cast<const int*>(bins)[32 + lane] : -1;
+    const double e_l = (d_l <= 0.0f && lane < nc) ? exp_safe(d_l, s_tab) : 0.0;
+    if (one_class) {
+      dstar = dhi;
+    } else {
+      double g = gbase;
+      int eq = 0;
+      for (int i = 0; i < nc; i++) {
+        const float o = __shfl_sync(FULL, d_l, i);
+        const double oe = __shfl_sync(FULL, e_l, i);
+        g += (o > d_l) ? oe : 0.0;
+        eq += (o == d_l) ? 1 : 0;
+      }
+      const bool cr = lane < nc && crossed(g + eq * e_l);
+      const uint32_t best = __reduce_min_sync(FULL, cr ? dkey_of(d_l) : 0xffffffffu);
+      if (best == 0xffffffffu) return 16;                    // rounding: nothing in the window crosses
+      const int who = __ffs(__ballot_sync(FULL, cr && dkey_of(d_l) == best)) - 1;
+      dstar = -__uint_as_float(best);
+      gb = __shfl_sync(FULL, g, who);
+      neq = __shfl_sync(FULL, eq, who);
+    }
+    // Several logits can share one d: a class that also has members outside the window is decided on the whole row
+    if (dstar == dA || dstar == scale_t(nextafterf(xB, -INFINITY), Tm) - m) return 16;
+    // the first member whose mass crosses (mode B keeps through it, mode A everything before it)
+    estar = exp_safe(dstar, s_tab);
+    if (!crossed(gb + neq * estar)) return 16;
+    int r = 1;
+    if (neq > 1) {
+      r = static_cast<int>(fmin(fmax(ceil((lim - gb) / estar), 1.0), static_cast<double>(neq)));
+      while (r > 1 && crossed(gb + (r - 1) * estar)) r--;
+      while (r < neq && !crossed(gb + r * estar)) r++;
+    }
+    const double etol = (1e-12 + 2.0 * plim * fabs(1.0 - plim) * sh.eps) * S;
+    if (fabs(gb + r * estar - lim) <= etol || fabs(gb + (r - 1) * estar - lim) <= etol) flags |= FLAG_TOPP_EDGE;
+    if (mode == 1 && r < neq) flags |= FLAG_TIE_CUT;         // the cut separates equal probabilities
+    const int kept = (mode == 0) ? r - 1 : r;
+    const unsigned long long dk = static_cast<unsigned long long>(dkey_of(dstar)) << 32;
+    ties_in = kept == neq;
+    cut_key = ties_in ? (dk | 0xffffffffull) : dk;
+    cut_incl = ties_in ? 1 : 0;
+    by_piece = kept > 0 && (one_class || !ties_in);
+    // ---- what the window adds to each warp's part of the row (lane w: warp w); where that already holds all of the window's mass, less
+    // all of it
+    if (low) for (int j = lane; j < cnt; j += 32) zsum -= (list[j] <= 0.0f) ? mass[j] : 0.0;
+    zsum = warp_sum_d(zsum);
+    __syncthreads();                                         // (the candidates have been read)
+    if (lane == 0) sh.zw[warp] = zsum;
+    if (by_piece) {
+      // members per piece, then which of them stay: the lowest indices in mode B, the highest in mode A
+      bins[tid] = 0u;
+      __syncthreads();
+      for (int j = lane, q = 0; j < cnt; j += 32) {
+        if (list[j] == dstar) {
+          while (from[q + 1] <= j) q++;
+          atomicAdd(&bins[warp * ppw + q], 1u);
+        }
+      }
+      __syncthreads();
+      const int have = (tid < W_NW * ppw) ? static_cast<int>(bins[tid]) : 0;
+      const int q = (mode == 0) ? neq - kept + 1 : kept;     // rank, from the lowest index, of the member at the edge
+      int incl = have;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(FULL, incl, o); if (lane >= o) incl += t; }
+      if (lane == 31) sc.i0[warp] = incl;
+      if (tid == 0) { sh.bc[0] = -1; sh.bc[2] = -1; }
+      __syncthreads();
+      const int pre = incl - have + __reduce_add_sync(FULL, (lane < warp && lane < W_NW) ? sc.i0[lane] : 0);
+      const int below = min(max(q - pre, 0), have), strictly = min(max(q - 1 - pre, 0), have);
+      bins[tid] = static_cast<uint32_t>((mode == 0) ? have - strictly : below);
+      if (have > 0 && pre < q && q <= pre + have) { sh.bc[0] = tid; sh.bc[1] = q - pre; }
+      __syncthreads();
+      if (!ties_in) {
+        // the member's index: one piece of the row again
+        const int pi = sh.bc[0], rank = sh.bc[1];
+        if (pi < 0) return 16;
+        constexpr int NV = (PV + W_NT - 1) / W_NT;
+        const int w = pi / ppw, vb = w * span + (pi - w * ppw) * PV, v = vb + tid * NV;
+        const int vend = min(min(vb + PV, w * span + span), rv.nvec);
+        uint32_t mask = 0u;
+        const int i0 = v * VEC - rv.shift;
+#pragma unroll
+        for (int h = 0; h < NV; h++) {
+          if (tid * NV + h < PV && v + h < vend) {
+            float x[VEC];
+            Elem<T>::unpack(__ldg(rv.vbase + v + h), x);
+#pragma unroll
+            for (int c = 0; c < VEC; c++) {
+              const int i = i0 + h * VEC + c;
+              if (i >= 0 && i < rv.V && x[c] >= xB && x[c] < xA && scale_t(x[c], Tm) - m == dstar) mask |= 1u << (h * VEC + c);
+            }
+          }
+        }
+        const int n = __popc(mask);
+        int inc = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) { const int t = __shfl_up_sync(FULL, inc, o); if (lane >= o) inc += t; }
+        if (lane == 31) sc.i1[warp] = inc;
+        __syncthreads();
+        const int ahead = inc - n + __reduce_add_sync(FULL, (lane < warp && lane < W_NW) ? sc.i1[lane] : 0);
+        if (ahead < rank && rank <= ahead + n) {
+          for (int z = rank - ahead; z > 1; z--) mask &= mask - 1u;
+          sh.bc[2] = i0 + __ffs(mask) - 1;
+        }
+        __syncthreads();
+        if (sh.bc[2] < 0) return 16;                         // (a list that disagrees with the row)
+        cut_key = zone_key(dstar, sh.bc[2], mode);
+        cut_incl = 1;
+      }
+    } else {
+      __syncthreads();
+    }
+    zw = mine ? sh.zw[lane] : 0.0;
+    if (!one_class) {
+      // candidates above the class, and the class when all of it stays, count with the warps that listed them
+      const double add = (lane < nc && (d_l > dstar || (d_l == dstar && ties_in))) ? e_l : 0.0;
+      for (int i = 0; i < nc; i++) {
+        const double ae = __shfl_sync(FULL, add, i);
+        if (__shfl_sync(FULL, from_l, i) == lane) zw += ae;
+      }
+    }
+    if (by_piece && mine) {
+      int stay = 0;
+      for (int q = 0; q < ppw; q++) stay += static_cast<int>(bins[lane * ppw + q]);
+      zw += estar * stay;
+    }
+  }
+  // ---- kept mass, and the warp in whose part of the row u falls: u < prefix / Re (generate.go:231-239) as u Re < prefix
+  const double wv = mine ? sh.kw[lane] * cf + zw : 0.0;
+  const double wi = warp_scan_incl_d(wv, lane);
+  const double Re = __shfl_sync(FULL, wi, W_NW - 1);
+  const double u = A.uniforms[row_id];
+  const double tgt = u * Re;
+  auto kept_mass = [&](float xv, int i) -> double {          // final rule for one logit: its kept mass (0 when cut away)
+    if (i < 0 || i >= rv.V) return 0.0;
+    const float d = (t_is_one ? xv : __fdiv_rn(xv, Tm)) - m;
+    if (cut_on && !(xv >= xA)) {
+      if (!(xv >= xB)) return 0.0;
+      const unsigned long long key = zone_key(d, i, mode);
+      if (!(key < cut_key || (cut_incl && key == cut_key))) return 0.0;
+    }
+    return exp_safe(d, s_tab);
+  };
+  if (!(Re > 0.0)) {                                         // mode A removed every token
+    wide_write_nothing_kept(A, row_id, m, S, 3, flags);
+    return 0;
+  }
+  WideResult res;
+  res.m = m; res.S = S; res.Re = Re; res.path = 3;
+  int psel = 0x7fffffff;
+  double before = Re;
+  const unsigned hit = __ballot_sync(FULL, mine && tgt < wi);
+  if (hit) {                                                 // uniform: the same bits in every warp
+    const int ws = __ffs(hit) - 1;
+    const double base = __shfl_sync(FULL, wi - wv, ws);
+    for (int q = warp; q < ppw; q += W_NW) {                 // that warp's pieces, by all warps
+      double zp = 0.0;
+      if (cut_on) {
+        const float* lw = reinterpret_cast<const float*>(dyn + W1_OFF_LIST) + ws * W1_WCAP;
+        const double* mw = reinterpret_cast<const double*>(dyn + W1_OFF_MASS) + ws * W1_WCAP;
+        const int* fw = reinterpret_cast<const int*>(dyn + W1_OFF_FROM) + ws * (W_MAX_PPW + 1);
+        const int j1 = fw[q + 1];
+        for (int j = fw[q] + lane; j < j1; j += 32) {
+          const float d = lw[j];
+          if (d <= 0.0f) {
+            const bool in = d > dstar || (d == dstar && ties_in && !by_piece);
+            zp += in ? (low ? 0.0 : mw[j]) : (low ? -mw[j] : 0.0);
+          }
+        }
+        zp = warp_sum_d(zp);
+        if (by_piece) zp += estar * static_cast<int>(bins[ws * ppw + q]);
+      }
+      if (lane == 0) sh.pm[q] = part[ws * ppw + q] * cf + zp;
+    }
+    __syncthreads();
+    const double pv = (lane < ppw) ? sh.pm[lane] : 0.0;
+    const double pi = base + warp_scan_incl_d(pv, lane);
+    const unsigned in = __ballot_sync(FULL, lane < ppw && tgt < pi);
+    const int q = in ? __ffs(in) - 1 : ppw - 1;              // (rounding: the warp's last piece, from which the walk goes on)
+    psel = ws * ppw + q;
+    before = __shfl_sync(FULL, pi - pv, q);
+  }
+  wide_draw<T>(A, row_id, rv, span, ppw, psel, before, u, res, flags, sh, kept_mass);
+  return 0;
+}
