@@ -9,28 +9,27 @@ namespace GS_N_NS {
 constexpr int N_NT = GS_N_NT;           // threads per CTA
 constexpr int N_NW = N_NT / 32;
 constexpr int N_WARM_ELEMS = 16 * N_NT; // logits of the warm-up chunk: 16 per thread, kept in registers
-// 256 threads: five CTAs per SM (48 registers, 42 KB of dynamic shared memory: the ring that the
-// stream is staged through, the candidate list, the hit list). 128 threads: eight CTAs per SM
-// (64 registers, 20 KB: candidate list, ring, hit list). What runs while no copy is in flight works in
-// memory that is dead by then: the prune in the ring; the finish in the ring (256 threads), or over
-// the candidate list and the ring, with the kept set in the hit list's place (128 threads).
+// 256 threads: five CTAs per SM (48 registers, 34 KB of dynamic shared memory: the candidate list, the ring that the
+// stream is staged through, the hit list). 128 threads: eight CTAs per SM (64 registers, 20 KB). What runs while no copy is in
+// flight works in memory that is dead by then: the prune in the ring; the finish over the candidate list and the ring, with
+// the kept set in the hit list's place. What the CTAs leave of an SM's memory is L1, which the greedy rows' register loads need
+// on their way: with a ring of 24 KB and work areas of its own the 256-thread instance left 28 KB (greedy rows,
+// 512 x 100,003 f32: 61 us against 46; 512 x 151,936 bf16: 49 against 39; top-k rows 1.00 to 1.09 times faster, but 256 x 100,003 f32, two
+// rows per SM, where the longer ring counted, 40.1 against 41.9).
 constexpr int N_CTAS_PER_SM = (N_NT == 256) ? 5 : 8;
 constexpr int N_CAP = (N_NT == 256) ? 1536 : 1024;   // candidate capacity (entries of 8 B)
 constexpr int N_KEEP = 768;                           // a prune must get below this
 constexpr int N_HITS = (N_NT == 256) ? 1536 : 1024;  // hit list: positions of lane-steps that hold a candidate (4 B each)
-constexpr int N_RING_BYTES = (N_NT == 256) ? 24576 : 8192;
-constexpr int N_RING_OFF = (N_NT == 256) ? 0 : 8192;
-constexpr int N_CAND_OFF = (N_NT == 256) ? 24576 : 0;
-constexpr int N_HITS_OFF = (N_NT == 256) ? N_CAND_OFF + N_CAP * 8 : 16384;
-constexpr int N_KEPT_OFF = (N_NT == 256) ? 0 : N_HITS_OFF;   // what the finish works on: KEEP_MAX entries
-constexpr int N_WORK_OFF = (N_NT == 256) ? 8192 : 0;         // its work arrays
-constexpr int N_TMP_OFF = (N_NT == 256) ? 8192 : 8192;    // the prune's buffer ...
-constexpr int N_TMP_CAP = (N_NT == 256) ? 2048 : 1024;    // ... and its entries
+constexpr int N_RING_BYTES = (N_NT == 256) ? 16384 : 8192;
+constexpr int N_CAND_OFF = 0;
+constexpr int N_RING_OFF = N_CAP * 8;
+constexpr int N_HITS_OFF = N_RING_OFF + N_RING_BYTES;
+constexpr int N_KEPT_OFF = N_HITS_OFF;                // what the finish works on: KEEP_MAX entries
+constexpr int N_WORK_OFF = 0;                         // its work arrays
+constexpr int N_TMP_OFF = N_RING_OFF;                 // the prune's buffer ...
+constexpr int N_TMP_CAP = N_RING_BYTES / 8;           // ... and its entries
 constexpr int N_DYN_BYTES = N_HITS_OFF + N_HITS * 4;
-static_assert((N_NT == 256) ? (N_KEPT_OFF + KEEP_MAX * 8 <= N_WORK_OFF && N_WORK_OFF + SS_WORK_BYTES <= N_RING_BYTES)
-                            : (KEEP_MAX * 8 <= N_HITS * 4 && N_WORK_OFF + SS_WORK_BYTES <= N_HITS_OFF),
-              "the finish works in memory that is dead by then");
-static_assert(N_TMP_OFF >= N_RING_OFF && N_TMP_OFF + N_TMP_CAP * 8 <= N_RING_OFF + N_RING_BYTES, "the prune's buffer lies in the ring");
+static_assert(KEEP_MAX * 8 <= N_HITS * 4 && N_WORK_OFF + SS_WORK_BYTES <= N_HITS_OFF, "the finish works in memory that is dead by then");
 static_assert(N_TMP_CAP >= N_KEEP && N_KEEP + 8 <= N_CAP, "a pruned list fits its buffer and leaves room for a portion of hits");
 
 // This thread's largest logit above -Inf, as (order key, ~vector): the lowest vector of equals; 0: none. NaNs are not
@@ -183,7 +182,7 @@ __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned c
   // cannot run that far ahead: in a rolled loop they share one scoreboard, so waiting for the
   // oldest waits for the newest too. The first copies go out now and fly during the selection.
   constexpr int EPI = 8 / VEC, SV = 32 * EPI;
-  constexpr int NQ = N_RING_BYTES / (EPI * N_NT * 16);       // stages: 6 of bf16, 3 of f32 (128 threads: 4 and 2)
+  constexpr int NQ = N_RING_BYTES / (EPI * N_NT * 16);       // stages: 4 of bf16, 2 of f32
   const int lane = tid & 31, warp = tid >> 5;
   const int rest = max(rv.nvec - warm, 0);
   const int span = (((rest + N_NW - 1) / N_NW + SV - 1) / SV) * SV;
