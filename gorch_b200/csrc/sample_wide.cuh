@@ -1,11 +1,8 @@
 // wide_rows_kernel: rows whose softmax runs over the whole vocabulary (top-k off).
 //
-// One row at a time per persistent CTA. Warp w owns one contiguous span of the row (1/W_NW of it,
-// rounded up to whole steps); in a step every lane handles eight logits (two 16-byte vectors
-// of f32, one of bf16), loaded straight into registers one or two steps ahead of their use
-// and asked from L2 two steps before that. Nothing is shared between threads inside a pass,
-// so a pass contains no barrier; the loads carry L2 cache hints (keep in pass 1, evict first
-// in pass 3), and the later passes find in L2 what has stayed there.
+// One row at a time per persistent CTA. Warp w owns one contiguous span of the row (1/W_NW of it, rounded up to whole steps);
+// in a step every lane handles eight logits (two 16-byte vectors of f32, one of bf16). Nothing is shared between threads inside
+// a pass, so a pass contains no barrier.
 //
 // This header has no include guard: it is included once per instance, with GS_W_NS naming the
 // instance's namespace inside gs and GS_W_NT its threads per CTA.
@@ -14,6 +11,8 @@
 //   1024: one CTA per SM. A row finishes about a quarter sooner: the instance for batches of at
 //         most one row per SM.
 //
+// Usually a row takes one pass (sample_wide_onepass.cuh). What that does not serve takes two, in this file (vectors loaded
+// straight into registers one or two steps ahead, with L2 cache hints):
 //   sample                     the first step of every warp: an upper estimate (anchor) of the
 //                              row's maximum and its range
 //   pass 1 (HBM)               max, min, NaN; with an active top-p cut also the count histogram
@@ -22,9 +21,9 @@
 //   bracket                    count-based lower/upper mass bounds bracket the cut to a zone of
 //                              buckets (a maximum above the anchor: pass 2 recounts exactly)
 //   pass 3 (L2)                exponentials. Mass of d >= dA (certainly kept) per piece of
-//                              four steps, zone logits (dB <= d < dA) into an exact list
-//   tail                       weighted selection inside the zone, prefix over the pieces,
-//                              rescan of the one piece that holds the drawn token
+//                              eight steps, zone logits (dB <= d < dA) into an exact list
+//   tail                       weighted selection inside the zone, prefix over the pieces
+// and either way the piece that holds the drawn token is looked at again with the exact rule (wide_draw).
 //
 // Row semantics: model/generate.go:147-240 (mode A), model/qwen/generate.go:92-153 (mode B).
 #include "sample_batch.cuh"   // includes row_stream.cuh
@@ -47,7 +46,7 @@ constexpr int W_D1 = 2;                 // steps of register prefetch in pass 1
 constexpr int W_G = 8;                  // steps per piece (power of two)
 constexpr int W_MAX_STEPS = (W_NT >= 512) ? 64 : 128;         // steps per warp and pass; longer rows go to the single-CTA kernel
 constexpr int W_MAX_PPW = W_MAX_STEPS / W_G;
-constexpr int W_MAX_PIECES = W_NW * W_MAX_PPW;                 // 512
+constexpr int W_MAX_PIECES = W_NW * W_MAX_PPW;                 // 128 (1024 threads: 256)
 constexpr int W_EB_REP = 16;            // copies of a table entry in the conflict-free layout
 constexpr int W_EB_REP_ENTRIES = 128;   // entries of that layout: d > -(128-1)/32
 constexpr int W_OFF_HIST = 0;
