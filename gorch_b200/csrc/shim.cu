@@ -43,20 +43,19 @@ constexpr int64_t kSliceCap = 109 * 1024 - gs::REGION_A - gs::REGION_B;
 // the cluster kernel (several CTAs per row), whose latency is lower while the GPU is not full. The rows' kinds are
 // on the device, so one line serves them all. us, batch | cluster, calls back to back on inputs that are not in L2, for rows with
 // top-k, greedy ones, the two mixed with nucleus rows, plain softmax rows, and rows with a top-p cut (f32):
-//   112 x 50,257: 30 | 23, 20 | 12, 40 | 27, 33 | 30, 50 | 67;  256 x 50,257: 33 | 41, 23 | 22, 49 | 48, 49 | 58, 75 | 128
-//   32 x 151,936: 39 | 18, 31 | 9, 57 | 23, 57 | 22, 82 | 49;  64: 41 | 27, 32 | 15, 59 | 35, 63 | 39, 83 | 84;  128: 43 | 43, 35 | 25, 65 | 54,
-//   75 | 72, 101 | 159
-// Rows with a cut change sides long before the others, and the line stays near theirs. Bytes follow that only roughly: from 40 to 60
-// rows of 151,936 f32 the clusters would serve every kind sooner (48: 40 | 21, 32 | 12, 60 | 29, 58 | 36, 82 | 77), and behind the line the
-// other kinds pay (128 x 50,257: 30 | 24, 19 | 12, 41 | 30, 33 | 32, for 51 | 69).
+//   112 x 50,257: 27 | 23, 16 | 11, 33 | 27, 21 | 30, 56 | 72;  256 x 50,257: 29 | 41, 16 | 20, 41 | 46, 25 | 57, 73 | 136
+//   32 x 151,936: 38 | 18, 18 | 8, 43 | 22, 29 | 23, 80 | 50;  64: 38 | 26, 18 | 13, 51 | 33, 29 | 37, 80 | 83;  128: 47 | 42, 26 | 22, 61 | 52,
+//   30 | 69, 97 | 157
+// Rows without top-k change sides long before the others, and the line stays near theirs. Bytes follow that only roughly: from 40 to 60
+// rows of 151,936 f32 the clusters would serve most kinds sooner (48: 38 | 20, 18 | 11, 43 | 28, 29 | 35, 85 | 75), and behind the line
+// top-k, greedy and mixed rows pay (128 x 50,257: 27 | 24, 14 | 11, 36 | 29, for 21 | 32, 57 | 74).
 // Short rows stay with the clusters for longer. Up to four rows per SM of 4,096 logits, two waves of clusters:
-//   592 x 4,096: 25 | 21, 14 | 10, 36 | 28, 27 | 24, 43 | 44 (8,000 logits, 512 rows: 27 | 21, 16 | 11, 39 | 28, 29 | 27, 48 | 53)
-// Beyond four rows per SM, the wide kernel's slots, the batch kernels start a second round of wide rows (592 x 12,000: 29 | 23, 19 | 12,
-// 44 | 32, 34 | 31, 53 | 65; 593: 31 | 29, 20 | 14, 44 | 32, 47 | 38, 81 | 80): up to six rows per SM of 16,384 logits
-//   888 x 4,000: 24 | 31, 14 | 15, 46 | 39, 42 | 35, 70 | 64;  768 x 16,000: 33 | 34, 20 | 18, 107 | 43, 62 | 51, 100 | 111
-//   889 x 16,384: 34 | 41, 22 | 20, 109 | 48, 71 | 58, 128 | 128
-// Mixed batches gain most there; rows with a cut give some of it back from 15,000 f32 or 8,000 bf16 logits on (700 x 16,000: 96 | 99, bf16:
-// 90 | 98), beyond five rows per SM from 10,000 and 5,000 on, where top-k rows by themselves do too.
+//   592 x 4,096: 24 | 20, 13 | 10, 37 | 28, 21 | 23, 45 | 40 (8,000 logits, 512 rows: 27 | 20, 13 | 10, 36 | 27, 20 | 26, 48 | 47)
+// Beyond four rows per SM, the wide kernel's slots, the batch kernels start a second round of wide rows (592 x 12,000: 27 | 22, 15 | 11,
+// 40 | 31, 23 | 30, 55 | 58; 593: 29 | 28, 15 | 13, 40 | 31, 27 | 36, 76 | 66): up to six rows per SM of 16,384 logits
+//   888 x 4,000: 24 | 29, 13 | 14, 44 | 38, 29 | 34, 73 | 60;  768 x 16,000: 29 | 33, 15 | 16, 100 | 41, 34 | 49, 99 | 94
+//   889 x 16,384: 31 | 40, 16 | 18, 102 | 46, 36 | 56, 106 | 105
+// Mixed batches and rows with a cut gain there; top-k rows by themselves and plain softmax rows give some of it back.
 // An argmax is one launch of the narrow kernel and keeps the lower line.
 constexpr int64_t kBatchModeRows = 384;
 constexpr int64_t kBatchModeBytes = 24ll << 20;
