@@ -350,11 +350,26 @@ struct WideShared {
   double pm[W_MAX_PPW];    // kept mass of one warp's pieces
 };
 
+// Why a row takes two passes (reserved[6] of its debug record), and which branches the one-pass form took with it (reserved[7]).
+enum { WHY_TEMPERATURE = 1,   // the quick quotient is not exact for it
+       WHY_SHORT,             // too short for a sample
+       WHY_NOT_FINITE,        // NaN or infinite, where looked at
+       WHY_HEAVY,             // a few tokens hold much of the mass: not for a sample to place the cut
+       WHY_WINDOW,            // the window holds more than the lists do
+       WHY_EMPTY_WINDOW,
+       WHY_NAN,               // a NaN in the row, or an infinite maximum
+       WHY_LIST,              // a list or a lane's buffer did not hold all
+       WHY_ANCHOR,            // the maximum lies too far from the anchor
+       WHY_SUM,
+       WHY_CUT_ABOVE,         // the window failed: the cut lies above it,
+       WHY_CUT_BELOW,         // ... or below, or too close to its end
+       WHY_LONG };            // longer than a warp's part can be
+enum { HOW_CUT = 1, HOW_LOW = 2, HOW_ONE_CLASS = 4, HOW_BY_PIECE = 8, HOW_INDEX = 16 };
 // How a row ends, from either form. `path`: 2 two passes, 3 one.
 struct WideResult {
   float m;                 // largest x / T
   double S, Re;            // all mass, kept mass
-  int path;
+  int path, why, how;
 };
 __device__ __forceinline__ void wide_write(const KernelArgs& A, int64_t row_id, const WideResult& r, int id, uint32_t flags,
                                            double lo, double hi, int kept) {
@@ -365,12 +380,14 @@ __device__ __forceinline__ void wide_write(const KernelArgs& A, int64_t row_id, 
     d.sum_exp = r.S; d.resum = r.Re / r.S; d.edge_lo = lo; d.edge_hi = hi; d.kept = kept;
     d.max_scaled = r.m; d.threshold = __int_as_float(0x7fc00000); d.path = r.path;
     for (int q = 0; q < 8; q++) d.reserved[q] = 0;
+    d.reserved[6] = static_cast<uint32_t>(r.why);
+    d.reserved[7] = static_cast<uint32_t>(r.how);
     A.out_debug[row_id] = d;
   }
 }
 // A row whose sum is no number (S NaN), or whose mode A cut removed every token (generate.go:221-227 divides by zero): every
 // comparison of the walk fails, result n-1 (:239).
-__device__ __noinline__ void wide_write_nothing_kept(const KernelArgs& A, int64_t row_id, float m, double S, int path, uint32_t flags) {
+__device__ __noinline__ void wide_write_nothing_kept(const KernelArgs& A, int64_t row_id, float m, double S, int path, int why, int how, uint32_t flags) {
   const double QNAN = __longlong_as_double(0x7ff8000000000000ll);
   if (A.out_probs) {
     double* pr = A.out_probs + row_id * static_cast<int64_t>(A.V);
@@ -378,7 +395,7 @@ __device__ __noinline__ void wide_write_nothing_kept(const KernelArgs& A, int64_
   }
   WideResult r;
   const bool number = S == S && S > 0.0;
-  r.m = m; r.S = number ? S : QNAN; r.Re = number ? 0.0 : r.S; r.path = path;
+  r.m = m; r.S = number ? S : QNAN; r.Re = number ? 0.0 : r.S; r.path = path; r.why = why; r.how = how;
   if (threadIdx.x == 0) wide_write(A, row_id, r, A.V - 1, flags | FLAG_NONFINITE | FLAG_FALLBACK, 0.0, 0.0, 0);
 }
 // The end of a row: u Re falls into piece `psel` or just behind it (rounding), `before` is the kept mass ahead of it
@@ -606,7 +623,7 @@ __device__ __noinline__ bool wide_big_zone(const WSpan& sp_in, const RowView<T>&
 
 // Two passes over the row: for what one pass does not serve.
 template <typename T>
-__device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t row_id, unsigned char* dyn, WideShared& sh,
+__device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t row_id, const int why, unsigned char* dyn, WideShared& sh,
                          unsigned long long pol_keep, unsigned long long pol_drop) {
   const KernelArgs& A = BA.k;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -705,7 +722,7 @@ __device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t
   // A NaN anywhere, or an infinite maximum, makes the softmax sum NaN upstream
   // (generate.go:173-181): every comparison of the walk fails, result n-1 (:239).
   if (anynan || !(fabsf(m) < INFINITY)) {
-    wide_write_nothing_kept(A, row_id, m, -1.0, 2, flags);
+    wide_write_nothing_kept(A, row_id, m, -1.0, 2, why, 0, flags);
     return;
   }
   dlow = scale_t(xmin, Tm) - m;                  // smallest d of the row (-Inf with a -Inf logit)
@@ -966,9 +983,9 @@ __device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t
   const double pm = (tid < npiece) ? part[tid] : 0.0;
   WideResult r;
   const double pex = bu::scan_excl_d<W_NW>(pm, r.Re, sc, tid);
-  r.m = m; r.S = S; r.path = 2;
+  r.m = m; r.S = S; r.path = 2; r.why = why; r.how = 0;
   if (!(S == S) || !(S > 0.0) || !(r.Re > 0.0)) {
-    wide_write_nothing_kept(A, row_id, m, S, 2, flags);
+    wide_write_nothing_kept(A, row_id, m, S, 2, why, 0, flags);
     return;
   }
   const int psel = bu::min_i<W_NW>((tid < npiece && u * r.Re < pex + pm) ? tid : 0x7fffffff, sc, tid);
@@ -1015,9 +1032,10 @@ __global__ void __launch_bounds__(W_NT, W_CTAS) wide_rows_kernel(const __grid_co
     // The narrow kernel may start: every CTA of this one has a row, or has gone. (Started together, the two kernels'
     // CTAs mix at random, and some SMs end up with more rows of this kind than others.)
     pdl_launch();
-    if (wide_onepass_row<T>(BA, row, dyn, sh) == 0) continue;
+    const int why = wide_onepass_row<T>(BA, row, dyn, sh);
+    if (why == 0) continue;
     __syncthreads();
-    wide_twopass_row<T>(BA, row, dyn, sh, pol_keep, pol_drop);
+    wide_twopass_row<T>(BA, row, why, dyn, sh, pol_keep, pol_drop);
   }
 }
 

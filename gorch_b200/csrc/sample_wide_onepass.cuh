@@ -288,7 +288,7 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
   // ---- the sample: 64-byte pieces spread evenly over the row, none of them at its edges; a thread looks at what it copied itself
   constexpr int J = W1_SAMPLE / (W_NT * VEC), PIECES = W_NT * J / 4;
   const int have = (sh.nvec - 2) / 4;                                     // whole pieces between the row's first and last vector
-  if (have < 2 * PIECES) return 2;                                        // short rows: nothing to gain
+  if (have < 2 * PIECES) return WHY_SHORT;                                      // short rows: nothing to gain
   {
     const uint4* src = sh.vbase + 1 + (tid & 3);
     const uint32_t dst = smem_addr(dyn) + static_cast<uint32_t>(tid) * 16u;
@@ -316,12 +316,12 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
   {
     uint32_t hi = okey(smax), lo = ~okey(smin), nan = (smax != smax) ? 1u : 0u;
     bu::max_u3<W_NW>(hi, lo, nan, sh.sc, tid);                            // (its barriers also publish the cleared bins)
-    if (nan) return 3;
+    if (nan) return WHY_NOT_FINITE;
     smax = okey_to_float(hi);
     smin = okey_to_float(~lo);
   }
   const float as = scale_t(smax, Tm);
-  if (!(fabsf(smax) < 1e30f) || !(fabsf(as) < 1e30f)) return 3;
+  if (!(fabsf(smax) < 1e30f) || !(fabsf(as) < 1e30f)) return WHY_NOT_FINITE;
   // ---- a count histogram of its upper 24 units of x / T (what lies lower has no mass to speak of, and shares the last bucket)
   const float range = fmaxf(fminf(smax - smin, 24.0f * Tm), 1e-6f * fmaxf(fabsf(smax), Tm));
   const float scale = static_cast<float>(W1_SBINS - 1) / range;
@@ -368,7 +368,7 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
     if (w < warp) { im += a; iq += b; in += sh.sc.i0[w]; }
     tot_m += a; tot_q += b;
   }
-  if (!(tot_m * 2.4e-3f >= 1.0f)) return 8;                               // heavy tokens (one above 1/400 of the mass): not for a sample to place
+  if (!(tot_m * 2.4e-3f >= 1.0f)) return WHY_HEAVY;                             // heavy tokens (one above 1/400 of the mass): not for a sample to place
   const float pl = static_cast<float>(plim), lim = pl * tot_m;
   if (im < lim && im + mass >= lim) wq[W_NW] = iq + sq;                   // one thread (none: nothing lies below the cut)
   __syncthreads();
@@ -403,10 +403,10 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
   const float seen = static_cast<float>(max(sh.bc[3] - sh.bc[2], 0));
   const float inside = fminf(2.0f * delta / ex2_approx(-(static_cast<float>(sh.bc[1]) + 0.5f) * wl2), seen + 3.0f * sqrtf(seen)), per_bucket = inside / static_cast<float>(max(sh.bc[1] - sh.bc[0] + 1, 1));
   const bool low = fits(static_cast<float>(W1_SAMPLE - sh.bc[2]) + per_bucket);
-  if (!low && !fits(inside + 2.0f * per_bucket)) return 10;
+  if (!low && !fits(inside + 2.0f * per_bucket)) return WHY_WINDOW;
   const float xA = smax - static_cast<float>(b1) / scale;
   const float xB = (low || b2 == W1_SBINS - 1) ? smax - 40.0f * Tm : smax - static_cast<float>(b2 + 1) / scale;
-  if (!(xA > xB)) return 11;
+  if (!(xA > xB)) return WHY_EMPTY_WINDOW;
   if (tid == 0) {
     sh.as = as; sh.xA = xA; sh.xB = xB; sh.low = low ? 1 : 0;
     sh.eps = W1_EPS_FIXED + W1_EPS_PER_D * fmin(9.7, static_cast<double>(range / Tm) + 2.0);
@@ -430,12 +430,12 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
   // and 1.5*float(p) is never that close to 1
   const bool cut_on = cfg.top_p > 0.0f && cfg.top_p < 1.0f && !(mode == 0 && plim >= 1.0);
   const bool t_is_one = (Tm == 1.0f);
-  if (!t_is_one && !(Tm >= 9.5367431640625e-7f && Tm <= 1048576.0f && (__float_as_uint(Tm) & 0x7fffffu) != 0x7fffffu)) return 1;
+  if (!t_is_one && !(Tm >= 9.5367431640625e-7f && Tm <= 1048576.0f && (__float_as_uint(Tm) & 0x7fffffu) != 0x7fffffu)) return WHY_TEMPERATURE;
   {
     RowView<T> rv;
     rv.init(static_cast<const T*>(A.logits) + row_id * A.row_stride, A.V);
     const int span = (((rv.nvec + W_NW - 1) / W_NW + SV - 1) / SV) * SV;   // a warp's part of the row, in whole steps
-    if (span / SV > W_MAX_STEPS) return 17;
+    if (span / SV > W_MAX_STEPS) return WHY_LONG;
     if (tid == 0) {
       sh.vbase = rv.vbase; sh.V = rv.V; sh.shift = rv.shift; sh.nvec = rv.nvec;
       sh.span = span; sh.ppw = (span / SV + W_G - 1) / W_G;
@@ -453,7 +453,7 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
       uint32_t top = okey(smax), nan = (smax != smax) ? 1u : 0u, none = 0u;
       bu::max_u3<W_NW>(top, nan, none, sc, tid);
       const float as = scale_t(okey_to_float(top), Tm);
-      if (nan || !(fabsf(as) < 1e30f)) return 3;
+      if (nan || !(fabsf(as) < 1e30f)) return WHY_NOT_FINITE;
       if (tid == 0) sh.as = as;
     }
   }
@@ -477,17 +477,17 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
   const int any = __reduce_or_sync(FULL, mine ? sc.i1[lane] : 0);
   double S = warp_sum_d(mine ? sc.d0[lane] : 0.0);
   double Ktot = warp_sum_d(mine ? sh.kw[lane] : 0.0);
-  if ((any & 1) || !(fabsf(m) < INFINITY)) return 12;                      // the two-pass form reports such rows
-  if (any & 2) return 5;
+  if ((any & 1) || !(fabsf(m) < INFINITY)) return WHY_NAN;                    // the two-pass form reports such rows
+  if (any & 2) return WHY_LIST;
   // with a cut the anchor is the sample's maximum: it must be close to the row's for the heavy logits to keep the error budget
-  if (cut_on && !(fabsf(m - sh.as) <= 2.0f)) return 13;
-  if (!(S > 0.0) || !(S < 1e300)) return 14;
+  if (cut_on && !(fabsf(m - sh.as) <= 2.0f)) return WHY_ANCHOR;
+  if (!(S > 0.0) || !(S < 1e300)) return WHY_SUM;
   // everything so far is relative to exp(anchor); from here on to exp(max)
   const double anchor = cut_on ? static_cast<double>(sh.as * P1_L2E) / static_cast<double>(P1_L2E) : static_cast<double>(sh.as);
   const double cf = exp(anchor - static_cast<double>(m));
   S *= cf;
   Ktot *= cf;
-  if (!(S > 0.0)) return 14;
+  if (!(S > 0.0)) return WHY_SUM;
   const int ppw = sh.ppw, span = sh.span;
   const float xA = sh.xA, xB = sh.xB;
   const int* from = reinterpret_cast<const int*>(dyn + W1_OFF_FROM);
@@ -503,6 +503,7 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
   int cut_incl = 0;
   float dstar = INFINITY;
   double estar = 0.0, zw = 0.0;            // mass of one member of the cut's class; lane w: what the window adds to warp w's part
+  bool one_class = false;                  // the candidates are a long run of equal d
   bool by_piece = false, ties_in = false;  // kept members of the class: counted per piece in bins[], or all of them
   if (cut_on) {
     const double lim = plim * S;
@@ -537,11 +538,10 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
       __syncthreads();
     }
     // the cut must lie below the window's upper end by more than the error of the sums
-    if (!(Ktot < lim - (1e-12 + 2.0 * plim * fabs(1.0 - plim) * sh.eps + 1e-9) * S)) return 15;
+    if (!(Ktot < lim - (1e-12 + 2.0 * plim * fabs(1.0 - plim) * sh.eps + 1e-9) * S)) return WHY_CUT_ABOVE;
     double gbase = Ktot;                                     // mass of everything above dhi
     double zsum = 0.0;                                       // this lane's window mass above the crossing's buckets
     int nc = 0;
-    bool one_class = false;
     for (int round = 0;; round++) {                          // uniform
       // The bucket of the crossing, from bounds of the mass through each bucket (a bucket's members lie between its edges): the
       // first that can cross, and the first that must. The slack covers the f32 sums and edges.
@@ -567,7 +567,7 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
         __syncthreads();
       }
       const int b1 = sh.bc[0], b2 = max(sh.bc[1], b1);
-      if (b1 == W1_BINS) return 16;                          // the window ends before the cut
+      if (b1 == W1_BINS) return WHY_CUT_BELOW;                          // the window ends before the cut
       // what lies above the crossing's buckets is kept; what lies in them is looked at one by one
       double sure = 0.0;
       float cmax = -INFINITY, cmin = 1.0f;
@@ -594,7 +594,7 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
       bu::max_u3<W_NW>(kmax, inv, none, sc, tid);
       dhi = -__uint_as_float(~inv); dlo = -__uint_as_float(kmax);
       if (dhi == dlo) { one_class = true; break; }           // a long run of equal d
-      if (round == 5) return 16;
+      if (round == 5) return WHY_CUT_BELOW;
       scale = fminf(static_cast<float>(W1_BINS) / (dhi - dlo), 1e30f);
       bins[tid] = 0u;
       if (tid == 0) { sh.bc[0] = W1_BINS; sh.bc[1] = W1_BINS - 1; sh.cnt = 0; }
@@ -624,17 +624,17 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
       }
       const bool cr = lane < nc && crossed(g + eq * e_l);
       const uint32_t best = __reduce_min_sync(FULL, cr ? dkey_of(d_l) : 0xffffffffu);
-      if (best == 0xffffffffu) return 16;                    // rounding: nothing in the window crosses
+      if (best == 0xffffffffu) return WHY_CUT_BELOW;                    // rounding: nothing in the window crosses
       const int who = __ffs(__ballot_sync(FULL, cr && dkey_of(d_l) == best)) - 1;
       dstar = -__uint_as_float(best);
       gb = __shfl_sync(FULL, g, who);
       neq = __shfl_sync(FULL, eq, who);
     }
     // Several logits can share one d: a class that also has members outside the window is decided on the whole row
-    if (dstar == dA || dstar == scale_t(nextafterf(xB, -INFINITY), Tm) - m) return 16;
+    if (dstar == dA || dstar == scale_t(nextafterf(xB, -INFINITY), Tm) - m) return WHY_CUT_BELOW;
     // the first member whose mass crosses (mode B keeps through it, mode A everything before it)
     estar = exp_safe(dstar, s_tab);
-    if (!crossed(gb + neq * estar)) return 16;
+    if (!crossed(gb + neq * estar)) return WHY_CUT_BELOW;
     int r = 1;
     if (neq > 1) {
       r = static_cast<int>(fmin(fmax(ceil((lim - gb) / estar), 1.0), static_cast<double>(neq)));
@@ -683,7 +683,7 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
       if (!ties_in) {
         // the member's index: one piece of the row again
         const int pi = sh.bc[0], rank = sh.bc[1];
-        if (pi < 0) return 16;
+        if (pi < 0) return WHY_CUT_BELOW;
         constexpr int NV = (PV + W_NT - 1) / W_NT;
         const int w = pi / ppw, vb = w * span + (pi - w * ppw) * PV, v = vb + tid * NV;
         const int vend = min(min(vb + PV, w * span + span), rv.nvec);
@@ -713,7 +713,7 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
           sh.bc[2] = i0 + __ffs(mask) - 1;
         }
         __syncthreads();
-        if (sh.bc[2] < 0) return 16;                         // (a list that disagrees with the row)
+        if (sh.bc[2] < 0) return WHY_CUT_BELOW;                         // (a list that disagrees with the row)
         cut_key = zone_key(dstar, sh.bc[2], mode);
         cut_incl = 1;
       }
@@ -751,12 +751,13 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
     }
     return exp_safe(d, s_tab);
   };
+  const int how = (cut_on ? HOW_CUT : 0) | (low ? HOW_LOW : 0) | (one_class ? HOW_ONE_CLASS : 0) | (by_piece ? HOW_BY_PIECE : 0) | (by_piece && !ties_in ? HOW_INDEX : 0);
   if (!(Re > 0.0)) {                                         // mode A removed every token
-    wide_write_nothing_kept(A, row_id, m, S, 3, flags);
+    wide_write_nothing_kept(A, row_id, m, S, 3, 0, how, flags);
     return 0;
   }
   WideResult res;
-  res.m = m; res.S = S; res.Re = Re; res.path = 3;
+  res.m = m; res.S = S; res.Re = Re; res.path = 3; res.why = 0; res.how = how;
   int psel = 0x7fffffff;
   double before = Re;
   const unsigned hit = __ballot_sync(FULL, mine && tgt < wi);

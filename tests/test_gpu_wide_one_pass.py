@@ -59,6 +59,28 @@ def test_one_pass_rows(wide, oracle, V, pad, bf16):
         assert paths[0] == 3 and paths[1] == 3                        # flat rows under a deep nucleus
 
 
+# reserved[6] of a wide row's debug record: why it took two passes
+WHY_TEMPERATURE, WHY_SHORT, WHY_NOT_FINITE, WHY_HEAVY, WHY_WINDOW, WHY_EMPTY_WINDOW, WHY_NAN, WHY_LIST, WHY_ANCHOR = range(1, 10)
+
+
+def test_reasons_for_two_passes(wide, oracle):
+    """The record says why a row was not served by one pass."""
+    rng = np.random.Generator(np.random.Philox(key=77))
+    V = 70000
+    z = lambda s: (rng.standard_normal(V) * s).astype(np.float32)
+    rows, cfgs, why = [], [], []
+    for x, T, p, w in ((z(0.25), 1.0, 0.995, 0), (z(2.0), 1.0, 0.0, 0), (z(0.25), 1.0, 0.5, WHY_WINDOW), (z(2.5), 1.0, 0.9, WHY_HEAVY),
+                       (z(0.25), np.nextafter(np.float32(2.0), np.float32(0.0)), 0.0, WHY_TEMPERATURE)):
+        rows.append(x); cfgs.append((T, 0, p, MODE_B)); why.append(w)
+    x = z(2.0); x[V // 2] = np.nan
+    rows.append(x); cfgs.append((1.0, 0, 0.0, MODE_B)); why.append(WHY_NAN)
+    x = z(0.25); x[:] = -np.inf
+    rows.append(x); cfgs.append((1.0, 0, 0.9, MODE_B)); why.append(WHY_NOT_FINITE)
+    gpu, _, _ = run_both(wide, oracle, np.stack(rows), np.array(cfgs, dtype=CFG_DTYPE), rng.random(len(rows)))
+    assert list(gpu["debug"]["reserved"][:, 6]) == why
+    assert list(gpu["debug"]["path"]) == [2 if w else 3 for w in why]
+
+
 def test_uniforms_at_the_ends(wide, oracle):
     """u = 0 takes the first kept logit, the largest u below 1 the last one."""
     rng = np.random.Generator(np.random.Philox(key=31))
