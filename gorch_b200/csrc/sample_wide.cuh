@@ -61,6 +61,7 @@ constexpr int W1_BINS = W_NT;
 constexpr int W1_OFF_LIST = 0;
 constexpr int W1_OFF_BUF = W1_OFF_LIST + W_NW * W1_WCAP * 4;
 constexpr int W1_OFF_RING = W1_OFF_BUF + W1_SLOTS * W_NT * 4;
+constexpr int W1_OFF_TAB = W1_OFF_LIST;                        // without a cut there are no lists: the exponential's table
 constexpr int W1_OFF_MASS = W1_OFF_BUF;                        // after the pass: the listed logits' masses
 constexpr int W1_OFF_BINS = W1_OFF_RING + W1_RING_BYTES;
 constexpr int W1_OFF_FROM = W1_OFF_BINS + W1_BINS * 4;
@@ -342,7 +343,9 @@ struct WideShared {
   const uint4* vbase;
   int V, shift, nvec;
   int span, ppw;           // vectors of a warp's part of the row, pieces in it
-  float as, Tm, xA, xB;    // anchor in units of x / T; above the window: x >= xA; the window: xB <= x < xA
+  float as, base;          // what the sums are relative to, in units of x / T: the anchor, or, for exact sums, the base
+  float Tm, xA, xB;        // above the window: x >= xA; the window: xB <= x < xA
+  int far;                 // a logit lies too far above the anchor
   int low;                 // the window reaches down to where no mass is
   double eps;              // relative error bound of the sums
   double kw[W_NW];         // the mass above the window in each warp's part of the row (all its mass where the window is low),
@@ -364,7 +367,7 @@ enum { WHY_TEMPERATURE = 1,   // the quick quotient is not exact for it
        WHY_CUT_ABOVE,         // the window failed: the cut lies above it,
        WHY_CUT_BELOW,         // ... or below, or too close to its end
        WHY_LONG };            // longer than a warp's part can be
-enum { HOW_CUT = 1, HOW_LOW = 2, HOW_ONE_CLASS = 4, HOW_BY_PIECE = 8, HOW_INDEX = 16 };
+enum { HOW_CUT = 1, HOW_LOW = 2, HOW_ONE_CLASS = 4, HOW_BY_PIECE = 8, HOW_INDEX = 16, HOW_EXACT = 32 };
 // How a row ends, from either form. `path`: 2 two passes, 3 one.
 struct WideResult {
   float m;                 // largest x / T

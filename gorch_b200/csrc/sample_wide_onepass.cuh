@@ -7,8 +7,11 @@
 // logits lie below the window, they are listed too and the rest of S is what is kept (P1_LOW: a quarter fewer instructions
 // in a loop that is bound by their issue where an SM has four rows). The sample only chooses the window: whether the cut really
 // lies inside is checked on the sums of the whole row, and a row whose window failed (or that the sample cannot place:
-// a few heavy tokens, NaN, a wide window) takes two passes (sample_wide.cuh). Rows without a cut (P1_ALL) need neither sample
-// nor window.
+// a few heavy tokens, NaN, a wide window) takes two passes (sample_wide.cuh). Rows without a cut need neither sample
+// nor window. Long ones whose maximum lies where a first look expects it are flat, many tokens share the mass, and the fast
+// exponential serves them (P1_ALL); short ones, and those in which a logit turns up more than 2 above that, get exact sums
+// (P1_EXACT), which cost twice the instructions. (us, flat rows, and rows with 16 peaks of 8 on a sigma of 2, the latter by exact sums and as two passes
+// over the row: 512 x 151,936 f32 68, 91, 210, bf16 52, 88, 161; 256 x 50,257 f32 23, 29, 51.)
 //
 // The lists. A window of 1 to 2 % of the logits puts one into a tenth of the lane-steps, so nearly every warp-step has a lane
 // that must list something, and slots from a shared counter cost every warp some ninety issue slots a step. So a lane has a
@@ -28,13 +31,15 @@
 // that carries mass). (C is the anchor times log2 e, rounded: the anchor that this stands for is what the sums are taken
 // back from.) The anchor must lie within 2 of the maximum. Without a cut the rounding of t is made up for (p1_exp2), which leaves
 // 6e-8 per unit: the anchor may lie W1_RISE below a logit for the same error.
-constexpr int P1_ALL = 0, P1_LOW = 1, P1_MID = 2;
+constexpr int P1_ALL = 0, P1_EXACT = 1, P1_LOW = 2, P1_MID = 3;
 constexpr int W1_SAMPLE = (W_NT >= 512) ? 16384 : 8192;        // logits of the sample
 constexpr int W1_SBINS = 1024;           // its histogram's buckets
 constexpr double W1_EPS_FIXED = 4.5e-7;
 constexpr double W1_EPS_PER_D = 2.0e-7;
-constexpr float W1_RISE = 6.0f;
-static_assert(W1_SBINS % W_NT == 0 && W1_BINS == W_NT && W1_SAMPLE * 4 + W1_SBINS * 4 <= W1_OFF_BINS, "a thread's share of the buckets; the sample and its buckets lie where lists and ring will be");
+constexpr int W1X_ENTRIES = 256, W1X_COPIES = 16;   // table of the exact exponential: 2^(j/256), a copy per pair of banks
+constexpr float W1X_FAR = 88.0f;         // the sums' base may lie this far below the maximum
+constexpr double W1X_STRETCH = 1.0 + 2.376e-12;   // what it takes the exponential of is stretched by this
+static_assert(W1_SBINS % W_NT == 0 && W1_BINS == W_NT && W1_SAMPLE * 4 + W1_SBINS * 4 <= W1_OFF_BINS && W1X_ENTRIES * W1X_COPIES * 8 <= W1_OFF_RING, "a thread's share of the buckets; the sample and its buckets lie where lists and ring will be, the table where lists and buffers are not");
 static_assert(W_MAX_PPW <= 32 && W_NW <= 32 && W_MAX_PIECES <= W1_BINS && W1_OFF_MASS + W_NW * W1_WCAP * 8 <= W1_OFF_BINS, "memory of the selection");
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
@@ -55,37 +60,70 @@ __device__ __forceinline__ f32x2_t div2_fast(f32x2_t X, float T, float y) {
   const f32x2_t R = fma2(Q0, pk2(-T, -T), X);
   return fma2(R, Y, Q0);
 }
+// Rows without a cut: quick sums first for rows of at least so many steps per warp whose first look spans no more than this, in units of x / T. Short
+// rows gain little (592 x 12,000 f32: 27 us exact, 32 in two passes). A wide span goes with tokens far above the rest, which a first look
+// does not see: the quick sums would be for nothing in most such rows.
+constexpr int W1_QUICK_STEPS = 8;
+constexpr float W1_QUICK_RANGE = 6.0f;
 constexpr float P1_L2E = 1.4426950408889634f;
-// exp of two, the rounding of the product with log2 e recovered exactly and applied to the result (arguments at or above -1e30).
-__device__ __forceinline__ f32x2_t p1_exp2(f32x2_t D) {
-  constexpr float L2E_LO = 1.925963033500011e-8f, LN2 = 0.6931471805599453f;
-  float t0, t1;
-  const f32x2_t NT2 = mul2(D, pk2(-P1_L2E, -P1_L2E));
-  f32x2_t R = fma2(D, pk2(P1_L2E, P1_L2E), NT2);
-  R = fma2(D, pk2(L2E_LO, L2E_LO), R);
-  upk2(NT2, t0, t1);
-  const f32x2_t P = pk2(ex2_approx(-t0), ex2_approx(-t1));
-  return fma2(P, mul2(R, pk2(LN2, LN2)), P);
-}
 
 struct P1Consts {
-  float as, C, Tm, yT;     // anchor in units of x / T, and times log2 e; temperature and its rounded reciprocal
+  float C, Tm, yT;         // the anchor times log2 e (without a cut: what the sums are relative to, in units of x / T); temperature and its rounded reciprocal
+  float xlow;              // P1_EXACT: logits below have no mass
+  uint32_t tab;            // P1_EXACT: shared-memory address of this lane's copy of the table
   float xA;                // above the window: x >= xA
   float xmid, xhalf;       // |x - xmid| <= xhalf is a superset of the window
   uint32_t buf, buf_end;   // shared-memory addresses of this lane's buffer: its first slot, and the one that leaves room for four logits
 };
 struct P1Acc {
-  double tot;              // all mass of the running piece (P1_MID: all mass so far)
+  double tot, tot2;        // all mass of the running piece (P1_MID: all mass so far); P1_EXACT: in two parts
   double kep;              // P1_MID: mass above the window of the running piece
   double stot;             // all mass of the pieces done
   float vmax;              // NaN-propagating running maximum
   uint32_t at;             // the lane's next slot
 };
 
-// Eight logits of a lane; masked logits are -Inf and add 0. Three f32 additions per sum, then f64. Logits near the window go
-// to the lane's buffer.
+// Eight logits of a lane of a row without a cut: exp(x/T - C) as f64. Table and short polynomial (Tang's scheme): with n the integer nearest to
+// s 256/ln2, s = n ln2/256 + r, exp = 2^(n/256) (1 + r + r^2/2 + r^3/6). ln2/256 is H + L with H of nine bits, so n H is exact up to
+// |s| = W1X_FAR and r is rounded once; 1 + ... is applied in f64. The error is at most 1.2e-10 (two roundings at |r| <= 2^-9.5), besides
+// that L's 24 bits make it exp(s W1X_STRETCH): the way back from C to the maximum is stretched too, and what is left is 2.4e-12 per
+// unit below the maximum. s = x/T - C is exact for what carries mass: C is 0 while the row's first look stays within 32 of 0, else
+// the next multiple of 32 on the side of 0. The table's exponent fields are reduced by j << 12, so that adding n << 12 leaves n div 256 there.
+// (Bound by the number of instructions: the conversion of r (1 + ...) to f64 done by shifts is slower, 92 against 87 us for 512 x 151,936 bf16.)
+template <bool TONE>
+__device__ __forceinline__ void p1_body_exact(const float* x, const P1Consts& k, P1Acc& a) {
+  a.vmax = max3nan(a.vmax, x[0], x[1]); a.vmax = max3nan(a.vmax, x[2], x[3]);
+  a.vmax = max3nan(a.vmax, x[4], x[5]); a.vmax = max3nan(a.vmax, x[6], x[7]);
+  constexpr float INV = 369.32993f, MAGIC = 12582912.0f, H = 355.0f / 131072.0f, L = -0x1.bd0106p-21f;
+#pragma unroll
+  for (int c = 0; c < 4; c++) {
+    f32x2_t S_ = pk2(fmaxf(x[2 * c], k.xlow), fmaxf(x[2 * c + 1], k.xlow));
+    if (!TONE) S_ = div2_fast(S_, k.Tm, k.yT);
+    S_ = add2(S_, pk2(-k.C, -k.C));
+    const f32x2_t F = fma2(S_, pk2(INV, INV), pk2(MAGIC, MAGIC));
+    const f32x2_t N = add2(F, pk2(-MAGIC, -MAGIC));
+    f32x2_t R = fma2(N, pk2(-H, -H), S_);
+    R = fma2(N, pk2(-L, -L), R);
+    const f32x2_t W = fma2(fma2(R, pk2(1.0f / 6.0f, 1.0f / 6.0f), pk2(0.5f, 0.5f)), mul2(R, R), R);
+    float f[2], w[2];
+    upk2(F, f[0], f[1]);
+    upk2(W, w[0], w[1]);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const uint32_t n = __float_as_uint(f[h]);
+      const double t = lds_f64(k.tab + (n & (W1X_ENTRIES - 1)) * (W1X_COPIES * 8));
+      const double E = __hiloint2double(__double2hiint(t) + static_cast<int>(n << 12), __double2loint(t));
+      double& sum = h ? a.tot2 : a.tot;
+      sum += fma(E, static_cast<double>(w[h]), E);
+    }
+  }
+}
+// Eight logits of a lane by ex2.approx; masked logits are -Inf and add 0. Three f32 additions per sum, then f64. With a cut, logits near
+// the window go to the lane's buffer.
 template <int VEC, bool TONE, int MODE>
 __device__ __forceinline__ void p1_body(const float* x, const P1Consts& k, P1Acc& a) {
+  constexpr bool CUT = MODE == P1_LOW || MODE == P1_MID;
+  if (MODE == P1_EXACT) { p1_body_exact<TONE>(x, k, a); return; }
   a.vmax = max3nan(a.vmax, x[0], x[1]); a.vmax = max3nan(a.vmax, x[2], x[3]);
   a.vmax = max3nan(a.vmax, x[4], x[5]); a.vmax = max3nan(a.vmax, x[6], x[7]);
   f32x2_t E[4], KK[2];
@@ -93,26 +131,23 @@ __device__ __forceinline__ void p1_body(const float* x, const P1Consts& k, P1Acc
   for (int c = 0; c < 4; c++) {
     const f32x2_t X = pk2(x[2 * c], x[2 * c + 1]);
     f32x2_t S_ = X;
-    if (!TONE || MODE == P1_ALL) S_ = pk2(fmaxf(x[2 * c], -1e30f), fmaxf(x[2 * c + 1], -1e30f));
-    if (!TONE) S_ = div2_fast(S_, k.Tm, k.yT);
-    if (MODE == P1_ALL) {
-      E[c] = p1_exp2(add2(S_, pk2(-k.as, -k.as)));
-    } else {
-      float t0, t1;
-      upk2(fma2(S_, pk2(P1_L2E, P1_L2E), pk2(-k.C, -k.C)), t0, t1);
-      E[c] = pk2(ex2_approx(t0), ex2_approx(t1));
-      if (MODE == P1_MID) {
-        const f32x2_t M = pk2(set_ge(x[2 * c], k.xA), set_ge(x[2 * c + 1], k.xA));
-        if ((c & 1) == 0) KK[c >> 1] = mul2(E[c], M); else KK[c >> 1] = fma2(E[c], M, KK[c >> 1]);
-      }
-      float z0, z1;
-      upk2(add2(X, pk2(-k.xmid, -k.xmid)), z0, z1);
-#pragma unroll
-      for (int h = 0; h < 2; h++)
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.le.f32 p, %2, %3;\n\t@p st.shared.f32 [%0], %1;\n\t@p add.u32 %0, %0, %4;\n\t}"
-                     : "+r"(a.at) : "f"(x[2 * c + h]), "f"(fabsf(h ? z1 : z0)), "f"(k.xhalf), "n"(W_NT * 4));
-      if (c & 1) a.at = min(a.at, k.buf_end);                   // a full buffer stays full: the row takes two passes
+    if (!TONE) S_ = div2_fast(pk2(fmaxf(x[2 * c], -1e30f), fmaxf(x[2 * c + 1], -1e30f)), k.Tm, k.yT);
+    float t0, t1;
+    if (CUT) upk2(fma2(S_, pk2(P1_L2E, P1_L2E), pk2(-k.C, -k.C)), t0, t1);
+    else upk2(mul2(add2(S_, pk2(-k.C, -k.C)), pk2(P1_L2E, P1_L2E)), t0, t1);
+    E[c] = pk2(ex2_approx(t0), ex2_approx(t1));
+    if (MODE == P1_MID) {
+      const f32x2_t M = pk2(set_ge(x[2 * c], k.xA), set_ge(x[2 * c + 1], k.xA));
+      if ((c & 1) == 0) KK[c >> 1] = mul2(E[c], M); else KK[c >> 1] = fma2(E[c], M, KK[c >> 1]);
     }
+    if (!CUT) continue;
+    float z0, z1;
+    upk2(add2(X, pk2(-k.xmid, -k.xmid)), z0, z1);
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      asm volatile("{\n\t.reg .pred p;\n\tsetp.le.f32 p, %2, %3;\n\t@p st.shared.f32 [%0], %1;\n\t@p add.u32 %0, %0, %4;\n\t}"
+                   : "+r"(a.at) : "f"(x[2 * c + h]), "f"(fabsf(h ? z1 : z0)), "f"(k.xhalf), "n"(W_NT * 4));
+    if (c & 1) a.at = min(a.at, k.buf_end);                     // a full buffer stays full: the row takes two passes
   }
   { float p, q; upk2(add2(add2(E[0], E[1]), add2(E[2], E[3])), p, q); a.tot += static_cast<double>(p + q); }
   if (MODE == P1_MID) {
@@ -130,31 +165,7 @@ __device__ __forceinline__ void p1_mask(float* x, int gv, int nvec, int shift, i
     if (!(g < nvec && i >= 0 && i < V)) x[c] = -INFINITY;
   }
 }
-// A piece of a row without a cut held a logit far above the warp's anchor: the anchor moves up to the warp's maximum, and the
-// piece (the n steps from that of gv) is summed again. A row of a few heavy tokens comes here a few times. Returns the lane's sum.
-template <typename T, bool TONE>
-__device__ __noinline__ double p1_raise_anchor(const WideShared& sh, int gv, int n, float vmax, float& as, float& xlim) {
-  constexpr int VEC = Elem<T>::VEC, EPI = 8 / VEC, SV = 32 * EPI;
-  const float wmax = okey_to_float(__reduce_max_sync(FULL, okey(vmax)));
-  const float up = scale_t(wmax, sh.Tm);
-  if (!(fabsf(up) < 1e30f)) { xlim = INFINITY; return 0.0; }   // the row's maximum is no number: it ends in the two-pass form
-  as = up;
-  xlim = (up + W1_RISE) * sh.Tm;
-  P1Consts k;
-  k.as = up; k.Tm = sh.Tm; k.yT = TONE ? 1.0f : __frcp_rn(sh.Tm);
-  P1Acc a;
-  a.tot = 0.0; a.vmax = -INFINITY;
-  for (int s = 0; s < n; s++, gv += SV) {
-    float x[8];
-#pragma unroll
-    for (int h = 0; h < EPI; h++) Elem<T>::unpack(__ldg(sh.vbase + min(gv + 32 * h, sh.nvec - 1)), x + h * VEC);
-    p1_mask<VEC>(x, gv, sh.nvec, sh.shift, sh.V);
-    p1_body<VEC, TONE, P1_ALL>(x, k, a);
-  }
-  return a.tot;
-}
-
-// The pass. Leaves in shared memory: part[warp * ppw + piece], the mass of each piece (P1_MID: of its logits above the window), relative to the anchor; the warps' lists, and in from[warp][piece] where a piece begins in its warp's;
+// The pass. Leaves in shared memory: part[warp * ppw + piece], the mass of each piece (P1_MID: of its logits above the window), relative to the anchor or base; the warps' lists, and in from[warp][piece] where a piece begins in its warp's;
 // per warp kw (sum of its pieces), sc.d0 (all mass), sc.i0 (order key of the maximum), sc.i1 (1: a NaN, 2: a list that did
 // not hold all).
 template <typename T, bool TONE, int MODE>
@@ -169,7 +180,10 @@ __device__ __noinline__ void wide_onepass_stream(unsigned char* dyn, WideShared&
   // steps [clean_lo, clean_hi) hold no logit outside the row: all their vectors exist, none is the row's first or last
   const int clean_lo = (first == 0) ? 1 : 0, clean_hi = min(nst, (nvec - 1 - first) / SV);
   P1Consts k;
-  k.as = sh.as; k.C = sh.as * P1_L2E; k.Tm = sh.Tm; k.yT = TONE ? 1.0f : __frcp_rn(sh.Tm);
+  constexpr bool CUT = MODE == P1_LOW || MODE == P1_MID;
+  k.C = CUT ? sh.as * P1_L2E : (MODE == P1_EXACT ? sh.base : sh.as); k.Tm = sh.Tm; k.yT = TONE ? 1.0f : __frcp_rn(sh.Tm);
+  k.xlow = (sh.base - 700.0f) * sh.Tm;
+  k.tab = smem_addr(dyn + W1_OFF_TAB) + 8u * (lane & (W1X_COPIES - 1));
   k.xA = sh.xA;
   k.xmid = 0.5f * sh.xA + 0.5f * sh.xB;
   k.xhalf = (0.5f * sh.xA - 0.5f * sh.xB) * 1.000001f + 1e-30f + 2.4e-7f * fabsf(k.xmid);
@@ -182,26 +196,16 @@ __device__ __noinline__ void wide_onepass_stream(unsigned char* dyn, WideShared&
   bool full = false;
   if (lane == 0) from[0] = 0;
   P1Acc a;
-  a.tot = 0.0; a.kep = 0.0; a.stot = 0.0; a.vmax = -INFINITY; a.at = k.buf;
-  // without a cut: sums are relative to the warp's anchor, and f brings them to the row's
-  float xlim = (k.as + W1_RISE) * k.Tm;
-  double f = 1.0;
+  a.tot = 0.0; a.tot2 = 0.0; a.kep = 0.0; a.stot = 0.0; a.vmax = -INFINITY; a.at = k.buf;
   // The ring: a thread copies the vectors it will take itself, and waits for its own copies only. A vector past the row's
   // end is replaced by the row's last one (masked below).
   const uint4* src = sh.vbase + first + lane;
   const int omax = nvec - 1 - first - lane;                    // of the offsets from src (negative: none of the warp's steps runs then)
   const uint32_t ring = smem_addr(dyn + W1_OFF_RING) + static_cast<uint32_t>(tid) * 16u;
   const uint4* ring_at = reinterpret_cast<const uint4*>(dyn + W1_OFF_RING) + tid;
+  volatile int* far = &sh.far;
   auto piece_end = [&](int st) {
-    if (MODE == P1_ALL) {
-      if (__any_sync(FULL, a.vmax > xlim)) {
-        float as = k.as, xl = xlim;
-        const int n = (st & (W_G - 1)) + 1;
-        a.tot = p1_raise_anchor<T, TONE>(sh, first + (st + 1 - n) * SV + lane, n, a.vmax, as, xl);
-        f = exp(static_cast<double>(as) - static_cast<double>(sh.as));
-        k.as = as; xlim = xl;
-      }
-    } else {
+    if (CUT) {
       full |= a.at >= k.buf_end;
       const int n = static_cast<int>((a.at - k.buf) / (W_NT * 4u));
       for (int r = 0;; r++) {
@@ -220,8 +224,9 @@ __device__ __noinline__ void wide_onepass_stream(unsigned char* dyn, WideShared&
     }
     double t = a.kep;
     if (MODE == P1_MID) a.kep = 0.0;
-    else { t = (MODE == P1_ALL) ? a.tot * f : a.tot; a.stot += t; a.tot = 0.0; }
-    const double kw = warp_sum_d(t);
+    else { t = (MODE == P1_EXACT) ? a.tot + a.tot2 : a.tot; a.stot += t; a.tot = a.tot2 = 0.0; }
+    double kw = warp_sum_d(t);
+    if (MODE == P1_EXACT && kw < 1e-270) kw = 0.0;               // -Inf throughout (each counts as exp(-700))
     if (lane == 0) part_w[st / W_G] = kw;
   };
   auto step = [&](int st, int slot, auto&& refill, bool clean) {
@@ -261,6 +266,12 @@ __device__ __noinline__ void wide_onepass_stream(unsigned char* dyn, WideShared&
         step(st, j % NQ, [&]() { put_any(j % NQ, st + NQ); }, st >= clean_lo && st < clean_hi);
     }
     piece_end(st - 1);
+    if (MODE == P1_ALL) {                                      // a logit far above the anchor: the row's sums will be exact ones
+      if (__any_sync(FULL, a.vmax > k.xA || *far != 0)) {
+        if (lane == 0) *far = 1;
+        break;
+      }
+    }
   }
   cp_wait<0>();
   if (lane == 0) {
@@ -273,7 +284,7 @@ __device__ __noinline__ void wide_onepass_stream(unsigned char* dyn, WideShared&
   const double kw = warp_sum_d((lane < ppw) ? part_w[lane] : 0.0);
   const double S = warp_sum_d(MODE == P1_MID ? a.tot : a.stot);
   const uint32_t wmax = __reduce_max_sync(FULL, okey(a.vmax));
-  const int odd = (__any_sync(FULL, a.vmax != a.vmax) ? 1 : 0) | ((MODE != P1_ALL && (listed > W1_WCAP || __any_sync(FULL, full))) ? 2 : 0);
+  const int odd = (__any_sync(FULL, a.vmax != a.vmax) ? 1 : 0) | ((CUT && (listed > W1_WCAP || __any_sync(FULL, full))) ? 2 : 0);
   if (lane == 0) { sh.kw[warp] = kw; sh.sc.d0[warp] = S; sh.sc.i0[warp] = static_cast<int>(wmax); sh.sc.i1[warp] = odd; }
   __syncthreads();
 }
@@ -430,6 +441,7 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
   // and 1.5*float(p) is never that close to 1
   const bool cut_on = cfg.top_p > 0.0f && cfg.top_p < 1.0f && !(mode == 0 && plim >= 1.0);
   const bool t_is_one = (Tm == 1.0f);
+  bool quick = false;                      // without a cut: the sums by ex2.approx, if the maximum turns out where it is expected
   if (!t_is_one && !(Tm >= 9.5367431640625e-7f && Tm <= 1048576.0f && (__float_as_uint(Tm) & 0x7fffffu) != 0x7fffffu)) return WHY_TEMPERATURE;
   {
     RowView<T> rv;
@@ -439,22 +451,24 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
     if (tid == 0) {
       sh.vbase = rv.vbase; sh.V = rv.V; sh.shift = rv.shift; sh.nvec = rv.nvec;
       sh.span = span; sh.ppw = (span / SV + W_G - 1) / W_G;
-      sh.Tm = Tm; sh.xA = 0.0f; sh.xB = 0.0f;
-      sh.eps = W1_EPS_FIXED + W1_EPS_PER_D * 9.7;
+      sh.Tm = Tm; sh.xA = 0.0f; sh.xB = 0.0f; sh.base = 0.0f;
     }
     if (!cut_on) {
-      // ---- the anchor: the largest logit of the warps' first steps
-      float smax = -INFINITY;
+      // ---- a first look: the warps' first steps. The row's maximum is expected an eighth of their range above theirs.
+      float smax = -INFINITY, smin = INFINITY;
 #pragma unroll
       for (int h = 0; h < 8 / VEC; h++) {
         const int g = warp * span + 32 * h + lane;
-        if (g < rv.nvec) rv.visit(g, [&](float xv, int) { smax = maxnan(smax, xv); });
+        if (g < rv.nvec) rv.visit(g, [&](float xv, int) { smax = maxnan(smax, xv); smin = fminf(smin, xv); });
       }
-      uint32_t top = okey(smax), nan = (smax != smax) ? 1u : 0u, none = 0u;
-      bu::max_u3<W_NW>(top, nan, none, sc, tid);
-      const float as = scale_t(okey_to_float(top), Tm);
-      if (nan || !(fabsf(as) < 1e30f)) return WHY_NOT_FINITE;
-      if (tid == 0) sh.as = as;
+      uint32_t top = okey(smax), nan = (smax != smax) ? 1u : 0u, inv = ~okey(smin);
+      bu::max_u3<W_NW>(top, nan, inv, sc, tid);
+      if (nan) return WHY_NOT_FINITE;
+      smax = okey_to_float(top);
+      smin = okey_to_float(~inv);
+      const float as = scale_t(smax + 0.125f * (smax - smin), Tm);
+      quick = rv.nvec >= W1_QUICK_STEPS * W_NW * SV && (smax - smin) / Tm <= W1_QUICK_RANGE && fabsf(as) < 1e30f;
+      if (tid == 0) { sh.as = quick ? as : scale_t(smax, Tm); sh.xA = (as + 2.0f) * Tm; sh.far = 0; }
     }
   }
   __syncthreads();
@@ -464,15 +478,34 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
   }
   __syncthreads();
   const bool low = cut_on && sh.low;
+  const bool mine = lane < W_NW;
+  bool exact = false;
   if (low) {
     if (t_is_one) wide_onepass_stream<T, true, P1_LOW>(dyn, sh); else wide_onepass_stream<T, false, P1_LOW>(dyn, sh);
   } else if (cut_on) {
     if (t_is_one) wide_onepass_stream<T, true, P1_MID>(dyn, sh); else wide_onepass_stream<T, false, P1_MID>(dyn, sh);
   } else {
-    if (t_is_one) wide_onepass_stream<T, true, P1_ALL>(dyn, sh); else wide_onepass_stream<T, false, P1_ALL>(dyn, sh);
+    float b = sh.as;
+    if (quick) {
+      if (t_is_one) wide_onepass_stream<T, true, P1_ALL>(dyn, sh); else wide_onepass_stream<T, false, P1_ALL>(dyn, sh);
+      if (__reduce_or_sync(FULL, mine ? sc.i1[lane] : 0)) return WHY_NAN;
+      b = scale_t(okey_to_float(__reduce_max_sync(FULL, mine ? static_cast<uint32_t>(sc.i0[lane]) : 0u)), Tm);   // the largest so far
+    }
+    exact = !quick || sh.far || !(fabsf(b - sh.as) <= 2.0f);
+    if (exact) {
+      if (!(fabsf(b) <= 1e6f)) return WHY_ANCHOR;              // (further out base - 700 is no f32)
+      if (tid == 0) sh.base = 32.0f * truncf(b * 0.03125f);
+      double* tab = reinterpret_cast<double*>(dyn + W1_OFF_TAB);
+      for (int j = tid; j < W1X_ENTRIES * W1X_COPIES; j += W_NT) {
+        const int e = j / W1X_COPIES;
+        const double t = s_tab[e];
+        tab[j] = __hiloint2double(__double2hiint(t) - (e << 12), __double2loint(t));
+      }
+      __syncthreads();
+      if (t_is_one) wide_onepass_stream<T, true, P1_EXACT>(dyn, sh); else wide_onepass_stream<T, false, P1_EXACT>(dyn, sh);
+    }
   }
   // ---- the row's sums and maximum
-  const bool mine = lane < W_NW;
   const float m = scale_t(okey_to_float(__reduce_max_sync(FULL, mine ? static_cast<uint32_t>(sc.i0[lane]) : 0u)), Tm);
   const int any = __reduce_or_sync(FULL, mine ? sc.i1[lane] : 0);
   double S = warp_sum_d(mine ? sc.d0[lane] : 0.0);
@@ -480,11 +513,11 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
   if ((any & 1) || !(fabsf(m) < INFINITY)) return WHY_NAN;                    // the two-pass form reports such rows
   if (any & 2) return WHY_LIST;
   // with a cut the anchor is the sample's maximum: it must be close to the row's for the heavy logits to keep the error budget
-  if (cut_on && !(fabsf(m - sh.as) <= 2.0f)) return WHY_ANCHOR;
+  if (exact ? !(m - sh.base <= W1X_FAR) : !(fabsf(m - sh.as) <= 2.0f)) return WHY_ANCHOR;
   if (!(S > 0.0) || !(S < 1e300)) return WHY_SUM;
   // everything so far is relative to exp(anchor); from here on to exp(max)
-  const double anchor = cut_on ? static_cast<double>(sh.as * P1_L2E) / static_cast<double>(P1_L2E) : static_cast<double>(sh.as);
-  const double cf = exp(anchor - static_cast<double>(m));
+  const double anchor = cut_on ? static_cast<double>(sh.as * P1_L2E) / static_cast<double>(P1_L2E) : static_cast<double>(exact ? sh.base : sh.as);
+  const double cf = exp((anchor - static_cast<double>(m)) * (exact ? W1X_STRETCH : 1.0));
   S *= cf;
   Ktot *= cf;
   if (!(S > 0.0)) return WHY_SUM;
@@ -751,7 +784,7 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
     }
     return exp_safe(d, s_tab);
   };
-  const int how = (cut_on ? HOW_CUT : 0) | (low ? HOW_LOW : 0) | (one_class ? HOW_ONE_CLASS : 0) | (by_piece ? HOW_BY_PIECE : 0) | (by_piece && !ties_in ? HOW_INDEX : 0);
+  const int how = (cut_on ? HOW_CUT : 0) | (low ? HOW_LOW : 0) | (one_class ? HOW_ONE_CLASS : 0) | (by_piece ? HOW_BY_PIECE : 0) | (by_piece && !ties_in ? HOW_INDEX : 0) | (exact ? HOW_EXACT : 0);
   if (!(Re > 0.0)) {                                         // mode A removed every token
     wide_write_nothing_kept(A, row_id, m, S, 3, 0, how, flags);
     return 0;

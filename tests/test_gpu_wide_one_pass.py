@@ -59,8 +59,9 @@ def test_one_pass_rows(wide, oracle, V, pad, bf16):
         assert paths[0] == 3 and paths[1] == 3                        # flat rows under a deep nucleus
 
 
-# reserved[6] of a wide row's debug record: why it took two passes
+# reserved[6] of a wide row's debug record: why it took two passes; reserved[7]: what one pass did
 WHY_TEMPERATURE, WHY_SHORT, WHY_NOT_FINITE, WHY_HEAVY, WHY_WINDOW, WHY_EMPTY_WINDOW, WHY_NAN, WHY_LIST, WHY_ANCHOR = range(1, 10)
+HOW_EXACT = 32
 
 
 def test_reasons_for_two_passes(wide, oracle):
@@ -79,6 +80,52 @@ def test_reasons_for_two_passes(wide, oracle):
     gpu, _, _ = run_both(wide, oracle, np.stack(rows), np.array(cfgs, dtype=CFG_DTYPE), rng.random(len(rows)))
     assert list(gpu["debug"]["reserved"][:, 6]) == why
     assert list(gpu["debug"]["path"]) == [2 if w else 3 for w in why]
+
+
+@pytest.mark.parametrize("bf16", [False, True], ids=["f32", "bf16"])
+@pytest.mark.parametrize("V", [300, 16391, 70001])
+def test_sums_without_a_cut(wide, oracle, V, bf16):
+    """The softmax denominator of rows without a cut against the sum in 64 bits, wherever the row lies. An exact exponential is off by
+    1.2e-10 + 2.4e-12 per unit below the maximum (of 30 that matter), and so is a sum of them; 1e-12 for 1e5 additions in f64."""
+    rng = np.random.Generator(np.random.Philox(key=91 + V))
+    z = lambda s: rng.standard_normal(V) * s
+    rows, T = [], []
+    for x, t in ((z(2.0), 1.0), (z(0.25), 0.8), (z(3.0) + 1000.0, 1.0), (z(3.0) - 1000.0, 1.3), (z(2.0), 0.07), (z(2.0) + 31.0, 1.0), (z(2.0) - 33.0, 1.0),
+                 (z(1.0) + 5e5, 1.0)):
+        rows.append(x); T.append(t)
+    x = z(1.0); x[V - 1] = 70.0                              # all but one token far below a maximum that the first look misses
+    rows.append(x); T.append(1.0)
+    x = z(2.0); x[: V // 2] = -np.inf
+    rows.append(x); T.append(0.7)
+    x = np.stack(rows).astype(np.float32)
+    cfgs = np.array([(t, 0, 0.0, MODE_B) for t in T], dtype=CFG_DTYPE)
+    bits = oracle.f32_to_bf16_bits(x) if bf16 else x
+    if bf16:
+        x = (bits.astype(np.uint32) << 16).view(np.float32)
+    gpu, _, _ = run_both(wide, oracle, bits, cfgs, rng.random(len(T)))
+    assert np.all(gpu["debug"]["path"] == 3)
+    exact = (gpu["debug"]["reserved"][:, 7] & HOW_EXACT) != 0
+    assert np.all(exact[[0, 2, 3, 4, 5, 6, 8]]) and (V > 16000 or np.all(exact))
+    s = (x / np.array(T, dtype=np.float32)[:, None]).astype(np.float64)
+    want = np.exp(s - s.max(axis=1, keepdims=True)).sum(axis=1)
+    err = np.abs(gpu["debug"]["sum_exp"] / want - 1.0)
+    assert np.max(err[exact]) <= 1.2e-10 + 30 * 2.4e-12 + 1e-12
+    assert np.all(err <= 4.5e-7 + 2.0e-7 * 9.7)             # the budget of the quick sums
+
+
+def test_maxima_far_from_the_first_look(wide, oracle):
+    """Short rows (and those whose first look spans much) take the exact sums at once, and a maximum more than 88 above their base leaves them to the two-pass form; a long
+    row's quick sums end at the first logit that is too far up, and the exact ones know it. Beyond 1e6 there are no exact sums."""
+    rng = np.random.Generator(np.random.Philox(key=5))
+    cfgs = np.array([(1.0, 0, 0.0, MODE_A)] * 5, dtype=CFG_DTYPE)
+    for V, path, why in ((10000, [3, 2, 2, 2, 3], [0, WHY_ANCHOR, WHY_ANCHOR, WHY_ANCHOR, 0]),
+                         (70000, [3] * 5, [0] * 5)):
+        x = (rng.standard_normal((5, V)) * 0.25).astype(np.float32)
+        x[0, V - 1] = 87.0; x[1, V - 1] = 89.0; x[2] += 2e6; x[3] -= 2e6
+        gpu, _, _ = run_both(wide, oracle, x, cfgs, rng.random(5))
+        assert list(gpu["debug"]["path"]) == path and list(gpu["debug"]["reserved"][:, 6]) == why
+        how = gpu["debug"]["reserved"][:, 7] & HOW_EXACT
+        assert list(how != 0) == ([True, False, False, False, True] if V == 10000 else [True, True, False, False, False])
 
 
 def test_uniforms_at_the_ends(wide, oracle):
