@@ -183,11 +183,14 @@ __device__ __forceinline__ void wide_steps(const WSpan& sp, const RowView<T>& rv
     if (sp.clean_hi < sp.nst) wide_steps<T, D, false>(sp, rv, pol, lane, sp.clean_hi, sp.nst, qa_, qb_, BODY(false)); \
   } while (0)
 
+__device__ __forceinline__ unsigned long long policy_keep() { unsigned long long p; asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p)); return p; }
+__device__ __forceinline__ unsigned long long policy_drop() { unsigned long long p; asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p)); return p; }
+
 // pass 1: max, min, NaN flag over the row's logits. With HIST it also counts the logits into the
 // histogram of q = s - anchor (an upper estimate of the row's maximum taken from a sample), so that
 // rows whose maximum stays below the anchor need no second pass for their histogram.
 template <typename T, bool HIST, bool TONE>
-__device__ __noinline__ void wide_pass1(const WSpan& sp_in, const RowView<T>& rv_in, unsigned long long pol, int lane,
+__device__ __noinline__ void wide_pass1(const WSpan& sp_in, const RowView<T>& rv_in, int lane,
                                         uint32_t hist_bias, float anchor, float Tm, float scale, float dclamp,
                                         float& xmax, float& xmin, bool& nan_seen) {
   const WSpan sp = sp_in;                // registers, not memory, inside the loop
@@ -213,6 +216,7 @@ __device__ __noinline__ void wide_pass1(const WSpan& sp_in, const RowView<T>& rv
         if (CL || ((valid >> c) & 1u)) asm volatile("red.shared.add.u32 [%0], 1;" :: "r"(a) : "memory"); \
       }                                                                                          \
     } }
+  const unsigned long long pol = policy_keep();
   GS_WIDE_STREAM(T, W_D1, sp, rv, pol, lane, GS_BODY1);
 #undef GS_BODY1
   xmax = vmax; xmin = vmin; nan_seen = (vmax != vmax);
@@ -221,7 +225,7 @@ __device__ __noinline__ void wide_pass1(const WSpan& sp_in, const RowView<T>& rv
 // pass 2: count histogram of d (logits outside the row are not counted).
 // hist_bias = shared address of the histogram - 0x4B000000 * 4 (mod 2^32): see exp_fast_s.
 template <typename T, bool TONE>
-__device__ __noinline__ void wide_pass2(const WSpan& sp_in, const RowView<T>& rv_in, unsigned long long pol, int lane,
+__device__ __noinline__ void wide_pass2(const WSpan& sp_in, const RowView<T>& rv_in, int lane,
                                         uint32_t hist_bias, float m, float Tm, float scale, float dclamp) {
   const WSpan sp = sp_in;
   const RowView<T> rv = rv_in;
@@ -232,6 +236,7 @@ __device__ __noinline__ void wide_pass2(const WSpan& sp_in, const RowView<T>& rv
       const uint32_t a = __float_as_uint(f) * 4u + hist_bias;                                    \
       if (CL || ((valid >> c) & 1u)) asm volatile("red.shared.add.u32 [%0], 1;" :: "r"(a) : "memory"); \
     } }
+  const unsigned long long pol = policy_keep();
   GS_WIDE_STREAM(T, 1, sp, rv, pol, lane, GS_BODY2);
 #undef GS_BODY2
 }
@@ -242,7 +247,7 @@ __device__ __noinline__ void wide_pass2(const WSpan& sp_in, const RowView<T>& rv
 // FAST: every logit of the row has d > -31.9 (bucket-table exponential, no range check);
 // TONE: temperature 1; CUT: a top-p cut is active.
 template <typename T, bool FAST, bool TONE, bool CUT>
-__device__ __noinline__ void wide_pass3(const WSpan& sp_in, const RowView<T>& rv_in, unsigned long long pol, int lane, int warp,
+__device__ __noinline__ void wide_pass3(const WSpan& sp_in, const RowView<T>& rv_in, int lane, int warp,
                                         float m, float Tm, float dA, float dB, uint32_t eb_mul, uint32_t eb_bias, const double* s_tab,
                                         double* part, int ppw, uint2* zl, int* zcnt, double& Ssum, double& Ksum) {
   constexpr int VEC = Elem<T>::VEC;
@@ -303,6 +308,7 @@ __device__ __noinline__ void wide_pass3(const WSpan& sp_in, const RowView<T>& rv
       if (lane == 0) { part[warp * ppw + (st / W_G)] = kw; ksum += kw; }                         \
       t0 = t1 = 0.0; sub = 0.0;                                                                  \
     } }
+  const unsigned long long pol = policy_drop();
   GS_WIDE_STREAM(T, 1, sp, rv, pol, lane, GS_BODY3);
 #undef GS_BODY3
   Ssum = stot; Ksum = ksum;
@@ -338,7 +344,7 @@ struct WideShared {
   double bcd[4];
   int bc[4];
   int cnt;
-  int row;
+  int row, why;
   // one pass: the row, its window, and what the pass and the cut find
   const uint4* vbase;
   int V, shift, nvec;
@@ -626,8 +632,8 @@ __device__ __noinline__ bool wide_big_zone(const WSpan& sp_in, const RowView<T>&
 
 // Two passes over the row: for what one pass does not serve.
 template <typename T>
-__device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t row_id, const int why, unsigned char* dyn, WideShared& sh,
-                         unsigned long long pol_keep, unsigned long long pol_drop) {
+__device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, unsigned char* dyn, WideShared& sh) {
+  const int64_t row_id = sh.row;
   const KernelArgs& A = BA.k;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int V = A.V;
@@ -713,9 +719,9 @@ __device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t
   bool nan_seen = false;
   {
     const uint32_t hb = smem_addr(hist) - 0x4B000000u * 4u;
-    if (!anchored) wide_pass1<T, false, true>(sp, rv, pol_keep, lane, hb, anchor, Tm, scale, dclamp, xmax, xmin, nan_seen);
-    else if (t_is_one) wide_pass1<T, true, true>(sp, rv, pol_keep, lane, hb, anchor, Tm, scale, dclamp, xmax, xmin, nan_seen);
-    else wide_pass1<T, true, false>(sp, rv, pol_keep, lane, hb, anchor, Tm, scale, dclamp, xmax, xmin, nan_seen);
+    if (!anchored) wide_pass1<T, false, true>(sp, rv, lane, hb, anchor, Tm, scale, dclamp, xmax, xmin, nan_seen);
+    else if (t_is_one) wide_pass1<T, true, true>(sp, rv, lane, hb, anchor, Tm, scale, dclamp, xmax, xmin, nan_seen);
+    else wide_pass1<T, true, false>(sp, rv, lane, hb, anchor, Tm, scale, dclamp, xmax, xmin, nan_seen);
   }
   __syncthreads();
   const int anynan = bu::max_i<W_NW>(nan_seen ? 1 : 0, sc, tid);
@@ -725,7 +731,7 @@ __device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t
   // A NaN anywhere, or an infinite maximum, makes the softmax sum NaN upstream
   // (generate.go:173-181): every comparison of the walk fails, result n-1 (:239).
   if (anynan || !(fabsf(m) < INFINITY)) {
-    wide_write_nothing_kept(A, row_id, m, -1.0, 2, why, 0, flags);
+    wide_write_nothing_kept(A, row_id, m, -1.0, 2, sh.why, 0, flags);
     return;
   }
   dlow = scale_t(xmin, Tm) - m;                  // smallest d of the row (-Inf with a -Inf logit)
@@ -745,8 +751,8 @@ __device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t
       __syncthreads();
       for (int j = tid; j < W_NB; j += W_NT) hist[j] = 0;
       __syncthreads();
-      if (t_is_one) wide_pass2<T, true>(sp, rv, pol_keep, lane, smem_addr(hist) - 0x4B000000u * 4u, m, Tm, scale, dclamp);
-      else wide_pass2<T, false>(sp, rv, pol_keep, lane, smem_addr(hist) - 0x4B000000u * 4u, m, Tm, scale, dclamp);
+      if (t_is_one) wide_pass2<T, true>(sp, rv, lane, smem_addr(hist) - 0x4B000000u * 4u, m, Tm, scale, dclamp);
+      else wide_pass2<T, false>(sp, rv, lane, smem_addr(hist) - 0x4B000000u * 4u, m, Tm, scale, dclamp);
     }
     __syncthreads();
     constexpr int PER = W_NB / W_NT;                         // buckets per thread
@@ -826,7 +832,7 @@ __device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t
   double Ssum = 0.0, Ksum = 0.0;
   const uint32_t eb_mul = eb_rep ? 8u * W_EB_REP : 8u;
   const uint32_t eb_bias = smem_addr(ebs) + (eb_rep ? 8u * (lane & (W_EB_REP - 1)) : 0u) - 0x4B000000u * eb_mul;
-#define GS_P3(F, O, C) wide_pass3<T, F, O, C>(sp, rv, pol_drop, lane, warp, m, Tm, dA, dB, eb_mul, eb_bias, s_tab, part, ppw, zl, &sh.cnt, Ssum, Ksum)
+#define GS_P3(F, O, C) wide_pass3<T, F, O, C>(sp, rv, lane, warp, m, Tm, dA, dB, eb_mul, eb_bias, s_tab, part, ppw, zl, &sh.cnt, Ssum, Ksum)
   if (cut_on) {
     if (fast_ok) { if (t_is_one) GS_P3(true, true, true); else GS_P3(true, false, true); }
     else         { if (t_is_one) GS_P3(false, true, true); else GS_P3(false, false, true); }
@@ -850,7 +856,7 @@ __device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t
   int cut_incl = 0;
   bool bad = false;
   if (big) {
-    if (!wide_big_zone<T>(sp, rv, pol_keep, sh, hist, part, s_tab, m, Tm, dA, dB, dlow, mode, plim, S, Ktot, fast_ok,
+    if (!wide_big_zone<T>(sp, rv, policy_keep(), sh, hist, part, s_tab, m, Tm, dA, dB, dlow, mode, plim, S, Ktot, fast_ok,
                           span, ppw, cut_key, cut_incl, flags)) {
       if (tid == 0) hand_to_single(BA, row_id);
       return;
@@ -986,9 +992,9 @@ __device__ __noinline__ void wide_twopass_row(const BatchArgs& BA, const int64_t
   const double pm = (tid < npiece) ? part[tid] : 0.0;
   WideResult r;
   const double pex = bu::scan_excl_d<W_NW>(pm, r.Re, sc, tid);
-  r.m = m; r.S = S; r.path = 2; r.why = why; r.how = 0;
+  r.m = m; r.S = S; r.path = 2; r.why = sh.why; r.how = 0;
   if (!(S == S) || !(S > 0.0) || !(r.Re > 0.0)) {
-    wide_write_nothing_kept(A, row_id, m, S, 2, why, 0, flags);
+    wide_write_nothing_kept(A, row_id, m, S, 2, sh.why, 0, flags);
     return;
   }
   const int psel = bu::min_i<W_NW>((tid < npiece && u * r.Re < pex + pm) ? tid : 0x7fffffff, sc, tid);
@@ -1015,9 +1021,6 @@ __global__ void __launch_bounds__(W_NT, W_CTAS) wide_rows_kernel(const __grid_co
   extern __shared__ __align__(16) unsigned char dyn[];
   __shared__ WideShared sh;
   if (threadIdx.x < 256) sh.tab[threadIdx.x] = BA.k.exp_table[threadIdx.x];
-  unsigned long long pol_keep, pol_drop;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_keep));
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_drop));
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1037,8 +1040,9 @@ __global__ void __launch_bounds__(W_NT, W_CTAS) wide_rows_kernel(const __grid_co
     pdl_launch();
     const int why = wide_onepass_row<T>(BA, row, dyn, sh);
     if (why == 0) continue;
+    if (threadIdx.x == 0) sh.why = why;
     __syncthreads();
-    wide_twopass_row<T>(BA, row, why, dyn, sh, pol_keep, pol_drop);
+    wide_twopass_row<T>(BA, dyn, sh);
   }
 }
 

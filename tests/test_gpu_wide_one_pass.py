@@ -13,6 +13,7 @@ pytestmark = pytest.mark.gpu
 @pytest.fixture(params=[4, 5], ids=["w256", "w1024"])
 def wide(request, _sampler_session):
     _sampler_session.set_kernel_variant(request.param, 0)
+    _sampler_session.one_pass_from = {4: 32832, 5: 65600}[request.param]   # shorter rows with a cut are not sampled
     yield _sampler_session
     _sampler_session.set_kernel_variant(0, 0)
 
@@ -56,7 +57,7 @@ def test_one_pass_rows(wide, oracle, V, pad, bf16):
     paths = gpu["debug"]["path"]
     assert np.all(paths[one & (cfgs["top_p"] == 0.0)] == 3)             # no cut: always one pass
     if V == 50257 and not bf16:
-        assert paths[0] == 3 and paths[1] == 3                        # flat rows under a deep nucleus
+        assert list(paths[:2]) == ([2, 2] if wide.one_pass_from > V else [3, 3])   # flat rows under a deep nucleus
 
 
 # reserved[6] of a wide row's debug record: why it took two passes; reserved[7]: what one pass did
@@ -126,6 +127,16 @@ def test_maxima_far_from_the_first_look(wide, oracle):
         assert list(gpu["debug"]["path"]) == path and list(gpu["debug"]["reserved"][:, 6]) == why
         how = gpu["debug"]["reserved"][:, 7] & HOW_EXACT
         assert list(how != 0) == ([True, False, False, False, True] if V == 10000 else [True, True, False, False, False])
+
+
+@pytest.mark.parametrize("bf16", [False, True], ids=["f32", "bf16"])
+def test_shortest_row_with_a_cut_in_one_pass(wide, oracle, bf16):
+    rng = np.random.Generator(np.random.Philox(key=12))
+    for V, pad, path, why in ((wide.one_pass_from - 1, 1, 2, WHY_SHORT), (wide.one_pass_from, 0, 3, 0), (wide.one_pass_from + 5, 3, 3, 0)):
+        x = (rng.standard_normal((6, V)) * 0.25).astype(np.float32)
+        cfgs = np.array([(T, 0, p, MODE_B) for T in (1.0, 0.8) for p in (0.99, 0.995, 0.999)], dtype=CFG_DTYPE)
+        gpu, _, _ = run_both(wide, oracle, oracle.f32_to_bf16_bits(x) if bf16 else x, cfgs, rng.random(6), pad=pad, allow_tie_cut=True)
+        assert np.all(gpu["debug"]["path"] == path) and np.all(gpu["debug"]["reserved"][:, 6] == why)
 
 
 def test_uniforms_at_the_ends(wide, oracle):
