@@ -628,9 +628,29 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
       uint32_t kmax = dkey_of(cmin), inv = ~dkey_of(cmax), none = 0u;      // (dkey falls as d rises)
       if (cmin > 0.0f) { kmax = 0u; inv = 0u; }                            // none here
       bu::max_u3<W_NW>(kmax, inv, none, sc, tid);
+      const float was_hi = dhi, was_lo = dlo;
       dhi = -__uint_as_float(~inv); dlo = -__uint_as_float(kmax);
       if (dhi == dlo) { one_class = true; break; }           // a long run of equal d
-      if (round == 5) return WHY_CUT_BELOW;
+      if (round == 7) return WHY_CUT_BELOW;
+      if (dhi == was_hi && dlo == was_lo) {
+        // The cut lies within the bounds' slack of where a long run of equal d ends: nothing came off either end. The upper run by
+        // itself, exactly (bf16 rows met this once in four thousand, and took two passes after all).
+        int run = 0;
+        float next = -INFINITY;
+        for (int j = lane; j < cnt; j += 32) {
+          const float d = list[j];
+          if (d == dhi) run++;
+          else if (d < dhi && d >= dlo) next = fmaxf(next, d);
+        }
+        const double e = exp_safe(dhi, s_tab);
+        nc = bu::sum_i<W_NW>(run, sc, tid);
+        if (crossed(gbase + nc * e)) { one_class = true; break; }
+        zsum += run * e;
+        gbase += nc * e;
+        uint32_t up = (next > -INFINITY) ? ~dkey_of(next) : 0u, none1 = 0u, none2 = 0u;
+        bu::max_u3<W_NW>(up, none1, none2, sc, tid);
+        dhi = -__uint_as_float(~up);
+      }
       scale = fminf(static_cast<float>(W1_BINS) / (dhi - dlo), 1e30f);
       bins[tid] = 0u;
       if (tid == 0) { sh.bc[0] = W1_BINS; sh.bc[1] = W1_BINS - 1; sh.cnt = 0; }

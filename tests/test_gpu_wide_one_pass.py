@@ -139,6 +139,26 @@ def test_shortest_row_with_a_cut_in_one_pass(wide, oracle, bf16):
         assert np.all(gpu["debug"]["path"] == path) and np.all(gpu["debug"]["reserved"][:, 6] == why)
 
 
+@pytest.mark.parametrize("T", [1.0, 0.8])
+def test_cut_at_the_end_of_a_run(wide, oracle, T):
+    """Long runs of equal logits, and a top-p within a few ulps of the mass through one of them: the bounds that look for the
+    cut's run cannot tell it from the next, and one pass has to find it all the same."""
+    rng = np.random.Generator(np.random.Philox(key=41))
+    V = 90000
+    base = (np.round(rng.standard_normal(V) * 0.25 * 64) / 64).astype(np.float32)
+    s = base / np.float32(T)
+    e = np.exp((s - s.max()).astype(np.float64))
+    vals, n = np.unique(s, return_counts=True)
+    through = np.cumsum((np.exp((vals - vals.max()).astype(np.float64)) * n)[::-1]) / e.sum()
+    cuts = through[np.flatnonzero((through > 0.988) & (through < 0.997) & (n[::-1] > 40))][:6]
+    assert len(cuts) >= 4
+    ps = [np.float32(c) + np.float32(k * 2.0 ** -24) for c in cuts for k in (-2, 0, 2)]
+    x = np.repeat(base[None], len(ps), axis=0)
+    cfgs = np.array([(T, 0, p, MODE_B) for p in ps], dtype=CFG_DTYPE)
+    gpu, _, _ = run_both(wide, oracle, x, cfgs, rng.random(len(ps)), allow_tie_cut=True)
+    assert list(gpu["debug"]["reserved"][:, 6]) == [0] * len(ps) and np.all(gpu["debug"]["path"] == 3)
+
+
 def test_uniforms_at_the_ends(wide, oracle):
     """u = 0 takes the first kept logit, the largest u below 1 the last one."""
     rng = np.random.Generator(np.random.Philox(key=31))
