@@ -591,7 +591,7 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
           const float a = __shfl_up_sync(FULL, hi, o), b = __shfl_up_sync(FULL, lo, o);
           if (lane >= o) { hi += a; lo += b; }
         }
-        float* wh = reinterpret_cast<float*>(sc.d0);
+        float* wh = reinterpret_cast<float*>(sc.u);          // (not sc.d0: a warp may still be reading sum_d's there)
         float* wl = reinterpret_cast<float*>(sc.d1);
         if (lane == 31) { wh[warp] = hi; wl[warp] = lo; }
         __syncthreads();
