@@ -352,7 +352,7 @@ struct WideShared {
   float as, base;          // what the sums are relative to, in units of x / T: the anchor, or, for exact sums, the base
   float Tm, xA, xB;        // above the window: x >= xA; the window: xB <= x < xA
   int far;                 // a logit lies too far above the anchor
-  int low;                 // the window reaches down to where no mass is
+  int placed;              // HOW_LOW: the window reaches down to where no mass is; HOW_OFTEN: the lanes' buffers are emptied more often; HOW_TWICE: twice the sample
   double eps;              // relative error bound of the sums
   double kw[W_NW];         // the mass above the window in each warp's part of the row (all its mass where the window is low),
   double zw[W_NW];         // what the window adds to it,
@@ -372,8 +372,9 @@ enum { WHY_TEMPERATURE = 1,   // the quick quotient is not exact for it
        WHY_SUM,
        WHY_CUT_ABOVE,         // the window failed: the cut lies above it,
        WHY_CUT_BELOW,         // ... or below, or too close to its end
-       WHY_LONG };            // longer than a warp's part can be
-enum { HOW_CUT = 1, HOW_LOW = 2, HOW_ONE_CLASS = 4, HOW_BY_PIECE = 8, HOW_INDEX = 16, HOW_EXACT = 32 };
+       WHY_LONG,              // longer than a warp's part can be
+       WHY_AGAIN };           // (not a reason: the sample is doubled)
+enum { HOW_CUT = 1, HOW_LOW = 2, HOW_ONE_CLASS = 4, HOW_BY_PIECE = 8, HOW_INDEX = 16, HOW_EXACT = 32, HOW_OFTEN = 64, HOW_TWICE = 128 };
 // How a row ends, from either form. `path`: 2 two passes, 3 one.
 struct WideResult {
   float m;                 // largest x / T

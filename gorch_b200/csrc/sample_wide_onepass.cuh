@@ -1,4 +1,4 @@
-// The wide kernel's usual way with a row: one pass over it. (Included by sample_wide.cuh inside its namespace, once per
+// The wide kernel's first way with a row: one pass over it, where the row is such that one pass can serve it. (Included by sample_wide.cuh inside its namespace, once per
 // instance.)
 //
 // One pass sums the mass of everything (S) with the fast exponential relative to an anchor near the row maximum. With a top-p
@@ -16,25 +16,26 @@
 // The lists. A window of 1 to 2 % of the logits puts one into a tenth of the lane-steps, so nearly every warp-step has a lane
 // that must list something, and slots from a shared counter cost every warp some ninety issue slots a step. So a lane has a
 // buffer of its own: a predicated store and a predicated addition per logit, no branch, no counter, consecutive lanes in
-// consecutive banks. At the end of a piece the warp moves what its lanes hold to its list, a vote per round. What is listed is
+// consecutive banks. At the end of a piece (of every turn of the ring, where the window is wide) the warp moves what its lanes hold to its list, a vote per round. What is listed is
 // the logit alone: its piece is known, and the few indices that the cut's ties need are found by looking at one piece again.
 //
 // The loads. Four CTAs' shared memory leaves some 28 KB of L1 per SM, too little for 64 KB of register loads on their way
 // (512 rows of 151,936 f32, loads alone: 65 us; 51 with L1 free), and the loop's loads share their scoreboards with its
 // exponentials. So sample and row come by asynchronous copies to shared memory, which take no L1 (53); asking L2
-// for lines further ahead made the pass slower (98 against 90 thousand cycles). Everything uniform lies in shared memory and nothing of a thread's on its stack: the stacks of a former version
-// wrote 59 MB to HBM per 311 MB read.
+// for lines further ahead made the pass slower. Everything uniform lies in shared memory and the pass has nothing on its stack: the stacks of a former
+// version wrote 59 MB to HBM per 311 MB read. (The code around it still spills some values, once a row.)
 //
 // Error budget of the fast sums against exp(d) in f64, d = x/T - max rounded to f32 as upstream. With a cut the argument of
-// 2^t is one FMA, x log2 e - C: ex2.approx 2.4e-7, three f32 additions per step before the f64 accumulators 1.8e-7, and per
+// 2^t is one FMA, x/T log2 e - C: ex2.approx 2.4e-7, three f32 additions per step before the f64 accumulators 1.8e-7, and per
 // unit of |x/T - anchor| the roundings of t, of log2 e and of upstream's d, 1.4e-7 together: W1_EPS_FIXED + W1_EPS_PER_D * (largest |d|
 // that carries mass). (C is the anchor times log2 e, rounded: the anchor that this stands for is what the sums are taken
-// back from.) The anchor must lie within 2 of the maximum. Without a cut the rounding of t is made up for (p1_exp2), which leaves
-// 6e-8 per unit: the anchor may lie W1_RISE below a logit for the same error.
+// back from.) The anchor must lie within 2 of the maximum. The quick sums without a cut take the same roundings, one more of x/T - C.
 constexpr int P1_ALL = 0, P1_EXACT = 1, P1_LOW = 2, P1_MID = 3;
 constexpr int W1_SAMPLE = (W_NT >= 512) ? 16384 : 8192;        // logits of the sample
 constexpr int W1_MIN_CUT = 4 * W1_SAMPLE + 64;                 // rows shorter than this are not sampled
 constexpr int W1_SBINS = 1024;           // its histogram's buckets
+constexpr float W1_MAX_WINDOW = 3328.0f; // logits of a window that takes more than the usual sample and buffers (wide_place_window)
+constexpr float W1_PER_VISIT = 1.5f;     // logits that a lane's buffer gets, on average, before it is emptied: the most
 constexpr double W1_EPS_FIXED = 4.5e-7;
 constexpr double W1_EPS_PER_D = 2.0e-7;
 constexpr int W1X_ENTRIES = 256, W1X_COPIES = 16;   // table of the exact exponential: 2^(j/256), a copy per pair of banks
@@ -169,7 +170,7 @@ __device__ __forceinline__ void p1_mask(float* x, int gv, int nvec, int shift, i
 // The pass. Leaves in shared memory: part[warp * ppw + piece], the mass of each piece (P1_MID: of its logits above the window), relative to the anchor or base; the warps' lists, and in from[warp][piece] where a piece begins in its warp's;
 // per warp kw (sum of its pieces), sc.d0 (all mass), sc.i0 (order key of the maximum), sc.i1 (1: a NaN, 2: a list that did
 // not hold all).
-template <typename T, bool TONE, int MODE>
+template <typename T, bool TONE, int MODE, bool OFTEN = false>
 __device__ __noinline__ void wide_onepass_stream(unsigned char* dyn, WideShared& sh) {
   constexpr int VEC = Elem<T>::VEC, EPI = 8 / VEC, SV = 32 * EPI;
   constexpr uint32_t STAGE = EPI * W_NT * 16;                  // ring: EPI vectors per thread and stage
@@ -205,24 +206,25 @@ __device__ __noinline__ void wide_onepass_stream(unsigned char* dyn, WideShared&
   const uint32_t ring = smem_addr(dyn + W1_OFF_RING) + static_cast<uint32_t>(tid) * 16u;
   const uint4* ring_at = reinterpret_cast<const uint4*>(dyn + W1_OFF_RING) + tid;
   volatile int* far = &sh.far;
-  auto piece_end = [&](int st) {
-    if (CUT) {
-      full |= a.at >= k.buf_end;
-      const int n = static_cast<int>((a.at - k.buf) / (W_NT * 4u));
-      for (int r = 0;; r++) {
-        const unsigned have = __ballot_sync(FULL, r < n);
-        if (have == 0u) break;
-        const int slot = listed + __popc(have & ((1u << lane) - 1u));
-        if (r < n && slot < W1_WCAP) {
-          float v;
-          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(k.buf + static_cast<uint32_t>(r) * (W_NT * 4u)));
-          list[slot] = v;
-        }
-        listed += __popc(have);
+  constexpr int VISIT = OFTEN ? NQ : W_G;                      // steps from one emptying of the buffers to the next
+  auto empty_buffers = [&]() {
+    full |= a.at >= k.buf_end;
+    const int n = static_cast<int>((a.at - k.buf) / (W_NT * 4u));
+    for (int r = 0;; r++) {
+      const unsigned have = __ballot_sync(FULL, r < n);
+      if (have == 0u) break;
+      const int slot = listed + __popc(have & ((1u << lane) - 1u));
+      if (r < n && slot < W1_WCAP) {
+        float v;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(k.buf + static_cast<uint32_t>(r) * (W_NT * 4u)));
+        list[slot] = v;
       }
-      a.at = k.buf;
-      if (lane == 0) from[st / W_G + 1] = min(listed, W1_WCAP);
+      listed += __popc(have);
     }
+    a.at = k.buf;
+  };
+  auto piece_end = [&](int st) {
+    if (CUT && lane == 0) from[st / W_G + 1] = min(listed, W1_WCAP);
     double t = a.kep;
     if (MODE == P1_MID) a.kep = 0.0;
     else { t = (MODE == P1_EXACT) ? a.tot + a.tot2 : a.tot; a.stot += t; a.tot = a.tot2 = 0.0; }
@@ -247,25 +249,27 @@ __device__ __noinline__ void wide_onepass_stream(unsigned char* dyn, WideShared&
   auto put_any = [&](int slot, int q) { if (q < nst) put(slot, src + min(q * SV, omax), src + min(q * SV + 32, omax)); };
 #pragma unroll
   for (int q = 0; q < NQ; q++) { put_any(q, q); cp_commit(); }
-  // Pieces that hold no step at the row's edges and whose refills are clean too run without a mask, a clamp or a test; W_G steps are
-  // a multiple of the ring's NQ.
+  // Pieces, or the parts of a piece between two emptyings, that hold no step at the row's edges and whose refills are clean too run without a
+  // mask, a clamp or a test; either is a multiple of the ring's NQ steps.
   static_assert(W_G % NQ == 0, "a piece begins at the ring's first slot");
   int st = 0;
 #pragma unroll 1
   while (st < nst) {
-    if (st >= clean_lo && st + W_G + NQ <= clean_hi) {
+    if (st >= clean_lo && st + VISIT + NQ <= clean_hi) {
       const uint4* p = src + (st + NQ) * SV;
 #pragma unroll 1
-      for (int j = 0; j < W_G; j += NQ, p += NQ * SV) {
+      for (int j = 0; j < VISIT; j += NQ, p += NQ * SV) {
 #pragma unroll
         for (int q = 0; q < NQ; q++) step(st, q, [&]() { put(q, p + q * SV, p + q * SV + 32); }, true);
       }
-      st += W_G;
+      st += VISIT;
     } else {
 #pragma unroll 1
-      for (int j = 0; j < W_G && st < nst; j++, st++)
+      for (int j = 0; j < VISIT && st < nst; j++, st++)
         step(st, j % NQ, [&]() { put_any(j % NQ, st + NQ); }, st >= clean_lo && st < clean_hi);
     }
+    if (CUT) empty_buffers();
+    if (OFTEN && st % W_G != 0 && st < nst) continue;
     piece_end(st - 1);
     if (MODE == P1_ALL) {                                      // a logit far above the anchor: the row's sums will be exact ones
       if (__any_sync(FULL, a.vmax > k.xA || *far != 0)) {
@@ -290,9 +294,16 @@ __device__ __noinline__ void wide_onepass_stream(unsigned char* dyn, WideShared&
   __syncthreads();
 }
 
-// Places the window of a row with a cut: sh.as, xA, xB, low and eps. 0, or why the row takes two passes.
+template <typename T, bool TONE, int MODE>
+__device__ __forceinline__ void pass_with_cut(unsigned char* dyn, WideShared& sh) {
+  if (sh.placed & HOW_OFTEN) wide_onepass_stream<T, TONE, MODE, true>(dyn, sh);
+  else wide_onepass_stream<T, TONE, MODE>(dyn, sh);
+}
+
+// Places the window of a row with a cut: sh.as, xA, xB, placed and eps. 0, or why the row takes two passes, or WHY_AGAIN: twice the sample may do,
+// and the next call (`again`) adds its other half to the buckets.
 template <typename T>
-__device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh, const double plim) {
+__device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh, const double plim, const bool again) {
   constexpr int VEC = Elem<T>::VEC;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float Tm = sh.Tm;
@@ -304,14 +315,15 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
     const uint4* src = sh.vbase + 1 + (tid & 3);
     const uint32_t dst = smem_addr(dyn) + static_cast<uint32_t>(tid) * 16u;
 #pragma unroll
-    for (int j = 0; j < J; j++) {
-      const int piece = static_cast<int>(static_cast<uint32_t>((static_cast<uint64_t>((j * W_NT + tid) >> 2) * static_cast<uint32_t>(have)) / PIECES));
+    for (int j = 0; j < J; j++) {                                         // (the other half's pieces lie between the first's)
+      const uint32_t at = 2u * static_cast<uint32_t>((j * W_NT + tid) >> 2) + (again ? 1u : 0u);
+      const int piece = static_cast<int>(static_cast<uint32_t>((static_cast<uint64_t>(at) * static_cast<uint32_t>(have)) / (2u * PIECES)));
       cp_async16(dst + j * W_NT * 16, src + piece * 4);
     }
     cp_commit();
   }
   uint32_t* bins = reinterpret_cast<uint32_t*>(dyn + W1_SAMPLE * 4);
-  for (int j = tid; j < W1_SBINS; j += W_NT) bins[j] = 0u;
+  if (!again) for (int j = tid; j < W1_SBINS; j += W_NT) bins[j] = 0u;
   auto each = [&](auto&& fn) {
 #pragma unroll 2
     for (int j = 0; j < J; j++) {
@@ -322,9 +334,9 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
     }
   };
   cp_wait<0>();
-  float smax = -INFINITY, smin = INFINITY;
-  each([&](float x) { smax = maxnan(smax, x); smin = fminf(smin, x); });
-  {
+  float smax = again ? sh.xA : -INFINITY, smin = again ? sh.xB : INFINITY;
+  if (!again) {
+    each([&](float x) { smax = maxnan(smax, x); smin = fminf(smin, x); });
     uint32_t hi = okey(smax), lo = ~okey(smin), nan = (smax != smax) ? 1u : 0u;
     bu::max_u3<W_NW>(hi, lo, nan, sh.sc, tid);                            // (its barriers also publish the cleared bins)
     if (nan) return WHY_NOT_FINITE;
@@ -336,10 +348,12 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
   // ---- a count histogram of its upper 24 units of x / T (what lies lower has no mass to speak of, and shares the last bucket)
   const float range = fmaxf(fminf(smax - smin, 24.0f * Tm), 1e-6f * fmaxf(fabsf(smax), Tm));
   const float scale = static_cast<float>(W1_SBINS - 1) / range;
-  each([&](float x) { atomicAdd(&bins[static_cast<int>(fminf((smax - x) * scale, static_cast<float>(W1_SBINS - 1)))], 1u); });
-  if (tid == 0) { sh.bc[0] = 0; sh.bc[1] = W1_SBINS - 1; sh.bc[2] = 0; sh.bc[3] = W1_SAMPLE; }
+  // (a logit of the second half may lie above smax: the pass finds out how far)
+  const int sampled = again ? 2 * W1_SAMPLE : W1_SAMPLE;
+  each([&](float x) { atomicAdd(&bins[static_cast<int>(fmaxf(fminf((smax - x) * scale, static_cast<float>(W1_SBINS - 1)), 0.0f))], 1u); });
+  if (tid == 0) { sh.bc[0] = 0; sh.bc[1] = W1_SBINS - 1; sh.bc[2] = 0; sh.bc[3] = sampled; }
   __syncthreads();
-  // ---- the window: where the sample's mass passes plim, give or take five standard errors of a mass fraction
+  // ---- the window: where the sample's mass passes plim, give or take 4.5 standard errors of a mass fraction
   // estimated from weighted logits (Var = ((1-p)^2 sum of squared weights above the cut + p^2 of those below) / (sum of
   // weights)^2). Placing it is a matter of speed, not of correctness (the pass checks it on the whole row): f32 does.
   constexpr int PER = W1_SBINS / W_NT;
@@ -384,8 +398,8 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
   if (im < lim && im + mass >= lim) wq[W_NW] = iq + sq;                   // one thread (none: nothing lies below the cut)
   __syncthreads();
   const float q_above = (wq[W_NW] >= 0.0f) ? wq[W_NW] : tot_q, q1 = 1.0f - pl;
-  const float fpc = 1.0f - static_cast<float>(W1_SAMPLE) / static_cast<float>(V);
-  const float delta = 5.0f * sqrtf(fmaxf(q1 * q1 * q_above + pl * pl * (tot_q - q_above), 0.0f) * fpc) + 2.0f;   // in units of mass: two top tokens more
+  const float fpc = 1.0f - static_cast<float>(sampled) / static_cast<float>(V);
+  const float delta = 4.5f * sqrtf(fmaxf(q1 * q1 * q_above + pl * pl * (tot_q - q_above), 0.0f) * fpc) + 2.0f;   // in units of mass: two top tokens more
   const float m_lo = lim - delta, m_hi = lim + delta;
   {
     float e = e0, acc = im;
@@ -402,24 +416,43 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
   }
   __syncthreads();
   const int b1 = max(sh.bc[0] - 1, 0), b2 = min(sh.bc[1] + 1, W1_SBINS - 1);   // a bucket of slack for the f32 sums
-  // How many logits of the row will be listed: the window's mass over that of its last logit, or the sample's count of a hundred
-  // or so (which by itself would be off by a tenth) and three standard deviations, whichever is less; and of the buckets of slack as
-  // many as the window's have on average. The lists hold five standard deviations more, and a lane's buffer of 12 for a piece is
-  // too small in less than one of 10^8 pieces. A window that reaches down to where no mass is saves instructions.
-  auto fits = [&](float logits) {
-    const float per_warp = logits * (static_cast<float>(V) / static_cast<float>(W1_SAMPLE * W_NW));
-    const float per_visit = per_warp / static_cast<float>(32 * max(sh.nvec / (W_NT * (8 / VEC) * W_G), 1));
-    return per_warp + 5.0f * sqrtf(per_warp) <= static_cast<float>(W1_WCAP) && per_visit <= 1.5f;
+  // How many logits of the row will be listed: as many as the sample's share of the window says, and of the buckets of slack as many as
+  // the window's have on average. The lists hold 4.5 standard deviations more, of the sample's count and of a warp's part; a lane's buffer, which
+  // counts as full at 12, is expected to get W1_PER_VISIT at most before it is emptied (full then: one lane in 4 x 10^7, one row of 151,936
+  // logits in 15,000). A list that does not hold all costs a pass: one such row made 512 rows of 151,936 (p = 0.98) take 188 us for 115.
+  // A window that reaches down to where no mass is saves instructions.
+  const float to_row = static_cast<float>(V) / static_cast<float>(sampled), to_warp = to_row * static_cast<float>(sh.span) / static_cast<float>(sh.nvec);
+  auto fits = [&](float logits, int visits) {
+    const float per_warp = logits * to_warp;
+    return per_warp + 4.5f * sqrtf(per_warp * (1.0f + to_warp)) <= static_cast<float>(W1_WCAP) && logits * to_row <= W1_PER_VISIT * static_cast<float>(visits);
   };
-  const float seen = static_cast<float>(max(sh.bc[3] - sh.bc[2], 0));
-  const float inside = fminf(2.0f * delta / ex2_approx(-(static_cast<float>(sh.bc[1]) + 0.5f) * wl2), seen + 3.0f * sqrtf(seen)), per_bucket = inside / static_cast<float>(max(sh.bc[1] - sh.bc[0] + 1, 1));
-  const bool low = fits(static_cast<float>(W1_SAMPLE - sh.bc[2]) + per_bucket);
-  if (!low && !fits(inside + 2.0f * per_bucket)) return WHY_WINDOW;
+  const float seen = static_cast<float>(max(sh.bc[3] - sh.bc[2], 0)), per_bucket = seen / static_cast<float>(max(sh.bc[1] - sh.bc[0] + 1, 1));
+  const float n_low = static_cast<float>(sampled - sh.bc[2]) + per_bucket, n_mid = seen + 2.0f * per_bucket;
+  // how often a lane empties its buffer: once a piece, or once for each turn of the ring
+  const int seldom = W_NT * max(sh.nvec / (W_NT * (8 / VEC) * W_G), 1), turns = V / (W1_RING_BYTES / (W_NT * static_cast<int>(sizeof(T))));
+  bool low = fits(n_low, seldom), often = false;
+  if (!low && !fits(n_mid, seldom)) {
+    // Wider windows are listed where an eighth of the row as sample, with the error of a plain share, leaves W1_MAX_WINDOW logits or fewer between
+    // the bounds. Beyond that the rows keep the exactness of the two-pass sums, which they always had (3e-10 against 4e-8).
+    // (us, flat f32 rows in two passes | one: 512 x 50,257, p = 0.95: 115 | 67; 512 x 100,003, 0.97: 164 | 88; 512 x 151,936, 0.98: 210 | 112;
+    // 128 x 100,003, 0.97: 76 | 44.)
+    const float by_eighth = tot_m * (5.0f * sqrtf(pl * fabsf(q1) * 8.0f / static_cast<float>(V)) + 32.0f / static_cast<float>(V));
+    if (seen * to_row * by_eighth > W1_MAX_WINDOW * delta) return WHY_WINDOW;
+    often = true;
+    low = fits(n_low, turns);
+    if (!low && !fits(n_mid, turns)) {
+      // Twice the sample makes the window narrower by sqrt(2), but for its slack: where that will do, and the sample is less than an eighth of
+      // the row, its other half too (10 us of 512 rows of 151,936 f32, for which two passes take 100 longer)
+      if (again || to_row <= 8.0f || !fits(0.78f * seen + 2.0f * per_bucket, turns)) return WHY_WINDOW;
+      if (tid == 0) { sh.xA = smax; sh.xB = smin; }
+      return WHY_AGAIN;
+    }
+  }
   const float xA = smax - static_cast<float>(b1) / scale;
   const float xB = (low || b2 == W1_SBINS - 1) ? smax - 40.0f * Tm : smax - static_cast<float>(b2 + 1) / scale;
   if (!(xA > xB)) return WHY_EMPTY_WINDOW;
   if (tid == 0) {
-    sh.as = as; sh.xA = xA; sh.xB = xB; sh.low = low ? 1 : 0;
+    sh.as = as; sh.xA = xA; sh.xB = xB; sh.placed = (low ? HOW_LOW : 0) | (often ? HOW_OFTEN : 0) | (again ? HOW_TWICE : 0);
     sh.eps = W1_EPS_FIXED + W1_EPS_PER_D * fmin(9.7, static_cast<double>(range / Tm) + 2.0);
   }
   return 0;
@@ -476,17 +509,21 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
   }
   __syncthreads();
   if (cut_on) {
-    const int why = wide_place_window<T>(dyn, sh, plim);
+    int why = wide_place_window<T>(dyn, sh, plim, false);
+    if (why == WHY_AGAIN) {
+      __syncthreads();                                         // (what the first call left in shared memory has been read)
+      why = wide_place_window<T>(dyn, sh, plim, true);
+    }
     if (why) return why;
   }
   __syncthreads();
-  const bool low = cut_on && sh.low;
+  const bool low = cut_on && (sh.placed & HOW_LOW) != 0;
   const bool mine = lane < W_NW;
   bool exact = false;
   if (low) {
-    if (t_is_one) wide_onepass_stream<T, true, P1_LOW>(dyn, sh); else wide_onepass_stream<T, false, P1_LOW>(dyn, sh);
+    if (t_is_one) pass_with_cut<T, true, P1_LOW>(dyn, sh); else pass_with_cut<T, false, P1_LOW>(dyn, sh);
   } else if (cut_on) {
-    if (t_is_one) wide_onepass_stream<T, true, P1_MID>(dyn, sh); else wide_onepass_stream<T, false, P1_MID>(dyn, sh);
+    if (t_is_one) pass_with_cut<T, true, P1_MID>(dyn, sh); else pass_with_cut<T, false, P1_MID>(dyn, sh);
   } else {
     float b = sh.as;
     if (quick) {
@@ -807,7 +844,7 @@ __device__ __noinline__ int wide_onepass_row(const BatchArgs& BA, const int64_t 
     }
     return exp_safe(d, s_tab);
   };
-  const int how = (cut_on ? HOW_CUT : 0) | (low ? HOW_LOW : 0) | (one_class ? HOW_ONE_CLASS : 0) | (by_piece ? HOW_BY_PIECE : 0) | (by_piece && !ties_in ? HOW_INDEX : 0) | (exact ? HOW_EXACT : 0);
+  const int how = (cut_on ? HOW_CUT | sh.placed : 0) | (one_class ? HOW_ONE_CLASS : 0) | (by_piece ? HOW_BY_PIECE : 0) | (by_piece && !ties_in ? HOW_INDEX : 0) | (exact ? HOW_EXACT : 0);
   if (!(Re > 0.0)) {                                         // mode A removed every token
     wide_write_nothing_kept(A, row_id, m, S, 3, 0, how, flags);
     return 0;

@@ -13,6 +13,7 @@ pytestmark = pytest.mark.gpu
 @pytest.fixture(params=[4, 5], ids=["w256", "w1024"])
 def wide(request, _sampler_session):
     _sampler_session.set_kernel_variant(request.param, 0)
+    _sampler_session.variant = request.param
     _sampler_session.one_pass_from = {4: 32832, 5: 65600}[request.param]   # shorter rows with a cut are not sampled
     yield _sampler_session
     _sampler_session.set_kernel_variant(0, 0)
@@ -60,9 +61,33 @@ def test_one_pass_rows(wide, oracle, V, pad, bf16):
         assert list(paths[:2]) == ([2, 2] if wide.one_pass_from > V else [3, 3])   # flat rows under a deep nucleus
 
 
+# Normal rows, their top-p, the passes they take, and by which means: the lanes' buffers emptied more often, or twice the sample. What a row's window holds is
+# known to a tenth, so every case lies that far from a line.
+REACH = {4: [(33000, 0.25, 0.9, 3, "often"), (50257, 0.25, 0.7, 2, ""), (50257, 0.25, 0.93, 3, "often"), (50257, 0.25, 0.99, 3, ""), (100003, 0.25, 0.9, 2, ""),
+             (100003, 0.25, 0.97, 3, "often"), (151936, 0.25, 0.9, 2, ""), (151936, 0.25, 0.98, 3, "twice"), (151936, 0.4, 0.99, 3, "twice"), (151936, 0.25, 0.99, 3, "")],
+         5: [(70001, 0.25, 0.7, 2, ""), (100003, 0.25, 0.97, 3, "often"), (151936, 0.25, 0.9, 2, ""), (151936, 0.25, 0.98, 3, "")]}
+HOW_CUT, HOW_LOW, HOW_ONE_CLASS, HOW_BY_PIECE, HOW_INDEX, HOW_EXACT, HOW_OFTEN, HOW_TWICE = (1 << i for i in range(8))
+
+
+@pytest.mark.parametrize("bf16", [False, True], ids=["f32", "bf16"])
+def test_reach_of_rows_with_a_cut(wide, oracle, bf16):
+    """Rows on both sides of the lines: the lanes' buffers emptied more often, the other half of the sample, windows too wide for the lists."""
+    rng = np.random.Generator(np.random.Philox(key=501))
+    for V, sigma, p, path, extra in REACH[wide.variant]:
+        x = (rng.standard_normal((4, V)) * sigma).astype(np.float32)
+        cfgs = np.array([(1.0, 0, p, MODE_B)] * 3 + [(1.25, 0, p / 1.5, MODE_A)], dtype=CFG_DTYPE)
+        x[3] *= np.float32(1.25)
+        gpu, _, _ = run_both(wide, oracle, oracle.f32_to_bf16_bits(x) if bf16 else x, cfgs, rng.random(4), pad=V % 4, allow_tie_cut=True, want_probs=False)
+        d = gpu["debug"]
+        assert list(d["path"]) == [path] * 4, (V, sigma, p)
+        how = d["reserved"][:, 7]
+        assert np.all(((how & HOW_OFTEN) != 0) == (extra == "often")) and np.all(((how & HOW_TWICE) != 0) == (extra == "twice")), (V, sigma, p)
+        if path == 2:
+            assert np.all(d["reserved"][:, 6] == WHY_WINDOW)
+
+
 # reserved[6] of a wide row's debug record: why it took two passes; reserved[7]: what one pass did
 WHY_TEMPERATURE, WHY_SHORT, WHY_NOT_FINITE, WHY_HEAVY, WHY_WINDOW, WHY_EMPTY_WINDOW, WHY_NAN, WHY_LIST, WHY_ANCHOR = range(1, 10)
-HOW_EXACT = 32
 
 
 def test_reasons_for_two_passes(wide, oracle):
