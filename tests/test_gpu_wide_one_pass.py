@@ -49,7 +49,7 @@ def _batch(V, seed):
 
 
 @pytest.mark.parametrize("bf16", [False, True], ids=["f32", "bf16"])
-@pytest.mark.parametrize("V,pad", [(300, 0), (16391, 0), (16403, 1), (20480, 0), (32777, 3), (50257, 2)])
+@pytest.mark.parametrize("V,pad", [(300, 0), (16391, 0), (16403, 1), (20480, 0), (32777, 3), (50257, 2), (70001, 1)])
 def test_one_pass_rows(wide, oracle, V, pad, bf16):
     x, cfgs, one, u = _batch(V, 7000 + V)
     if bf16:
@@ -57,8 +57,9 @@ def test_one_pass_rows(wide, oracle, V, pad, bf16):
     gpu, _, _ = run_both(wide, oracle, x, cfgs, u, pad=pad, allow_tie_cut=True)
     paths = gpu["debug"]["path"]
     assert np.all(paths[one & (cfgs["top_p"] == 0.0)] == 3)             # no cut: always one pass
-    if V == 50257 and not bf16:
-        assert list(paths[:2]) == ([2, 2] if wide.one_pass_from > V else [3, 3])   # flat rows under a deep nucleus
+    if V >= 50257:                                                      # flat rows under a deep nucleus, with short runs and with masked logits too
+        assert np.all(paths[[0, 1, 3, 6, 10]] == (2 if wide.one_pass_from > V else 3))
+        assert paths[12] == 2                                           # (the maximum far above the sample's)
 
 
 # Normal rows, their top-p, the passes they take, and by which means: the lanes' buffers emptied more often, or twice the sample. What a row's window holds is
@@ -84,6 +85,26 @@ def test_reach_of_rows_with_a_cut(wide, oracle, bf16):
         assert np.all(((how & HOW_OFTEN) != 0) == (extra == "often")) and np.all(((how & HOW_TWICE) != 0) == (extra == "twice")), (V, sigma, p)
         if path == 2:
             assert np.all(d["reserved"][:, 6] == WHY_WINDOW)
+
+
+@pytest.mark.parametrize("bf16", [False, True], ids=["f32", "bf16"])
+def test_cut_inside_runs(wide, oracle, bf16):
+    """The cut divides runs of 2 to 32 equal logits (steps of 1/1,024, f32), which the selection looks at one by one, and runs of hundreds (1/64), in
+    both modes: all of it in one pass, the member's index from a piece that is read again."""
+    rng = np.random.Generator(np.random.Philox(key=502))
+    V = {4: 50257, 5: 66001}[wide.variant]
+    rows, cfgs = [], []
+    for q in (1024, 64):
+        for p, mode in ((0.99, MODE_B), (0.987, MODE_B), (0.985, MODE_B), (0.66, MODE_A), (0.658, MODE_A), (0.6565, MODE_A)):
+            rows.append(np.round(rng.standard_normal(V) * 0.25 * q) / q)
+            cfgs.append((1.0, 0, p, mode))
+    x = np.stack(rows).astype(np.float32)
+    gpu, _, _ = run_both(wide, oracle, oracle.f32_to_bf16_bits(x) if bf16 else x, np.array(cfgs, dtype=CFG_DTYPE), rng.random(len(rows)), allow_tie_cut=True)
+    how = gpu["debug"]["reserved"][:, 7]
+    assert np.all(gpu["debug"]["path"] == 3)
+    for b in (0, 3, 6, 9):                                   # (a cut may fall on the end of a run)
+        assert np.sum((how[b:b + 3] & (HOW_BY_PIECE | HOW_INDEX)) == (HOW_BY_PIECE | HOW_INDEX)) >= 2
+    assert np.all(how[6:] & HOW_ONE_CLASS) and (bf16 or not np.any(how[:6] & HOW_ONE_CLASS))
 
 
 # reserved[6] of a wide row's debug record: why it took two passes; reserved[7]: what one pass did
@@ -187,8 +208,20 @@ def test_cut_at_the_end_of_a_run(wide, oracle, T):
 def test_uniforms_at_the_ends(wide, oracle):
     """u = 0 takes the first kept logit, the largest u below 1 the last one."""
     rng = np.random.Generator(np.random.Philox(key=31))
-    V = 40000
+    V = 70000
     x = np.repeat((rng.standard_normal((1, V)) * 0.25).astype(np.float32), 6, axis=0)
     cfgs = np.array([(1.0, 0, 0.99, MODE_B), (1.0, 0, 0.0, MODE_B)] * 3, dtype=CFG_DTYPE)
     u = np.array([0.0, 0.0, np.nextafter(1.0, 0.0), np.nextafter(1.0, 0.0), 0.5, 0.5])
-    run_both(wide, oracle, x, cfgs, u)
+    gpu, _, _ = run_both(wide, oracle, x, cfgs, u)
+    assert np.all(gpu["debug"]["path"] == 3)
+
+
+def test_finite_logits_far_out(wide, oracle):
+    """A finite maximum of 1e32, outside what a first look sees, without a cut: no base serves the row, and two passes take that very token."""
+    rng = np.random.Generator(np.random.Philox(key=33))
+    for V in (10000, 70000):
+        x = (rng.standard_normal((2, V)) * 0.25).astype(np.float32)
+        x[:, V // 2 + 100] = 1e32
+        gpu, _, _ = run_both(wide, oracle, x, np.array([(1.0, 0, 0.0, MODE_A), (0.9, 0, 0.0, MODE_B)], dtype=CFG_DTYPE), rng.random(2))
+        assert np.all(gpu["ids"] == V // 2 + 100)
+        assert np.all(gpu["debug"]["path"] == 2) and np.all(gpu["debug"]["reserved"][:, 6] == WHY_ANCHOR)
