@@ -7,8 +7,8 @@
 //                          persistent kernel walks ALL rows with its own atomic
 //                          cursor and takes the rows of its kind, so no separate
 //                          classification launch and no per-kind lists exist.
-//   narrow_rows_kernel     (sample_narrow.cuh, two instances: 256 threads x five CTAs per SM,
-//                          128 threads x eight). One streaming pass per row: the first
+//   narrow_rows_kernel     (sample_narrow.cuh, three instances: 256 threads x five CTAs per SM,
+//                          or three with a longer ring, 128 threads x eight). One streaming pass per row: the first
 //                          16 logits per thread give a threshold (from the per-thread
 //                          maxima: a lower bound of the k-th largest logit, or a tighter
 //                          estimate that is checked at the row's end); then every warp
@@ -90,19 +90,34 @@ __device__ __forceinline__ void hand_to_single(const BatchArgs& BA, int64_t row_
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
-// The narrow kernel, compiled twice from one source (sample_narrow.cuh): n256 with 256 threads and
+// The narrow kernel, compiled three times from one source (sample_narrow.cuh): n256 with 256 threads and
 // five CTAs per SM for batches of at most one row per CTA slot (a row is then streamed by eight
-// warps), n128 with 128 threads and eight CTAs per SM beyond that (1184 rows in flight: the phases
+// warps), n256d with a longer ring for f32 batches of at most two rows per SM, n128 with 128 threads and eight CTAs per SM beyond that (1184 rows in flight: the phases
 // before and after a row's stream then run once per slot instead of twice).
 #define GS_N_NS n256
 #define GS_N_NT 256
+#define GS_N_CTAS 5
+#define GS_N_RING 16384
+#include "sample_narrow.cuh"
+#undef GS_N_NS
+#undef GS_N_CTAS
+#undef GS_N_RING
+#define GS_N_NS n256d
+#define GS_N_CTAS 3
+#define GS_N_RING 32768
 #include "sample_narrow.cuh"
 #undef GS_N_NS
 #undef GS_N_NT
+#undef GS_N_CTAS
+#undef GS_N_RING
 #define GS_N_NS n128
 #define GS_N_NT 128
+#define GS_N_CTAS 8
+#define GS_N_RING 8192
 #include "sample_narrow.cuh"
 #undef GS_N_NS
 #undef GS_N_NT
+#undef GS_N_CTAS
+#undef GS_N_RING
 
 }  // namespace gs

@@ -1,6 +1,6 @@
 // The narrow kernel of the sorted-batch path (greedy and top-k <= 256 rows, one streaming pass
-// each), written once and compiled for two CTA sizes: the including file defines GS_N_NS (the
-// instance's namespace inside gs) and GS_N_NT (threads per CTA: 256 or 128). No include guard.
+// each), written once and compiled three times: the including file defines GS_N_NS (the instance's namespace
+// inside gs), GS_N_NT (threads per CTA: 256 or 128), GS_N_CTAS (CTAs per SM) and GS_N_RING (bytes of the ring). No include guard.
 // Row semantics: model/generate.go:134-260 (mode A), model/qwen/generate.go:77-181 (mode B).
 
 // (included inside namespace gs)
@@ -9,18 +9,19 @@ namespace GS_N_NS {
 constexpr int N_NT = GS_N_NT;           // threads per CTA
 constexpr int N_NW = N_NT / 32;
 constexpr int N_WARM_ELEMS = 16 * N_NT; // logits of the warm-up chunk: 16 per thread, kept in registers
-// 256 threads: five CTAs per SM (48 registers, 34 KB of dynamic shared memory: the candidate list, the ring that the
-// stream is staged through, the hit list). 128 threads: eight CTAs per SM (64 registers, 20 KB). What runs while no copy is in
+// n256, 256 threads: five CTAs per SM (48 registers, 34 KB of dynamic shared memory: the candidate list, the ring that the
+// stream is staged through, the hit list); n256d: three (80 registers, 50 KB). n128, 128 threads: eight CTAs per SM (64 registers, 20 KB). What runs while no copy is in
 // flight works in memory that is dead by then: the prune in the ring; the finish over the candidate list and the ring, with
 // the kept set in the hit list's place. What the CTAs leave of an SM's memory is L1, which the greedy rows' register loads need
 // on their way: with a ring of 24 KB and work areas of its own the 256-thread instance left 28 KB (greedy rows,
-// 512 x 100,003 f32: 61 us against 46; 512 x 151,936 bf16: 49 against 39; top-k rows 1.00 to 1.09 times faster, but 256 x 100,003 f32, two
-// rows per SM, where the longer ring counted, 40.1 against 41.9).
-constexpr int N_CTAS_PER_SM = (N_NT == 256) ? 5 : 8;
+// 512 x 100,003 f32: 61 us against 46; 512 x 151,936 bf16: 49 against 39; top-k rows 1.00 to 1.09 times faster). Where an SM has two rows at most the
+// bytes that one row has on their way count: n256d's ring holds four f32 steps instead of two, and its registers let greedy rows ask for all their vectors at
+// once (launch_narrow has the figures).
+constexpr int N_CTAS_PER_SM = GS_N_CTAS;
 constexpr int N_CAP = (N_NT == 256) ? 1536 : 1024;   // candidate capacity (entries of 8 B)
 constexpr int N_KEEP = 768;                           // a prune must get below this
 constexpr int N_HITS = (N_NT == 256) ? 1536 : 1024;  // hit list: positions of lane-steps that hold a candidate (4 B each)
-constexpr int N_RING_BYTES = (N_NT == 256) ? 16384 : 8192;
+constexpr int N_RING_BYTES = GS_N_RING;
 constexpr int N_CAND_OFF = 0;
 constexpr int N_RING_OFF = N_CAP * 8;
 constexpr int N_HITS_OFF = N_RING_OFF + N_RING_BYTES;
@@ -182,7 +183,7 @@ __device__ void narrow_row(const BatchArgs& BA, const int64_t row_id, unsigned c
   // cannot run that far ahead: in a rolled loop they share one scoreboard, so waiting for the
   // oldest waits for the newest too. The first copies go out now and fly during the selection.
   constexpr int EPI = 8 / VEC, SV = 32 * EPI;
-  constexpr int NQ = N_RING_BYTES / (EPI * N_NT * 16);       // stages: 4 of bf16, 2 of f32
+  constexpr int NQ = N_RING_BYTES / (EPI * N_NT * 16);       // stages: 4 of bf16, 2 of f32 (n256d: 4)
   const int lane = tid & 31, warp = tid >> 5;
   const int rest = max(rv.nvec - warm, 0);
   const int span = (((rest + N_NW - 1) / N_NW + SV - 1) / SV) * SV;

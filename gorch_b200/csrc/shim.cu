@@ -43,19 +43,19 @@ constexpr int64_t kSliceCap = 109 * 1024 - gs::REGION_A - gs::REGION_B;
 // the cluster kernel (several CTAs per row), whose latency is lower while the GPU is not full. The rows' kinds are
 // on the device, so one line serves them all. us, batch | cluster, calls back to back on inputs that are not in L2, for rows with
 // top-k, greedy ones, the two mixed with nucleus rows, plain softmax rows, and rows with a top-p cut (f32):
-//   112 x 50,257: 27 | 23, 16 | 11, 33 | 27, 21 | 30, 56 | 72;  256 x 50,257: 29 | 41, 16 | 20, 41 | 46, 25 | 57, 73 | 136
-//   32 x 151,936: 38 | 18, 18 | 8, 43 | 22, 29 | 23, 80 | 50;  64: 38 | 26, 18 | 13, 51 | 33, 29 | 37, 80 | 83;  128: 47 | 42, 26 | 22, 61 | 52,
-//   30 | 69, 97 | 157
-// Rows without top-k change sides long before the others, and the line stays near theirs. Bytes follow that only roughly: from 40 to 60
-// rows of 151,936 f32 the clusters would serve most kinds sooner (48: 38 | 20, 18 | 11, 43 | 28, 29 | 35, 85 | 75), and behind the line
-// top-k, greedy and mixed rows pay (128 x 50,257: 27 | 24, 14 | 11, 36 | 29, for 21 | 32, 57 | 74).
+//   112 x 50,257: 28 | 23, 17 | 12, 35 | 27, 25 | 31, 54 | 72;  256 x 50,257: 31 | 41, 20 | 22, 44 | 49, 31 | 58, 79 | 136
+//   32 x 151,936: 36 | 19, 21 | 10, 47 | 23, 35 | 23, 83 | 49;  64: 37 | 27, 23 | 15, 51 | 35, 35 | 40, 85 | 85;  128: 40 | 44, 25 | 26, 55 | 55,
+//   39 | 72, 99 | 160
+// At 50,257 columns rows without top-k change sides long before the others, and the line stays near theirs. Bytes follow that only roughly: up to 48
+// rows of 151,936 f32 the clusters would serve nearly every kind sooner (48: 37 | 22, 22 | 13, 50 | 30, 35 | 36, 83 | 77), and behind the line
+// top-k, greedy and mixed rows pay (128 x 50,257: 28 | 24, 17 | 13, 37 | 30, for 25 | 32, 54 | 76).
 // Short rows stay with the clusters for longer. Up to four rows per SM of 4,096 logits, two waves of clusters:
-//   592 x 4,096: 24 | 20, 13 | 10, 37 | 28, 21 | 23, 45 | 40 (8,000 logits, 512 rows: 27 | 20, 13 | 10, 36 | 27, 20 | 26, 48 | 47)
-// Beyond four rows per SM, the wide kernel's slots, the batch kernels start a second round of wide rows (592 x 12,000: 27 | 22, 15 | 11,
-// 40 | 31, 23 | 30, 55 | 58; 593: 29 | 28, 15 | 13, 40 | 31, 27 | 36, 76 | 66): up to six rows per SM of 16,384 logits
-//   888 x 4,000: 24 | 29, 13 | 14, 44 | 38, 29 | 34, 73 | 60;  768 x 16,000: 29 | 33, 15 | 16, 100 | 41, 34 | 49, 99 | 94
-//   889 x 16,384: 31 | 40, 16 | 18, 102 | 46, 36 | 56, 106 | 105
-// Mixed batches and rows with a cut gain there; top-k rows by themselves and plain softmax rows give some of it back.
+//   592 x 4,096: 25 | 20, 15 | 10, 36 | 29, 23 | 24, 45 | 41 (8,000 logits, 512 rows: 28 | 21, 16 | 11, 39 | 29, 23 | 27, 49 | 48)
+// Beyond four rows per SM, the wide kernel's slots, the batch kernels start a second round of wide rows (592 x 12,000: 30 | 23, 18 | 13,
+// 44 | 33, 27 | 31, 57 | 60; 593: 31 | 30, 19 | 15, 44 | 33, 35 | 38, 81 | 68): up to six rows per SM of 16,384 logits
+//   888 x 4,000: 25 | 29, 15 | 15, 47 | 40, 34 | 35, 75 | 60;  768 x 16,000: 35 | 35, 21 | 18, 107 | 44, 40 | 51, 104 | 98
+//   889 x 16,384: 37 | 41, 23 | 21, 108 | 49, 43 | 59, 108 | 109
+// Mixed batches gain most there, rows with a cut some; top-k rows by themselves give a few us back, plain softmax rows up to a quarter.
 // An argmax is one launch of the narrow kernel and keeps the lower line.
 constexpr int64_t kBatchModeRows = 384;
 constexpr int64_t kBatchModeBytes = 24ll << 20;
@@ -386,11 +386,16 @@ int batch_lists(Ctx* c, int64_t B, int32_t** base, char** errOut) {
   return GORCH_CUDA_OK;
 }
 
-// The narrow kernel's two instances: 256-thread CTAs (five per SM) while every row gets a CTA slot
-// of its own, 128-thread CTAs (eight per SM) beyond that. Variants 6 / 7 force one of them (tests).
+// The narrow kernel's instances: 256-thread CTAs (five per SM) while every row gets a CTA slot
+// of its own, 128-thread CTAs (eight per SM) beyond that. Variants 6 / 7 force one of them (tests). Where no SM gets more than two rows of
+// f32, 256 threads with a longer ring and more registers (n256d). us, n256 | n256d, top-k of 50: 64 x 151,936: 46.1 | 36.0, 148 x 100,003:
+// 40.0 | 32.7, 256 x 50,257: 33.0 | 29.3, 296 x 100,003: 46.1 | 40.4; greedy, 148 x 151,936: 36.8 | 27.2, 256 x 100,003: 32.5 | 27.3; mixed, 256 x 50,257: 46.3 | 42.4,
+// 148 x 151,936: 70.6 | 58.0. Beyond, the two come together (330 x 151,936: 63.7 | 65.1, 400: 71.5 | 70.2). bf16 rows have four steps on their way in either, and
+// mixed batches of them are slower beside the wide kernel (256 x 100,003: 49.4 | 50.6, 330: 51.9 | 54.7).
 static cudaError_t launch_narrow(Ctx* c, const gs::BatchArgs& ba, int dtype, int64_t B, bool dependent) {
   const int64_t slots256 = static_cast<int64_t>(gs::n256::N_CTAS_PER_SM) * c->sm_count;
   const bool small_ctas = c->variant == 6 || (c->variant != 7 && B > slots256);
+  const bool deep = !small_ctas && c->variant != 7 && dtype == GORCH_CUDA_F32 && B <= 2ll * c->sm_count;
   const int64_t slots = small_ctas ? static_cast<int64_t>(gs::n128::N_CTAS_PER_SM) * c->sm_count : slots256;
   const unsigned g = static_cast<unsigned>(B < slots ? B : slots);
   const bool diag = ba.k.out_probs || ba.k.out_debug;
@@ -399,6 +404,7 @@ static cudaError_t launch_narrow(Ctx* c, const gs::BatchArgs& ba, int dtype, int
   auto pick = [&](auto type) {
     typedef decltype(type) E;
     if (small_ctas) go(diag ? gs::n128::narrow_rows_kernel<E, true> : gs::n128::narrow_rows_kernel<E, false>, gs::n128::N_NT, gs::n128::N_DYN_BYTES);
+    else if (deep) go(diag ? gs::n256d::narrow_rows_kernel<float, true> : gs::n256d::narrow_rows_kernel<float, false>, gs::n256d::N_NT, gs::n256d::N_DYN_BYTES);
     else go(diag ? gs::n256::narrow_rows_kernel<E, true> : gs::n256::narrow_rows_kernel<E, false>, gs::n256::N_NT, gs::n256::N_DYN_BYTES);
   };
   if (dtype == GORCH_CUDA_F32) pick(float()); else pick(uint16_t());
@@ -808,6 +814,8 @@ GorchCudaCtxRef gorch_cuda_create_ctx(int device, char** errOut) {
   if ((e = cudaFuncSetAttribute(gs::n256::narrow_rows_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n256::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::n256::narrow_rows_kernel<uint16_t, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n256::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::n256::narrow_rows_kernel<uint16_t, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n256::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::n256d::narrow_rows_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n256d::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
+  if ((e = cudaFuncSetAttribute(gs::n256d::narrow_rows_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n256d::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::n128::narrow_rows_kernel<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n128::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::n128::narrow_rows_kernel<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n128::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
   if ((e = cudaFuncSetAttribute(gs::n128::narrow_rows_kernel<uint16_t, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, gs::n128::N_DYN_BYTES)) != cudaSuccess) return fail("cudaFuncSetAttribute", e);
