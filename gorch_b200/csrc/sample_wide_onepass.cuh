@@ -351,7 +351,7 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
   // (a logit of the second half may lie above smax: the pass finds out how far)
   const int sampled = again ? 2 * W1_SAMPLE : W1_SAMPLE;
   each([&](float x) { atomicAdd(&bins[static_cast<int>(fmaxf(fminf((smax - x) * scale, static_cast<float>(W1_SBINS - 1)), 0.0f))], 1u); });
-  if (tid == 0) { sh.bc[0] = 0; sh.bc[1] = W1_SBINS - 1; sh.bc[2] = 0; sh.bc[3] = sampled; }
+  if (tid == 0) { sh.bc[0] = 0; sh.bc[1] = 0; }
   __syncthreads();
   // ---- the window: where the sample's mass passes plim, give or take 4.5 standard errors of a mass fraction
   // estimated from weighted logits (Var = ((1-p)^2 sum of squared weights above the cut + p^2 of those below) / (sum of
@@ -383,7 +383,7 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
   float* wm = reinterpret_cast<float*>(sh.sc.d0);
   float* wq = reinterpret_cast<float*>(sh.sc.d1);
   if (lane == 31) { wm[warp] = im; wq[warp] = iq; sh.sc.i0[warp] = in; }
-  if (tid == 0) wq[W_NW] = -1.0f;
+  if (tid == 0) wq[W_NW] = 0.0f;
   __syncthreads();
   float tot_m = 0.0f, tot_q = 0.0f;
   im -= mass; iq -= sq; in -= n;                                          // exclusive
@@ -395,27 +395,37 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
   }
   if (!(tot_m * 2.4e-3f >= 1.0f)) return WHY_HEAVY;                             // heavy tokens (one above 1/400 of the mass): not for a sample to place
   const float pl = static_cast<float>(plim), lim = pl * tot_m;
-  if (im < lim && im + mass >= lim) wq[W_NW] = iq + sq;                   // one thread (none: nothing lies below the cut)
+  // Where a limit is passed: in the last thread whose prefix lies below it, found as a maximum. (A thread's own end and the next one's prefix are rounded
+  // differently, and a limit between the two is passed by neither: one row in 17,000 got a window from the row's first bucket that way.)
+  auto last_below = [&](int mine, int* slot) {
+    const int top = __reduce_max_sync(FULL, mine);
+    if (lane == 0) atomicMax(slot, top);
+  };
+  last_below(im < lim ? __float_as_int(iq + sq) : 0, reinterpret_cast<int*>(wq + W_NW));
   __syncthreads();
-  const float q_above = (wq[W_NW] >= 0.0f) ? wq[W_NW] : tot_q, q1 = 1.0f - pl;
+  const float q_above = wq[W_NW], q1 = 1.0f - pl;
   const float fpc = 1.0f - static_cast<float>(sampled) / static_cast<float>(V);
   const float delta = 4.5f * sqrtf(fmaxf(q1 * q1 * q_above + pl * pl * (tot_q - q_above), 0.0f) * fpc) + 2.0f;   // in units of mass: two top tokens more
   const float m_lo = lim - delta, m_hi = lim + delta;
   {
     float e = e0, acc = im;
-    int c = in;
+    int c = in, lo = 0, hi = 0;                                           // bucket << 16 | logits of the sample above it, or through it
 #pragma unroll
-    for (int j = 0; j < PER; j++) {                                       // prefixes grow: one bucket passes either limit first
-      const float next = acc + weight(j, e);
-      if (acc < m_lo && next >= m_lo) { sh.bc[0] = tid * PER + j; sh.bc[2] = c; }
-      if (acc < m_hi && next >= m_hi) { sh.bc[1] = tid * PER + j; sh.bc[3] = c + cnt[j]; }
+    for (int j = 0; j < PER; j++) {
+      const int at = (tid * PER + j) << 16;
+      if (acc < m_lo) lo = at | c;
       c += cnt[j];
-      acc = next;
+      if (acc < m_hi) hi = at | c;
+      acc += weight(j, e);
       e *= ratio;
     }
+    last_below(lo, &sh.bc[0]);
+    last_below(hi, &sh.bc[1]);
   }
   __syncthreads();
-  const int b1 = max(sh.bc[0] - 1, 0), b2 = min(sh.bc[1] + 1, W1_SBINS - 1);   // a bucket of slack for the f32 sums
+  static_assert(2 * W1_SAMPLE < 65536, "counts of the sample in 16 bits");
+  const int from_bin = sh.bc[0] >> 16, above = sh.bc[0] & 0xffff, to_bin = sh.bc[1] >> 16, through = sh.bc[1] & 0xffff;
+  const int b1 = max(from_bin - 1, 0), b2 = min(to_bin + 1, W1_SBINS - 1);   // a bucket of slack for the f32 sums
   // How many logits of the row will be listed: as many as the sample's share of the window says, and of the buckets of slack as many as
   // the window's have on average. The lists hold 4.5 standard deviations more, of the sample's count and of a warp's part; a lane's buffer, which
   // counts as full at 12, is expected to get W1_PER_VISIT at most before it is emptied (full then: one lane in 4 x 10^7, one row of 151,936
@@ -426,8 +436,8 @@ __device__ __noinline__ int wide_place_window(unsigned char* dyn, WideShared& sh
     const float per_warp = logits * to_warp;
     return per_warp + 4.5f * sqrtf(per_warp * (1.0f + to_warp)) <= static_cast<float>(W1_WCAP) && logits * to_row <= W1_PER_VISIT * static_cast<float>(visits);
   };
-  const float seen = static_cast<float>(max(sh.bc[3] - sh.bc[2], 0)), per_bucket = seen / static_cast<float>(max(sh.bc[1] - sh.bc[0] + 1, 1));
-  const float n_low = static_cast<float>(sampled - sh.bc[2]) + per_bucket, n_mid = seen + 2.0f * per_bucket;
+  const float seen = static_cast<float>(max(through - above, 0)), per_bucket = seen / static_cast<float>(max(to_bin - from_bin + 1, 1));
+  const float n_low = static_cast<float>(sampled - above) + per_bucket, n_mid = seen + 2.0f * per_bucket;
   // how often a lane empties its buffer: once a piece, or once for each turn of the ring
   const int seldom = W_NT * max(sh.nvec / (W_NT * (8 / VEC) * W_G), 1), turns = V / (W1_RING_BYTES / (W_NT * static_cast<int>(sizeof(T))));
   bool low = fits(n_low, seldom), often = false;

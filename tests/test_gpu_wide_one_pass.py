@@ -225,3 +225,11 @@ def test_finite_logits_far_out(wide, oracle):
         gpu, _, _ = run_both(wide, oracle, x, np.array([(1.0, 0, 0.0, MODE_A), (0.9, 0, 0.0, MODE_B)], dtype=CFG_DTYPE), rng.random(2))
         assert np.all(gpu["ids"] == V // 2 + 100)
         assert np.all(gpu["debug"]["path"] == 2) and np.all(gpu["debug"]["reserved"][:, 6] == WHY_ANCHOR)
+
+
+def test_limit_between_two_threads(wide, oracle):
+    """Rows whose window's limit falls into the rounding between one thread's prefix of the sample's mass and the next one's."""
+    V, keys = {4: (50257, (9803, 11332)), 5: (70001, (2272, 5846))}[wide.variant]
+    x = np.stack([np.random.Generator(np.random.Philox(key=k)).standard_normal(V, dtype=np.float32) * np.float32(0.25) for k in keys])
+    gpu, _, _ = run_both(wide, oracle, x, np.array([(1.0, 0, 0.99, MODE_B)] * len(keys), dtype=CFG_DTYPE), np.full(len(keys), 0.5))
+    assert list(gpu["debug"]["reserved"][:, 6]) == [0] * len(keys) and np.all(gpu["debug"]["path"] == 3)
