@@ -52,7 +52,7 @@ template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.as
 __device__ __forceinline__ float ex2_approx(float t) { float e; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t)); return e; }
 __device__ __forceinline__ float set_ge(float a, float b) { float r; asm("set.ge.f32.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b)); return r; }   // 1.0f or 0.0f
 
-// x / T in IEEE f32 round-to-nearest by q0 = x y, r = fma(-q0, T, x), q = fma(r, y, q0) with y = RN(1/T):
+// x / T in IEEE f32 round-to-nearest by q0 = x y, r = fma(-q0, T, x), q = fma(r, y, q0) with y = RN(1/T) (Markstein's correction):
 // the correctly rounded quotient whenever T's significand is not all ones and nothing over- or underflows
 // (the caller takes this form for 2^-20 <= T <= 2^20 only and clamps x at -1e30: whatever lies below has
 // mass 0 either way).
